@@ -86,19 +86,16 @@ __device__ __forceinline__ unsigned long long make_desc(unsigned saddr) {
 }
 /* instruction descriptor: D = f32 (bit 4), A = B = f16 (0), both K-major, N = 128 (>>3 at bit 17), M = 128 (>>4 at bit 24) */
 constexpr unsigned kIdesc = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-__device__ __forceinline__ void tmem_ld32(unsigned taddr, unsigned (&r)[32]) {
+/* 32 columns of the warp's lanes; the registers are valid after tmem_ld_wait (several loads can be in flight before it) */
+__device__ __forceinline__ void tmem_ld32_nowait(unsigned taddr, unsigned *r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
                    "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-/* the same load without the wait: several loads can be in flight before one tcgen05.wait::ld */
-__device__ __forceinline__ void tmem_ld32_nowait(unsigned taddr, unsigned (&r)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr) : "memory");
+/* waits for all loads of the thread; the operands make every use of the registers depend on it */
+__device__ __forceinline__ void tmem_ld_wait(unsigned *r) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]) :: "memory");
 }
 __device__ __forceinline__ void tmem_st32(unsigned taddr, const unsigned (&r)[32]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
@@ -123,6 +120,72 @@ __device__ __forceinline__ void umma_commit_lead(unsigned bar, unsigned lead) {
 __device__ __forceinline__ float fmax3(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
 __device__ __forceinline__ float ex2f(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ unsigned pack_h2(float lo, float hi) { unsigned r; asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo)); return r; }
+
+/* ---- packed fp32 pairs (one instruction for two values) */
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 w, x, y, z;\n mov.b64 {%0, %1}, w;\n}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 w, x, y;\n mov.b64 {%0, %1}, w;\n}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 splat(float a) { return make_float2(a, a); }
+/* 2^t of a pair on the FMA pipe (the exponential unit takes 16 values per clock and SM, which the softmax of two tiles fills):
+ * t = n + f, n = round(t), 2^f on [-1/2, 1/2] by the Taylor polynomial of e^(f ln 2) of degree 6 (remainder below 2e-8 relative,
+ * i.e. fp32 rounding), n added to the exponent field.  t is clamped at -126 (masked keys: 2^-126 instead of 0, which is 0 in
+ * fp16 and nothing beside a denominator >= 2^-8). */
+__device__ __forceinline__ float2 ex2_fma(float2 t) {
+    const float magic = 12582912.f;    /* 1.5 * 2^23: adding it rounds to an integer and leaves it in the low mantissa bits */
+    t.x = fmaxf(t.x, -126.f); t.y = fmaxf(t.y, -126.f);
+    const float2 z = add2(t, splat(magic)), n = add2(z, splat(-magic)), f = fma2(n, splat(-1.f), t);
+    float2 p = fma2(splat(1.5403530e-4f), f, splat(1.3333558e-3f));
+    p = fma2(p, f, splat(9.6181291e-3f));
+    p = fma2(p, f, splat(5.5504109e-2f));
+    p = fma2(p, f, splat(2.4022651e-1f));
+    p = fma2(p, f, splat(6.9314718e-1f));
+    p = fma2(p, f, splat(1.f));
+    return make_float2(__uint_as_float(__float_as_uint(p.x) + (__float_as_uint(z.x) << 23)), __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(z.y) << 23)));
+}
+__device__ __forceinline__ float row_max(const unsigned (&v)[64]) {
+    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      /* four independent chains */
+#pragma unroll
+    for (int i = 0; i < 64; i += 2) mx[(i >> 1) & 3] = fmax3(mx[(i >> 1) & 3], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+    return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+}
+/* Turns on the exponential unit: tile A and tile B compute their exponentials alternately.  Left alone the two tiles fall into
+ * step -- both wait, load and reduce at the same time and then share the unit at half speed (1 250 clocks for 64 columns of both,
+ * in a period of 1 985 clocks per step); with turns one tile's exponentials run under the other's waits: 1 560-1 620 clocks. */
+__device__ __forceinline__ void turn_wait(int x) { asm volatile("bar.sync %0, 256;" ::"r"(1 + x) : "memory"); }
+__device__ __forceinline__ void turn_pass(int x) { asm volatile("bar.arrive %0, 256;" ::"r"(2 - x) : "memory"); }
+__device__ __forceinline__ float ex2v(float x) { float r; asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+/* P = 2^(s * scale - m) of a row's 64 scores as packed fp16 pairs; returns the (pairwise) sum of the unrounded values (the fp16
+ * rounding of P is a zero-mean 2^-12 relative error per term, far below the tolerance).  One pair in eight goes through the FMA
+ * pipe: 512 tokens behind 4 096 take 75 us with none, 69-70 us with one, 74-76 us with two or more (the FMA form costs issue
+ * slots that the waiting tile's maximum wants). */
+__device__ __forceinline__ float2 softmax_exp(const unsigned (&v)[64], float m, unsigned (&pk)[32], int x, bool pass) {
+    const float2 sc = splat(kScaleLog2), nm = splat(-m);
+    float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, t[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) t[i] = fma2(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sc, nm);
+    turn_wait(x);
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        if ((i & 7) == 7) t[i] = ex2_fma(t[i]);
+        else { t[i].x = ex2v(t[i].x); t[i].y = ex2v(t[i].y); }
+    }
+    if (pass) turn_pass(x);
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        pk[i] = pack_h2(t[i].x, t[i].y);
+        ls[i & 1] = add2(ls[i & 1], t[i]);
+    }
+    return add2(ls[0], ls[1]);
+}
 
 /* ---- pass 1: pages -> dense fp16 K [head][tok][128] and V^T [head][128][tok] ------------------- */
 template <int DT>
@@ -352,72 +415,57 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const bool row_valid = (tq0 + t_local) < a.nq;
         const unsigned lane_base = (unsigned)((warp & 3) * 32) << 16; /* this warp's quarter of the TMEM lanes */
         const unsigned tm_o = tmem + 256u + 128u * x + lane_base;
-        float m = -INFINITY, l = 0.f;
+        float m = -INFINITY;
+        float2 l2 = make_float2(0.f, 0.f);
         bool ok = true;
-        for (int j = 0; j < ntiles && ok; j++) {
+        if (x == 1) turn_pass(1);                /* tile A has the first turn */
+        for (int j = 0; j < ntiles; j++) {       /* to the end also after a wait ran out: the turns have to match */
             const unsigned tm_s = tmem + 128u * x + 64u * (j & 1) + lane_base;
             ok = __all_sync(0xffffffffu, mbar_wait_blocking(BAR(B3_SF + 2 * x + (j & 1)), (unsigned)(j >> 1) & 1u, s_abort, a.err, 30u));   /* keep the warp together */
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int k0 = j * kKeys3;
             const bool masked = (k0 + kKeys3 - 1 > a.base + tq0);   /* the tile crosses the diagonal of some row */
-            unsigned v0[32], v1[32];
-            tmem_ld32_nowait(tm_s, v0);
-            tmem_ld32_nowait(tm_s + 32u, v1);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            unsigned v[64];
+            tmem_ld32_nowait(tm_s, v);
+            tmem_ld32_nowait(tm_s + 32u, v + 32);
+            tmem_ld_wait(v);
+            tmem_ld_wait(v + 32);
             if (masked) {      /* only the tiles on the diagonal pay for the causal test */
 #pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    if (k0 + i > qpos) v0[i] = 0xff800000u;
-                    if (k0 + 32 + i > qpos) v1[i] = 0xff800000u;
-                }
+                for (int i = 0; i < 64; i++) if (k0 + i > qpos) v[i] = 0xff800000u;
             }
             /* the maximum is taken over the raw scores (the scale is positive) and the scale is folded into the exponent's
-             * argument: one FFMA per element.  Four independent chains keep the dependent-issue latency hidden. */
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-            for (int i = 0; i < 32; i++) mx4[i & 3] = fmax3(mx4[i & 3], __uint_as_float(v0[i]), __uint_as_float(v1[i]));
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * kScaleLog2;
-            /* a tile that is masked for the whole row (its keys all lie behind the row's query; only in the last tiles of
-             * the CTA) has mx = -inf: nothing moves and all its P are 0 */
+             * argument.  A tile that is masked for the whole row (its keys all lie behind the row's query; only in the last
+             * tiles of the CTA) has mx = -inf: nothing moves and all its P are 0 */
+            const float mx = row_max(v) * kScaleLog2;
             const bool grow = mx > m + kPfThreshold;              /* true while m == -inf (key 0 is never masked) */
-            const float m_new = grow ? mx : m;
-            const float neg_m = -m_new;
-            unsigned pk[32];
-            float ls[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-                /* the denominator sums the unrounded values: the fp16 rounding of P is a zero-mean 2^-12 relative error per
-                 * term, far below the tolerance */
-                const float e0 = ex2f(fmaf(__uint_as_float(v0[i]), kScaleLog2, neg_m)), e1 = ex2f(fmaf(__uint_as_float(v0[i + 1]), kScaleLog2, neg_m));
-                const float e2 = ex2f(fmaf(__uint_as_float(v1[i]), kScaleLog2, neg_m)), e3 = ex2f(fmaf(__uint_as_float(v1[i + 1]), kScaleLog2, neg_m));
-                pk[i >> 1] = pack_h2(e0, e1); pk[16 + (i >> 1)] = pack_h2(e2, e3);
-                ls[0] += e0; ls[1] += e1; ls[2] += e2; ls[3] += e3;
-            }
-            const float lsum = (ls[0] + ls[1]) + (ls[2] + ls[3]);
-            /* tcgen05.ld / .st are warp-collective: the whole warp rescales its 32 rows as soon as one of them moved its
-             * reference (the others multiply by exactly 1).  O_x is only ours when P_x(j-1).V_(j-1) has completed. */
-            const float alpha = grow ? ex2f(m - m_new) : 1.f;     /* 0 on the first tile (m = -inf) */
             if (__any_sync(0xffffffffu, grow)) {
+                /* tcgen05.ld / .st are warp-collective: the whole warp rescales its 32 rows as soon as one of them moved its
+                 * reference (the others multiply by exactly 1).  O_x is only ours when P_x(j-1).V_(j-1) has completed:
+                 * S_x(j+1) was issued behind P_x(j-1).V, and a commit covers everything its thread issued before */
+                const float m_new = grow ? mx : m, alpha = grow ? ex2f(m - m_new) : 1.f;     /* 0 on the first tile (m = -inf) */
                 if (j > 0) {
-                    /* S_x(j+1) was issued behind P_x(j-1).V, and a commit covers everything its thread issued before */
                     ok = __all_sync(0xffffffffu, j + 1 < ntiles ? mbar_wait_blocking(BAR(B3_SF + 2 * x + ((j + 1) & 1)), (unsigned)((j + 1) >> 1) & 1u, s_abort, a.err, 31u)
                                                                : mbar_wait_blocking(BAR(B3_O + 2 * x), 0u, s_abort, a.err, 31u));
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (ok) {
-#pragma unroll
+#pragma unroll 1
                         for (int c = 0; c < 4; c++) {
-                            unsigned v[32];
-                            tmem_ld32(tm_o + 32u * c, v);
+                            unsigned o[32];
+                            tmem_ld32_nowait(tm_o + 32u * c, o);
+                            tmem_ld_wait(o);
 #pragma unroll
-                            for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                            tmem_st32(tm_o + 32u * c, v);
+                            for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                            tmem_st32(tm_o + 32u * c, o);
                         }
                     }
                 }
-                l *= alpha;
+                l2.x *= alpha; l2.y *= alpha;
                 m = m_new;
             }
-            l += lsum;
+            unsigned pk[32];
+            const float2 ls = softmax_exp(v, m, pk, x, x == 0 || j + 1 < ntiles);
+            l2 = add2(l2, ls);
             /* P over the first 32 columns of this S buffer (column c = keys 2c, 2c+1) */
             tmem_st32(tm_s, pk);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -425,6 +473,7 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR(B3_P + 2 * x + (j & 1)));
         }
+        const float l = l2.x + l2.y;
         /* epilogue: O / l.  The issuer commits P.V of the last two tiles on barriers of their own, which therefore complete
          * exactly once (a parity wait on a barrier that runs through many phases can only tell the last completed phase
          * from the one before it, and a waiter here could be two behind).  The last commit covers all earlier MMAs. */
@@ -436,7 +485,8 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 unsigned v[32];
-                tmem_ld32(tm_o + 32u * c, v);
+                tmem_ld32_nowait(tm_o + 32u * c, v);
+                tmem_ld_wait(v);
                 if (row_valid)
 #pragma unroll
                 for (int i = 0; i < 32; i += 4)
