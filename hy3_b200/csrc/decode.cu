@@ -5,7 +5,7 @@
  * Replaces attention_split_kv[_int4]_kernel + attention_reduce_kernel of the reference
  * (hy3_gpu.cu:183-247, :274-325).  The reference runs one warp per (query head, split),
  * so every KV byte is fetched once per query head of its group (8x) with 4-byte loads at
- * an 83 KB stride.  Here a warp processes 16 tokens of one KV head for ALL 8 query heads
+ * an 83 KB stride.  Here a warp processes 16 or 32 tokens of one KV head for ALL 8 query heads
  * of the group at once, on tensor cores, so each KV byte is read exactly once:
  *
  *   S[16 x 8]   = Q2[16 x 128] . K^T    rows 0-7 = the 8 heads, rows 8-15 = a residual of the
@@ -28,7 +28,7 @@
  * serves every length (lengths come from device memory; nothing is baked into a captured
  * graph, cf. hy3_gpu.cu:774-789).  A producer warp streams the CTA's pages into a shared-
  * memory ring with bulk asynchronous copies (cp.async.bulk + mbarrier transaction counts);
- * the consumer warps take the 16-token granules of the pages round-robin.  The piece a CTA
+ * the consumer warps take the 16- or 32-token granules of the pages round-robin.  The piece a CTA
  * computes for a (row, head) segment is folded in shared memory; if the segment spans
  * several CTAs each writes an {m, l, acc} record and the LAST CTA to arrive (atomic
  * counter) folds them -- the LSE-merge epilogue, no second launch.
@@ -54,6 +54,7 @@ constexpr int kFixedML = ((kWarps * 8 * 2 * 4) + 127) / 128 * 128;
 constexpr int kFixedQ = 8 * 32 * 16;
 constexpr int kBarBytes = 256;      /* mbarriers of the page ring: empty[8], full[16] */
 constexpr int kFixed = kFixedO + kFixedML + kFixedQ;   /* bytes of shared memory in front of the page-count prefix */
+static_assert(16 / 8 * 8 >= 8 + 3 && 16 / 7 * 7 >= 7 + 3 && 16 / 6 * 6 >= 6 + 3 && kWarps <= 12, "rounds of the full barriers: see the consumer loop");
 constexpr bool kPSplit = true;                         /* carry the fp16 residual of P in MMA rows 8-15 */
 constexpr int kRecFloats = HY3A_REC_FLOATS;             /* floats per head record in the merge scratch (130 used) */
 constexpr int kShardBatch = 5;                          /* ranks polled at once by the sharded epilogue */
@@ -133,7 +134,14 @@ struct warp_state {
 
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
 
-/* One 16-token granule of one warp: loads, S = Q.K^T, online softmax, O += P.V.
+/* Tokens a consumer warp takes at a time.  An INT4 page costs instructions, not bytes (16.9 KB per 128 tokens): with 32 tokens
+ * the Q fragments, the maximum's shuffles, the rescale test and the ring bookkeeping are paid half as often and four
+ * independent score chains cover each other's latency: 262 144 positions 82.9 -> 73.8 us a layer (3.3 -> 3.75 TB/s), 8 ragged
+ * sequences of up to 8 000 tokens 27.3 -> 26.2 us.  FP16 keeps 16: its K and V registers would not fit twice. */
+template <int DT> constexpr int kGran = DT == 2 ? 32 : 16;
+template <int DT> constexpr int kGranPage = HY3A_PT / kGran<DT>;
+
+/* One granule of one warp: loads, S = Q.K^T, online softmax, O += P.V.
  * SM: operands come from a shared-memory copy of the page (32-bit shared addresses) instead
  * of global memory.  FULL: all 16 tokens are valid (no masking).  sq: shared address of this
  * lane's Q fragments; qf: score factor of this lane's head (integer-MMA path).             */
@@ -143,29 +151,37 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
                                         float pscale) {
     static_assert(DT == 0 || DT == 2, "INT8 caches are served by decode_umma.cu");
     constexpr int NK = DT == 0 ? 4 : 1;
-    constexpr int NV = DT == 0 ? 8 : 2;
+    constexpr int NV = DT == 0 ? 8 : 2;                      /* V chunks per 16 tokens */
+    constexpr int NB = kGran<DT> / 8, NT = kGran<DT> / 16;   /* 8-token blocks, 16-token halves */
     /* page-relative byte offsets of granule gi (16 tokens = 16 K rows = 8 V pair-rows) */
-    const int gk = gi * 16 * geom.k_row, gv = geom.v_off + gi * (DT == 0 ? 16 : 8) * geom.v_prow, gs = gi * 32;
-    uint4 kr[2][NK];
+    const int gk = gi * kGran<DT> * geom.k_row, gv = geom.v_off + gi * (DT == 0 ? 16 : 8 * NT) * geom.v_prow, gs = gi * 2 * kGran<DT>;
+    uint4 kr[NB][NK];
 #pragma unroll
-    for (int nb = 0; nb < 2; nb++) {
+    for (int nb = 0; nb < NB; nb++) {
+        const int o = gk + (nb >> 1) * 16 * geom.k_row;
 #pragma unroll
-        for (int i = 0; i < NK; i++) kr[nb][i] = SM ? lds16(spage + gk + k_off[nb][i]) : ld16(gpage + gk + k_off[nb][i]);
+        for (int i = 0; i < NK; i++) kr[nb][i] = SM ? lds16(spage + o + k_off[nb & 1][i]) : ld16(gpage + o + k_off[nb & 1][i]);
     }
-    unsigned ksw[2] = {0, 0}, vsw[2] = {0, 0};
+    unsigned ksw[NB], vsw[NB];
+#pragma unroll
+    for (int nb = 0; nb < NB; nb++) ksw[nb] = vsw[nb] = 0;
     if (DT != 0) {
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++) {
-            ksw[nb] = SM ? lds4(spage + geom.ks_off + gs + sc_off[nb]) : ld4(gpage + geom.ks_off + gs + sc_off[nb]);
-            vsw[nb] = SM ? lds4(spage + geom.vs_off + gs + sc_off[nb]) : ld4(gpage + geom.vs_off + gs + sc_off[nb]);
+        for (int nb = 0; nb < NB; nb++) {
+            const int o = gs + (nb >> 1) * 32 + sc_off[nb & 1];
+            ksw[nb] = SM ? lds4(spage + geom.ks_off + o) : ld4(gpage + geom.ks_off + o);
+            vsw[nb] = SM ? lds4(spage + geom.vs_off + o) : ld4(gpage + geom.vs_off + o);
         }
     }
-    uint4 vr[NV];
+    uint4 vr[NT * NV];
 #pragma unroll
-    for (int i = 0; i < NV; i++) vr[i] = SM ? lds16(spage + gv + v_off[i]) : ld16(gpage + gv + v_off[i]);
+    for (int i = 0; i < NT * NV; i++) {
+        const int o = gv + (i / NV) * 8 * geom.v_prow + v_off[i % NV];
+        vr[i] = SM ? lds16(spage + o) : ld16(gpage + o);
+    }
 
-    /* ---- raw scores r[nb][e] of head g for tokens 16gi + 8nb + 2tig + e (before the K scale) */
-    float r[2][2];
+    /* ---- raw scores r[nb][e] of head g for tokens kGran gi + 8nb + 2tig + e (before the K scale) */
+    float r[NB][2];
     if (DT == 0) {
         unsigned qa[8][4];
 #pragma unroll
@@ -187,33 +203,33 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
         uint4 qa[4];
 #pragma unroll
         for (int kk = 0; kk < 4; kk++) qa[kk] = lds16(sq + kk * 512);
-        int ce[2][4], co[2][4];     /* even / odd k-steps: four independent integer-MMA chains */
+        int c[NB][4];               /* four independent integer-MMA chains */
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++) { ce[nb][0] = ce[nb][1] = ce[nb][2] = ce[nb][3] = 0; co[nb][0] = co[nb][1] = co[nb][2] = co[nb][3] = 0; }
+        for (int nb = 0; nb < NB; nb++) c[nb][0] = c[nb][1] = c[nb][2] = c[nb][3] = 0;
 #pragma unroll
         for (int kk = 0; kk < 4; kk++) {
 #pragma unroll
-            for (int nb = 0; nb < 2; nb++) {
+            for (int nb = 0; nb < NB; nb++) {
                 /* two's-complement nibbles: moving a nibble to the top of its byte gives 16 x code as int8 */
                 const unsigned w = kk == 0 ? kr[nb][0].x : (kk == 1 ? kr[nb][0].y : (kk == 2 ? kr[nb][0].z : kr[nb][0].w));
                 const unsigned b0 = (w << 4) & 0xF0F0F0F0u, b1 = w & 0xF0F0F0F0u;
-                imma16832((kk & 1) ? co[nb] : ce[nb], qa[kk], b0, b1);
+                imma16832(c[nb], qa[kk], b0, b1);
             }
         }
         /* rows 0-7 carry the high digit of q, rows 8-15 the low digit: q ~ sq*(hi + lo/254) */
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++) {
-            r[nb][0] = (float)((ce[nb][0] + co[nb][0]) * 254 + (ce[nb][2] + co[nb][2])) * qf;
-            r[nb][1] = (float)((ce[nb][1] + co[nb][1]) * 254 + (ce[nb][3] + co[nb][3])) * qf;
+        for (int nb = 0; nb < NB; nb++) {
+            r[nb][0] = (float)(c[nb][0] * 254 + c[nb][2]) * qf;
+            r[nb][1] = (float)(c[nb][1] * 254 + c[nb][3]) * qf;
         }
     }
     /* ---- logits (base 2) and V scales */
-    float s[2][2], vs[2][2];
+    float s[NB][2], vs[NB][2];
 #pragma unroll
-    for (int nb = 0; nb < 2; nb++) {
+    for (int nb = 0; nb < NB; nb++) {
         float2 kf = make_float2(1.f, 1.f), vf = make_float2(1.f, 1.f);
         if (DT != 0) { kf = unpack_h2(ksw[nb]); vf = unpack_h2(vsw[nb]); }
-        const int t0 = 16 * gi + 8 * nb + 2 * tig;
+        const int t0 = kGran<DT> * gi + 8 * nb + 2 * tig;
         s[nb][0] = (FULL || t0 < valid) ? r[nb][0] * kf.x : -INFINITY;
         s[nb][1] = (FULL || t0 + 1 < valid) ? r[nb][1] * kf.y : -INFINITY;
         vs[nb][0] = (FULL || t0 < valid) ? vf.x * pscale : 0.f;
@@ -223,8 +239,10 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
      * the granule's max exceeds the reference by more than 2^8; until then p <= 2^8, which the
      * fp16 range of P has room for (pscale leaves 2^8 of headroom).                           */
     float mx = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+#pragma unroll
+    for (int nb = 2; nb < NB; nb += 2) mx = fmaxf(mx, fmaxf(fmaxf(s[nb][0], s[nb][1]), fmaxf(s[nb + 1][0], s[nb + 1][1])));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));   /* finite: token 16gi of this granule is valid */
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));   /* finite: the first token of this granule is valid */
     const bool grow = mx > st.m + kRescaleThreshold;       /* also true while st.m == -inf */
     if (__any_sync(0xffffffffu, grow)) {
         const float m_new = grow ? mx : st.m;
@@ -234,52 +252,56 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
         for (int jn = 0; jn < 16; jn++) { st.o[jn][0] *= alpha; st.o[jn][1] *= alpha; st.o[jn][2] *= alpha; st.o[jn][3] *= alpha; }
         st.m = m_new;
     }
-    unsigned pa[4];
-    {
-        float w[2][2];
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++) {
+    for (int nt = 0; nt < NT; nt++) {      /* 16 tokens: one k-step of P.V */
+        unsigned pa[4];
+        {
+            float w[2][2], pe[2][2];
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const float pe = ex2(s[nb][e] - st.m); /* -inf -> 0 */
-                st.l += pe;
-                w[nb][e] = pe * vs[nb][e];
+            for (int nb = 0; nb < 2; nb++) {
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    pe[nb][e] = ex2(s[2 * nt + nb][e] - st.m); /* -inf -> 0 */
+                    w[nb][e] = pe[nb][e] * vs[2 * nt + nb][e];
+                }
+            }
+            st.l += (pe[0][0] + pe[0][1]) + (pe[1][0] + pe[1][1]);
+            pa[0] = pack_h2(w[0][0], w[0][1]);
+            pa[2] = pack_h2(w[1][0], w[1][1]);
+            if (kPSplit) {
+                float2 h0 = unpack_h2(pa[0]), h1 = unpack_h2(pa[2]);
+                pa[1] = pack_h2(w[0][0] - h0.x, w[0][1] - h0.y);
+                pa[3] = pack_h2(w[1][0] - h1.x, w[1][1] - h1.y);
+            } else {
+                pa[1] = pa[3] = 0u;
             }
         }
-        pa[0] = pack_h2(w[0][0], w[0][1]);
-        pa[2] = pack_h2(w[1][0], w[1][1]);
-        if (kPSplit) {
-            float2 h0 = unpack_h2(pa[0]), h1 = unpack_h2(pa[2]);
-            pa[1] = pack_h2(w[0][0] - h0.x, w[0][1] - h0.y);
-            pa[3] = pack_h2(w[1][0] - h1.x, w[1][1] - h1.y);
-        } else {
-            pa[1] = pa[3] = 0u;
-        }
-    }
-    /* ---- O += P.V over 16 n-blocks of 8 output dims */
-    if (DT == 2) {
-        unsigned a4[4] = {vr[0].x, vr[0].y, vr[0].z, vr[0].w};
-        unsigned b4[4] = {vr[1].x, vr[1].y, vr[1].z, vr[1].w};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const unsigned xa = a4[k], xb = b4[k], xah = xa >> 8, xbh = xb >> 8;
-            mma16816(st.o[4 * k + 0], pa, cvt_u4_lo(xa), cvt_u4_lo(xb));
-            mma16816(st.o[4 * k + 1], pa, cvt_u4_hi(xa), cvt_u4_hi(xb));
-            mma16816(st.o[4 * k + 2], pa, cvt_u4_lo(xah), cvt_u4_lo(xbh));
-            mma16816(st.o[4 * k + 3], pa, cvt_u4_hi(xah), cvt_u4_hi(xbh));
-        }
-    } else {
-#pragma unroll
-        for (int half = 0; half < 2; half++) {
-            /* vr[2t + half]: token t (A,B = b0 pair; C,D = b1 pair), chunk g + 8*half */
-            unsigned tA[4] = {vr[0 + half].x, vr[0 + half].y, vr[0 + half].z, vr[0 + half].w};
-            unsigned tB[4] = {vr[2 + half].x, vr[2 + half].y, vr[2 + half].z, vr[2 + half].w};
-            unsigned tC[4] = {vr[4 + half].x, vr[4 + half].y, vr[4 + half].z, vr[4 + half].w};
-            unsigned tD[4] = {vr[6 + half].x, vr[6 + half].y, vr[6 + half].z, vr[6 + half].w};
+        /* ---- O += P.V over 16 n-blocks of 8 output dims */
+        if (DT == 2) {
+            const uint4 va = vr[nt * NV], vb = vr[nt * NV + 1];
+            unsigned a4[4] = {va.x, va.y, va.z, va.w};
+            unsigned b4[4] = {vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                mma16816(st.o[8 * half + 2 * k], pa, prmt(tA[k], tB[k], 0x5410u), prmt(tC[k], tD[k], 0x5410u));
-                mma16816(st.o[8 * half + 2 * k + 1], pa, prmt(tA[k], tB[k], 0x7632u), prmt(tC[k], tD[k], 0x7632u));
+                const unsigned xa = a4[k], xb = b4[k], xah = xa >> 8, xbh = xb >> 8;
+                mma16816(st.o[4 * k + 0], pa, cvt_u4_lo(xa), cvt_u4_lo(xb));
+                mma16816(st.o[4 * k + 1], pa, cvt_u4_hi(xa), cvt_u4_hi(xb));
+                mma16816(st.o[4 * k + 2], pa, cvt_u4_lo(xah), cvt_u4_lo(xbh));
+                mma16816(st.o[4 * k + 3], pa, cvt_u4_hi(xah), cvt_u4_hi(xbh));
+            }
+        } else {
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                /* vr[2t + half]: token t (A,B = b0 pair; C,D = b1 pair), chunk g + 8*half */
+                unsigned tA[4] = {vr[0 + half].x, vr[0 + half].y, vr[0 + half].z, vr[0 + half].w};
+                unsigned tB[4] = {vr[2 + half].x, vr[2 + half].y, vr[2 + half].z, vr[2 + half].w};
+                unsigned tC[4] = {vr[4 + half].x, vr[4 + half].y, vr[4 + half].z, vr[4 + half].w};
+                unsigned tD[4] = {vr[6 + half].x, vr[6 + half].y, vr[6 + half].z, vr[6 + half].w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    mma16816(st.o[8 * half + 2 * k], pa, prmt(tA[k], tB[k], 0x5410u), prmt(tC[k], tD[k], 0x5410u));
+                    mma16816(st.o[8 * half + 2 * k + 1], pa, prmt(tA[k], tB[k], 0x7632u), prmt(tC[k], tD[k], 0x7632u));
+                }
             }
         }
     }
@@ -321,8 +343,8 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         s_prefix[0] = 0;
         s_abort = 0;
         if (STAGED) {
-            for (int i = 0; i < a.stages; i++) mbar_init(bar_base + 8 * i, 256);          /* empty[stage]: every thread of the 8 warps that share a page */
-            for (int i = 0; i < 2 * a.stages; i++) mbar_init(bar_base + 64 + 8 * i, 1);   /* full[page mod 2 stages]: the producer's expect_tx */
+            for (int i = 0; i < a.stages; i++) mbar_init(bar_base + 8 * i, 32 * kGranPage<DT>);   /* empty[stage]: every thread of the warps that share a page */
+            for (int i = 0; i < 16; i++) mbar_init(bar_base + 64 + 8 * i, 1);   /* full[page mod n_full]: the producer's expect_tx */
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
@@ -403,6 +425,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
      * slot, scratch records), so wait for it -- except the producer lane, which first starts the
      * copies of pages that lie wholly below the newest slot (append-only cache: immutable).       */
     const bool is_producer = STAGED && warp == kWarps;
+    const unsigned n_full = STAGED ? 16u / (unsigned)a.stages * (unsigned)a.stages : 1u;   /* "full" barriers: a multiple of the stages */
     if (!is_producer) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         /* Only now may the NEXT kernel in the stream start its prologue: it then knows that everything
@@ -462,7 +485,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                     ok = mbar_wait(bar_base + 8 * stage, phase ^ 1u, &s_abort, a.err, 1u);
                     if (!ok) break;
                     const uint8_t *page = cache.pool + hy3a_page_index(cache, block, a.layer, sg.hl) * (size_t)cache.page_bytes;
-                    const unsigned full = bar_base + 64 + 8 * (it % (2u * (unsigned)a.stages));
+                    const unsigned full = bar_base + 64 + 8 * (it % n_full);
                     mbar_expect_tx(full, (unsigned)geom.page_bytes);
                     bulk_g2s(ring_base + stage * (unsigned)geom.page_bytes, page, (unsigned)geom.page_bytes, full, pol);
                 }
@@ -473,7 +496,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 /* gave up: let the copies already issued land before the CTA's shared memory goes away */
                 const unsigned first = it > (unsigned)a.stages ? it - (unsigned)a.stages : 0u;
                 for (unsigned j = first; j < it; j++) {
-                    const unsigned fb = j % (2u * (unsigned)a.stages), fphase = (j / (2u * (unsigned)a.stages)) & 1u;
+                    const unsigned fb = j % n_full, fphase = (j / n_full) & 1u;
                     for (unsigned spin = 0; spin < (1u << 20) && !mbar_test(bar_base + 64 + 8 * fb, fphase); spin++) __nanosleep(64);
                 }
             }
@@ -623,25 +646,39 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
 #pragma unroll
         for (int jn = 0; jn < 16; jn++) { st.o[jn][0] = st.o[jn][1] = st.o[jn][2] = st.o[jn][3] = 0.f; }
 
-        /* granule slot x = 8*(ring position of the page) + granule-in-page; warp w takes slots
-         * x = w (mod kWarps), so any number of consumer warps shares the 8 granules of a page and
-         * each page is released by exactly 8 warps (one arrival per thread per slot).            */
+        /* granule slot x = GP*(ring position of the page) + granule-in-page; warp w takes slots
+         * x = w (mod kWarps), so any number of consumer warps shares the GP granules of a page and
+         * each page is released by exactly GP warps (one arrival per thread per slot).            */
+        constexpr unsigned GP = kGranPage<DT>;
+        constexpr int GT = kGran<DT>;
         const unsigned it_end = it + (unsigned)(sg.p_end - sg.p_begin);
-        for (unsigned x = it * 8u + ((unsigned)warp + kWarps - (it * 8u) % kWarps) % kWarps; x < it_end * 8u; x += kWarps) {
-            const unsigned pit = x >> 3;
-            const int gi = (int)(x & 7u), p = sg.p_begin + (int)(pit - it);
+        unsigned x = it * GP + ((unsigned)warp + kWarps - (it * GP) % kWarps) % kWarps, pit = x / GP;
+        /* ring position of page pit, its "full" barrier and that barrier's phase, carried along (no divisions per granule) */
+        unsigned stage = STAGED ? pit % (unsigned)a.stages : 0u, fb = pit % n_full, fphase = (pit / n_full) & 1u;
+        auto advance = [&]() {
+            x += kWarps;
+            const unsigned d = x / GP - pit;
+            pit += d;
+            if (STAGED) {
+                stage += d;
+                while (stage >= (unsigned)a.stages) stage -= (unsigned)a.stages;
+                fb += d;
+                if (fb >= n_full) { fb -= n_full; fphase ^= 1u; }
+            }
+        };
+        for (; x < it_end * GP; advance()) {
+            const int gi = (int)(x % GP), p = sg.p_begin + (int)(pit - it);
             const int valid = min(HY3A_PT, sg.len - p * HY3A_PT);
             if (STAGED) {
-                const unsigned q2 = pit / (2u * (unsigned)a.stages), r2 = pit - q2 * 2u * (unsigned)a.stages;   /* ring round pair, position in it */
-                const unsigned stage = r2 < (unsigned)a.stages ? r2 : r2 - (unsigned)a.stages;
                 const unsigned spage = ring_base + stage * (unsigned)geom.page_bytes;
-                /* the page's "full" barrier is one of 2 x stages: a warp holds granules in 8 of every 11 pages, so it may skip a
-                 * use of a stage, and an mbarrier wait only knows the parity of a phase.  With one barrier per stage the warp's next
-                 * wait on that stage could pass on the stale phase while the skipped page is still landing (seen with the two-stage
-                 * ring of FP16 pages).  With two barriers per stage the phase a warp can miss is two ring rounds old: every page the
-                 * warp has consumed since was filled after that one had been filled, consumed and its stage filled again. */
-                mbar_wait(bar_base + 64 + 8 * r2, q2 & 1u, &s_abort, a.err, 2u);
-                if (a.fused && a.k_in && p == ((sg.len - 1) >> 7) && gi == (((sg.len - 1) & 127) >> 4)) {
+                /* A warp holds granules in GP of every 11 pages, so it may skip a use of a stage, and an mbarrier wait only knows
+                 * the parity of a phase: with one "full" barrier per stage the warp's next wait on that stage could pass on the
+                 * stale phase while the skipped page is still landing (seen with the two-stage ring of FP16 pages).  So the
+                 * barriers are cycled over n_full pages: page pit - n_full, whose phase a wait for pit could mistake, has long
+                 * been consumed, because this warp's last page pit' >= pit - ceil(11 / GP) was issued after page pit' - stages
+                 * had been consumed, and n_full >= stages + ceil(11 / GP). */
+                mbar_wait(bar_base + 64 + 8 * fb, fphase, &s_abort, a.err, 2u);
+                if (a.fused && a.k_in && p == ((sg.len - 1) >> 7) && gi == ((sg.len - 1) & 127) / GT) {
                     /* fused append: this warp holds the only granule that contains the newest slot.  It
                      * normalises, rotates and quantises the new K row and quantises the new V row exactly
                      * as the append kernel does, writes them to the page in HBM (for later steps) and into
@@ -663,11 +700,11 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                     if (DT != 0 && lane == 0) atomicMax(cache.vs_max + a.layer * G + hl, sb);
                     __syncwarp();
                 }
-                if (16 * gi + 16 <= valid) granule<DT, true, true>(st, sq, qf, nullptr, spage, geom, k_off, v_off, sc_off, gi, tig, valid, pscale);
-                else if (16 * gi < valid) granule<DT, true, false>(st, sq, qf, nullptr, spage, geom, k_off, v_off, sc_off, gi, tig, valid, pscale);
-                mbar_arrive(bar_base + 8 * stage); /* every thread of the 8 warps that share a page releases it */
+                if (GT * gi + GT <= valid) granule<DT, true, true>(st, sq, qf, nullptr, spage, geom, k_off, v_off, sc_off, gi, tig, valid, pscale);
+                else if (GT * gi < valid) granule<DT, true, false>(st, sq, qf, nullptr, spage, geom, k_off, v_off, sc_off, gi, tig, valid, pscale);
+                mbar_arrive(bar_base + 8 * stage); /* every thread of the warps that share a page releases it */
             } else {
-                if (16 * gi >= valid) continue; /* warp-uniform */
+                if (GT * gi >= valid) continue; /* warp-uniform */
                 const int block = cache.block_table[(size_t)sg.seq * cache.max_blocks_per_seq + p];
                 const uint8_t *page = cache.pool + hy3a_page_index(cache, block, a.layer, hl) * (size_t)cache.page_bytes;
                 granule<DT, false, false>(st, sq, qf, page, 0u, geom, k_off, v_off, sc_off, gi, tig, valid, pscale);

@@ -95,6 +95,33 @@ def test_decode_is_bitwise_repeatable(cuda, dt):
     assert differing == 0, "%d of 360 launches differ from the first" % differing
 
 
+@pytest.mark.parametrize("dt", ["int4", "fp16"])
+@pytest.mark.parametrize("n", [40017, 351])
+def test_ring_depth_does_not_matter(cuda, dt, n, monkeypatch):
+    """Every depth of the page ring gives the same bits, back to back (a consumer warp skips pages: up to two INT4 pages lie
+    between its 32-token granules), and 32-token granules end anywhere in the last page."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    q = torch.randn((1, 64, 128), device=cuda, generator=torch.Generator(device=cuda).manual_seed(6))
+    ref = None
+    for stages in (None, 2) if dt == "fp16" else (None, 2, 3, 5, 7):
+        if stages is None:
+            monkeypatch.delenv("HY3A_DECODE_STAGES", raising=False)
+        else:
+            monkeypatch.setenv("HY3A_DECODE_STAGES", str(stages))
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_batch=1, max_tokens=n + 128)
+        ctx.fill_random(0, 0, 0, n, 9)
+        outs = []
+        for m in (n, n - 1, n - 15, n - 16, n - 17, n - 31, n - 32, n - 33):
+            ctx.batch_set([0], [m - 1])
+            outs += [ctx.decode(0, q).clone() for _ in range(8)]
+        ctx.sync()
+        ctx.close()
+        ref = ref or outs
+        assert all(torch.equal(a, b) for a, b in zip(outs, ref)), "stages=%s" % stages
+        assert all(torch.equal(outs[i], outs[i - i % 8]) for i in range(len(outs)))
+
+
 def test_decode_ragged_batch_and_poison(cuda, oracle):
     """Several sequences of different lengths in one launch; cache bytes past each length are poison."""
     import torch
