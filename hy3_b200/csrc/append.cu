@@ -115,103 +115,180 @@ __global__ void __launch_bounds__(256) hy3a_append_kernel(hy3a_cache_view cache,
 }
 
 /* ---- the same work for a chunk of rows (prefill): blocks shaped for throughput -----------------------------------
- * With hundreds of rows the per-row blocks above are bound by their own latency (5 120 blocks for 512 rows, each with a
- * cosf/sinf stage in front of one 512-byte load per warp).  Here all blocks of a chunk are resident at once:
- *   blocks [0, n)            one row each: the 64 query heads, 8 per warp, loads issued up front, RoPE coefficients once
- *                            per row;
- *   blocks [n, n + kvh*ng)   one owned KV head x 8 consecutive rows (ng = ceil(n / 8)), warp = row: K and V of that head.
- *                            Eight consecutive tokens of one head in one block make the write-through of the
- *                            TRANSPOSED V operand a 16-byte store per head dim (staged in shared memory).
- * The arithmetic is the per-row kernel's (same rowops functions), so codes, scales and queries are identical bits. */
+ * blocks [0, ng*hg)    8 consecutive rows (warp = row) x hpb <= 4 owned KV heads: K and V of those heads; ng = ceil(n / 8),
+ *                      hg = ceil(kv_heads / hpb); hpb grows with the rows, so that short chunks spread over the SMs.  Eight consecutive tokens in one block make the transposed V codes of INT8
+ *                      pages an 8-byte store and the write-through of the transposed V operand a 16-byte store per head dim
+ *                      (staged in shared memory), and the running V scale maximum one atomic per head.
+ * blocks [ng*hg, +n)   one row each: the 64 query heads, 8 per warp, loads issued up front.
+ * Issue slots bound this kernel more than bytes (512 rows move 29 MB), so:
+ *   - cos / sin are computed once per row and block by all threads (64 full-range pairs a row), before the wait for the
+ *     preceding kernel: they need only what the host wrote;
+ *   - a lane of a query warp holds dims {2 lane, 2 lane + 1} and their rotate_half partners, so RoPE needs no exchange, and
+ *     the sums of squares of the warp's 8 heads are reduced together: at each level of the tree a lane hands half of its
+ *     sums to its partner and keeps the other half: 25 shuffles for 8 heads instead of 192.
+ * Every sum has the per-row kernel's operands at every level of the tree, so queries, codes and scales are identical bits. */
+constexpr int kChunkHeads = 4;
 template <int DT>
-__global__ void __launch_bounds__(256) hy3a_append_chunk_kernel(hy3a_cache_view cache, hy3a_batch_view batch, hy3a_rope_params rope, append_args a, int aligned8) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__global__ void __launch_bounds__(256, 4) hy3a_append_chunk_kernel(hy3a_cache_view cache, hy3a_batch_view batch, hy3a_rope_params rope, append_args a, int kv_blocks, int hpb, int contig8) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = batch.n;
-    const int half = lane >> 4, idx = lane & 15, d0 = half * 64 + idx * 4;
     const hy3a_geom g = hy3a_make_geom(DT);
-    if ((int)blockIdx.x < n) {
-        /* ---- query block */
-        const int row = blockIdx.x;
-        __shared__ float s_cos[64], s_sin[64];
-        if (threadIdx.x < 64) {
-            const int ti = batch.pos[row];
+    const bool is_qb = (int)blockIdx.x >= kv_blocks;
+    const int hg = (cache.kv_heads + hpb - 1) / hpb, grp = (int)blockIdx.x / hg;
+    __shared__ __align__(16) float s_cos[8][64], s_sin[8][64];
+    {
+        const int rows = is_qb ? 1 : 8, row0 = is_qb ? (int)blockIdx.x - kv_blocks : grp * 8;
+        for (int i = threadIdx.x; i < rows * 64; i += 256) {
+            const int r = i >> 6, d = i & 63;
+            if (row0 + r >= n) continue;
+            const int ti = batch.pos[row0 + r];
             const int pos = (ti + (ti >= rope.pos_jump_at ? rope.pos_jump : 0)) * rope.pos_stride;
-            const float fr = (float)pos * rope.inv_freq[threadIdx.x];
-            s_cos[threadIdx.x] = cosf(fr) * rope.attn_factor;
-            s_sin[threadIdx.x] = sinf(fr) * rope.attn_factor;
+            const float fr = (float)pos * rope.inv_freq[d];
+            s_cos[r][d] = cosf(fr) * rope.attn_factor;
+            s_sin[r][d] = sinf(fr) * rope.attn_factor;
         }
-        float4 xv[8];
-        const float *src = a.q_in + (size_t)row * a.q_stride + d0;
+    }
+    if (is_qb) {
+        /* ---- query block */
+        const int row = blockIdx.x - kv_blocks, d = 2 * lane;
+        const float2 wl = *reinterpret_cast<const float2 *>(a.norm_w + d), wh = *reinterpret_cast<const float2 *>(a.norm_w + 64 + d);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        float2 xl[8], xh[8];
+        const float *src = a.q_in + (size_t)row * a.q_stride + d;
 #pragma unroll
-        for (int i = 0; i < 8; i++) xv[i] = *reinterpret_cast<const float4 *>(src + (size_t)(warp + 8 * i) * HY3A_D);
-        const float4 wv = *reinterpret_cast<const float4 *>(a.norm_w + d0);
+        for (int i = 0; i < 8; i++) {
+            xl[i] = *reinterpret_cast<const float2 *>(src + (size_t)(warp + 8 * i) * HY3A_D);
+            xh[i] = *reinterpret_cast<const float2 *>(src + (size_t)(warp + 8 * i) * HY3A_D + 64);
+        }
+        /* sums of squares in the reference's tree order (hy3_gpu.cu:155-157): (d, d+64) in the lane, then lane bits 4..0 for
+         * 32, 16, 8, 4, 2, then the even and the odd dims */
+        float v[16];                 /* [head][parity] */
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            v[2 * i] = __fadd_rn(__fmul_rn(xl[i].x, xl[i].x), __fmul_rn(xh[i].x, xh[i].x));
+            v[2 * i + 1] = __fadd_rn(__fmul_rn(xl[i].y, xl[i].y), __fmul_rn(xh[i].y, xh[i].y));
+        }
+#pragma unroll
+        for (int o = 16, k = 8; o > 1; o >>= 1, k >>= 1) {
+            const bool up = lane & o;          /* keeps the upper half of the sums */
+#pragma unroll
+            for (int i = 0; i < k; i++) {
+                const float send = up ? v[i] : v[k + i], keep = up ? v[k + i] : v[i];
+                v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, o));
+            }
+        }
+        v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
+        const float ss = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], 2));      /* of head (lane bits 4, 3, 2) */
+        const float rr = rsqrtf(ss / (float)HY3A_D + a.eps);
         __syncthreads();
-        const float4 cv4 = *reinterpret_cast<const float4 *>(s_cos + idx * 4), sv4 = *reinterpret_cast<const float4 *>(s_sin + idx * 4);
-        const float c[4] = {cv4.x, cv4.y, cv4.z, cv4.w}, sn[4] = {sv4.x, sv4.y, sv4.z, sv4.w};
+        const float2 c = *reinterpret_cast<const float2 *>(&s_cos[0][d]), sn = *reinterpret_cast<const float2 *>(&s_sin[0][d]);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const int head = warp + 8 * i;
-            float y[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
-            norm_rope_apply(y, wv, a.eps, c, sn, lane);
-            if (a.q_out) *reinterpret_cast<float4 *>(a.q_out + (size_t)row * a.q_out_stride + (size_t)head * HY3A_D + d0) = make_float4(y[0], y[1], y[2], y[3]);
+            const float r = __shfl_sync(0xffffffffu, rr, 4 * i);
+            const float l0 = xl[i].x * r * wl.x, l1 = xl[i].y * r * wl.y, h0 = xh[i].x * r * wh.x, h1 = xh[i].y * r * wh.y;
+            /* the per-row kernel's contractions, spelled out: own dim x cos is the fused product in both halves */
+            const float2 yl = make_float2(__fmaf_rn(l0, c.x, -__fmul_rn(h0, sn.x)), __fmaf_rn(l1, c.y, -__fmul_rn(h1, sn.y)));
+            const float2 yh = make_float2(__fmaf_rn(h0, c.x, __fmul_rn(l0, sn.x)), __fmaf_rn(h1, c.y, __fmul_rn(l1, sn.y)));
+            if (a.q_out) {
+                float *dst = a.q_out + (size_t)row * a.q_out_stride + (size_t)head * HY3A_D + d;
+                *reinterpret_cast<float2 *>(dst) = yl;
+                *reinterpret_cast<float2 *>(dst + 64) = yh;
+            }
             if (a.q_out16) {
-                __half2 h01 = __floats2half2_rn(y[0], y[1]), h23 = __floats2half2_rn(y[2], y[3]);
-                uint2 w2;
-                w2.x = *reinterpret_cast<unsigned *>(&h01);
-                w2.y = *reinterpret_cast<unsigned *>(&h23);
-                *reinterpret_cast<uint2 *>(a.q_out16 + ((size_t)row * 64 + head) * HY3A_D + d0) = w2;
+                __half *dst = a.q_out16 + ((size_t)row * 64 + head) * HY3A_D + d;
+                *reinterpret_cast<__half2 *>(dst) = __floats2half2_rn(yl.x, yl.y);
+                *reinterpret_cast<__half2 *>(dst + 64) = __floats2half2_rn(yh.x, yh.y);
             }
         }
         return;
     }
-    /* ---- K/V block: owned head hl, rows 8 grp .. 8 grp + 7 (warp = row) */
-    const int kb = blockIdx.x - n, hl = kb % cache.kv_heads, grp = kb / cache.kv_heads;
-    const int head = cache.kv_head_begin + hl, row = grp * 8 + warp;
+    /* ---- K/V block: owned heads h0 .. h0 + nh - 1, rows 8 grp .. 8 grp + 7 (warp = row) */
+    const int half = lane >> 4, idx = lane & 15, d0 = half * 64 + idx * 4;
+    const int h0 = ((int)blockIdx.x - grp * hg) * hpb, nh = min(hpb, cache.kv_heads - h0), row = grp * 8 + warp;
     const bool live = row < n;
-    __shared__ __align__(16) __half s_vt[HY3A_D][8];
-    int slot = 0;
+    /* 8 whole, aligned, consecutive token columns of one sequence: the transposed stores are staged */
+    const bool whole8 = contig8 && grp * 8 + 8 <= n;
+    __shared__ __align__(16) __half s_vt[kChunkHeads][HY3A_D][8];
+    __shared__ __align__(8) uint8_t s_vc[kChunkHeads][HY3A_D][8];
+    __shared__ unsigned s_vmax[kChunkHeads];
+    if (threadIdx.x < kChunkHeads) s_vmax[threadIdx.x] = 0u;
+    const float4 wv = *reinterpret_cast<const float4 *>(a.norm_w + HY3A_D + d0);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    float4 kx = make_float4(0.f, 0.f, 0.f, 0.f), vx = kx;
+    int slot = 0, seq = 0;
+    const float *ks = nullptr, *vs = nullptr;
     if (live) {
-        const int seq = batch.seq[row], ti = batch.pos[row];
-        slot = batch.slot[row];
-        const float4 kx = *reinterpret_cast<const float4 *>(a.k_in + (size_t)row * a.k_stride + (size_t)head * HY3A_D + d0);
-        const float4 vx = *reinterpret_cast<const float4 *>(a.v_in + (size_t)row * a.v_stride + (size_t)head * HY3A_D + d0);
-        uint8_t *page = page_ptr(cache, seq, slot, a.layer, hl);
-        int codes[4];
-        {
-            float y[4] = {kx.x, kx.y, kx.z, kx.w};
-            norm_rope_row(y, a.norm_w + HY3A_D, a.eps, rope, ti, lane);
-            const unsigned sb = store_row<DT>(page, g, slot & 127, false, y, d0, lane, nullptr, codes);
-            if (a.mirror_k) {
-                __half hv[4];
-                const float sc = DT == 0 ? 0.f : __half2float(__ushort_as_half((unsigned short)sb));
-#pragma unroll
-                for (int j = 0; j < 4; j++) hv[j] = DT == 0 ? __float2half_rn(y[j]) : __float2half_rn((float)codes[j] * sc);
-                *reinterpret_cast<uint2 *>(a.mirror_k + ((size_t)hl * a.mirror_stride + slot) * HY3A_D + d0) = *reinterpret_cast<uint2 *>(hv);
+        seq = batch.seq[row]; slot = batch.slot[row];
+        const size_t off = (size_t)(cache.kv_head_begin + h0) * HY3A_D + d0;
+        ks = a.k_in + (size_t)row * a.k_stride + off;
+        vs = a.v_in + (size_t)row * a.v_stride + off;
+        kx = *reinterpret_cast<const float4 *>(ks);
+        vx = *reinterpret_cast<const float4 *>(vs);
+    }
+    __syncthreads();
+    if (live) {
+        const float4 cv4 = *reinterpret_cast<const float4 *>(&s_cos[warp][idx * 4]), sv4 = *reinterpret_cast<const float4 *>(&s_sin[warp][idx * 4]);
+        const float c[4] = {cv4.x, cv4.y, cv4.z, cv4.w}, sn[4] = {sv4.x, sv4.y, sv4.z, sv4.w};
+        uint8_t *page = page_ptr(cache, seq, slot, a.layer, h0);
+        /* not unrolled: straight-line code for 4 heads is fetched from L2 once per launch, which cost more than the loop */
+#pragma unroll 1
+        for (int i = 0; i < nh; i++, page += cache.page_bytes) {
+            const float4 kc = kx, vc = vx;
+            if (i + 1 < nh) {
+                kx = *reinterpret_cast<const float4 *>(ks + (i + 1) * HY3A_D);
+                vx = *reinterpret_cast<const float4 *>(vs + (i + 1) * HY3A_D);
             }
-        }
-        {
-            float y[4] = {vx.x, vx.y, vx.z, vx.w};
-            const unsigned sb = store_row<DT>(page, g, slot & 127, true, y, d0, lane, nullptr, codes);
-            if (DT != 0 && lane == 0) atomicMax(cache.vs_max + a.layer * cache.kv_heads + hl, sb);
-            if (a.mirror_k) {
-                const float sc = DT == 0 ? 0.f : __half2float(__ushort_as_half((unsigned short)sb));
+            const int hl = h0 + i;
+            int codes[4];
+            {
+                float y[4] = {kc.x, kc.y, kc.z, kc.w};
+                norm_rope_apply(y, wv, a.eps, c, sn, lane);
+                const unsigned sb = store_row<DT>(page, g, slot & 127, false, y, d0, lane, nullptr, codes);
+                if (a.mirror_k) {
+                    __half hv[4];
+                    const float sc = DT == 0 ? 0.f : __half2float(__ushort_as_half((unsigned short)sb));
 #pragma unroll
-                for (int j = 0; j < 4; j++) s_vt[d0 + j][warp] = DT == 0 ? __float2half_rn(y[j]) : __float2half_rn((float)codes[j] * sc);
+                    for (int j = 0; j < 4; j++) hv[j] = DT == 0 ? __float2half_rn(y[j]) : __float2half_rn((float)codes[j] * sc);
+                    *reinterpret_cast<uint2 *>(a.mirror_k + ((size_t)hl * a.mirror_stride + slot) * HY3A_D + d0) = *reinterpret_cast<uint2 *>(hv);
+                }
+            }
+            {
+                float y[4] = {vc.x, vc.y, vc.z, vc.w};
+                const unsigned sb = store_row<DT>(page, g, slot & 127, true, y, d0, lane, nullptr, codes, DT == 1 && whole8);
+                if (DT != 0 && lane == 0) atomicMax(&s_vmax[i], sb);
+                if (DT == 1 && whole8) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) s_vc[i][d0 + j][warp] = (uint8_t)(codes[j] & 0xFF);
+                }
+                if (a.mirror_k) {
+                    const float sc = DT == 0 ? 0.f : __half2float(__ushort_as_half((unsigned short)sb));
+#pragma unroll
+                    for (int j = 0; j < 4; j++) s_vt[i][d0 + j][warp] = DT == 0 ? __float2half_rn(y[j]) : __float2half_rn((float)codes[j] * sc);
+                }
             }
         }
     }
-    if (!a.mirror_k) return;      /* uniform over the block */
     __syncthreads();
-    if (threadIdx.x < HY3A_D) {
-        /* rows of a mirrored chunk are consecutive slots of one sequence: the block's 8 tokens are 8 adjacent columns */
-        const int d = threadIdx.x, slot_base = batch.slot[grp * 8];
-        __half *dst = a.mirror_v + ((size_t)hl * HY3A_D + d) * a.mirror_stride + slot_base;
-        const int nrow = min(8, n - grp * 8);
-        if (aligned8 && nrow == 8) {
-            *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(&s_vt[d][0]);
+    if (DT != 0 && (int)threadIdx.x < nh) atomicMax(cache.vs_max + a.layer * cache.kv_heads + h0 + threadIdx.x, s_vmax[threadIdx.x]);
+    if (DT == 1 && whole8) {
+        const int s0 = batch.slot[grp * 8], q0 = batch.seq[grp * 8];
+        for (int e = threadIdx.x; e < nh * HY3A_D; e += 256) {
+            const int i = e / HY3A_D, d = e % HY3A_D;
+            *reinterpret_cast<uint2 *>(page_ptr(cache, q0, s0, a.layer, h0 + i) + g.v_off + hy3a_vt_off(d, s0 & 127)) = *reinterpret_cast<const uint2 *>(&s_vc[i][d][0]);
+        }
+    }
+    if (!a.mirror_k) return;
+    /* rows of a mirrored chunk are consecutive slots of one sequence: the block's tokens are adjacent columns */
+    const int slot_base = batch.slot[grp * 8], nrow = min(8, n - grp * 8);
+    for (int e = threadIdx.x; e < nh * HY3A_D; e += 256) {
+        const int i = e / HY3A_D, d = e % HY3A_D;
+        __half *dst = a.mirror_v + ((size_t)(h0 + i) * HY3A_D + d) * a.mirror_stride + slot_base;
+        if (whole8) {
+            *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(&s_vt[i][d][0]);
         } else {
-            for (int t = 0; t < nrow; t++) dst[t] = s_vt[d][t];
+            for (int t = 0; t < nrow; t++) dst[t] = s_vt[i][d][t];
         }
     }
 }
@@ -355,13 +432,17 @@ int hy3a_launch_append(hy3a_ctx *ctx, int layer, const float *q_in, size_t q_str
     cfg.attrs = attr; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
     cudaError_t e;
     if (ctx->batch_n >= 32) {      /* a chunk: the throughput-shaped kernel */
-        const int n = ctx->batch_n, kv_blocks = k_in ? ctx->cfg.kv_head_count * ((n + 7) / 8) : 0;
-        const int aligned8 = a.mirror_k && (ctx->batch_slot0 % 8 == 0) && (ctx->pf_mcap[layer] % 8 == 0);
+        const int n = ctx->batch_n, ng = (n + 7) / 8, kvh = ctx->cfg.kv_head_count;
+        int hpb = 1;      /* KV heads per block: as many as leave two blocks per SM (a block's heads run one after the other) */
+        while (hpb < kChunkHeads && ng * ((kvh + 2 * hpb - 1) / (2 * hpb)) >= 2 * ctx->sm_count) hpb *= 2;
+        const int kv_blocks = k_in ? (kvh + hpb - 1) / hpb * ng : 0;
+        /* groups of 8 rows are 8 aligned columns of one sequence (mirror strides are multiples of 1 024) */
+        const int contig8 = ctx->batch_contig && ctx->batch_slot0 % 8 == 0;
         cfg.gridDim = dim3(n + kv_blocks);
         switch (ctx->geom.dtype) {
-            case 0: e = cudaLaunchKernelEx(&cfg, hy3a_append_chunk_kernel<0>, cv, bv, ctx->rope, a, aligned8); break;
-            case 1: e = cudaLaunchKernelEx(&cfg, hy3a_append_chunk_kernel<1>, cv, bv, ctx->rope, a, aligned8); break;
-            default: e = cudaLaunchKernelEx(&cfg, hy3a_append_chunk_kernel<2>, cv, bv, ctx->rope, a, aligned8); break;
+            case 0: e = cudaLaunchKernelEx(&cfg, hy3a_append_chunk_kernel<0>, cv, bv, ctx->rope, a, kv_blocks, hpb, contig8); break;
+            case 1: e = cudaLaunchKernelEx(&cfg, hy3a_append_chunk_kernel<1>, cv, bv, ctx->rope, a, kv_blocks, hpb, contig8); break;
+            default: e = cudaLaunchKernelEx(&cfg, hy3a_append_chunk_kernel<2>, cv, bv, ctx->rope, a, kv_blocks, hpb, contig8); break;
         }
         ctx->launches++;
         ctx->bulk_write_pending = 1;

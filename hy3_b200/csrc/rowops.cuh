@@ -28,7 +28,8 @@ __device__ __forceinline__ uint8_t *page_ptr(const hy3a_cache_view &c, int seq, 
 template <int DT>
 __device__ __forceinline__ unsigned store_row(uint8_t *page, const hy3a_geom &g, int tok, bool is_v, const float y[4], int d0, int lane,
                                               uint8_t *scale_page = nullptr /* where the scale goes, if not into `page` (a shared-memory copy split in two) */,
-                                              int *codes_out = nullptr /* the lane's 4 codes (quantised caches) */) {
+                                              int *codes_out = nullptr /* the lane's 4 codes (quantised caches) */,
+                                              bool skip_vt = false /* INT8 V: leave the transposed code bytes to the caller */) {
     if (DT == 0) {
         __half2 h01 = __floats2half2_rn(y[0], y[1]);
         __half2 h23 = __floats2half2_rn(y[2], y[3]);
@@ -56,7 +57,7 @@ __device__ __forceinline__ unsigned store_row(uint8_t *page, const hy3a_geom &g,
         if (!is_v) {
             unsigned w = (unsigned)(c[0] & 0xFF) | ((unsigned)(c[1] & 0xFF) << 8) | ((unsigned)(c[2] & 0xFF) << 16) | ((unsigned)(c[3] & 0xFF) << 24);
             *reinterpret_cast<unsigned *>(page + hy3a_k_dim_off<1>(tok, d0)) = w;
-        } else {
+        } else if (!skip_vt) {
             /* V codes go into the transposed tile: one byte per (head dim, token) */
 #pragma unroll
             for (int j = 0; j < 4; j++) page[g.v_off + hy3a_vt_off(d0 + j, tok)] = (uint8_t)(c[j] & 0xFF);

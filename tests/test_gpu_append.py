@@ -179,3 +179,37 @@ def test_chunk_kernel_equals_row_kernel(cuda, oracle, dt, heads):
         ctx.close()
     for a, b, what in zip(res[0], res[1], ("q fp32", "q fp16", "K slots", "V slots")):
         assert np.array_equal(a, b), what
+
+
+@pytest.mark.parametrize("seqs", [1, 2])
+@pytest.mark.parametrize("heads", [(0, 8), (3, 5), (7, 1)])
+@pytest.mark.parametrize("dt", ["int8", "int4", "fp16"])
+def test_chunk_kernel_aligned_columns(cuda, oracle, dt, heads, seqs):
+    """The chunk kernel's staged stores (8 aligned consecutive slots; pages crossed; a ragged tail; head groups of 4 + 1) and
+    a batch of two sequences that must not take them, against the per-row kernel: identical bytes."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    n, slot0 = 75, 104
+    q = oracle.fill_normal((n, 64, 128), SEED, 811)
+    k = oracle.fill_normal((n, 8, 128), SEED, 812)
+    v = oracle.fill_normal((n, 8, 128), SEED, 813)
+    v[5] = 0.0
+    sid = [0] * n if seqs == 1 else [i % 2 for i in range(n)]
+    slots = [slot0 + (i if seqs == 1 else i // 2) for i in range(n)]
+    tq, tk, tv = (torch.from_numpy(a).to(cuda) for a in (q, k, v))
+    res = []
+    for step in (n, 25):
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_seqs=2, max_batch=n, max_tokens=1024, max_tokens_per_seq=512, kv_head_begin=heads[0], kv_head_count=heads[1])
+        qo = torch.empty((n, 64, 128), device=cuda)
+        for b in range(0, n, step):
+            e = min(n, b + step)
+            ctx.batch_set(sid[b:e], slots[b:e], [3 * x for x in slots[b:e]])
+            ctx.append(0, tq[b:e], tk[b:e], tv[b:e], q_out=qo[b:e])
+        ctx.sync()
+        out = [qo.cpu().numpy()]
+        for s in range(seqs):
+            out += list(ctx.export_kv(0, s, slot0, sid.count(s)))
+        res.append(out)
+        ctx.close()
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
