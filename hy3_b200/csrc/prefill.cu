@@ -312,6 +312,10 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         for (int i = 0; i < 4; i++) mbar_init(BAR(B3_O + i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == 8 && lane < 3) {   /* the descriptors' first use is then no miss behind the wait for the preceding kernel */
+        const CUtensorMap *m = lane == 0 ? &tm_q : (lane == 1 ? &tm_k : &tm_v);
+        asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
+    }
     if (warp == 0) {   /* one warp allocates all 512 TMEM columns (1 CTA per SM) */
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + kOff3Bar + 256), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -409,10 +413,9 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
     } else {
         /* ===================== softmax warps: tile x = warp / 4; thread = one row of Q tile x ===================== */
-        const int x = warp >> 2, r = tid & 127, t_local = r >> 3, h = r & 7;
+        const int x = warp >> 2, t_local = (tid & 127) >> 3;
         const int tq0 = q0 + x * kQTok;                          /* first query token of this tile */
         const int qpos = a.base + tq0 + t_local;                 /* global index of this row's query */
-        const bool row_valid = (tq0 + t_local) < a.nq;
         const unsigned lane_base = (unsigned)((warp & 3) * 32) << 16; /* this warp's quarter of the TMEM lanes */
         const unsigned tm_o = tmem + 256u + 128u * x + lane_base;
         float m = -INFINITY;
@@ -480,18 +483,33 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         if (ok && ntiles > 0) ok = mbar_wait_blocking(BAR(B3_O + 2 * x + 1), 0u, s_abort, a.err, 32u);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (__all_sync(0xffffffffu, ok) && ntiles > 0) {      /* warp-uniform: tcgen05.ld is warp-collective */
+            /* A thread holds a row, so storing from the registers touches 32 rows per instruction; the warp's 32 rows go through
+             * shared memory instead, 64 columns at a time (its quarter of Q_x, which P.V's last commit says is read; 16-byte
+             * chunk c of row r at c ^ (r & 7): conflict-free both ways), and leave as two rows of 256 contiguous bytes per
+             * instruction. */
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            float *orow = a.out + (size_t)(tq0 + t_local) * a.out_stride + (size_t)((a.kv_head_begin + hl) * 8 + h) * HY3A_D;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                unsigned v[32];
-                tmem_ld32_nowait(tm_o + 32u * c, v);
+            uint8_t *stage = sm + kOff3Q + x * kTileBytes + (warp & 3) * 8192;
+            const int t0 = tq0 + (warp & 3) * 4, nrow = min(32, (a.nq - t0) * 8);          /* rows of valid query tokens (none: <= 0) */
+            float *o0 = a.out + (size_t)t0 * a.out_stride + (size_t)((a.kv_head_begin + hl) * 8) * HY3A_D + (lane & 15) * 4;
+#pragma unroll 1
+            for (int c = 0; c < 2; c++) {
+                unsigned v[64];
+                tmem_ld32_nowait(tm_o + 64u * c, v);
+                tmem_ld32_nowait(tm_o + 64u * c + 32u, v + 32);
                 tmem_ld_wait(v);
-                if (row_valid)
+                tmem_ld_wait(v + 32);
 #pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                    *reinterpret_cast<float4 *>(orow + 32 * c + i) = make_float4(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv,
-                                                                                   __uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
+                for (int i = 0; i < 16; i++)
+                    *reinterpret_cast<float4 *>(stage + lane * 256 + ((i ^ (lane & 7)) << 4)) =
+                        make_float4(__uint_as_float(v[4 * i]) * inv, __uint_as_float(v[4 * i + 1]) * inv, __uint_as_float(v[4 * i + 2]) * inv, __uint_as_float(v[4 * i + 3]) * inv);
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int r2 = 2 * i + (lane >> 4);
+                    if (r2 < nrow) *reinterpret_cast<float4 *>(o0 + (size_t)(r2 >> 3) * a.out_stride + (r2 & 7) * HY3A_D + 64 * c) =
+                        *reinterpret_cast<const float4 *>(stage + r2 * 256 + (((lane & 15) ^ (r2 & 7)) << 4));
+                }
+                __syncwarp();
             }
         }
     }
