@@ -242,3 +242,14 @@ def decode_schedule(kv_lens, kv_heads, n_ctas, cta):
     if rc:
         raise Hy3AttnError(rc, "bad schedule arguments")
     return tot.value, u0.value, u1.value
+
+
+def prefill_schedule(base_slot, nq, kv_heads, sms=148, max_records=512):
+    """Pure host arithmetic of the prefill's cut into CTAs: int32 rows {query block, first step, steps, first record, piece,
+    pieces of the block} of one KV head in launch order (no rows: uncut blocks in descending order)."""
+    lib = load_library()
+    buf = np.zeros((256, 6), np.int32)
+    n = lib.hy3a_prefill_schedule(base_slot, nq, kv_heads, sms, max_records, buf.ctypes.data_as(C.POINTER(C.c_int)), 256)
+    if n < 0:
+        raise Hy3AttnError(n, "bad schedule arguments")
+    return buf[:n]

@@ -115,6 +115,18 @@ int hy3a_decode_schedule(int n, const int *kv_lens, int kv_heads, int n_ctas, in
     return 0;
 }
 
+int hy3a_prefill_schedule(int base_slot, int nq, int kv_heads, int sms, int max_records, int *pieces, int cap) {
+    if (base_slot < 0 || nq < 1 || kv_heads < 1 || kv_heads > HY3A_N_KV_HEAD || sms < 1 || max_records < 0 || max_records > HY3A_PF_MAX_SLOTS || !pieces || cap < 0) return HY3A_EINVAL;
+    hy3a_pf_table t;
+    hy3a_pf_plan(base_slot, nq, kv_heads, sms, max_records, &t);
+    for (int i = 0; i < t.count && i < cap; i++) {
+        const hy3a_pf_piece &e = t.e[i];
+        const int row[6] = {e.qblk, e.j0, e.n, e.rec, e.piece, e.np};
+        memcpy(pieces + 6 * i, row, sizeof(row));
+    }
+    return t.count;
+}
+
 void hy3a_destroy(hy3a_ctx *ctx) {
     if (!ctx) return;
     int prev = -1;
@@ -123,7 +135,7 @@ void hy3a_destroy(hy3a_ctx *ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->pool); cudaFree(ctx->d_block_table); cudaFree(ctx->d_vs_max); cudaFree(ctx->d_inv_freq);
     cudaFree(ctx->d_norm_w); cudaFree(ctx->d_batch); cudaFree(ctx->d_partials); cudaFree(ctx->d_counters); cudaFree(ctx->d_err);
-    cudaFree(ctx->d_pf_k); cudaFree(ctx->d_pf_v);
+    cudaFree(ctx->d_pf_k); cudaFree(ctx->d_pf_v); cudaFree(ctx->d_pf_rec); cudaFree(ctx->d_pf_cnt);
     for (int l = 0; l < HY3A_MAX_LAYERS; l++) { cudaFree(ctx->pf_mk[l]); cudaFree(ctx->pf_mv[l]); }
     hy3a_shard_disconnect(ctx);
     cudaFree(ctx->shard_local);
@@ -215,6 +227,15 @@ int hy3a_create(const hy3a_config *cfg, hy3a_ctx **out) {
     CREATE_CUDA(cudaMemsetAsync(ctx->d_counters, 0, (size_t)2 * cfg->max_batch * cfg->kv_head_count * sizeof(unsigned), ctx->stream));
     CREATE_CUDA(cudaMalloc(&ctx->d_err, HY3A_ERR_WORDS * sizeof(unsigned)));
     CREATE_CUDA(cudaMemsetAsync(ctx->d_err, 0, HY3A_ERR_WORDS * sizeof(unsigned), ctx->stream));
+    /* records of the chunked prefill's cut blocks (contexts that take chunks; without room the blocks stay uncut) */
+    if (cfg->max_batch >= 16) {
+        if (cudaMalloc(&ctx->d_pf_rec, (size_t)HY3A_PF_MAX_SLOTS * HY3A_PF_REC_BYTES) != cudaSuccess || cudaMalloc(&ctx->d_pf_cnt, (size_t)HY3A_PF_MAX_SLOTS * 8 * sizeof(unsigned)) != cudaSuccess ||
+            cudaMemsetAsync(ctx->d_pf_cnt, 0, (size_t)HY3A_PF_MAX_SLOTS * 8 * sizeof(unsigned), ctx->stream) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(ctx->d_pf_rec); cudaFree(ctx->d_pf_cnt);
+            ctx->d_pf_rec = NULL; ctx->d_pf_cnt = NULL;
+        }
+    }
     /* operand mirrors of the chunked prefill, sized for a whole sequence, when a context that takes chunks (max_batch >= 16:
      * one query tile) can hold all layers' mirrors within the budget: hy3a_prefill then never allocates.  Zeroed once:
      * columns past a sequence's end are read by the last tile (and masked), so they must never hold a NaN or Inf pattern. */
@@ -295,6 +316,7 @@ int hy3a_sync(hy3a_ctx *ctx) {
         cudaMemsetAsync(ctx->d_err, 0, HY3A_ERR_WORDS * sizeof(unsigned), ctx->stream);
         /* a kernel that gave up may have left merge counters behind */
         cudaMemsetAsync(ctx->d_counters, 0, (size_t)2 * ctx->cfg.max_batch * ctx->cfg.kv_head_count * sizeof(unsigned), ctx->stream);
+        if (ctx->d_pf_cnt) cudaMemsetAsync(ctx->d_pf_cnt, 0, (size_t)HY3A_PF_MAX_SLOTS * 8 * sizeof(unsigned), ctx->stream);
         return hy3a_fail(ctx, HY3A_ETIMEOUT, "device-side bounded wait or bounds check failed (code %u, where %u, detail %u %u)", code, where, w2, w3);
     }
     return HY3A_OK;

@@ -7,6 +7,7 @@
 
 #include "../../include/hy3_attn.h"
 #include "layout.h"
+#include "prefill_plan.h"
 
 #define HY3A_MAX_LAYERS 128
 #ifndef HY3A_DECODE_WARPS
@@ -77,6 +78,10 @@ struct hy3a_ctx {
     int pf_mntok[HY3A_MAX_LAYERS];  /* tokens converted and still valid */
     int pf_mseq;                    /* the sequence all mirrors belong to, -1 = none */
     size_t pf_mbytes, pf_mbudget;   /* allocated / allowed bytes of mirrors (HY3A_PF_MIRROR_MB, 0 = no mirrors) */
+    float *d_pf_rec;        /* prefill: records of cut blocks, NULL = blocks stay uncut (prefill_plan.h) */
+    unsigned int *d_pf_cnt; /* their arrival counters (self-resetting) */
+    hy3a_pf_table pf_plan;  /* the cut of the chunk (pf_plan_base, pf_plan_nq): a function of these sizes alone */
+    int pf_plan_base, pf_plan_nq;
     unsigned int *d_err;  /* HY3A_ERR_WORDS words: kernels record bounded-wait timeouts / bad indices here */
     size_t partial_records;
 

@@ -167,8 +167,10 @@ __device__ __forceinline__ float ex2v(float x) { float r; asm volatile("ex2.appr
  * rounding of P is a zero-mean 2^-12 relative error per term, far below the tolerance).  One pair in eight goes through the FMA
  * pipe: 512 tokens behind 4 096 take 75 us with none, 69-70 us with one, 74-76 us with two or more (the FMA form costs issue
  * slots that the waiting tile's maximum wants). */
+template <bool CUT>
 __device__ __forceinline__ float2 softmax_exp(const unsigned (&v)[64], float m, unsigned (&pk)[32], int x, bool pass) {
-    const float2 sc = splat(kScaleLog2), nm = splat(-m);
+    /* m == -inf: every key of the row so far is masked; the arguments are then -inf, not NaN, and all P are 0 */
+    const float2 sc = splat(kScaleLog2), nm = splat(CUT && m == -INFINITY ? 0.f : -m);
     float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, t[32];
 #pragma unroll
     for (int i = 0; i < 32; i++) t[i] = fma2(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sc, nm);
@@ -256,9 +258,14 @@ __global__ void __launch_bounds__(256) hy3a_kv_to_f16_kernel(hy3a_cache_view cac
 struct prefill_args {
     float *out;
     size_t out_stride;
-    int base, nq, kv_head_begin;
+    int base, nq, kv_head_begin, kv_heads, entries, group;   /* entries per head (blocks, or pieces of cut blocks), dealt to the heads in groups */
     unsigned *err;
+    float *rec;             /* records of cut blocks: [slot][8 warps][kRecWarp] */
+    unsigned *cnt;          /* arrivals: [slot][8 warps], left at zero */
 };
+/* record of one softmax warp: O as [32 column quads][32 rows] float4 (a warp stores 512 contiguous bytes), then {m, l} per row */
+constexpr int kRecWarp = 32 * 128 + 64;
+static_assert(8 * kRecWarp * 4 == HY3A_PF_REC_BYTES, "record size");
 
 /* ---- pass 2: the attention kernel -------------------------------------------------------------------------------------
  * One CTA = 32 query tokens x the 8 query heads of one KV head = two 128-row Q tiles A and B that share every K/V tile
@@ -272,8 +279,13 @@ struct prefill_args {
  * Warps 0-3 / 4-7: softmax of tile A / B; warp 8: TMA producer (4-stage rings of 16 KB K and V tiles); warps 9 / 10:
  * MMA issuers of tile A / B, each in uniform control flow with one lane elected once (one thread issues an MMA every
  * ~26 ns at best, which a single issuer for both tiles would be bound by).                                       */
-constexpr int kQTok2 = 32;                     /* query tokens per CTA = two tiles of kQTok */
-constexpr int kKeys3 = 64;
+constexpr int kQTok2 = HY3A_PF_QTOK;           /* query tokens per CTA = two tiles of kQTok */
+constexpr int kKeys3 = HY3A_PF_KEYS;
+/* Neighbouring CTAs (the two SMs of a TPC, a GPC) should walk the same head: they ask L2 for the same K/V lines at the same time.  So
+ * a grid that is resident at once goes head by head, and a larger one in groups of 8 blocks per head, the groups in descending
+ * order of length, because the longest blocks must not start last.  512 tokens behind 4 096: 72 us, heads alternating every block 82, every 2 blocks 82, every 4 to 16 72-76; 2 048 fresh
+ * tokens: 96 us in ascending order, 86 in this. */
+constexpr int kGroup = 8;
 constexpr int kK3Bytes = kKeys3 * 128 * 2;      /* one K tile = two sub-tiles [64 keys][64 dims]; one V^T tile = [128 dims][64 keys] */
 constexpr int kSt3 = 4;                         /* ring stages */
 constexpr int kPf3Threads = 352;
@@ -288,8 +300,16 @@ __device__ __forceinline__ void umma_f16_n64_lead(unsigned d_tmem, unsigned long
     asm volatile("{\n .reg .pred p, e;\n setp.ne.b32 e, %5, 0;\n setp.ne.b32 p, %4, 0;\n @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdescN64), "r"(accumulate), "r"(lead) : "memory");
 }
-__global__ void __launch_bounds__(kPf3Threads, 1)
-hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, prefill_args a) {
+/* where a CTA's piece lies; an uncut block is one piece from step 0 */
+struct pf_where { int hl, qblk, j0, ntiles, piece, np, rec0; };
+/* CTA -> (entry, head) */
+__device__ __forceinline__ void entry_of(const prefill_args &a, int &ent, int &hl) {
+    const int per = a.group * a.kv_heads, grp = blockIdx.x / per, in = blockIdx.x - grp * per, gsz = min(a.group, a.entries - grp * a.group);
+    hl = in / gsz;
+    ent = grp * a.group + in - hl * gsz;
+}
+template <bool CUT>
+__device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUtensorMap &tm_k, const CUtensorMap &tm_v, const prefill_args &a, const pf_where &w) {
     extern __shared__ uint8_t s_raw[];
     uint8_t *sm = s_raw + ((1024u - (smem_u32(s_raw) & 1023u)) & 1023u);
     const unsigned sbase = smem_u32(sm);
@@ -299,9 +319,8 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #define BAR(i) (bar0 + 8u * (unsigned)(i))
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int q0 = blockIdx.x * kQTok2, hl = blockIdx.y;
-    const int kv_end = min(a.base + q0 + kQTok2, a.base + a.nq);   /* keys [0, kv_end) matter for this CTA */
-    const int ntiles = (kv_end + kKeys3 - 1) / kKeys3;
+    const int hl = w.hl, qblk = w.qblk, ntiles = w.ntiles, j0 = CUT ? w.j0 : 0, np = CUT ? w.np : 1, piece = w.piece, rec0 = w.rec0;
+    const int q0 = qblk * kQTok2;
 
     if (tid == 0) {
         *s_abort = 0;
@@ -342,8 +361,8 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
              * so the issuers need both at the same time and wait for them once) */
             for (int j = 0; j < 2 && j < ntiles; j++) {
                 mbar_expect_tx(BAR(B3_K0F + j), kK3Bytes);
-                tma_load_3d(sbase + kOff3K + j * kK3Bytes, &tm_k, BAR(B3_K0F + j), 0, j * kKeys3, hl);
-                tma_load_3d(sbase + kOff3K + j * kK3Bytes + 8192, &tm_k, BAR(B3_K0F + j), 64, j * kKeys3, hl);
+                tma_load_3d(sbase + kOff3K + j * kK3Bytes, &tm_k, BAR(B3_K0F + j), 0, (j0 + j) * kKeys3, hl);
+                tma_load_3d(sbase + kOff3K + j * kK3Bytes + 8192, &tm_k, BAR(B3_K0F + j), 64, (j0 + j) * kKeys3, hl);
             }
             for (int j = 0; j < ntiles; j++) {
                 const int st = j & (kSt3 - 1), j2 = j + 2, st2 = j2 & (kSt3 - 1); const unsigned ph = (unsigned)(j / kSt3) & 1u;
@@ -352,10 +371,10 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 if (!mbar_wait_blocking(BAR(B3_DE + st), ph ^ 1u, s_abort, a.err, 10u)) break;
                 if ((j == 2 || j == 3) && j2 < ntiles && !mbar_wait_blocking(BAR(B3_K0E + j - 2), 0u, s_abort, a.err, 11u)) break;
                 mbar_expect_tx(BAR(B3_DF + st), j2 < ntiles ? 2 * kK3Bytes : kK3Bytes);
-                tma_load_3d(sbase + kOff3V + st * kK3Bytes, &tm_v, BAR(B3_DF + st), j * kKeys3, 0, hl);
+                tma_load_3d(sbase + kOff3V + st * kK3Bytes, &tm_v, BAR(B3_DF + st), (j0 + j) * kKeys3, 0, hl);
                 if (j2 < ntiles) {
-                    tma_load_3d(sbase + kOff3K + st2 * kK3Bytes, &tm_k, BAR(B3_DF + st), 0, j2 * kKeys3, hl);
-                    tma_load_3d(sbase + kOff3K + st2 * kK3Bytes + 8192, &tm_k, BAR(B3_DF + st), 64, j2 * kKeys3, hl);
+                    tma_load_3d(sbase + kOff3K + st2 * kK3Bytes, &tm_k, BAR(B3_DF + st), 0, (j0 + j2) * kKeys3, hl);
+                    tma_load_3d(sbase + kOff3K + st2 * kK3Bytes + 8192, &tm_k, BAR(B3_DF + st), 64, (j0 + j2) * kKeys3, hl);
                 }
             }
         }
@@ -426,7 +445,7 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             const unsigned tm_s = tmem + 128u * x + 64u * (j & 1) + lane_base;
             ok = __all_sync(0xffffffffu, mbar_wait_blocking(BAR(B3_SF + 2 * x + (j & 1)), (unsigned)(j >> 1) & 1u, s_abort, a.err, 30u));   /* keep the warp together */
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int k0 = j * kKeys3;
+            const int k0 = (j0 + j) * kKeys3;
             const bool masked = (k0 + kKeys3 - 1 > a.base + tq0);   /* the tile crosses the diagonal of some row */
             unsigned v[64];
             tmem_ld32_nowait(tm_s, v);
@@ -441,7 +460,7 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
              * argument.  A tile that is masked for the whole row (its keys all lie behind the row's query; only in the last
              * tiles of the CTA) has mx = -inf: nothing moves and all its P are 0 */
             const float mx = row_max(v) * kScaleLog2;
-            const bool grow = mx > m + kPfThreshold;              /* true while m == -inf (key 0 is never masked) */
+            const bool grow = mx > m + kPfThreshold;              /* true while m == -inf, unless all keys so far are masked (last piece of a cut block) */
             if (__any_sync(0xffffffffu, grow)) {
                 /* tcgen05.ld / .st are warp-collective: the whole warp rescales its 32 rows as soon as one of them moved its
                  * reference (the others multiply by exactly 1).  O_x is only ours when P_x(j-1).V_(j-1) has completed:
@@ -467,7 +486,7 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 m = m_new;
             }
             unsigned pk[32];
-            const float2 ls = softmax_exp(v, m, pk, x, x == 0 || j + 1 < ntiles);
+            const float2 ls = softmax_exp<CUT>(v, m, pk, x, x == 0 || j + 1 < ntiles);
             l2 = add2(l2, ls);
             /* P over the first 32 columns of this S buffer (column c = keys 2c, 2c+1) */
             tmem_st32(tm_s, pk);
@@ -482,7 +501,8 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
          * from the one before it, and a waiter here could be two behind).  The last commit covers all earlier MMAs. */
         if (ok && ntiles > 0) ok = mbar_wait_blocking(BAR(B3_O + 2 * x + 1), 0u, s_abort, a.err, 32u);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (__all_sync(0xffffffffu, ok) && ntiles > 0) {      /* warp-uniform: tcgen05.ld is warp-collective */
+        ok = __all_sync(0xffffffffu, ok);                     /* warp-uniform: tcgen05.ld is warp-collective */
+        if (np == 1 && ok) {
             /* A thread holds a row, so storing from the registers touches 32 rows per instruction; the warp's 32 rows go through
              * shared memory instead, 64 columns at a time (its quarter of Q_x, which P.V's last commit says is read; 16-byte
              * chunk c of row r at c ^ (r & 7): conflict-free both ways), and leave as two rows of 256 contiguous bytes per
@@ -511,6 +531,77 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
                 __syncwarp();
             }
+        } else if (np > 1 && tq0 + (warp & 3) * 4 < a.nq) {   /* a warp without query tokens leaves no record */
+            /* a piece of a cut block: every softmax warp leaves the record of its 32 rows, and the last of the np warps with
+             * these rows to arrive folds the records in the order of the pieces (the result does not depend on who is last) */
+            const size_t slot0 = (size_t)rec0 * a.kv_heads + hl;          /* record of piece p: slot0 + p * kv_heads */
+            const size_t rec_step = (size_t)a.kv_heads * 8 * kRecWarp;
+            float *rec = a.rec + (slot0 * 8 + warp) * kRecWarp;
+            if (ok) {
+                float4 *dst = reinterpret_cast<float4 *>(rec + piece * rec_step);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    unsigned v[32];
+                    tmem_ld32_nowait(tm_o + 32u * c, v);
+                    tmem_ld_wait(v);
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        __stcg(dst + (8 * c + i) * 32 + lane, make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]), __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3])));
+                }
+                __stcg(reinterpret_cast<float2 *>(dst + 1024) + lane, make_float2(m, l));
+            }
+            __threadfence();
+            __syncwarp();
+            unsigned old = 0;
+            if (lane == 0) old = atomicAdd(a.cnt + slot0 * 8 + warp, 1u);
+            old = __shfl_sync(0xffffffffu, old, 0);
+            if (old == (unsigned)np - 1u) {
+                __threadfence();
+                if (lane == 0) a.cnt[slot0 * 8 + warp] = 0u;              /* ready for the next launch */
+                /* the loads of four records are in flight at once (indices past the end read the last record again) */
+                auto ml_of = [&](int p) { return __ldcg(reinterpret_cast<const float2 *>(rec + min(p, np - 1) * rec_step + 4096) + lane); };
+                float M = -INFINITY, L = 0.f;
+                for (int p = 0; p < np; p += 4) {
+                    float2 ml[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) ml[i] = ml_of(p + i);
+                    /* finite from the first record on: key 0 is never masked */
+                    const float m_new = fmaxf(fmaxf(fmaxf(M, ml[0].x), ml[1].x), fmaxf(ml[2].x, ml[3].x));
+                    L *= ex2f(M - m_new);
+                    M = m_new;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) if (p + i < np) L += ml[i].y * ex2f(ml[i].x - M);     /* a record of masked keys has weight 0 */
+                }
+                const float inv = L > 0.f ? 1.f / L : 0.f;
+                const bool row_valid = tq0 + t_local < a.nq;
+                float *orow = a.out + (size_t)(tq0 + t_local) * a.out_stride + (size_t)((a.kv_head_begin + hl) * 8 + (tid & 7)) * HY3A_D;
+#pragma unroll 1
+                for (int c = 0; c < 4; c++) {
+                    float4 acc[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+                    for (int p = 0; p < np; p += 2) {       /* two records in flight: a trip to L2 is most of a round */
+                        const bool two = p + 1 < np;
+                        const float *r0 = rec + p * rec_step, *r1 = two ? r0 + rec_step : r0;
+                        float4 v0[8], v1[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            v0[i] = __ldcg(reinterpret_cast<const float4 *>(r0) + (8 * c + i) * 32 + lane);
+                            v1[i] = __ldcg(reinterpret_cast<const float4 *>(r1) + (8 * c + i) * 32 + lane);
+                        }
+                        const float f0 = ex2f(ml_of(p).x - M) * inv, f1 = two ? ex2f(ml_of(p + 1).x - M) * inv : 0.f;
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            acc[i].x = fmaf(v1[i].x, f1, fmaf(v0[i].x, f0, acc[i].x)); acc[i].y = fmaf(v1[i].y, f1, fmaf(v0[i].y, f0, acc[i].y));
+                            acc[i].z = fmaf(v1[i].z, f1, fmaf(v0[i].z, f0, acc[i].z)); acc[i].w = fmaf(v1[i].w, f1, fmaf(v0[i].w, f0, acc[i].w));
+                        }
+                    }
+                    if (row_valid)
+#pragma unroll
+                    for (int i = 0; i < 8; i++) *reinterpret_cast<float4 *>(orow + 32 * c + 4 * i) = acc[i];
+                }
+            }
         }
     }
     /* ---- common exit: everybody arrives here, also after a wait ran out; release TMEM */
@@ -524,6 +615,27 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 #undef BAR
+}
+/* blocks uncut (full grids) */
+__global__ void __launch_bounds__(kPf3Threads, 1)
+hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ prefill_args a) {
+    pf_where w = {0, 0, 0, 0, 0, 1, 0};
+    int ent;
+    entry_of(a, ent, w.hl);
+    w.qblk = a.entries - 1 - ent;
+    w.ntiles = (min(a.base + (w.qblk + 1) * kQTok2, a.base + a.nq) + kKeys3 - 1) / kKeys3;      /* keys behind these do not matter for this CTA */
+    prefill_body<false>(tm_q, tm_k, tm_v, a, w);
+}
+/* blocks cut along the keys (grids that would leave SMs idle); a separate kernel, because the offsets and the -inf test of its
+ * inner loop cost the other one 5 % */
+__global__ void __launch_bounds__(kPf3Threads, 1)
+hy3a_prefill_cut_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ prefill_args a,
+                        const __grid_constant__ hy3a_pf_table tab) {
+    int ent, hl;
+    entry_of(a, ent, hl);
+    const hy3a_pf_piece pc = tab.e[ent];
+    const pf_where w = {hl, pc.qblk, pc.j0, pc.n, pc.piece, pc.np, pc.rec};
+    prefill_body<true>(tm_q, tm_k, tm_v, a, w);
 }
 
 
@@ -649,16 +761,26 @@ int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq
     bool &attr_set = attr_dev[ctx->device & 63];
     if (!attr_set) {
         HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
+        HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_cut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
         attr_set = true;
     }
-    prefill_args a;
+    prefill_args a = {};
     a.out = out; a.out_stride = out_stride; a.base = base_slot; a.nq = nq; a.kv_head_begin = ctx->cfg.kv_head_begin; a.err = ctx->d_err;
+    a.kv_heads = kvh; a.rec = ctx->d_pf_rec; a.cnt = ctx->d_pf_cnt;
     {
+        /* the cut depends on the chunk's sizes alone; the layers of a chunk share it */
+        if (ctx->pf_plan_base != base_slot || ctx->pf_plan_nq != nq) {
+            hy3a_pf_plan(base_slot, nq, kvh, ctx->sm_count, ctx->d_pf_rec ? HY3A_PF_MAX_SLOTS : 0, &ctx->pf_plan);
+            ctx->pf_plan_base = base_slot; ctx->pf_plan_nq = nq;
+        }
+        const int entries = ctx->pf_plan.count ? ctx->pf_plan.count : (nq + kQTok2 - 1) / kQTok2;
+        a.entries = entries; a.group = entries * kvh <= ctx->sm_count ? entries : kGroup;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((nq + kQTok2 - 1) / kQTok2, kvh); cfg.stream = ctx->stream;
+        cfg.gridDim = dim3(entries * kvh); cfg.stream = ctx->stream;
         cfg.blockDim = dim3(kPf3Threads); cfg.dynamicSmemBytes = kPf3Smem;
         cfg.attrs = attr; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
-        HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_kernel, tq, tk, tv, a));
+        if (ctx->pf_plan.count) HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_cut_kernel, tq, tk, tv, a, ctx->pf_plan));
+        else HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_kernel, tq, tk, tv, a));
     }
     ctx->launches++;
     ctx->bulk_write_pending = 1;

@@ -1,0 +1,126 @@
+/*
+ * prefill_plan.h -- how the chunked prefill is cut into CTAs (host code, no CUDA).
+ *
+ * A block is 32 query tokens of one KV head; it walks ceil(keys / 64) steps of 64 keys.  A chunk has
+ * ceil(nq / 32) x heads blocks whose lengths grow with the query index, and one CTA occupies an SM, so blocks alone can leave
+ * most SMs idle: 45 tokens are 16 blocks, 128 are 32.  A block may therefore be cut along the keys into pieces of M steps
+ * (the last takes the rest); every piece of a cut block leaves a {m, l, O} record and the last to arrive folds them.  M is
+ * chosen per chunk by list scheduling in units of steps, longest pieces first.
+ */
+#ifndef HY3A_PREFILL_PLAN_H
+#define HY3A_PREFILL_PLAN_H
+
+#include <stdint.h>
+#include <string.h>
+
+#include <algorithm>
+
+#define HY3A_PF_MAX_PIECES 256   /* table entries (pieces of one head); longer chunks run uncut */
+#define HY3A_PF_MAX_SLOTS 512    /* piece records in the scratch */
+#define HY3A_PF_REC_BYTES (8 * (32 * 128 + 64) * 4)   /* 8 warps x 32 rows x {O[128], m, l} fp32 */
+#define HY3A_PF_QTOK 32
+#define HY3A_PF_KEYS 64
+
+struct hy3a_pf_piece {
+    uint16_t qblk;               /* query block: tokens 32 qblk .. */
+    uint16_t j0, n;              /* steps [j0, j0 + n) of 64 keys */
+    uint16_t rec;                /* index of the block's first record per head (cut blocks) */
+    uint8_t piece, np;           /* this piece, pieces of the block */
+    uint16_t pad;
+};
+struct hy3a_pf_table {
+    int count;                   /* 0: uncut blocks in descending order, no table needed */
+    hy3a_pf_piece e[HY3A_PF_MAX_PIECES];
+};
+
+/* costs in steps (one step of both query tiles = 0.84 us): start and end of a CTA, writing a record, folding one record */
+constexpr float kPfCostCta = 8.0f, kPfCostRecord = 5.0f, kPfCostFold = 1.5f;
+
+static inline int hy3a_pf_steps(int base, int nq, int qblk) {
+    const int end = std::min(base + (qblk + 1) * HY3A_PF_QTOK, base + nq);
+    return (end + HY3A_PF_KEYS - 1) / HY3A_PF_KEYS;
+}
+
+/* when the last CTA of the table ends, in steps (list scheduling on a heap of SM groups that divide the heads evenly); gives
+ * up as soon as the end is known to be no earlier than `limit` */
+static inline float hy3a_pf_makespan(const hy3a_pf_table *t, int heads, int sms, float limit) {
+    int unit = heads;
+    while (unit > 1 && (sms % unit || heads % unit)) unit--;
+    const int ng = std::min(sms / unit, 256), reps = heads / unit;
+    float load[256];
+    for (int i = 0; i < ng; i++) load[i] = 0.f;
+    float end = 0.f;
+    for (int c = 0; c < t->count; c++) {
+        const hy3a_pf_piece &e = t->e[c];
+        const float cost = kPfCostCta + e.n + (e.np > 1 ? kPfCostRecord : 0.f), fold = e.np > 1 ? kPfCostFold * e.np : 0.f;
+        for (int r = 0; r < reps; r++) {
+            const float v = load[0] + cost;       /* the least loaded group is at the root */
+            if (v + fold > end) { end = v + fold; if (end >= limit) return end; }
+            int i = 0;
+            for (int k = 1; k < ng; k = 2 * i + 1) {
+                if (k + 1 < ng && load[k + 1] < load[k]) k++;
+                if (load[k] >= v) break;
+                load[i] = load[k]; i = k;
+            }
+            load[i] = v;
+        }
+    }
+    return end;
+}
+
+/* pieces of at most M steps in descending order of length; false: does not fit the table or the records, or the work alone
+ * fills the SMs up to `limit` */
+static inline bool hy3a_pf_cut(int base, int nq, int heads, int sms, int M, int max_slots, float limit, hy3a_pf_table *t) {
+    const int nqb = (nq + HY3A_PF_QTOK - 1) / HY3A_PF_QTOK;
+    int rec = 0, count = 0;
+    float work = 0.f;
+    for (int q = nqb - 1; q >= 0; q--) {
+        const int nt = hy3a_pf_steps(base, nq, q), np = (nt + M - 1) / M;
+        if (np > 255 || count + np > HY3A_PF_MAX_PIECES || (np > 1 && (rec + np) * heads > max_slots)) return false;
+        work += nt + np * (kPfCostCta + (np > 1 ? kPfCostRecord : 0.f));
+        int j0 = 0;
+        for (int p = 0; p < np; p++) {
+            hy3a_pf_piece &e = t->e[count++];
+            e.qblk = (uint16_t)q; e.j0 = (uint16_t)j0; e.n = (uint16_t)std::min(M, nt - j0);
+            e.rec = (uint16_t)(np > 1 ? rec : 0); e.piece = (uint8_t)p; e.np = (uint8_t)np; e.pad = 0;
+            j0 += e.n;
+        }
+        if (np > 1) rec += np;
+    }
+    if (work * heads >= limit * sms) return false;
+    t->count = count;
+    std::sort(t->e, t->e + count, [](const hy3a_pf_piece &a, const hy3a_pf_piece &b) { return a.n != b.n ? a.n > b.n : (a.qblk != b.qblk ? a.qblk > b.qblk : a.piece < b.piece); });
+    return true;
+}
+
+/* the plan of a chunk; max_slots = 0: no records, i.e. uncut blocks */
+static inline void hy3a_pf_plan(int base, int nq, int heads, int sms, int max_slots, hy3a_pf_table *out) {
+    out->count = 0;
+    const int nqb = (nq + HY3A_PF_QTOK - 1) / HY3A_PF_QTOK, longest = hy3a_pf_steps(base, nq, nqb - 1);
+    if (nqb > HY3A_PF_MAX_PIECES || longest > 65535) return;
+    long long total = 0;
+    for (int q = 0; q < nqb; q++) total += hy3a_pf_steps(base, nq, q);
+    const float share = (float)(total * heads) / sms;                 /* steps per SM */
+    int cand[16], nc = 0;
+    cand[nc++] = longest;                                             /* uncut */
+    if (max_slots > 0 && longest > 1) {
+        /* pieces a little above the even share (or an integral part of it), whose rests fill the remaining SMs; equal pieces */
+        static const float f[8] = {1.06f, 1.12f, 1.0f, 0.56f, 0.52f, 0.36f, 0.27f, 1.2f};
+        for (int i = 0; i < 8; i++) { const int M = (int)(share * f[i] + 0.5f * kPfCostCta); if (M >= 2 && M < longest) cand[nc++] = M; }
+        for (int k = 2; k <= 6; k++) { const int M = (longest + k - 1) / k; if (M >= 2) cand[nc++] = M; }
+    }
+    hy3a_pf_table t;
+    float best = 3e38f;
+    for (int i = 0; i < nc; i++) {
+        /* the kernel for cut blocks is 5 % slower a step, and rests that share an SM with others cost more than this model says */
+        const float limit = best * (i == 0 ? 1.f : (out->count == 0 ? 0.88f : 0.98f));
+        if (!hy3a_pf_cut(base, nq, heads, sms, cand[i], max_slots, limit, &t)) continue;
+        const float m = hy3a_pf_makespan(&t, heads, sms, limit);
+        if (m < limit) {
+            best = m;
+            if (i) memcpy(out, &t, sizeof(int) + sizeof(hy3a_pf_piece) * (size_t)t.count);      /* uncut: no table */
+        }
+    }
+}
+
+#endif

@@ -237,6 +237,11 @@ uint64_t hy3a_launch_count(const hy3a_ctx *ctx);
  * of page units, and for CTA `cta` of `n_ctas` its unit range [*u0, *u1).               */
 int hy3a_decode_schedule(int n, const int *kv_lens, int kv_heads, int n_ctas, int cta, long long *total_units,
                          long long *u0, long long *u1);
+/* How hy3a_prefill cuts a chunk into CTAs (pure host arithmetic, no GPU): the pieces of one KV head in launch order, six
+ * ints each {query block of 32 tokens, first step, steps (of 64 keys), first record, piece, pieces of the block}.  `sms` SMs,
+ * `max_records` piece records over all heads (0: blocks stay uncut).  Writes at most cap pieces, returns their number
+ * (0: uncut blocks in descending order) or a negative error.                                                         */
+int hy3a_prefill_schedule(int base_slot, int nq, int kv_heads, int sms, int max_records, int *pieces, int cap);
 /* Library build info, e.g. "hy3attn sm_100a <date>". */
 const char *hy3a_version(void);
 

@@ -55,6 +55,16 @@ def test_prefill_chunk_over_prefix(cuda, oracle, dt):
     run_case(cuda, oracle, dt, 1536, 512, rows=[0, 1, 15, 16, 127, 128, 255, 256, 500, 511])
 
 
+@pytest.mark.parametrize("dt", ["fp16", "int8", "int4"])
+@pytest.mark.parametrize("base,nq", [(2047, 1), (3970, 45), (4090, 37), (4060, 129), (3999, 33)])
+def test_prefill_cut_along_the_keys(cuda, oracle, dt, base, nq):
+    """Chunks whose blocks are cut into several pieces (records + fold): warps without queries, rows whose keys in the last
+    piece are all masked, odd bases."""
+    from hy3_b200.attn import prefill_schedule
+    assert (prefill_schedule(base, nq, 8)[:, 5] > 1).any()
+    run_case(cuda, oracle, dt, base, nq, rows=sorted({0, nq // 2, max(nq - 2, 0), nq - 1, min(31, nq - 1), min(32, nq - 1)}))
+
+
 def _chunked(cuda, oracle, dt, chunks, mirror_mb, monkeypatch, redo=None):
     """Feeds `chunks` (token counts) one after the other through append + prefill on ONE context; `redo` =
     (keep_ntok, n): after the last chunk the sequence is cut back to keep_ntok tokens and n DIFFERENT tokens follow.

@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from hy3_b200.attn import decode_schedule
+from hy3_b200.attn import decode_schedule, prefill_schedule
 
 
 @pytest.mark.parametrize("lens,heads,ctas", [([32768], 8, 148), ([1], 8, 148), ([128, 129, 0, 5000], 8, 148),
@@ -67,3 +67,29 @@ def test_plan_eval_follows_the_reference_walk():
     e = read_env({"HY3_KV_INT4": "1", "HY3_PREFILL_CHUNK": "abc", "HY3_POS_STRIDE": "-3", "HY3_POS_JUMP": "7"})
     assert e == {"kv_dtype": "int4", "chunk": 0, "pos_stride": 1, "pos_jump": 7, "pos_jump_at": 0}
     assert read_env({})["kv_dtype"] == "int8" and read_env({"HY3_KV_FP16": "1"})["kv_dtype"] == "fp16"
+
+
+@pytest.mark.parametrize("base,nq", [(0, 1), (0, 32), (0, 33), (1001, 45), (5, 59), (31, 64), (4096, 512), (0, 2048), (2048, 953), (16000, 128),
+                                     (262143, 1), (262000, 2048), (1000, 1000), (0, 8192), (100, 8193), (4194304, 7)])
+@pytest.mark.parametrize("heads", [8, 4, 3, 1])
+@pytest.mark.parametrize("records", [512, 16, 0])
+def test_prefill_schedule_covers_every_step_once(base, nq, heads, records):
+    """The pieces of a block are its steps [0, n) without gap or overlap, the records of cut blocks are disjoint and within the
+    scratch, and the table is in descending order of length."""
+    t = prefill_schedule(base, nq, heads, 148, records)
+    nqb = -(-nq // 32)
+    if len(t) == 0:      # uncut
+        assert records < 512 or (base, nq, heads) != (16000, 128, 8)
+        return
+    assert (np.diff(t[:, 2]) <= 0).all() and (t[:, 2] >= 1).all()
+    used = np.zeros(records // heads + 1, int)
+    for b in range(nqb):
+        p = t[t[:, 0] == b]
+        p = p[np.argsort(p[:, 4])]
+        assert (p[:, 5] == len(p)).all() and (p[:, 4] == np.arange(len(p))).all()
+        assert (p[:, 1] == np.concatenate([[0], np.cumsum(p[:-1, 2])])).all()
+        assert p[:, 2].sum() == -(-min(base + 32 * b + 32, base + nq) // 64)
+        if len(p) > 1:
+            assert (p[:, 3] == p[0, 3]).all() and (p[0, 3] + len(p)) * heads <= records
+            used[p[0, 3]:p[0, 3] + len(p)] += 1
+    assert used.max() <= 1 and len(t) == sum((t[:, 0] == b).sum() for b in range(nqb))
