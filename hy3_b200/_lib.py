@@ -39,7 +39,7 @@ PROTOTYPES = {
     "hy3a_seq_release": (_i, [_vp, _i, _i]),
     "hy3a_seq_capacity": (_i, [_vp, _i]),
     "hy3a_free_blocks": (_i, [_vp]),
-    "hy3a_batch_set": (_i, [_vp, _i, _ip, _ip, _ip]),
+    "hy3a_batch_set": (_i, [_vp, _i, _vp, _vp, _vp]),
     "hy3a_append": (_i, [_vp, _i, _vp, _sz, _vp, _sz, _vp, _sz, _vp, _sz, _vp]),
     "hy3a_decode": (_i, [_vp, _i, _vp, _sz, _vp, _sz, _vp]),
     "hy3a_decode_step": (_i, [_vp, _i, _vp, _sz, _vp, _sz, _vp, _sz, _vp, _sz, _vp, _sz, _vp]),

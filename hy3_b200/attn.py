@@ -12,8 +12,24 @@ PARTIAL_FLOATS = 130
 KV_DTYPES = {"fp16": 0, "int8": 1, "int4": 2}
 
 
+_f32 = None     # torch.float32, fetched with the first tensor (the module itself does not need torch)
+
+
 def _ptr(t):
-    return C.c_void_p(0 if t is None else t.data_ptr())
+    return None if t is None else t.data_ptr()
+
+
+def _rows(t, n):
+    """Row stride of an fp32 tensor of n rows whose heads are dense (0 for None)."""
+    if t is None:
+        return 0
+    global _f32
+    if _f32 is None:
+        import torch
+        _f32 = torch.float32
+    st = t.stride()
+    assert len(t) == n and t.dtype is _f32 and st[-1] == 1 and st[-2] == D
+    return st[0]
 
 
 class Hy3Attn:
@@ -116,29 +132,31 @@ class Hy3Attn:
         t = np.ascontiguousarray(slots, np.int32)
         p = t if rope_pos is None else np.ascontiguousarray(rope_pos, np.int32)
         assert s.size == t.size == p.size
-        ip = C.POINTER(C.c_int)
-        self._chk(self.lib.hy3a_batch_set(self.h, s.size, s.ctypes.data_as(ip), t.ctypes.data_as(ip), p.ctypes.data_as(ip)))
+        rc = self.lib.hy3a_batch_set(self.h, s.size, *(a.__array_interface__["data"][0] for a in (s, t, p)))
+        if rc:
+            self._chk(rc)
         self.batch_n = int(s.size)
 
     # ---- hot path
     def append(self, layer, q, k, v, q_out=None, q_out16=None):
         """q [n,64,128] / k,v [n,8,128] fp32 (row stride free, rows dense).  Returns q_out (fp32); q_out=False with a
         q_out16 buffer writes the 16-bit queries only (the chunked prefill reads nothing else)."""
-        import torch
         n = self.batch_n
         assert (k is None) == (v is None)
-        for t in (q, k, v):
-            assert t is None or (t.shape[0] == n and t.dtype == torch.float32 and t.stride(-1) == 1 and t.stride(-2) == D)
+        sq, sk, sv = _rows(q, n), _rows(k, n), _rows(v, n)
         if q_out is False:
             assert q_out16 is not None
             q_out = None
         elif q_out is None:
+            import torch
             q_out = torch.empty((n, H, D), dtype=torch.float32, device=q.device)
         if q_out16 is not None:
+            import torch
             assert q_out16.dtype == torch.float16 and q_out16.is_contiguous() and q_out16.numel() == n * H * D
-        self._chk(self.lib.hy3a_append(self.h, layer, _ptr(q), q.stride(0), _ptr(k), 0 if k is None else k.stride(0),
-                                       _ptr(v), 0 if v is None else v.stride(0),
-                                       _ptr(q_out), 0 if q_out is None else q_out.stride(0), _ptr(q_out16)))
+        rc = self.lib.hy3a_append(self.h, layer, q.data_ptr(), sq, _ptr(k), sk, _ptr(v), sv, _ptr(q_out),
+                                  0 if q_out is None else q_out.stride(0), _ptr(q_out16))
+        if rc:
+            self._chk(rc)
         return q_out
 
     def decode(self, layer, q, out=None, partials=None):
@@ -156,17 +174,17 @@ class Hy3Attn:
 
     def decode_step(self, layer, q, k, v, out=None, q_out=None, partials=None):
         """Fused append + decode of one new token per batch row (pre-norm q [n,64,128], k/v [n,8,128])."""
-        import torch
         n = self.batch_n
         assert (k is None) == (v is None)
-        for t in (q, k, v):
-            assert t is None or (t.shape[0] == n and t.dtype == torch.float32 and t.stride(-1) == 1 and t.stride(-2) == D)
+        sq, sk, sv = _rows(q, n), _rows(k, n), _rows(v, n)
         if partials is None and out is None:
+            import torch
             out = torch.zeros((n, H, D), dtype=torch.float32, device=q.device)
-        self._chk(self.lib.hy3a_decode_step(self.h, layer, _ptr(q), q.stride(0), _ptr(k), 0 if k is None else k.stride(0),
-                                            _ptr(v), 0 if v is None else v.stride(0), _ptr(q_out),
-                                            0 if q_out is None else q_out.stride(0), _ptr(out),
-                                            0 if out is None else out.stride(0), _ptr(partials)))
+        rc = self.lib.hy3a_decode_step(self.h, layer, q.data_ptr(), sq, _ptr(k), sk, _ptr(v), sv, _ptr(q_out),
+                                       0 if q_out is None else q_out.stride(0), _ptr(out),
+                                       0 if out is None else out.stride(0), _ptr(partials))
+        if rc:
+            self._chk(rc)
         return out if partials is None else partials
 
     # ---- sequence sharding over peer memory
