@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(256) hy3a_append_kernel(hy3a_cache_view cache,
  *   - a lane of a query warp holds dims {2 lane, 2 lane + 1} and their rotate_half partners, so RoPE needs no exchange, and
  *     the sums of squares of the warp's 8 heads are reduced together: at each level of the tree a lane hands half of its
  *     sums to its partner and keeps the other half: 25 shuffles for 8 heads instead of 192.
- * Every sum has the per-row kernel's operands at every level of the tree, so queries, codes and scales are identical bits. */
+ * Every sum has the per-row kernel's operands at every level of the tree, so queries, codes and scales are identical bits.
+ * Measured between two prefill launches: 512 rows 16.0 -> 8.3 us (floor 4.5), 2 048 rows 50 -> 29 us (floor 18). */
 constexpr int kChunkHeads = 4;
 template <int DT>
 __global__ void __launch_bounds__(256, 4) hy3a_append_chunk_kernel(hy3a_cache_view cache, hy3a_batch_view batch, hy3a_rope_params rope, append_args a, int kv_blocks, int hpb, int contig8) {

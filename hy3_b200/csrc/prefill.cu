@@ -506,7 +506,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
             /* A thread holds a row, so storing from the registers touches 32 rows per instruction; the warp's 32 rows go through
              * shared memory instead, 64 columns at a time (its quarter of Q_x, which P.V's last commit says is read; 16-byte
              * chunk c of row r at c ^ (r & 7): conflict-free both ways), and leave as two rows of 256 contiguous bytes per
-             * instruction. */
+             * instruction (one step of 32 tokens 9.7 -> 7.4 us a launch, 512 fresh tokens 17.4 -> 15.3 us). */
             const float inv = l > 0.f ? 1.f / l : 0.f;
             uint8_t *stage = sm + kOff3Q + x * kTileBytes + (warp & 3) * 8192;
             const int t0 = tq0 + (warp & 3) * 4, nrow = min(32, (a.nq - t0) * 8);          /* rows of valid query tokens (none: <= 0) */
