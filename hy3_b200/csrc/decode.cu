@@ -368,12 +368,13 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
     const long long U = (long long)G * s_prefix[n];
     bool idle = (U == 0);
     /* Two ways to cut the units into per-CTA ranges:
-     *  - few segments (n*G < grid): every segment gets its own whole number of CTAs, roughly in
-     *    proportion to its pages, so no CTA straddles two segments (a straddling CTA pays the
+     *  - few segments (n*G < grid): every segment gets its own whole number of CTAs, for pieces of at
+     *    most L pages or (1 row, more than 32) roughly in proportion to its pages, so no CTA straddles two segments (a straddling CTA pays the
      *    query set-up and the fold twice and becomes the critical path of a small batch);
      *  - many segments: one contiguous, equally sized range per CTA over all units.
      * In both, never more CTAs than units, and the CTAs sharing a segment are contiguous.       */
-    const bool aligned = (long long)n * G < (long long)gridDim.x && aligned_split_balanced(s_prefix, n, G, gridDim.x, lane);
+    const unsigned L = even_piece_pages(s_prefix, n, G, gridDim.x, lane);      /* 0: shares in proportion to the pages */
+    const bool aligned = split_is_aligned(s_prefix, n, G, gridDim.x, lane, L);
     int C = (long long)gridDim.x < U ? (int)gridDim.x : (int)U;
     long long u_begin = 0, u_end = 0;
     int al_first = 0, al_pieces = 1;
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         for (int r = 0; r < n && !found; r++) {
             const int p = s_prefix[r + 1] - s_prefix[r];
             if (p == 0) continue;
-            int c = 1 + (int)(spare * p / (P * G));
+            int c = L ? (p + (int)L - 1) / (int)L : 1 + (int)(spare * p / (P * G));
             c = c < p ? c : p;
             if (cta < base + G * c) {
                 const int idx = cta - base, hl = idx / c, k = idx % c;
