@@ -122,6 +122,31 @@ def test_ring_depth_does_not_matter(cuda, dt, n, monkeypatch):
         assert all(torch.equal(outs[i], outs[i - i % 8]) for i in range(len(outs)))
 
 
+@pytest.mark.parametrize("dt", ["int4", "fp16"])
+@pytest.mark.parametrize("heads", [8, 3])
+@pytest.mark.parametrize("lens", [[3007, 129, 1, 4097, 640], [300] * 17, [1, 5000, 128, 2, 3, 257, 127, 255, 31, 33, 700, 900, 11]])
+def test_few_rows_in_even_pieces(cuda, oracle, dt, heads, lens):
+    """2 to 32 rows with fewer than four CTAs per segment: whole CTAs per segment in pieces of even size (or, where that is
+    unbalanced, the equal split); every row against the oracle."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    B = len(lens)
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_seqs=B, max_batch=B, kv_head_count=heads, max_tokens=sum(lens) + 128 * B, max_tokens_per_seq=8192)
+    for i, n in enumerate(lens):
+        ctx.fill_random(0, i, 0, n, 70 + i)
+    q = oracle.fill_normal((B, 64, 128), SEED, 441)
+    ctx.batch_set(list(range(B)), [n - 1 for n in lens])
+    out = ctx.decode(0, torch.from_numpy(q).to(cuda))
+    ctx.sync()
+    out = out.cpu().numpy()
+    for i, n in enumerate(lens):
+        ks, vs = ctx.export_kv(0, i, 0, n)
+        Kf, Vf = slots_to_float(oracle, ks, dt), slots_to_float(oracle, vs, dt)
+        want = oracle.attention(q[i], Kf, Vf)
+        check_attention(out[i][:8 * heads], want[:8 * heads], "%s row %d len %d" % (dt, i, n))
+    ctx.close()
+
+
 def test_decode_ragged_batch_and_poison(cuda, oracle):
     """Several sequences of different lengths in one launch; cache bytes past each length are poison."""
     import torch
