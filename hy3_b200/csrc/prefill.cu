@@ -134,14 +134,24 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
         : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return d;
 }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 w, x, y;\n mov.b64 {%0, %1}, w;\n}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
 __device__ __forceinline__ float2 splat(float a) { return make_float2(a, a); }
+/* maximum that keeps a NaN operand (fmaxf returns the other one) */
+__device__ __forceinline__ float fmax_nan(float a, float b) { float r; asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
 /* 2^t of a pair on the FMA pipe (the exponential unit takes 16 values per clock and SM, which the softmax of two tiles fills):
- * t = n + f, n = round(t), 2^f on [-1/2, 1/2] by the Taylor polynomial of e^(f ln 2) of degree 6 (remainder below 2e-8 relative,
- * i.e. fp32 rounding), n added to the exponent field.  t is clamped at -126 (masked keys: 2^-126 instead of 0, which is 0 in
- * fp16 and nothing beside a denominator >= 2^-8). */
+ * t = n + f, n = round(t), 2^f on [-1/2, 1/2] by the Taylor polynomial of e^(f ln 2) of degree 6 (relative error up to 1.6e-7 in
+ * fp64 with these constants, 2.2e-7 in fp32 steps; the first missing term is (ln 2 / 2)^7 / 7! = 1.2e-7), times 2^n, whose bits are put together from n.  t is
+ * clamped at -126 (masked keys: 2^-126 instead of 0, which is 0 in fp16 and nothing beside a denominator >= 2^-8).  A NaN (a NaN
+ * score, or a row whose maximum is +inf) stays one, as in ex2.approx: the clamp keeps it, and 2^n is a factor and not added to
+ * the exponent field, where it would leave a finite pattern. */
 __device__ __forceinline__ float2 ex2_fma(float2 t) {
     const float magic = 12582912.f;    /* 1.5 * 2^23: adding it rounds to an integer and leaves it in the low mantissa bits */
-    t.x = fmaxf(t.x, -126.f); t.y = fmaxf(t.y, -126.f);
+    t.x = fmax_nan(t.x, -126.f); t.y = fmax_nan(t.y, -126.f);
     const float2 z = add2(t, splat(magic)), n = add2(z, splat(-magic)), f = fma2(n, splat(-1.f), t);
     float2 p = fma2(splat(1.5403530e-4f), f, splat(1.3333558e-3f));
     p = fma2(p, f, splat(9.6181291e-3f));
@@ -149,7 +159,7 @@ __device__ __forceinline__ float2 ex2_fma(float2 t) {
     p = fma2(p, f, splat(2.4022651e-1f));
     p = fma2(p, f, splat(6.9314718e-1f));
     p = fma2(p, f, splat(1.f));
-    return make_float2(__uint_as_float(__float_as_uint(p.x) + (__float_as_uint(z.x) << 23)), __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(z.y) << 23)));
+    return mul2(p, make_float2(__uint_as_float((__float_as_uint(z.x) << 23) + 0x3f800000u), __uint_as_float((__float_as_uint(z.y) << 23) + 0x3f800000u)));
 }
 __device__ __forceinline__ float row_max(const unsigned (&v)[64]) {
     float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      /* four independent chains */

@@ -4,7 +4,7 @@ hy3.c:617-652) -- evaluated on the SAME stored K/V and the same fp16 queries."""
 import numpy as np
 import pytest
 
-from helpers import SEED, check_attention, slots_to_float
+from helpers import SEED, check_attention, make_slots, slots_to_float
 
 pytestmark = pytest.mark.gpu
 
@@ -63,6 +63,50 @@ def test_prefill_cut_along_the_keys(cuda, oracle, dt, base, nq):
     from hy3_b200.attn import prefill_schedule
     assert (prefill_schedule(base, nq, 8)[:, 5] > 1).any()
     run_case(cuda, oracle, dt, base, nq, rows=sorted({0, nq // 2, max(nq - 2, 0), nq - 1, min(31, nq - 1), min(32, nq - 1)}))
+
+
+@pytest.mark.parametrize("kind", ["nan", "+inf", "-inf"])
+@pytest.mark.parametrize("base,nq,first", [(0, 96, 16), (4060, 37, 4000)])
+def test_prefill_non_finite_scores(cuda, oracle, base, nq, first, kind):
+    """A key whose score is NaN or +inf makes every query that sees it NaN, wherever the key lies in a step (64 positions), uncut and
+    cut; a score of -inf is a weight of 0.  Against softmax in 64 bits."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    from hy3_b200.attn import prefill_schedule
+    assert (len(prefill_schedule(base, nq, 8)) > 0) == (base > 0)
+    ntok = base + nq
+    q = oracle.fill_normal((nq, 64, 128), SEED, 521).astype(np.float16)
+    q[:, :, 0] = 1.0
+    k = oracle.fill_normal((ntok, 8, 128), SEED, 522).astype(np.float16)
+    v = oracle.fill_normal((ntok, 8, 128), SEED, 523)
+    vs = make_slots(oracle, v, "fp16")
+    tq = torch.from_numpy(q).to(cuda)
+    ctx = Hy3Attn(kv_dtype="fp16", n_layers=1, max_batch=max(nq, 16), max_tokens=ntok + 128)
+    v64 = v.astype(np.float16).astype(np.float64)
+    seen = np.arange(ntok)[None, :] <= base + np.arange(nq)[:, None]
+    for r in range(8):
+        kk = k.copy()
+        for h in range(8):                                    # a key of its own for every KV head
+            kk[first + 8 * r + h, h, 0] = np.float16(kind)
+        ctx.import_kv(0, 0, 0, np.ascontiguousarray(kk).view(np.uint8).reshape(ntok, 2048), vs)
+        out = ctx.prefill(0, 0, base, tq)
+        ctx.sync()
+        out = out.cpu().numpy()
+        for h in range(8):
+            s = np.einsum("qgd,td->qgt", q[:, 8 * h:8 * h + 8].astype(np.float64), kk[:, h].astype(np.float64)) / np.sqrt(128.0)
+            s = np.where(seen[:, None, :], s, -np.inf)
+            with np.errstate(invalid="ignore"):
+                w = np.exp(s - s.max(axis=2, keepdims=True))
+            want = np.einsum("qgt,td->qgd", w / w.sum(axis=2, keepdims=True), v64[:, h])
+            got = out[:, 8 * h:8 * h + 8]
+            hit = base + np.arange(nq) >= first + 8 * r + h
+            what = "%s at key %d" % (kind, first + 8 * r + h)
+            if kind != "-inf":
+                assert np.isnan(want[hit]).all() and np.isnan(got[hit]).all(), what + ": the key was dropped"
+                got, want = got[~hit], want[~hit]
+            if len(got):
+                check_attention(got, want, what)
+    ctx.close()
 
 
 def _chunked(cuda, oracle, dt, chunks, mirror_mb, monkeypatch, redo=None):
