@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(256) hy3a_append_kernel(hy3a_cache_view cache,
         }
         return;
     }
+    if (slot < 0) return;      /* a row without keys here: nothing to store (and no block-table entry to look up) */
     const int hl = head - cache.kv_head_begin;
     uint8_t *page = page_ptr(cache, seq, slot, a.layer, hl);
     int codes[4];
@@ -207,7 +208,8 @@ __global__ void __launch_bounds__(256, 4) hy3a_append_chunk_kernel(hy3a_cache_vi
     /* ---- K/V block: owned heads h0 .. h0 + nh - 1, rows 8 grp .. 8 grp + 7 (warp = row) */
     const int half = lane >> 4, idx = lane & 15, d0 = half * 64 + idx * 4;
     const int h0 = ((int)blockIdx.x - grp * hg) * hpb, nh = min(hpb, cache.kv_heads - h0), row = grp * 8 + warp;
-    const bool live = row < n;
+    const int slot = row < n ? batch.slot[row] : -1;
+    const bool live = slot >= 0;      /* slot -1: a row without keys here, nothing to store */
     /* 8 whole, aligned, consecutive token columns of one sequence: the transposed stores are staged */
     const bool whole8 = contig8 && grp * 8 + 8 <= n;
     __shared__ __align__(16) __half s_vt[kChunkHeads][HY3A_D][8];
@@ -218,10 +220,10 @@ __global__ void __launch_bounds__(256, 4) hy3a_append_chunk_kernel(hy3a_cache_vi
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     float4 kx = make_float4(0.f, 0.f, 0.f, 0.f), vx = kx;
-    int slot = 0, seq = 0;
+    int seq = 0;
     const float *ks = nullptr, *vs = nullptr;
     if (live) {
-        seq = batch.seq[row]; slot = batch.slot[row];
+        seq = batch.seq[row];
         const size_t off = (size_t)(cache.kv_head_begin + h0) * HY3A_D + d0;
         ks = a.k_in + (size_t)row * a.k_stride + off;
         vs = a.v_in + (size_t)row * a.v_stride + off;

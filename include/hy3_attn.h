@@ -110,7 +110,9 @@ int hy3a_free_blocks(hy3a_ctx *ctx);
  * Replaces the h_pos -> d_pos hand-off (hy3_gpu.cu:872-873) and iota_kernel (:364);
  * like there, the position is supplied by the caller on every call -- the context keeps
  * no private counter, so rolling back (hy3.c:1514) is just passing smaller positions.
- * Reserves capacity for the slots.                                                    */
+ * Reserves capacity for the slots.  slots[i] == -1: the row has no keys in this context (a
+ * rank without tokens of the sequence): nothing is stored for it, and decode returns zeros
+ * (or an empty partial record).                                                        */
 int hy3a_batch_set(hy3a_ctx *ctx, int n, const int *seq_ids, const int *slots, const int *rope_pos);
 
 /* ---- hot path ----------------------------------------------------------------------*/

@@ -213,3 +213,39 @@ def test_chunk_kernel_aligned_columns(cuda, oracle, dt, heads, seqs):
         ctx.close()
     for a, b in zip(*res):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [8, 40])
+@pytest.mark.parametrize("dt", ["int8", "int4", "fp16"])
+def test_rows_without_a_slot_store_nothing(cuda, oracle, dt, n):
+    """Rows with slot -1 (no keys in this context) among live ones, in both kernels: their queries come out as usual, no cache byte
+    changes but those of the live rows, and the running V scale is the live rows'."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    q = oracle.fill_normal((n, 64, 128), SEED, 821)
+    k = oracle.fill_normal((n, 8, 128), SEED, 822)
+    v = oracle.fill_normal((n, 8, 128), SEED, 823)
+    dead = np.arange(n) % 3 != 1
+    v[dead] *= 1e4
+    sid = [i % 4 for i in range(n)]                          # every sequence has rows of both kinds
+    slots = [-1 if dead[i] else 120 + i for i in range(n)]
+    tq, tk, tv = (torch.from_numpy(a).to(cuda) for a in (q, k, v))
+    res = []
+    for keep in (np.arange(n), np.flatnonzero(~dead)):
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_seqs=4, max_batch=n, max_tokens=4 * 256, max_tokens_per_seq=256)
+        for s_ in range(4):
+            ctx.fill_random(0, s_, 0, 256, 30 + s_)
+        ctx.batch_set([sid[i] for i in keep], [slots[i] for i in keep], list(keep))
+        idx = torch.from_numpy(keep).to(cuda)
+        qo = ctx.append(0, tq[idx], tk[idx], tv[idx])
+        out = ctx.decode(0, qo)
+        ctx.sync()
+        live = torch.from_numpy(~dead[keep]).to(cuda)
+        res.append([qo[live].cpu().numpy(), out[live].cpu().numpy()] + [a for s_ in range(4) for a in ctx.export_kv(0, s_, 0, 256)])
+        if len(keep) == n:
+            assert not out[~live].any()
+            ctx.batch_set([0] * n, [0] * n, list(range(n)))   # the queries of all rows, from a batch without dead ones
+            assert torch.equal(ctx.append(0, tq, None, None), qo)
+        ctx.close()
+    for what, a, b in zip(["queries", "outputs"] + ["cache"] * 8, *res):
+        assert np.array_equal(a, b) if what != "outputs" else np.abs(a - b).max() < 1e-3, what
