@@ -1003,16 +1003,28 @@ int hy3a_decode_ring_capacity(int page_bytes, int max_batch) {
 int hy3a_decode_max_ctas(void) { return kFixedO / 64; }
 static_assert(kRecFloats >= HY3A_PARTIAL_FLOATS && (kRecFloats * 4) % 16 == 0, "a head's record must start on a 16-byte boundary");
 
+/* Folders per segment of the spread fold (0: the last CTA to arrive folds).  It pays off where the epilogue is the cross-GPU
+ * exchange (several CTAs store to the peers instead of one); on one GPU the folders only hold their SMs longer, which delays the
+ * next launch's CTAs there.  Its folders wait for the other pieces, so every CTA of the grid must be resident.  4 measured best
+ * on 8 GPUs (8: 28.8, 4: 27.8, 2: 27.8, 1: 29.2 us per layer).  A folder lands 8 / F heads x pieces records in the page ring: a
+ * segment has up to CTAs / KV heads pieces, and with one KV head on 148 CTAs 2 x 148 records (156 KB) exceed the rings of FP16
+ * and INT4 pages (131 and 135 KB).  Then 8 folders take one head each; a ring too small for that too keeps the plain fold.
+ * (Segments of fewer than F pieces have fewer folders: 4 heads x 3 pieces = 6.3 KB at most.) */
+static int spread_folders(const hy3a_ctx *ctx) {
+    if (ctx->shard_slot < 0 || ctx->decode_ctas > ctx->sm_count) return 0;
+    const size_t ring = (size_t)(ctx->geom.dtype == HY3A_KV_INT8 ? HY3A_UMMA_STAGES : ctx->decode_stages) * ctx->geom.page_bytes;
+    const size_t pieces = (size_t)(ctx->decode_ctas / ctx->cfg.kv_head_count);
+    for (int f = 4; f <= 8; f *= 2) if ((size_t)(8 / f) * pieces * kRecFloats * 4 <= ring) return f;
+    return 0;
+}
+
 int hy3a_launch_decode(hy3a_ctx *ctx, int layer, const float *q, size_t q_stride, float *out, size_t out_stride, float *partials,
                        const hy3a_step_inputs *step) {
     decode_args a;
     memset(&a, 0, sizeof(a));
     a.q = q; a.q_stride = q_stride; a.out = out; a.out_stride = out_stride; a.user_partials = partials;
     a.scratch = ctx->d_partials; a.counters = ctx->d_counters; a.n_counters = ctx->cfg.max_batch * ctx->cfg.kv_head_count; a.err = ctx->d_err; a.layer = layer;
-    /* the spread fold pays off where the epilogue is the cross-GPU exchange (8 CTAs store to the peers instead of one); on one
-     * GPU the folders only hold their SMs longer, which delays the next launch's CTAs there.  Its folders wait for the other
-     * pieces, so every CTA of the grid must be resident */
-    a.spread = (ctx->shard_slot >= 0 && ctx->decode_ctas <= ctx->sm_count) ? 4 : 0;   /* folders per segment: 4 measured best on 8 GPUs (8: 28.8, 4: 27.8, 2: 27.8, 1: 29.2 us per layer) */
+    a.spread = spread_folders(ctx);
     a.early_prefetch = ctx->use_pdl && !ctx->bulk_write_pending;
     if (ctx->shard_slot >= 0) {   /* set by hy3a_decode_step_sharded around this call */
         const int W = ctx->shard_world, slot = ctx->shard_slot;

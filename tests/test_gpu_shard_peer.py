@@ -56,6 +56,39 @@ def test_world1_push_and_merge_equals_decode_step(cuda, oracle, dt):
     assert np.array_equal(res["plain"], res["pushed"]), "max diff %.3g" % np.abs(res["plain"] - res["pushed"]).max()
 
 
+@pytest.mark.parametrize("dt,heads,lens0,stages", [("fp16", 1, [20000], None), ("int4", 1, [20000], None), ("int8", 1, [20000], None),
+                                                   ("int4", 2, [20000], 2), ("int4", 4, [300, 9000], 3)])
+def test_world1_segments_of_many_pieces(cuda, oracle, dt, heads, lens0, stages, monkeypatch):
+    """Few KV heads: up to 148 pieces of a segment, whose records have to fit the page ring that the folders land them in (4 folders
+    of two heads each, 8 of one, or the plain fold).  Equal to hy3a_decode_step bit for bit."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    if stages is not None:
+        monkeypatch.setenv("HY3A_DECODE_STAGES", str(stages))
+    B, steps = len(lens0), 4
+    q, k, v = (torch.from_numpy(oracle.fill_normal((steps, B, h, 128), SEED, 531 + h)).to(cuda) for h in (64, 8, 8))
+    res = []
+    for pushed in (False, True):
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_seqs=B, max_batch=B, kv_head_begin=8 - heads, kv_head_count=heads,
+                      max_tokens=sum(lens0) + 256 * B, max_tokens_per_seq=max(lens0) + 256)
+        for s_, n0 in enumerate(lens0):
+            ctx.fill_random(0, s_, 0, n0, 60 + s_)
+        if pushed:
+            ctx.shard_connect([ctx.shard_init(0, 1, 1, B)])
+        out = torch.zeros((steps, B, 64, 128), device=cuda)
+        for t in range(steps):
+            ctx.batch_set(list(range(B)), [n0 + t for n0 in lens0])
+            if pushed:
+                ctx.decode_step_sharded(0, 0, q[t], k[t], v[t], out=out[t])
+            else:
+                ctx.decode_step(0, q[t], k[t], v[t], out=out[t])
+        ctx.sync()
+        res.append(out)
+        ctx.close()
+    assert torch.equal(*res)
+    assert res[0][:, :, 64 - 8 * heads:].abs().max() > 0
+
+
 def test_wait_for_a_silent_peer_runs_out_with_a_status(cuda, oracle):
     """world = 2 with a stand-in for rank 1 that never pushes: the kernel's wait must give up after about a
     second, hy3a_sync must report HY3A_ETIMEOUT, and the context must still decode correctly afterwards."""
