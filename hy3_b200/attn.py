@@ -250,13 +250,13 @@ class Hy3Attn:
         self._chk(self.lib.hy3a_fill_random(self.h, layer, seq, t0, n, C.c_uint64(seed)))
 
 
-def decode_schedule(kv_lens, kv_heads, n_ctas, cta):
-    """Pure host arithmetic of the decode kernel's unit split (no GPU needed)."""
+def decode_schedule(kv_lens, kv_heads, n_ctas, cta, kv_dtype="int8"):
+    """Pure host arithmetic of the decode kernels' unit split (no GPU needed); INT8 caches are split differently from FP16 / INT4."""
     lib = load_library()
     lens = np.ascontiguousarray(kv_lens, np.int32)
     tot, u0, u1 = C.c_longlong(), C.c_longlong(), C.c_longlong()
-    rc = lib.hy3a_decode_schedule(lens.size, lens.ctypes.data_as(C.POINTER(C.c_int)), kv_heads, n_ctas, cta,
-                                  C.byref(tot), C.byref(u0), C.byref(u1))
+    rc = lib.hy3a_decode_schedule_kv(KV_DTYPES[kv_dtype], lens.size, lens.ctypes.data_as(C.POINTER(C.c_int)), kv_heads, n_ctas,
+                                     cta, C.byref(tot), C.byref(u0), C.byref(u1))
     if rc:
         raise Hy3AttnError(rc, "bad schedule arguments")
     return tot.value, u0.value, u1.value

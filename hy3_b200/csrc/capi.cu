@@ -15,6 +15,7 @@
 #include <string.h>
 
 #include "ctx.h"
+#include "decode_plan.h"
 
 static thread_local char g_create_err[512];   /* message of the last failed hy3a_create of this thread */
 
@@ -66,43 +67,54 @@ size_t hy3a_block_bytes(const hy3a_config *cfg) {
     return (size_t)cfg->n_layers * cfg->kv_head_count * g.page_bytes;
 }
 
-int hy3a_decode_schedule(int n, const int *kv_lens, int kv_heads, int n_ctas, int cta, long long *total_units, long long *u0,
-                         long long *u1) {
-    /* the same arithmetic as the head of hy3a_decode_kernel (the INT8 kernel moves a few pages between the pieces of the last
-     * segment of a single-row grid on top of it: decode_umma.cu; the FP16 / INT4 kernel cuts 2 to 32 rows with fewer than four
-     * CTAs per segment into pieces of even size: even_piece_pages in decode_common.cuh) */
-    if (n < 0 || kv_heads < 1 || n_ctas < 1 || cta < 0 || cta >= n_ctas) return HY3A_EINVAL;
-    long long P = 0;
+static long long pages_of(int len) { return len > 0 ? (len + (long long)HY3A_PAGE_TOKENS - 1) / HY3A_PAGE_TOKENS : 0; }
+
+int hy3a_decode_schedule_kv(int kv_dtype, int n, const int *kv_lens, int kv_heads, int n_ctas, int cta, long long *total_units,
+                            long long *u0, long long *u1) {
+    /* the same arithmetic as the heads of hy3a_decode_kernel and hy3a_decode_umma_kernel; the rules they share are in decode_plan.h */
+    if (kv_dtype < 0 || kv_dtype > 2 || n < 0 || (n && !kv_lens) || kv_heads < 1 || n_ctas < 1 || cta < 0 || cta >= n_ctas) return HY3A_EINVAL;
+    long long P = 0, longest = 0;
     int rows_ne = 0;
-    for (int i = 0; i < n; i++) { long long p = kv_lens[i] > 0 ? (kv_lens[i] + HY3A_PAGE_TOKENS - 1) / HY3A_PAGE_TOKENS : 0; P += p; rows_ne += p > 0; }
-    const long long U = P * kv_heads;
+    for (int i = 0; i < n; i++) { const long long p = pages_of(kv_lens[i]); P += p; rows_ne += p > 0; if (p > longest) longest = p; }
+    const long long U = P * kv_heads, spare = (long long)n_ctas - (long long)rows_ne * kv_heads;
     if (total_units) *total_units = U;
-    long long b = U, e = U;
+    long long b = U, e = U, L = 0;
     bool aligned = U > 0 && (long long)n * kv_heads < n_ctas;
-    if (aligned && (long long)n * kv_heads * 4 > n_ctas) {
-        /* the aligned split is kept only while its rounding leaves no CTA more than 5/4 of the even share */
-        const long long spare = (long long)n_ctas - (long long)rows_ne * kv_heads, PG = P * kv_heads;
+    if (aligned && kv_dtype != HY3A_KV_INT8 && hy3a_even_applies(n, kv_heads, (unsigned)n_ctas)) {
+        const unsigned cap = (unsigned)(n_ctas / kv_heads);
+        L = hy3a_least_piece((unsigned)((P + cap - 1) / cap), (unsigned)longest, cap, [&](unsigned len) {
+            unsigned c = 0;
+            for (int i = 0; i < n; i++) c += (unsigned)((pages_of(kv_lens[i]) + len - 1) / len);
+            return c;
+        });
+        aligned = hy3a_even_accepted((unsigned)L, (unsigned)P, kv_heads, (unsigned)n_ctas);
+    } else if (aligned && (long long)n * kv_heads * 4 > n_ctas) {
+        /* shares in proportion are kept only while their rounding leaves no CTA more than 5/4 of the even share */
         long long worst = 0;
         for (int r = 0; r < n; r++) {
-            long long p = kv_lens[r] > 0 ? (kv_lens[r] + HY3A_PAGE_TOKENS - 1) / HY3A_PAGE_TOKENS : 0;
+            const long long p = pages_of(kv_lens[r]);
             if (p == 0) continue;
-            long long c = 1 + spare * p / PG;
+            long long c = 1 + spare * p / U;
             if (c > p) c = p;
             if ((p + c - 1) / c > worst) worst = (p + c - 1) / c;
         }
-        aligned = worst * 4 <= (PG + n_ctas - 1) / n_ctas * 5 + 4;
+        aligned = worst * 4 <= (U + n_ctas - 1) / n_ctas * 5 + 4;
     }
     if (aligned) {
-        const long long spare = (long long)n_ctas - (long long)rows_ne * kv_heads;
         long long base = 0, pre = 0;
         for (int r = 0; r < n; r++) {
-            long long p = kv_lens[r] > 0 ? (kv_lens[r] + HY3A_PAGE_TOKENS - 1) / HY3A_PAGE_TOKENS : 0;
+            const long long p = pages_of(kv_lens[r]);
             if (p == 0) continue;
-            long long c = 1 + spare * p / (P * kv_heads);
+            long long c = L ? (p + L - 1) / L : 1 + spare * p / U;
             if (c > p) c = p;
             if (cta < base + kv_heads * c) {
-                long long idx = cta - base, hl = idx / c, k = idx % c, seg0 = kv_heads * pre + hl * p;
+                const long long idx = cta - base, hl = idx / c, k = idx % c, seg0 = kv_heads * pre + hl * p, late = c - HY3A_LATE;
                 b = seg0 + k * p / c; e = seg0 + (k + 1) * p / c;
+                if (kv_dtype == HY3A_KV_INT8 && rows_ne == 1 && hl == kv_heads - 1 && c > 2 * (long long)HY3A_LATE && p >= 8 * c && P < (1 << 23)) {
+                    const long long pp = p + HY3A_LATE * HY3A_LATE_CUT;
+                    b = seg0 + k * pp / c - HY3A_LATE_CUT * (k > late ? k - late : 0);
+                    e = seg0 + (k + 1) * pp / c - HY3A_LATE_CUT * (k + 1 > late ? k + 1 - late : 0);
+                }
                 break;
             }
             base += kv_heads * c; pre += p;
@@ -114,6 +126,10 @@ int hy3a_decode_schedule(int n, const int *kv_lens, int kv_heads, int n_ctas, in
     if (u0) *u0 = b;
     if (u1) *u1 = e;
     return 0;
+}
+
+int hy3a_decode_schedule(int n, const int *kv_lens, int kv_heads, int n_ctas, int cta, long long *total_units, long long *u0, long long *u1) {
+    return hy3a_decode_schedule_kv(HY3A_KV_INT8, n, kv_lens, kv_heads, n_ctas, cta, total_units, u0, u1);
 }
 
 int hy3a_prefill_schedule(int base_slot, int nq, int kv_heads, int sms, int max_records, int *pieces, int cap) {

@@ -11,6 +11,7 @@
 #include <math.h>
 
 #include "ctx.h"
+#include "decode_plan.h"
 
 /* Argument block of the decode kernels (filled by hy3a_launch_decode / hy3a_decode_noalloc in decode.cu). */
 struct hy3a_decode_args {
@@ -121,33 +122,26 @@ __device__ __forceinline__ bool aligned_split_balanced(const int *s_prefix, int 
     return (unsigned long long)worst * 4ull <= even * 5ull + 4ull;
 }
 
-/* 2 to 32 rows with fewer than four CTAs per segment: the least number of pages L for which pieces of at most L pages fit the grid (sum of ceil(pages / L) over the rows
- * <= CTAs per head), found by bisection with a lane per row; 0: not this case.  Shares in proportion (above) round down, and a row
- * that just misses its second CTA holds the launch up: 8 rows of 22 to 56 pages x 8 heads on 148 CTAs get at most 24 pages a CTA
- * that way, 19 this way (INT4: 27.3 -> 21.1 us a layer with the straddling split that 24 pages fall back to; 12 rows of up to 2 646
- * tokens 27.1 -> 17.7, FP16 24.9 -> 20.6).  The FP16 / INT4 kernel only: the INT8 kernel gains as much there, but its batch-1
- * launch loses 0.4 % to the registers of this code.  The result is the same in every warp. */
-constexpr unsigned kStraddlePages = 5;     /* a second segment in a CTA (queries, fold, record: about 6 us) costs more than this many pages */
+/* 2 to 32 rows with fewer than four CTAs per segment: the least number of pages L for which pieces of at most L pages fit the
+ * grid (sum of ceil(pages / L) over the rows <= CTAs per head), a lane per row; 0: not this case.  Shares in proportion (above)
+ * round down, and a row that just misses its second CTA holds the launch up: 8 rows of 22 to 56 pages x 8 heads on 148 CTAs get at
+ * most 24 pages a CTA that way, 19 this way (INT4: 27.3 -> 21.1 us a layer with the straddling split that 24 pages fall back to;
+ * 12 rows of up to 2 646 tokens 27.1 -> 17.7, FP16 24.9 -> 20.6).  The FP16 / INT4 kernel only: the INT8 kernel gains as much
+ * there, but its batch-1 launch loses 0.4 % to the registers of this code.  The result is the same in every warp. */
 __device__ __noinline__ unsigned even_piece_search(const int *s_prefix, int n, int G, unsigned grid, int lane) {
     const unsigned P = (unsigned)s_prefix[n], cap = grid / (unsigned)G, p = lane < n ? (unsigned)(s_prefix[lane + 1] - s_prefix[lane]) : 0u;
     if (P == 0u) return 0u;
-    unsigned lo = (P + cap - 1u) / cap, hi = __reduce_max_sync(0xffffffffu, p);
-    for (int i = 0; i < 8 && lo < hi; i++) {      /* hi always fits; 8 rounds bring it within 1 % of the least */
-        const unsigned mid = (lo + hi) >> 1;
-        if (__reduce_add_sync(0xffffffffu, (p + mid - 1u) / mid) <= cap) hi = mid; else lo = mid + 1u;
-    }
-    return hi;
+    return hy3a_least_piece((P + cap - 1u) / cap, __reduce_max_sync(0xffffffffu, p), cap,
+                            [&](unsigned L) { return __reduce_add_sync(0xffffffffu, (p + L - 1u) / L); });
 }
 __device__ __forceinline__ unsigned even_piece_pages(const int *s_prefix, int n, int G, unsigned grid, int lane) {
-    if (n < 2 || n > 32 || (unsigned)(n * G) >= grid || (unsigned)(n * G) * 4u <= grid) return 0u;   /* four CTAs a segment round well enough */
-    return even_piece_search(s_prefix, n, G, grid, lane);
+    return hy3a_even_applies(n, G, grid) ? even_piece_search(s_prefix, n, G, grid, lane) : 0u;
 }
 /* whether segments get whole CTAs; `L` from above */
 __device__ __forceinline__ bool split_is_aligned(const int *s_prefix, int n, int G, unsigned grid, int lane, unsigned L) {
     if (!((long long)n * G < (long long)grid)) return false;
     if (L == 0u) return aligned_split_balanced(s_prefix, n, G, grid, lane);
-    const unsigned long long even = ((unsigned long long)(unsigned)s_prefix[n] * (unsigned)G + grid - 1ull) / grid;
-    return L * 4ull <= even * 5ull + 4ull || L <= even + kStraddlePages;
+    return hy3a_even_accepted(L, (unsigned)s_prefix[n], G, grid);
 }
 
 /* ---- shared-memory / mbarrier / bulk-copy primitives ---------------------------------- */

@@ -79,7 +79,7 @@ constexpr int kOffPt = 0;                            /* kSlots x [16 rows][128 B
 constexpr int kOffAcc = 0;                           /* [8 heads][128 dims] fp32: the finished piece, handed to the epilogue */
 constexpr int kOffLand = 0;                          /* landing zone of records / exchange lines when the page ring is not idle */
 constexpr int kLandBytes = kSlots * 2048;
-constexpr unsigned kLate = 4, kLateCut = 2;      /* the last pieces of a single-row grid start late: they take fewer pages */
+constexpr unsigned kLate = HY3A_LATE, kLateCut = HY3A_LATE_CUT;      /* the last pieces of a single-row grid start late: they take fewer pages */
 constexpr int kOffQ = kOffPt + kSlots * 2048;        /* Q fragments [4 k-steps][32 lanes] x 16 B */
 constexpr int kOffQ8 = kOffQ + 2048;                 /* Q digits [2][8][128] int8 */
 constexpr int kOffMisc = kOffQ8 + 2048;

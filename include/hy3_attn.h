@@ -236,7 +236,11 @@ int hy3a_fill_random(hy3a_ctx *ctx, int layer, int seq, int t0, int n, uint64_t 
 /* Number of kernels this library has launched on ctx since creation. */
 uint64_t hy3a_launch_count(const hy3a_ctx *ctx);
 /* Decode schedule for a batch (pure host arithmetic, no GPU): given n lengths, the number
- * of page units, and for CTA `cta` of `n_ctas` its unit range [*u0, *u1).               */
+ * of page units, and for CTA `cta` of `n_ctas` its unit range [*u0, *u1).  The kernels split
+ * the units differently for INT8 and for FP16 / INT4 caches; hy3a_decode_schedule is the
+ * schedule of an INT8 cache (the default).                                               */
+int hy3a_decode_schedule_kv(int kv_dtype, int n, const int *kv_lens, int kv_heads, int n_ctas, int cta,
+                            long long *total_units, long long *u0, long long *u1);
 int hy3a_decode_schedule(int n, const int *kv_lens, int kv_heads, int n_ctas, int cta, long long *total_units,
                          long long *u0, long long *u1);
 /* How hy3a_prefill cuts a chunk into CTAs (pure host arithmetic, no GPU): the pieces of one KV head in launch order, six

@@ -93,3 +93,58 @@ def test_prefill_schedule_covers_every_step_once(base, nq, heads, records):
             assert (p[:, 3] == p[0, 3]).all() and (p[0, 3] + len(p)) * heads <= records
             used[p[0, 3]:p[0, 3] + len(p)] += 1
     assert used.max() <= 1 and len(t) == sum((t[:, 0] == b).sum() for b in range(nqb))
+
+
+def _few_row_batches():
+    rng = np.random.default_rng(17)
+    out = [([262144] + [100] * 4, 8), ([262144] + [128] * 31, 2), ([0, 5, 0, 9000, 0, 7, 3, 1], 8), ([1] * 18, 8), ([4096] * 17, 8), ([0] * 6, 8)]
+    for n in (2, 3, 5, 8, 17, 18, 31, 32, 33, 40):
+        for heads in (8, 5, 4, 3, 2, 1):
+            for hi in (300, 3000, 60000):
+                lens = rng.integers(1, hi, n)
+                lens[rng.random(n) < 0.15] = 0
+                if rng.random() < 0.3:
+                    lens[int(rng.integers(n))] = 20 * hi
+                out.append(([int(x) for x in lens], heads))
+    return out
+
+
+@pytest.mark.parametrize("dt", ["int4", "fp16", "int8"])
+def test_schedule_of_few_rows(dt):
+    """Ragged batches around the 2 to 32 rows that the FP16 / INT4 kernel cuts into pieces of even size: every page of every segment
+    in exactly one CTA, ranges in order; either no CTA straddles two segments, and then no piece is far above the even share, or the
+    ranges are equal."""
+    ctas, even_seen = 148, 0
+    for lens, heads in _few_row_batches():
+        pages = [-(-n // 128) for n in lens]
+        total = sum(pages) * heads
+        got = [decode_schedule(lens, heads, ctas, c, kv_dtype=dt) for c in range(ctas)]
+        assert all(g[0] == total for g in got)
+        r = [(u0, u1) for _, u0, u1 in got if u1 > u0]
+        assert [u0 for u0, _ in r] == [0] * bool(r) + [u1 for _, u1 in r[:-1]] and (r[-1][1] if r else 0) == total
+        if not r:
+            continue
+        sizes = [b - a for a, b in r]
+        bounds = np.cumsum([p for p in pages for _ in range(heads)])
+        straddles = any(((bounds > a) & (bounds < b)).any() for a, b in r)
+        even, segs = -(-total // ctas), len(lens) * heads
+        if straddles:
+            assert max(sizes) - min(sizes) <= 1
+        elif dt != "int8" and 2 <= len(lens) <= 32 and segs < ctas < 4 * segs:
+            even_seen += max(sizes) - min(sizes) > 1
+            assert max(sizes) * 4 <= even * 5 + 4 or max(sizes) <= even + 5
+        elif segs < ctas < 4 * segs and max(sizes) - min(sizes) > 1:
+            assert max(sizes) * 4 <= even * 5 + 4
+    assert (even_seen >= 10) == (dt != "int8")      # the batches above do reach the even pieces
+
+
+def test_schedule_depends_on_the_cache_type():
+    """8 rows of 22 to 56 pages x 8 heads on 148 CTAs: whole CTAs per segment with at most 19 pages each (FP16 / INT4), or equal ranges
+    (INT8); and the shortened last pieces of an INT8 single-row grid."""
+    lens = [3006, 7075, 3290, 3374, 6828, 2718, 2910, 3288]
+    for dt, worst in (("int4", 19), ("fp16", 19), ("int8", 14)):
+        r = [decode_schedule(lens, 8, 148, c, kv_dtype=dt)[1:] for c in range(148)]
+        assert max(b - a for a, b in r) == worst, dt
+    one = {dt: [b - a for _, a, b in (decode_schedule([32768], 8, 148, c, kv_dtype=dt) for c in range(126, 144))] for dt in ("int8", "int4")}
+    assert sum(one["int8"]) == sum(one["int4"]) == 256 and min(one["int4"]) == 14
+    assert one["int8"][-4:] == [13, 12, 13, 13] and min(one["int8"][:-4]) >= 14, one
