@@ -82,7 +82,7 @@ int hy3a_decode_schedule_kv(int kv_dtype, int n, const int *kv_lens, int kv_head
     bool aligned = U > 0 && (long long)n * kv_heads < n_ctas;
     if (aligned && kv_dtype != HY3A_KV_INT8 && hy3a_even_applies(n, kv_heads, (unsigned)n_ctas)) {
         const unsigned cap = (unsigned)(n_ctas / kv_heads);
-        L = hy3a_least_piece((unsigned)((P + cap - 1) / cap), (unsigned)longest, cap, [&](unsigned len) {
+        L = hy3a_least_piece((unsigned)((P + cap - 1) / cap), hy3a_piece_bound((unsigned)P, cap, (unsigned)n, (unsigned)longest), cap, [&](unsigned len) {
             unsigned c = 0;
             for (int i = 0; i < n; i++) c += (unsigned)((pages_of(kv_lens[i]) + len - 1) / len);
             return c;

@@ -131,7 +131,7 @@ __device__ __forceinline__ bool aligned_split_balanced(const int *s_prefix, int 
 __device__ __noinline__ unsigned even_piece_search(const int *s_prefix, int n, int G, unsigned grid, int lane) {
     const unsigned P = (unsigned)s_prefix[n], cap = grid / (unsigned)G, p = lane < n ? (unsigned)(s_prefix[lane + 1] - s_prefix[lane]) : 0u;
     if (P == 0u) return 0u;
-    return hy3a_least_piece((P + cap - 1u) / cap, __reduce_max_sync(0xffffffffu, p), cap,
+    return hy3a_least_piece((P + cap - 1u) / cap, hy3a_piece_bound(P, cap, (unsigned)n, __reduce_max_sync(0xffffffffu, p)), cap,
                             [&](unsigned L) { return __reduce_add_sync(0xffffffffu, (p + L - 1u) / L); });
 }
 __device__ __forceinline__ unsigned even_piece_pages(const int *s_prefix, int n, int G, unsigned grid, int lane) {

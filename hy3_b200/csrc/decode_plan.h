@@ -20,11 +20,20 @@ constexpr unsigned HY3A_STRADDLE_PAGES = 5;
 HY3A_HD bool hy3a_even_applies(int n, int G, unsigned grid) {
     return n >= 2 && n <= 32 && (unsigned)(n * G) < grid && (unsigned)(n * G) * 4u > grid;
 }
-/* The least L in [lo, hi] for which pieces(L) <= cap, by bisection; hi fits. */
+/* Most pages that the bisection has to look at: with n rows, pieces of ceil(P / (cap - n + 1)) pages always fit, because
+ * sum ceil(p / L) <= ceil(P / L) + n - 1; nor is more than the longest row of use.  n <= cap. */
+HY3A_HD unsigned hy3a_piece_bound(unsigned P, unsigned cap, unsigned n, unsigned longest) {
+    const unsigned d = cap - n + 1u, b = (P + d - 1u) / d;
+    return b < longest ? b : longest;
+}
+/* The least L in [lo, hi] for which pieces(L) <= cap, by bisection; hi fits.  Exact, in at most log2(hi - lo) + 1 rounds: a search
+ * stopped after 8 ends up to 17 % above the least with one very long row among short ones, and the rule below then refuses the
+ * split (100 000 tokens and 9 x 128, 4 KV heads: INT4 82.0 us a layer that way, 27.5 with the least; FP16 63.1 and 44.0; 8 rows
+ * of 2 718 to 7 075 tokens 21.1 and 20.8). */
 template <class Pieces>
 HY3A_HD unsigned hy3a_least_piece(unsigned lo, unsigned hi, unsigned cap, Pieces pieces) {
-    for (int i = 0; i < 8 && lo < hi; i++) {
-        const unsigned mid = (lo + hi) >> 1;
+    while (lo < hi) {
+        const unsigned mid = lo + ((hi - lo) >> 1);
         if (pieces(mid) <= cap) hi = mid; else lo = mid + 1u;
     }
     return hi;

@@ -148,3 +148,30 @@ def test_schedule_depends_on_the_cache_type():
     one = {dt: [b - a for _, a, b in (decode_schedule([32768], 8, 148, c, kv_dtype=dt) for c in range(126, 144))] for dt in ("int8", "int4")}
     assert sum(one["int8"]) == sum(one["int4"]) == 256 and min(one["int4"]) == 14
     assert one["int8"][-4:] == [13, 12, 13, 13] and min(one["int8"][:-4]) >= 14, one
+
+
+@pytest.mark.parametrize("dt", ["int4", "fp16"])
+def test_even_pieces_are_the_least_that_fit(dt):
+    """The piece size is the least for which the pieces fit the grid, also with one very long row among short ones, and a split that
+    the rule accepts is not lost."""
+    rng = np.random.default_rng(23)
+    batches = _few_row_batches()
+    for n, heads in ((5, 8), (10, 4), (20, 2), (32, 2), (18, 8)):
+        for long_pages in (500, 2048, 8192):
+            batches.append(([128 * long_pages] + [128] * (n - 1), heads))
+            batches.append(([128 * int(x) for x in rng.integers(1, 40, n - 1)] + [128 * long_pages], heads))
+    seen = 0
+    for lens, heads in batches:
+        n, P = len(lens), [-(-x // 128) for x in lens]
+        if not (2 <= n <= 32 and n * heads < 148 < 4 * n * heads) or sum(P) == 0:
+            continue
+        cap, even = 148 // heads, -(-sum(P) * heads // 148)
+        least = next(L for L in range(-(-sum(P) // cap), max(P) + 1) if sum(-(-p // L) for p in P) <= cap)
+        r = [decode_schedule(lens, heads, 148, c, kv_dtype=dt)[1:] for c in range(148)]
+        sizes = [b - a for a, b in r if b > a]
+        if least * 4 <= even * 5 + 4 or least <= even + 5:
+            assert max(sizes) <= least and len(sizes) == heads * sum(-(-p // least) for p in P), (lens, heads)
+            seen += 1
+        else:
+            assert max(sizes) - min(sizes) <= 1
+    assert seen > 20
