@@ -185,7 +185,7 @@ def test_chunk_kernel_equals_row_kernel(cuda, oracle, dt, heads):
 @pytest.mark.parametrize("heads", [(0, 8), (3, 5), (7, 1)])
 @pytest.mark.parametrize("dt", ["int8", "int4", "fp16"])
 def test_chunk_kernel_aligned_columns(cuda, oracle, dt, heads, seqs):
-    """The chunk kernel's staged stores (8 aligned consecutive slots; pages crossed; a ragged tail; head groups of 4 + 1) and
+    """The chunk kernel's staged stores (8 aligned consecutive slots; pages crossed; a ragged tail; one KV head per block) and
     a batch of two sequences that must not take them, against the per-row kernel: identical bytes."""
     import torch
     from hy3_b200 import Hy3Attn
@@ -249,3 +249,34 @@ def test_rows_without_a_slot_store_nothing(cuda, oracle, dt, n):
         ctx.close()
     for what, a, b in zip(["queries", "outputs"] + ["cache"] * 8, *res):
         assert np.array_equal(a, b) if what != "outputs" else np.abs(a - b).max() < 1e-3, what
+
+
+@pytest.mark.parametrize("slot0", [8, 3])
+@pytest.mark.parametrize("n,heads", [(1203, (0, 8)), (1203, (3, 5)), (601, (0, 8))])
+@pytest.mark.parametrize("dt", ["int8", "int4", "fp16"])
+def test_chunk_kernel_head_groups(cuda, oracle, dt, n, heads, slot0, monkeypatch):
+    """Chunks long enough for several KV heads per block (groups of 4 + 4, 4 + 1 and 2 x 4 on 148 SMs), with and without aligned
+    slots, a ragged tail: identical cache bytes and queries to the per-row kernel; and the prefill operands that the chunk kernel
+    writes through give the same attention bits as operands rebuilt from the pages."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    ntok = slot0 + n
+    q = torch.from_numpy(oracle.fill_normal((ntok, 64, 128), SEED, 831)).to(cuda)
+    k = torch.from_numpy(oracle.fill_normal((ntok, 8, 128), SEED, 832)).to(cuda)
+    v = torch.from_numpy(oracle.fill_normal((ntok, 8, 128), SEED, 833)).to(cuda)
+    w = (1.0 + 0.02 * oracle.fill_normal((2, 128), SEED, 3)).astype(np.float32)
+    res = []
+    for step, mirror_mb in ((n, "8192"), (25, "0")):
+        monkeypatch.setenv("HY3A_PF_MIRROR_MB", mirror_mb)
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_batch=n, max_tokens=ntok + 128, kv_head_begin=heads[0], kv_head_count=heads[1])
+        ctx.set_norm_weights(0, w[0], w[1])
+        q16 = torch.empty((ntok, 64, 128), dtype=torch.float16, device=cuda)
+        for b, e in [(0, slot0)] + [(b, min(ntok, b + step)) for b in range(slot0, ntok, step)]:
+            ctx.batch_set([0] * (e - b), list(range(b, e)))
+            ctx.append(0, q[b:e], k[b:e], v[b:e], q_out=False, q_out16=q16[b:e])
+        out = ctx.prefill(0, 0, slot0, q16[slot0:])
+        ctx.sync()
+        res.append([q16.cpu().numpy(), out.cpu().numpy()] + list(ctx.export_kv(0, 0, 0, ntok)))
+        ctx.close()
+    for what, a, b in zip(("queries", "attention", "K slots", "V slots"), *res):
+        assert np.array_equal(a, b), what
