@@ -109,6 +109,64 @@ def test_prefill_non_finite_scores(cuda, oracle, base, nq, first, kind):
     ctx.close()
 
 
+@pytest.mark.parametrize("dt,base,nq,heads,cut", [
+    ("fp16", 0, 2048, (0, 8), False), ("int8", 2048, 953, (0, 8), False), ("int4", 40, 700, (0, 8), False), ("fp16", 9930, 97, (0, 8), True),
+    ("int8", 1001, 512, (2, 4), True), ("fp16", 500, 1000, (6, 2), True), ("int4", 3000, 200, (7, 1), True), ("fp16", 3000, 300, (5, 3), True),
+    ("int8", 100, 2900, (4, 3), False)])
+def test_prefill_every_block_and_head(cuda, oracle, dt, base, nq, heads, cut):
+    """Grids in several groups of blocks (more CTAs than SMs) with a ragged last group, uncut and cut, and contexts that own some of
+    the KV heads: one query of every 32-token block, every owned head, into an output that starts as NaN; heads of others are not
+    written.  Repeated and interleaved with a chunk of another shape on the same records: identical bits."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    from hy3_b200.attn import prefill_schedule
+    h0, nh = heads
+    plan = prefill_schedule(base, nq, nh)
+    assert (len(plan) > 0) == cut
+    ntok = base + nq
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_batch=nq, max_tokens=ntok + 128, kv_head_begin=h0, kv_head_count=nh)
+    ctx.fill_random(0, 0, 0, ntok, 77)
+    q16 = torch.from_numpy(oracle.fill_normal((nq, 64, 128), SEED, 531).astype(np.float16)).to(cuda)
+    outs = []
+    for _ in range(3):
+        outs.append(ctx.prefill(0, 0, base, q16, out=torch.full((nq, 64, 128), float("nan"), device=cuda)))
+        ctx.prefill(0, 0, ntok - 33, q16[:33])
+    ctx.sync()
+    ks, vs = ctx.export_kv(0, 0, 0, ntok)
+    ctx.close()
+    own = slice(8 * h0, 8 * (h0 + nh))
+    assert all(torch.equal(o[:, own], outs[0][:, own]) for o in outs[1:])
+    assert torch.isfinite(outs[0][:, own]).all()
+    assert torch.isnan(outs[0][:, :8 * h0]).all() and torch.isnan(outs[0][:, 8 * (h0 + nh):]).all()
+    rows = sorted({min(32 * b + (7 * b) % 32, nq - 1) for b in range(-(-nq // 32))} | {0, nq - 1})
+    Kf, Vf = slots_to_float(oracle, ks, dt), slots_to_float(oracle, vs, dt)
+    want = oracle.prefill_causal(q16.float().cpu().numpy(), Kf, Vf, base, rows=rows)
+    got = outs[0].cpu().numpy()
+    for i in rows:
+        for h in range(h0, h0 + nh):
+            check_attention(got[i, 8 * h:8 * h + 8], want[i, 8 * h:8 * h + 8], "%s base=%d nq=%d row %d KV head %d" % (dt, base, nq, i, h))
+
+
+def test_prefill_without_records(cuda, oracle):
+    """A context without piece records (max_batch < 16) runs uncut what another one cuts."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    from hy3_b200.attn import prefill_schedule
+    base, nq = 3970, 45
+    assert len(prefill_schedule(base, nq, 8)) > 0 and len(prefill_schedule(base, nq, 8, 148, 0)) == 0
+    q16 = torch.from_numpy(oracle.fill_normal((nq, 64, 128), SEED, 541).astype(np.float16)).to(cuda)
+    ctx = Hy3Attn(kv_dtype="int8", n_layers=1, max_batch=8, max_tokens=4096 + 128)
+    ctx.fill_random(0, 0, 0, base + nq, 78)
+    out = ctx.prefill(0, 0, base, q16)
+    ctx.sync()
+    ks, vs = ctx.export_kv(0, 0, 0, base + nq)
+    ctx.close()
+    rows = [0, 15, 16, 31, 32, 44]
+    want = oracle.prefill_causal(q16.float().cpu().numpy(), slots_to_float(oracle, ks, "int8"), slots_to_float(oracle, vs, "int8"), base, rows=rows)
+    for i in rows:
+        check_attention(out[i].cpu().numpy(), want[i], "row %d" % i)
+
+
 def _chunked(cuda, oracle, dt, chunks, mirror_mb, monkeypatch, redo=None):
     """Feeds `chunks` (token counts) one after the other through append + prefill on ONE context; `redo` =
     (keep_ntok, n): after the last chunk the sequence is cut back to keep_ntok tokens and n DIFFERENT tokens follow.
