@@ -57,10 +57,14 @@ def test_world1_push_and_merge_equals_decode_step(cuda, oracle, dt):
 
 
 @pytest.mark.parametrize("dt,heads,lens0,stages", [("fp16", 1, [20000], None), ("int4", 1, [20000], None), ("int8", 1, [20000], None),
-                                                   ("int4", 2, [20000], 2), ("int4", 4, [300, 9000], 3)])
+                                                   ("int4", 2, [20000], 2), ("int4", 4, [300, 9000], 3),
+                                                   ("int4", 8, [3007, 129, 0, 4097, 640, 2000, 900], None),
+                                                   ("fp16", 8, [3007, 129, 0, 4097, 640, 2000, 900], None),
+                                                   ("int4", 8, [9000] + [100] * 8, None)])
 def test_world1_segments_of_many_pieces(cuda, oracle, dt, heads, lens0, stages, monkeypatch):
     """Few KV heads: up to 148 pieces of a segment, whose records have to fit the page ring that the folders land them in (4 folders
-    of two heads each, 8 of one, or the plain fold).  Equal to hy3a_decode_step bit for bit."""
+    of two heads each, 8 of one, or the plain fold).  And 7 or 9 rows of all heads, in pieces of even size or straddling.  Equal to
+    hy3a_decode_step bit for bit."""
     import torch
     from hy3_b200 import Hy3Attn
     if stages is not None:
@@ -72,7 +76,8 @@ def test_world1_segments_of_many_pieces(cuda, oracle, dt, heads, lens0, stages, 
         ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_seqs=B, max_batch=B, kv_head_begin=8 - heads, kv_head_count=heads,
                       max_tokens=sum(lens0) + 256 * B, max_tokens_per_seq=max(lens0) + 256)
         for s_, n0 in enumerate(lens0):
-            ctx.fill_random(0, s_, 0, n0, 60 + s_)
+            if n0:
+                ctx.fill_random(0, s_, 0, n0, 60 + s_)
         if pushed:
             ctx.shard_connect([ctx.shard_init(0, 1, 1, B)])
         out = torch.zeros((steps, B, 64, 128), device=cuda)
