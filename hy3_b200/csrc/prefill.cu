@@ -175,8 +175,8 @@ __device__ __forceinline__ void turn_pass(int x) { asm volatile("bar.arrive %0, 
 __device__ __forceinline__ float ex2v(float x) { float r; asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 /* P = 2^(s * scale - m) of a row's 64 scores as packed fp16 pairs; returns the (pairwise) sum of the unrounded values (the fp16
  * rounding of P is a zero-mean 2^-12 relative error per term, far below the tolerance).  One pair in eight goes through the FMA
- * pipe: 512 tokens behind 4 096 take 75 us with none, 69-70 us with one, 74-76 us with two or more (the FMA form costs issue
- * slots that the waiting tile's maximum wants). */
+ * pipe: 512 tokens behind 4 096 take 73.0 us with none, 70.8 with one, 73.0 with two (the FMA form costs issue slots that the
+ * waiting tile's maximum wants); 2 048 fresh tokens 82.1 / 81.6 / 82.3. */
 template <bool CUT>
 __device__ __forceinline__ float2 softmax_exp(const unsigned (&v)[64], float m, unsigned (&pk)[32], int x, bool pass) {
     /* m == -inf: every key of the row so far is masked; the arguments are then -inf, not NaN, and all P are 0 */
@@ -293,8 +293,10 @@ constexpr int kQTok2 = HY3A_PF_QTOK;           /* query tokens per CTA = two til
 constexpr int kKeys3 = HY3A_PF_KEYS;
 /* Neighbouring CTAs (the two SMs of a TPC, a GPC) should walk the same head: they ask L2 for the same K/V lines at the same time.  So
  * a grid that is resident at once goes head by head, and a larger one in groups of 8 blocks per head, the groups in descending
- * order of length, because the longest blocks must not start last.  512 tokens behind 4 096: 72 us, heads alternating every block 82, every 2 blocks 82, every 4 to 16 72-76; 2 048 fresh
- * tokens: 96 us in ascending order, 86 in this. */
+ * order of length, because the longest blocks must not start last: 2 048 fresh tokens 94.5 us in ascending order, 81.6 in this.
+ * The size of the group matters little (operands from HBM, heads alternating every 1 / 2 / 4 / 8 / 16 blocks): 953 tokens behind
+ * 2 048 take 82.0 / 82.1 / 81.8 / 80.8 / 82.7 us, 2 048 fresh ones 80.5 / 80.7 / 81.1 / 81.6 / 83.3; 512 behind 4 096, resident at
+ * once, 70.8 head by head and 72.3 alternating. */
 constexpr int kGroup = 8;
 constexpr int kK3Bytes = kKeys3 * 128 * 2;      /* one K tile = two sub-tiles [64 keys][64 dims]; one V^T tile = [128 dims][64 keys] */
 constexpr int kSt3 = 4;                         /* ring stages */
@@ -516,7 +518,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
             /* A thread holds a row, so storing from the registers touches 32 rows per instruction; the warp's 32 rows go through
              * shared memory instead, 64 columns at a time (its quarter of Q_x, which P.V's last commit says is read; 16-byte
              * chunk c of row r at c ^ (r & 7): conflict-free both ways), and leave as two rows of 256 contiguous bytes per
-             * instruction (one step of 32 tokens 9.7 -> 7.4 us a launch, 512 fresh tokens 17.4 -> 15.3 us). */
+             * instruction (one step of 32 tokens 8.4 -> 6.4 us a launch, 512 fresh tokens 16.4 -> 14.3 us). */
             const float inv = l > 0.f ? 1.f / l : 0.f;
             uint8_t *stage = sm + kOff3Q + x * kTileBytes + (warp & 3) * 8192;
             const int t0 = tq0 + (warp & 3) * 4, nrow = min(32, (a.nq - t0) * 8);          /* rows of valid query tokens (none: <= 0) */

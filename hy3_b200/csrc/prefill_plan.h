@@ -33,7 +33,10 @@ struct hy3a_pf_table {
     hy3a_pf_piece e[HY3A_PF_MAX_PIECES];
 };
 
-/* costs in steps (one step of both query tiles = 0.84 us): start and end of a CTA, writing a record, folding one record */
+/* Costs in steps of both query tiles (0.79 us in a CTA by itself, 0.9 with 128 CTAs): start and end of a CTA, writing a record,
+ * folding one record.  To derive them again: a one-step launch takes 6.5 us; 32 tokens behind 4 064 (8 CTAs uncut, 56.9 us) in 2 /
+ * 4 / 8 / 16 pieces a block take 42.5 / 32.1 / 28.1 / 33.6 us, i.e. 10.7 / 13.0 / 15.3 / 24 us beside the steps and the 6.5, where
+ * 5 + 1.5 pieces say 6.3 / 8.7 / 13.4 / 22.9.  The model is 2 to 4 us low for few pieces, which the 0.88 below allows for. */
 constexpr float kPfCostCta = 8.0f, kPfCostRecord = 5.0f, kPfCostFold = 1.5f;
 
 static inline int hy3a_pf_steps(int base, int nq, int qblk) {

@@ -58,7 +58,8 @@ typedef struct {
     int kv_head_begin;      /* first KV head owned by this context (KV-head sharding); 0 */
     int kv_head_count;      /* KV heads owned; 8 when unsharded */
     int max_seqs;           /* sequences that can hold KV at once (1 for the reference's loop) */
-    int max_batch;          /* rows per hy3a_batch_set (decode batch or prefill chunk) */
+    int max_batch;          /* rows per hy3a_batch_set (decode batch or prefill chunk).  16 or more: hy3a_create also takes, where
+                             * there is room beside the pool, 68 MB of scratch for hy3a_prefill and its fp16 operands */
     int max_blocks;         /* pool capacity in 128-token blocks (a block spans all layers and owned heads) */
     int max_blocks_per_seq; /* longest sequence, in blocks */
     int device;             /* CUDA device ordinal, -1 = current device */
@@ -213,7 +214,11 @@ int hy3a_decode_step_sharded(hy3a_ctx *ctx, int layer, int slot, const float *q_
  * of sequence seq attends keys [0, base_slot + i]; the chunk's own K/V must already have
  * been appended (the reference does the same, hy3_gpu.cu:823-832).  Replaces
  * prefill_attn_int8/int4_kernel (hy3_gpu.cu:383, :415).  q16: IEEE fp16 [nq][64][128]
- * dense (hy3a_append's q_out16); out: fp32 [nq][64][128] with row stride out_stride.   */
+ * dense (hy3a_append's q_out16); out: fp32 [nq][64][128] with row stride out_stride.
+ * Chunks that would leave SMs idle are cut along the keys (hy3a_prefill_schedule) and the
+ * pieces folded in a fixed order: the same call on the same context gives the same bits,
+ * but the cut depends on kv_head_count, base_slot, nq and the number of SMs, so a context
+ * that owns some of the KV heads, or another chunking, may differ in the last bits.      */
 int hy3a_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq, const void *q16, float *out,
                  size_t out_stride);
 
