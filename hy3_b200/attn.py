@@ -229,6 +229,13 @@ class Hy3Attn:
         self._chk(self.lib.hy3a_prefill(self.h, layer, seq, base_slot, nq, _ptr(q16), _ptr(out), out.stride(0)))
         return out
 
+    def prefill_cluster(self, base_slot, nq):
+        """CTAs per block of 32 query tokens of such a chunk: 2, 4 or 8 as a cluster, 1: `prefill_schedule`."""
+        n = self.lib.hy3a_prefill_cluster(self.h, base_slot, nq)
+        if n < 0:
+            self._chk(n)
+        return n
+
     # ---- import / export (host numpy)
     def slot_bytes(self):
         return int(self.lib.hy3a_slot_bytes(KV_DTYPES[self.kv_dtype]))

@@ -82,6 +82,7 @@ struct hy3a_ctx {
     unsigned int *d_pf_cnt; /* their arrival counters (self-resetting) */
     hy3a_pf_table pf_plan;  /* the cut of the chunk (pf_plan_base, pf_plan_nq): a function of these sizes alone */
     int pf_plan_base, pf_plan_nq;
+    int pf_plan_cluster;    /* > 1: its blocks run as clusters of that many CTAs instead */
     unsigned int *d_err;  /* HY3A_ERR_WORDS words: kernels record bounded-wait timeouts / bad indices here */
     size_t partial_records;
 

@@ -320,7 +320,22 @@ __device__ __forceinline__ void entry_of(const prefill_args &a, int &ent, int &h
     hl = in / gsz;
     ent = grp * a.group + in - hl * gsz;
 }
-template <bool CUT>
+/* blocks whole / cut, records through memory / cut over the CTAs of a cluster */
+enum { PF_WHOLE = 0, PF_CUT = 1, PF_CLUSTER = 2 };
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ unsigned cluster_addr(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster16(unsigned addr, float a, float b, float c, float d) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void st_cluster8(unsigned addr, float a, float b) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
+}
+template <int MODE, int CL>
 __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUtensorMap &tm_k, const CUtensorMap &tm_v, const prefill_args &a, const pf_where &w) {
     extern __shared__ uint8_t s_raw[];
     uint8_t *sm = s_raw + ((1024u - (smem_u32(s_raw) & 1023u)) & 1023u);
@@ -331,7 +346,8 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
 #define BAR(i) (bar0 + 8u * (unsigned)(i))
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int hl = w.hl, qblk = w.qblk, ntiles = w.ntiles, j0 = CUT ? w.j0 : 0, np = CUT ? w.np : 1, piece = w.piece, rec0 = w.rec0;
+    constexpr bool CUT = MODE != PF_WHOLE;
+    const int hl = w.hl, qblk = w.qblk, ntiles = w.ntiles, j0 = CUT ? w.j0 : 0, np = MODE == PF_CUT ? w.np : 1, piece = w.piece, rec0 = w.rec0;
     const int q0 = qblk * kQTok2;
 
     if (tid == 0) {
@@ -413,7 +429,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
         /* tile B starts when the first softmax of tile A is through: half a period out of phase, the MMAs of one tile
          * run while the other tile's issuer is between two steps and its softmax warps have the SM's exponential
          * unit to themselves (nothing pulls the two loops apart by itself when they start together) */
-        if (ok && x == 1) ok = mbar_wait_blocking(BAR(B3_P + 0), 0u, s_abort, a.err, 22u);
+        if (ok && x == 1 && (MODE != PF_CLUSTER || ntiles > 0)) ok = mbar_wait_blocking(BAR(B3_P + 0), 0u, s_abort, a.err, 22u);
         for (int j = 0; j < 2 && j < ntiles && ok; j++) {
             ok = __all_sync(0xffffffffu, mbar_wait_blocking(BAR(B3_K0F + j), 0u, s_abort, a.err, 21u));
             if (!ok) break;
@@ -452,7 +468,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
         float m = -INFINITY;
         float2 l2 = make_float2(0.f, 0.f);
         bool ok = true;
-        if (x == 1) turn_pass(1);                /* tile A has the first turn */
+        if (x == 1 && (MODE != PF_CLUSTER || ntiles > 0)) turn_pass(1);      /* tile A has the first turn (a piece of a cluster may have no steps) */
         for (int j = 0; j < ntiles; j++) {       /* to the end also after a wait ran out: the turns have to match */
             const unsigned tm_s = tmem + 128u * x + 64u * (j & 1) + lane_base;
             ok = __all_sync(0xffffffffu, mbar_wait_blocking(BAR(B3_SF + 2 * x + (j & 1)), (unsigned)(j >> 1) & 1u, s_abort, a.err, 30u));   /* keep the warp together */
@@ -514,7 +530,73 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
         if (ok && ntiles > 0) ok = mbar_wait_blocking(BAR(B3_O + 2 * x + 1), 0u, s_abort, a.err, 32u);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         ok = __all_sync(0xffffffffu, ok);                     /* warp-uniform: tcgen05.ld is warp-collective */
-        if (np == 1 && ok) {
+        if (MODE == PF_CLUSTER) {
+            /* The CL pieces of a block meet in shared memory: CTA r of the cluster finishes columns [128 r / CL, 128 (r + 1) / CL) of
+             * all 256 rows.  Every piece sends the others their columns of its O and every row's {m, l}; the zones lie over the Q
+             * tiles and the K ring, which are free in all CTAs once all have arrived behind their last P.V.  Bound by the bytes
+             * between the SMs (98 KB out of and into each CTA of 4): 45 tokens behind 1 001 take 14.3 us a launch, 21.0 with
+             * records through memory, and 19.0 with chunks of a row side by side (a store then crosses as 32 pieces of 16 bytes). */
+            constexpr int W4 = 32 / CL;                          /* float4 chunks of a row that a CTA finishes */
+            constexpr int kZone = W4 * 4096;                     /* one source's zone: [W4 chunks][256 rows] */
+            constexpr int kOffMl = CL * kZone, kOffWt = kOffMl + CL * 256 * 8;
+            static_assert(kOffWt + CL * 256 * 4 <= kOff3Bar, "the zones overlap the barriers");
+            const int me = w.piece, row = tid;
+            /* chunk c of all rows is contiguous, so that a warp's store crosses as 512 consecutive bytes; rows are permuted within
+             * groups of 8 by the chunk, so that 8 lanes which read a row's chunks (CL = 8: two rows') hit all banks */
+            auto zone_off = [](int r, int c) { return c * 4096 + ((r & ~7) | ((r ^ (CL == 8 ? 2 * c : c)) & 7)) * 16; };
+            const bool live = tq0 + (warp & 3) * 4 < a.nq;       /* the warp has query tokens: else nothing to send or finish */
+            cluster_arrive();
+            cluster_wait();
+#pragma unroll 1
+            for (int c = 0; c < 4 && live; c++) {
+                unsigned v[32];
+#pragma unroll
+                for (int i = 0; i < 32; i++) v[i] = 0u;          /* a piece without steps has no O */
+                if (ntiles > 0 && ok) {
+                    tmem_ld32_nowait(tm_o + 32u * c, v);
+                    tmem_ld_wait(v);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int c4 = 8 * c + i;                    /* chunk of the whole row */
+                    st_cluster16(cluster_addr(sbase + me * kZone + zone_off(row, c4 % W4), c4 / W4),
+                                 __uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]), __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < CL; r++) if (live) st_cluster8(cluster_addr(sbase + kOffMl + (me * 256 + row) * 8, r), m, l);
+            cluster_arrive();
+            cluster_wait();
+            /* weights of the pieces for this thread's row (a piece of masked keys has m = -inf: weight 0; key 0 is never masked) */
+            if (live) {
+                float2 ml[CL];
+#pragma unroll
+                for (int r = 0; r < CL; r++) ml[r] = *reinterpret_cast<const float2 *>(sm + kOffMl + (r * 256 + row) * 8);
+                float M = ml[0].x, L = 0.f;
+#pragma unroll
+                for (int r = 1; r < CL; r++) M = fmaxf(M, ml[r].x);
+#pragma unroll
+                for (int r = 0; r < CL; r++) { ml[r].x = ex2f(ml[r].x - M); L += ml[r].y * ml[r].x; }
+                const float inv = L > 0.f ? 1.f / L : 0.f;
+#pragma unroll
+                for (int r = 0; r < CL; r++) *reinterpret_cast<float *>(sm + kOffWt + (r * 256 + row) * 4) = ml[r].x * inv;
+            }
+            __syncwarp();                                        /* a warp folds its own 32 rows */
+            const int c = lane % W4;
+            float *o0 = a.out + (size_t)((a.kv_head_begin + hl) * 8) * HY3A_D + (me * W4 + c) * 4;
+#pragma unroll
+            for (int i = 0; i < W4 && live; i++) {
+                const int r = warp * 32 + i * (32 / W4) + lane / W4, t = q0 + (r >> 3);
+                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int p = 0; p < CL; p++) {
+                    const float4 v = *reinterpret_cast<const float4 *>(sm + p * kZone + zone_off(r, c));
+                    const float f = *reinterpret_cast<const float *>(sm + kOffWt + (p * 256 + r) * 4);
+                    acc.x = fmaf(v.x, f, acc.x); acc.y = fmaf(v.y, f, acc.y); acc.z = fmaf(v.z, f, acc.z); acc.w = fmaf(v.w, f, acc.w);
+                }
+                if (t < a.nq) *reinterpret_cast<float4 *>(o0 + (size_t)t * a.out_stride + (r & 7) * HY3A_D) = acc;
+            }
+        } else if (np == 1 && ok) {
             /* A thread holds a row, so storing from the registers touches 32 rows per instruction; the warp's 32 rows go through
              * shared memory instead, 64 columns at a time (its quarter of Q_x, which P.V's last commit says is read; 16-byte
              * chunk c of row r at c ^ (r & 7): conflict-free both ways), and leave as two rows of 256 contiguous bytes per
@@ -616,6 +698,11 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
             }
         }
     }
+    if (MODE == PF_CLUSTER && warp >= 8) {       /* the other roles arrive for the two meetings of the epilogue */
+        __syncwarp();
+        cluster_arrive(); cluster_wait();
+        cluster_arrive(); cluster_wait();
+    }
     /* ---- common exit: everybody arrives here, also after a wait ran out; release TMEM */
     if (*s_abort && warp == 8 && lane == 0) {
         /* copies already issued must land before the shared memory goes away */
@@ -636,7 +723,7 @@ hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     entry_of(a, ent, w.hl);
     w.qblk = a.entries - 1 - ent;
     w.ntiles = (min(a.base + (w.qblk + 1) * kQTok2, a.base + a.nq) + kKeys3 - 1) / kKeys3;      /* keys behind these do not matter for this CTA */
-    prefill_body<false>(tm_q, tm_k, tm_v, a, w);
+    prefill_body<PF_WHOLE, 1>(tm_q, tm_k, tm_v, a, w);
 }
 /* blocks cut along the keys (grids that would leave SMs idle); a separate kernel, because the offsets and the -inf test of its
  * inner loop cost the other one 5 % */
@@ -647,11 +734,29 @@ hy3a_prefill_cut_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     entry_of(a, ent, hl);
     const hy3a_pf_piece pc = tab.e[ent];
     const pf_where w = {hl, pc.qblk, pc.j0, pc.n, pc.piece, pc.np, pc.rec};
-    prefill_body<true>(tm_q, tm_k, tm_v, a, w);
+    prefill_body<PF_CUT, 1>(tm_q, tm_k, tm_v, a, w);
+}
+/* blocks cut into CL pieces, one per CTA of a cluster */
+template <int CL>
+__global__ void __launch_bounds__(kPf3Threads, 1)
+hy3a_prefill_cluster_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ prefill_args a) {
+    pf_where w = {0, 0, 0, 0, 0, 1, 0};
+    const int blk = blockIdx.x / CL, ent = blk / a.kv_heads;      /* longest blocks first */
+    w.piece = blockIdx.x - blk * CL;                              /* = rank in the cluster */
+    w.hl = blk - ent * a.kv_heads;
+    w.qblk = a.entries - 1 - ent;
+    const int nt = (min(a.base + (w.qblk + 1) * kQTok2, a.base + a.nq) + kKeys3 - 1) / kKeys3;
+    w.j0 = w.piece * nt / CL;
+    w.ntiles = (w.piece + 1) * nt / CL - w.j0;
+    prefill_body<PF_CLUSTER, CL>(tm_q, tm_k, tm_v, a, w);
 }
 
 
 } /* namespace */
+
+static const void *pf_cluster_fn(int cl) {
+    return cl == 2 ? (const void *)hy3a_prefill_cluster_kernel<2> : cl == 4 ? (const void *)hy3a_prefill_cluster_kernel<4> : (const void *)hy3a_prefill_cluster_kernel<8>;
+}
 
 typedef CUresult (*hy3a_encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                          const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -677,6 +782,51 @@ static int make_map(hy3a_ctx *ctx, CUtensorMap *map, void *base, const cuuint64_
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return hy3a_fail(ctx, HY3A_ECUDA, "prefill: cuTensorMapEncodeTiled failed (%d)", (int)r);
     return HY3A_OK;
+}
+
+/* Attributes of the attention kernels on the context's device (they are per device), and how many clusters of 2^i CTAs fit on it at
+ * once (148 SMs of a B200: 74 of 2, 33 of 4, 15 of 8). */
+static int prefill_device(hy3a_ctx *ctx, const int **cap) {
+    static bool done_dev[64];
+    static int cap_dev[64][4];
+    const int dev = ctx->device & 63;
+    if (!done_dev[dev]) {
+        HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
+        HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_cut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
+        for (int i = 1; i < 4; i++) {
+            const void *f = pf_cluster_fn(1 << i);
+            HY3A_CUDA(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 1 << i; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(64 << i); cfg.blockDim = dim3(kPf3Threads); cfg.dynamicSmemBytes = kPf3Smem; cfg.attrs = at; cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, f, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }   /* no clusters of this size */
+            cap_dev[dev][i] = n;
+        }
+        done_dev[dev] = true;
+    }
+    *cap = cap_dev[dev];
+    return HY3A_OK;
+}
+
+/* the cut depends on the chunk's sizes alone; the layers of a chunk share it */
+static void plan_chunk(hy3a_ctx *ctx, const int *cap, int base_slot, int nq) {
+    if (ctx->pf_plan_base == base_slot && ctx->pf_plan_nq == nq) return;
+    float end = 0.f;
+    hy3a_pf_plan(base_slot, nq, ctx->cfg.kv_head_count, ctx->sm_count, ctx->d_pf_rec ? HY3A_PF_MAX_SLOTS : 0, &ctx->pf_plan, &end);
+    ctx->pf_plan_cluster = hy3a_pf_cluster(base_slot, nq, ctx->cfg.kv_head_count, cap, end, ctx->pf_plan.count > 0);
+    ctx->pf_plan_base = base_slot; ctx->pf_plan_nq = nq;
+}
+
+extern "C" int hy3a_prefill_cluster(hy3a_ctx *ctx, int base_slot, int nq) {
+    if (!ctx) return HY3A_EINVAL;
+    if (base_slot < 0 || nq < 1) return hy3a_fail(ctx, HY3A_EINVAL, "prefill_cluster: base_slot %d, nq %d", base_slot, nq);
+    const int *cap = NULL;
+    int rc = prefill_device(ctx, &cap);
+    if (rc) return rc;
+    plan_chunk(ctx, cap, base_slot, nq);
+    return ctx->pf_plan_cluster;
 }
 
 int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq, const void *q16, float *out, size_t out_stride) {
@@ -769,30 +919,36 @@ int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq
         rc = make_map(ctx, &tv, ws_v, dv, sv, bv);
         if (rc) return rc;
     }
-    static bool attr_dev[64];   /* function attributes are per device */
-    bool &attr_set = attr_dev[ctx->device & 63];
-    if (!attr_set) {
-        HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
-        HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_cut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
-        attr_set = true;
+    const int *cl_cap = NULL;
+    {
+        int rc = prefill_device(ctx, &cl_cap);
+        if (rc) return rc;
     }
     prefill_args a = {};
     a.out = out; a.out_stride = out_stride; a.base = base_slot; a.nq = nq; a.kv_head_begin = ctx->cfg.kv_head_begin; a.err = ctx->d_err;
     a.kv_heads = kvh; a.rec = ctx->d_pf_rec; a.cnt = ctx->d_pf_cnt;
     {
-        /* the cut depends on the chunk's sizes alone; the layers of a chunk share it */
-        if (ctx->pf_plan_base != base_slot || ctx->pf_plan_nq != nq) {
-            hy3a_pf_plan(base_slot, nq, kvh, ctx->sm_count, ctx->d_pf_rec ? HY3A_PF_MAX_SLOTS : 0, &ctx->pf_plan);
-            ctx->pf_plan_base = base_slot; ctx->pf_plan_nq = nq;
-        }
-        const int entries = ctx->pf_plan.count ? ctx->pf_plan.count : (nq + kQTok2 - 1) / kQTok2;
-        a.entries = entries; a.group = entries * kvh <= ctx->sm_count ? entries : kGroup;
+        plan_chunk(ctx, cl_cap, base_slot, nq);
+        const int cl = ctx->pf_plan_cluster, blocks = (nq + kQTok2 - 1) / kQTok2;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(entries * kvh); cfg.stream = ctx->stream;
-        cfg.blockDim = dim3(kPf3Threads); cfg.dynamicSmemBytes = kPf3Smem;
-        cfg.attrs = attr; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
-        if (ctx->pf_plan.count) HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_cut_kernel, tq, tk, tv, a, ctx->pf_plan));
-        else HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_kernel, tq, tk, tv, a));
+        cfg.stream = ctx->stream; cfg.blockDim = dim3(kPf3Threads); cfg.dynamicSmemBytes = kPf3Smem;
+        cudaLaunchAttribute at[2];
+        at[0] = attr[0];
+        cfg.attrs = at; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
+        if (cl > 1) {
+            a.entries = blocks;
+            cudaLaunchAttribute &ca = at[cfg.numAttrs++];
+            ca.id = cudaLaunchAttributeClusterDimension; ca.val.clusterDim.x = cl; ca.val.clusterDim.y = ca.val.clusterDim.z = 1;
+            cfg.gridDim = dim3(blocks * kvh * cl);
+            void *args[4] = {&tq, &tk, &tv, &a};
+            HY3A_CUDA(ctx, cudaLaunchKernelExC(&cfg, pf_cluster_fn(cl), args));
+        } else {
+            const int entries = ctx->pf_plan.count ? ctx->pf_plan.count : blocks;
+            a.entries = entries; a.group = entries * kvh <= ctx->sm_count ? entries : kGroup;
+            cfg.gridDim = dim3(entries * kvh);
+            if (ctx->pf_plan.count) HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_cut_kernel, tq, tk, tv, a, ctx->pf_plan));
+            else HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_kernel, tq, tk, tv, a));
+        }
     }
     ctx->launches++;
     ctx->bulk_write_pending = 1;

@@ -5,7 +5,8 @@
  * ceil(nq / 32) x heads blocks whose lengths grow with the query index, and one CTA occupies an SM, so blocks alone can leave
  * most SMs idle: 45 tokens are 16 blocks, 128 are 32.  A block may therefore be cut along the keys into pieces of M steps
  * (the last takes the rest); every piece of a cut block leaves a {m, l, O} record and the last to arrive folds them.  M is
- * chosen per chunk by list scheduling in units of steps, longest pieces first.
+ * chosen per chunk by list scheduling in units of steps, longest pieces first.  Or the CTAs of a cluster share a block
+ * (hy3a_pf_cluster, below).
  */
 #ifndef HY3A_PREFILL_PLAN_H
 #define HY3A_PREFILL_PLAN_H
@@ -46,7 +47,7 @@ static inline int hy3a_pf_steps(int base, int nq, int qblk) {
 
 /* when the last CTA of the table ends, in steps (list scheduling on a heap of SM groups that divide the heads evenly); gives
  * up as soon as the end is known to be no earlier than `limit` */
-static inline float hy3a_pf_makespan(const hy3a_pf_table *t, int heads, int sms, float limit) {
+static inline float hy3a_pf_makespan(const hy3a_pf_table *t, int heads, int sms, float limit, float extra = 0.f) {
     int unit = heads;
     while (unit > 1 && (sms % unit || heads % unit)) unit--;
     const int ng = std::min(sms / unit, 256), reps = heads / unit;
@@ -55,7 +56,7 @@ static inline float hy3a_pf_makespan(const hy3a_pf_table *t, int heads, int sms,
     float end = 0.f;
     for (int c = 0; c < t->count; c++) {
         const hy3a_pf_piece &e = t->e[c];
-        const float cost = kPfCostCta + e.n + (e.np > 1 ? kPfCostRecord : 0.f), fold = e.np > 1 ? kPfCostFold * e.np : 0.f;
+        const float cost = kPfCostCta + extra + e.n + (e.np > 1 ? kPfCostRecord : 0.f), fold = e.np > 1 ? kPfCostFold * e.np : 0.f;
         for (int r = 0; r < reps; r++) {
             const float v = load[0] + cost;       /* the least loaded group is at the root */
             if (v + fold > end) { end = v + fold; if (end >= limit) return end; }
@@ -97,7 +98,7 @@ static inline bool hy3a_pf_cut(int base, int nq, int heads, int sms, int M, int 
 }
 
 /* the plan of a chunk; max_slots = 0: no records, i.e. uncut blocks */
-static inline void hy3a_pf_plan(int base, int nq, int heads, int sms, int max_slots, hy3a_pf_table *out) {
+static inline void hy3a_pf_plan(int base, int nq, int heads, int sms, int max_slots, hy3a_pf_table *out, float *end = nullptr) {
     out->count = 0;
     const int nqb = (nq + HY3A_PF_QTOK - 1) / HY3A_PF_QTOK, longest = hy3a_pf_steps(base, nq, nqb - 1);
     if (nqb > HY3A_PF_MAX_PIECES || longest > 65535) return;
@@ -121,9 +122,45 @@ static inline void hy3a_pf_plan(int base, int nq, int heads, int sms, int max_sl
         const float m = hy3a_pf_makespan(&t, heads, sms, limit);
         if (m < limit) {
             best = m;
+            if (end) *end = m;
             if (i) memcpy(out, &t, sizeof(int) + sizeof(hy3a_pf_piece) * (size_t)t.count);      /* uncut: no table */
         }
     }
+}
+
+/* CTAs per block (1: what the plan above says, whose end in steps is `end`, with blocks cut into records or not).  The blocks of a short chunk may run as clusters of 2,
+ * 4 or 8 CTAs that share a block's keys evenly and meet in shared memory instead of through records; cap[i]: clusters of 2^i CTAs
+ * that fit at once.  The meeting costs kPfCostMeet[i] steps when all 32 query tokens of a block are in use and less in proportion
+ * to the softmax warps that hold some (4 tokens each).  Measured, us a launch, 8 heads, whole / with records / clusters of 2 / 4 / 8:
+ *    45 behind  1 001   21.0  21.0  16.2  14.3  24.9      32 behind  4 064   56.9  28.6  36.2  23.9  20.6
+ *     2 behind  1 001   18.2  18.2  13.0   9.3   7.6     128 behind  2 000   35.5  27.1  23.9  19.8  48.7
+ *   200 behind  1 000   22.9  23.0  18.1  30.2  60.7     128 behind 16 000  230.6  72.9 110.1  67.8 119.5
+ *    30 behind    300   11.1  11.1  10.8  11.1  13.9      64 behind  8 192  113.4  39.6  64.2  39.1  53.1
+ *   600 behind  4 000  116.1 116.0 107.5 130.7      600 behind 16 000  435.7 324.7 350.1 336.2
+ * Clusters of 4 and 8 only where all fit at once.  Records stay the better way for few tokens behind a very long history (more than
+ * 8 pieces per block) and for a little more than one block per SM. */
+constexpr float kPfCostMeet[4] = {0.f, 3.5f, 5.5f, 10.f};
+static inline int hy3a_pf_cluster(int base, int nq, int heads, const int cap[4], float end, bool records) {
+    const int nqb = (nq + HY3A_PF_QTOK - 1) / HY3A_PF_QTOK;
+    if (nqb > HY3A_PF_MAX_PIECES || end <= 0.f || hy3a_pf_steps(base, nq, nqb - 1) > 65535) return 1;
+    int best = 1;
+    const float used = std::min(8, (nq + 3) / 4) * 0.125f;
+    hy3a_pf_table t;
+    t.count = nqb;
+    for (int i = 1; i < 4; i++) {
+        const int cl = 1 << i;
+        const bool at_once = nqb * heads <= cap[i];
+        if (cap[i] < 1 || (cl > 2 && !at_once)) continue;
+        for (int c = 0; c < nqb; c++) {
+            t.e[c].n = (uint16_t)((hy3a_pf_steps(base, nq, nqb - 1 - c) + cl - 1) / cl);
+            t.e[c].np = 1;
+        }
+        /* the model of the records is 2 to 4 us low (above), that of several rounds of clusters on every SM a few percent */
+        const float limit = best == 1 ? end * (at_once ? (records ? 1.15f : 1.f) : 0.97f) : end;
+        const float m = hy3a_pf_makespan(&t, heads, cap[i], limit, kPfCostMeet[i] * used);
+        if (m < limit) { best = cl; end = m; }
+    }
+    return best;
 }
 
 #endif

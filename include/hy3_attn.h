@@ -215,9 +215,9 @@ int hy3a_decode_step_sharded(hy3a_ctx *ctx, int layer, int slot, const float *q_
  * been appended (the reference does the same, hy3_gpu.cu:823-832).  Replaces
  * prefill_attn_int8/int4_kernel (hy3_gpu.cu:383, :415).  q16: IEEE fp16 [nq][64][128]
  * dense (hy3a_append's q_out16); out: fp32 [nq][64][128] with row stride out_stride.
- * Chunks that would leave SMs idle are cut along the keys (hy3a_prefill_schedule) and the
- * pieces folded in a fixed order: the same call on the same context gives the same bits,
- * but the cut depends on kv_head_count, base_slot, nq and the number of SMs, so a context
+ * Chunks that would leave SMs idle are cut along the keys (hy3a_prefill_cluster,
+ * hy3a_prefill_schedule) and the pieces folded in a fixed order: the same call on the same
+ * context gives the same bits, but the cut depends on kv_head_count, base_slot, nq and the number of SMs, so a context
  * that owns some of the KV heads, or another chunking, may differ in the last bits.      */
 int hy3a_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq, const void *q16, float *out,
                  size_t out_stride);
@@ -248,7 +248,10 @@ int hy3a_decode_schedule_kv(int kv_dtype, int n, const int *kv_lens, int kv_head
                             long long *total_units, long long *u0, long long *u1);
 int hy3a_decode_schedule(int n, const int *kv_lens, int kv_heads, int n_ctas, int cta, long long *total_units,
                          long long *u0, long long *u1);
-/* How hy3a_prefill cuts a chunk into CTAs (pure host arithmetic, no GPU): the pieces of one KV head in launch order, six
+/* CTAs that hy3a_prefill gives each block of 32 query tokens and KV head of such a chunk on this context's device: 2, 4 or 8 that
+ * share the block's keys as a thread-block cluster, or 1 (hy3a_prefill_schedule), or a negative error. */
+int hy3a_prefill_cluster(hy3a_ctx *ctx, int base_slot, int nq);
+/* How hy3a_prefill cuts a chunk that does not run as clusters into CTAs (pure host arithmetic, no GPU): the pieces of one KV head in launch order, six
  * ints each {query block of 32 tokens, first step, steps (of 64 keys), first record, piece, pieces of the block}.  `sms` SMs,
  * `max_records` piece records over all heads (0: blocks stay uncut).  Writes at most cap pieces, returns their number
  * (0: uncut blocks in descending order) or a negative error.                                                         */

@@ -147,6 +147,51 @@ def test_prefill_every_block_and_head(cuda, oracle, dt, base, nq, heads, cut):
             check_attention(got[i, 8 * h:8 * h + 8], want[i, 8 * h:8 * h + 8], "%s base=%d nq=%d row %d KV head %d" % (dt, base, nq, i, h))
 
 
+@pytest.mark.parametrize("dt,base,nq,heads,size", [
+    ("fp16", 1001, 1, (0, 8), 8), ("int8", 0, 500, (0, 2), 2), ("int4", 449, 31, (0, 8), 2), ("fp16", 1001, 45, (0, 8), 4),
+    ("int8", 1000, 200, (0, 8), 2), ("int4", 4064, 32, (0, 8), 8), ("fp16", 900, 33, (3, 5), 4), ("int8", 2500, 70, (7, 1), 8),
+    ("fp16", 0, 1200, (6, 1), 2), ("int4", 40, 900, (2, 1), 4)])
+def test_prefill_clusters(cuda, oracle, dt, base, nq, heads, size):
+    """Blocks shared by the CTAs of a cluster: tokens that fill no softmax warp, one, or the last partly; fewer steps than CTAs (pieces
+    without keys, or with masked ones only); several heads and blocks per launch; every owned row finite and the others untouched;
+    one query per 4 tokens against the oracle; repeated launches bit for bit; a context without records takes the same path."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    h0, nh = heads
+    ntok = base + nq
+    q16 = torch.from_numpy(oracle.fill_normal((nq, 64, 128), SEED, 551).astype(np.float16)).to(cuda)
+    outs = []
+    for batch in (max(nq, 16), 8):
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_batch=batch, max_tokens=ntok + 128, kv_head_begin=h0, kv_head_count=nh)
+        ctx.fill_random(0, 0, 0, ntok, 79)
+        assert ctx.prefill_cluster(base, nq) > 1      # `size` on 148 SMs in the usual GPCs
+        for _ in range(3):
+            outs.append(ctx.prefill(0, 0, base, q16, out=torch.full((nq, 64, 128), float("nan"), device=cuda)))
+        ctx.sync()
+        ks, vs = ctx.export_kv(0, 0, 0, ntok)
+        ctx.close()
+    own = slice(8 * h0, 8 * (h0 + nh))
+    assert all(torch.equal(o[:, own], outs[0][:, own]) for o in outs[1:3]) and all(torch.equal(o[:, own], outs[3][:, own]) for o in outs[4:])
+    assert all(torch.isfinite(o[:, own]).all() for o in outs)
+    assert torch.isnan(outs[0][:, :8 * h0]).all() and torch.isnan(outs[0][:, 8 * (h0 + nh):]).all()
+    rows = sorted({min(4 * b + b % 4, nq - 1) for b in range(-(-nq // 4))} | {0, nq - 1})
+    want = oracle.prefill_causal(q16.float().cpu().numpy(), slots_to_float(oracle, ks, dt), slots_to_float(oracle, vs, dt), base, rows=rows)
+    for o in (outs[0], outs[3]):
+        got = o.cpu().numpy()
+        for i in rows:
+            check_attention(got[i, own], want[i, own], "%s base=%d nq=%d row %d" % (dt, base, nq, i))
+
+
+@pytest.mark.parametrize("dt,base,nq,heads", [("int8", 2500, 500, (3, 5)), ("int4", 500, 1500, (2, 2)), ("fp16", 4500, 150, (0, 8))])
+def test_prefill_records_where_no_cluster_pays(cuda, oracle, dt, base, nq, heads):
+    """Chunks that still leave records: the checks of the grids above."""
+    from hy3_b200 import Hy3Attn
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_batch=nq, max_tokens=base + nq, kv_head_begin=heads[0], kv_head_count=heads[1])
+    assert ctx.prefill_cluster(base, nq) == 1
+    ctx.close()
+    test_prefill_every_block_and_head(cuda, oracle, dt, base, nq, heads, True)
+
+
 def test_prefill_without_records(cuda, oracle):
     """A context without piece records (max_batch < 16) runs uncut what another one cuts."""
     import torch
