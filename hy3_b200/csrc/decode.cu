@@ -47,13 +47,14 @@
 namespace {
 
 constexpr int kWarps = HY3A_DECODE_WARPS;              /* consumer warps */
-static_assert(kWarps >= 8, "the Q packing and the reductions use the first 8 consumer warps");
+static_assert(kWarps >= 11, "eight warps for the queries and the reductions, one each for the new V row's scale and the new K and V rows");
 constexpr int kThreads = kWarps * 32;
 constexpr int kFixedO = kWarps * 8 * HY3A_D * 4;
 constexpr int kFixedML = ((kWarps * 8 * 2 * 4) + 127) / 128 * 128;
 constexpr int kFixedQ = 8 * 32 * 16;
+constexpr int kFixedNew = 2 * HY3A_D * 4;
 constexpr int kBarBytes = 256;      /* mbarriers of the page ring: empty[8], full[16] */
-constexpr int kFixed = kFixedO + kFixedML + kFixedQ;   /* bytes of shared memory in front of the page-count prefix */
+constexpr int kFixed = kFixedO + kFixedML + kFixedQ + kFixedNew;   /* bytes of shared memory in front of the page-count prefix */
 static_assert(16 / 8 * 8 >= 8 + 3 && 16 / 7 * 7 >= 7 + 3 && 16 / 6 * 6 >= 6 + 3 && kWarps <= 12, "rounds of the full barriers: see the consumer loop");
 constexpr bool kPSplit = true;                         /* carry the fp16 residual of P in MMA rows 8-15 */
 constexpr int kRecFloats = HY3A_REC_FLOATS;             /* floats per head record in the merge scratch (130 used) */
@@ -314,11 +315,12 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
  * single-GPU kernel's register allocation is untouched by it. */
 template <int DT, bool STAGED, bool SHARD = false>
 __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_kernel(hy3a_cache_view cache, hy3a_batch_view batch, decode_args a) {
-    /* dynamic shared memory: [s_o | s_ml | s_q | page-count prefix | full[8] empty[8] | ring of pages] */
+    /* dynamic shared memory: [s_o | s_ml | s_q | s_new | page-count prefix | full[8] empty[8] | ring of pages] */
     extern __shared__ __align__(128) uint8_t s_dyn[];
     float (*s_o)[8][HY3A_D] = reinterpret_cast<float (*)[8][HY3A_D]>(s_dyn);                       /* per-warp unnormalised outputs */
     float (*s_ml)[8][2] = reinterpret_cast<float (*)[8][2]>(s_dyn + kFixedO);                      /* per-warp {m, l} */
     uint4 (*s_q)[32] = reinterpret_cast<uint4 (*)[32]>(s_dyn + kFixedO + kFixedML);                /* Q fragments: [k-step][lane] */
+    float (*s_new)[HY3A_D] = reinterpret_cast<float (*)[HY3A_D]>(s_dyn + kFixedO + kFixedML + kFixedQ);   /* fused step: the new K row (normalised, rotated) and V row */
     __shared__ float s_qf[8];
     __shared__ unsigned s_vnew;
     __shared__ int s_flag;
@@ -410,14 +412,14 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         if (idle) u_begin = u_end = 0;
     }
     /* ---- fused step, still before the wait: what the query set-up needs besides the queries themselves
-     * (norm weights, RoPE table, the row's position -> cos/sin) comes from the host, so warps 0-7 fetch
-     * and compute it now, off the critical path.                                                       */
+     * (norm weights, RoPE table, the row's position -> cos/sin) comes from the host, so warps 0-7 (queries)
+     * and 9 (new K row) fetch and compute it now, off the critical path.                               */
     const int rl_d0 = (lane >> 4) * 64 + (lane & 15) * 4;
     float4 pre_w = make_float4(1.f, 1.f, 1.f, 1.f);
     float pre_c[4] = {1.f, 1.f, 1.f, 1.f}, pre_s[4] = {0.f, 0.f, 0.f, 0.f};
     int pre_row = -1;
-    if (a.fused && !idle && warp < 8) {
-        pre_w = *reinterpret_cast<const float4 *>(a.norm_w + rl_d0);
+    if (a.fused && !idle && (warp < 8 || warp == 9)) {
+        pre_w = *reinterpret_cast<const float4 *>(a.norm_w + (warp == 9 ? HY3A_D : 0) + rl_d0);
         pre_row = locate(s_prefix, batch, n, G, u_begin, u_end).row;
         hy3a_rowops::rope_coeffs(pre_c, pre_s, a.rope, batch.pos[pre_row], lane);
     }
@@ -544,6 +546,12 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
          * first applies the per-head RMSNorm and RoPE (same code as the append kernel).  The softmax
          * scale 1/sqrt(128) (hy3_gpu.cu:193) and log2(e) are folded into the fragments.            */
         float qf = 1.f;
+        /* what the scales of P and the append need from memory: issued with the loads of the queries */
+        const unsigned vs_old = DT != 0 ? cache.vs_max[a.layer * G + hl] : 0u;
+        const int new_page = (sg.len - 1) >> 7;
+        const bool has_new = a.fused && a.k_in && new_page >= sg.p_begin && new_page < sg.p_end;
+        int new_block = 0;
+        if (has_new) new_block = cache.block_table[(size_t)sg.seq * cache.max_blocks_per_seq + new_page];
         float *s_qx = reinterpret_cast<float *>(s_dyn);                 /* FP16 cache: [8][128] fp32 staging */
         signed char *s_q8 = reinterpret_cast<signed char *>(s_dyn);     /* INT8/INT4: [2][8][128] int8 digits */
         if (warp < 8) {
@@ -594,6 +602,19 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 vb = (unsigned)__half_as_ushort(__float2half(__fadd_rn(__fdiv_rn(m, 7.f), 1e-8f)));
             }
             if (lane == 0) s_vnew = vb;
+        } else if (has_new) {
+            /* the new rows, ready by the time their page is: the warp that holds the newest slot then only quantises and stores
+             * (loading, normalising and rotating them there cost every launch 1 to 2 us behind the last page) */
+            const size_t kvh = (size_t)(cache.kv_head_begin + hl) * HY3A_D + rl_d0;
+            if (warp == 9) {
+                const float4 k4 = *reinterpret_cast<const float4 *>(a.k_in + (size_t)row * a.ki_stride + kvh);
+                float y[4] = {k4.x, k4.y, k4.z, k4.w};
+                if (row != pre_row) { hy3a_rowops::rope_coeffs(pre_c, pre_s, a.rope, batch.pos[row], lane); pre_row = row; }
+                hy3a_rowops::norm_rope_apply(y, pre_w, a.eps, pre_c, pre_s, lane);
+                *reinterpret_cast<float4 *>(&s_new[0][rl_d0]) = make_float4(y[0], y[1], y[2], y[3]);
+            } else if (warp == 10) {
+                *reinterpret_cast<float4 *>(&s_new[1][rl_d0]) = *reinterpret_cast<const float4 *>(a.v_in + (size_t)row * a.vi_stride + kvh);
+            }
         }
         consumer_sync();
         if (DT == 0) {
@@ -630,8 +651,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         {
             int E = 6;
             if (DT != 0) {
-                unsigned vb = cache.vs_max[a.layer * G + hl];
-                vb = vb > vnew ? vb : vnew;   /* positive fp16 bit patterns order like the numbers */
+                const unsigned vb = vs_old > vnew ? vs_old : vnew;   /* positive fp16 bit patterns order like the numbers */
                 __half_raw hr; hr.x = (unsigned short)vb;
                 float vmax = __half2float(__half(hr));
                 int ex;
@@ -679,25 +699,21 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                  * been consumed, because this warp's last page pit' >= pit - ceil(11 / GP) was issued after page pit' - stages
                  * had been consumed, and n_full >= stages + ceil(11 / GP). */
                 mbar_wait(bar_base + 64 + 8 * fb, fphase, &s_abort, a.err, 2u);
-                if (a.fused && a.k_in && p == ((sg.len - 1) >> 7) && gi == ((sg.len - 1) & 127) / GT) {
-                    /* fused append: this warp holds the only granule that contains the newest slot.  It
-                     * normalises, rotates and quantises the new K row and quantises the new V row exactly
-                     * as the append kernel does, writes them to the page in HBM (for later steps) and into
-                     * the shared-memory copy it is about to read.                                         */
-                    const int d0 = (lane >> 4) * 64 + (lane & 15) * 4, tok = (sg.len - 1) & 127;
-                    const int block = cache.block_table[(size_t)sg.seq * cache.max_blocks_per_seq + p];
-                    uint8_t *gp = cache.pool + hy3a_page_index(cache, block, a.layer, hl) * (size_t)cache.page_bytes;
+                if (has_new && p == new_page && gi == ((sg.len - 1) & 127) / GT) {
+                    /* fused append: this warp holds the only granule that contains the newest slot.  It quantises the new rows
+                     * exactly as the append kernel does and writes them into the shared-memory copy it is about to read and to
+                     * the page in HBM (for later steps). */
+                    const int tok = (sg.len - 1) & 127;
+                    uint8_t *gp = cache.pool + hy3a_page_index(cache, new_block, a.layer, hl) * (size_t)cache.page_bytes;
                     uint8_t *sp = s_dyn + kFixed + a.prefix_bytes + kBarBytes + (size_t)stage * geom.page_bytes;
-                    const int kvh = cache.kv_head_begin + hl;
-                    float4 kv4 = *reinterpret_cast<const float4 *>(a.k_in + (size_t)row * a.ki_stride + (size_t)kvh * HY3A_D + d0);
-                    float y[4] = {kv4.x, kv4.y, kv4.z, kv4.w};
-                    hy3a_rowops::norm_rope_row(y, a.norm_w + HY3A_D, a.eps, a.rope, batch.pos[row], lane);
-                    hy3a_rowops::store_row<DT>(gp, geom, tok, false, y, d0, lane);
-                    hy3a_rowops::store_row<DT>(sp, geom, tok, false, y, d0, lane);
-                    kv4 = *reinterpret_cast<const float4 *>(a.v_in + (size_t)row * a.vi_stride + (size_t)kvh * HY3A_D + d0);
-                    y[0] = kv4.x; y[1] = kv4.y; y[2] = kv4.z; y[3] = kv4.w;
-                    const unsigned sb = hy3a_rowops::store_row<DT>(gp, geom, tok, true, y, d0, lane);
-                    hy3a_rowops::store_row<DT>(sp, geom, tok, true, y, d0, lane);
+                    float4 r4 = *reinterpret_cast<const float4 *>(&s_new[0][rl_d0]);
+                    float y[4] = {r4.x, r4.y, r4.z, r4.w};
+                    hy3a_rowops::store_row<DT>(sp, geom, tok, false, y, rl_d0, lane);
+                    hy3a_rowops::store_row<DT>(gp, geom, tok, false, y, rl_d0, lane);
+                    r4 = *reinterpret_cast<const float4 *>(&s_new[1][rl_d0]);
+                    y[0] = r4.x; y[1] = r4.y; y[2] = r4.z; y[3] = r4.w;
+                    const unsigned sb = hy3a_rowops::store_row<DT>(sp, geom, tok, true, y, rl_d0, lane);
+                    hy3a_rowops::store_row<DT>(gp, geom, tok, true, y, rl_d0, lane);
                     if (DT != 0 && lane == 0) atomicMax(cache.vs_max + a.layer * G + hl, sb);
                     __syncwarp();
                 }
