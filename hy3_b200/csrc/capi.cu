@@ -14,6 +14,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "ctx.h"
 #include "decode_plan.h"
 
@@ -237,6 +239,7 @@ int hy3a_create(const hy3a_config *cfg, hy3a_ctx **out) {
     CREATE_CUDA(cudaMemsetAsync(ctx->d_vs_max, 0, (size_t)cfg->n_layers * cfg->kv_head_count * sizeof(unsigned), ctx->stream));
     CREATE_CUDA(cudaMalloc(&ctx->d_inv_freq, 64 * sizeof(float)));
     CREATE_CUDA(cudaMalloc(&ctx->d_norm_w, (size_t)cfg->n_layers * 2 * HY3A_D * sizeof(float)));
+    hy3a_decode_cluster_init(ctx);
     CREATE_CUDA(cudaMalloc(&ctx->d_batch, (size_t)3 * cfg->max_batch * sizeof(int)));
     ctx->partial_records = (size_t)ctx->decode_ctas + (size_t)cfg->max_batch * cfg->kv_head_count;
     CREATE_CUDA(cudaMalloc(&ctx->d_partials, ctx->partial_records * 8 * HY3A_REC_FLOATS * sizeof(float)));
@@ -444,6 +447,12 @@ int hy3a_batch_set(hy3a_ctx *ctx, int n, const int *seq_ids, const int *slots, c
     ctx->batch_n = n;
     ctx->batch_seq0 = seq_ids[0]; ctx->batch_slot0 = slots[0]; ctx->batch_contig = slots[0] >= 0;
     for (int i = 1; i < n && ctx->batch_contig; i++) ctx->batch_contig = seq_ids[i] == seq_ids[0] && slots[i] == slots[0] + i;
+    ctx->batch_pages = 0; ctx->batch_pages_all = 0;
+    for (int i = 0; i < n; i++) {
+        const int pages = slots[i] < 0 ? 0 : slots[i] / HY3A_PAGE_TOKENS + 1;
+        ctx->batch_pages = std::max(ctx->batch_pages, pages);
+        ctx->batch_pages_all += pages;
+    }
     ctx->batch_seq_uniform = 1; ctx->batch_slot_min = slots[0] < 0 ? 0 : slots[0];
     for (int i = 1; i < n; i++) {
         if (seq_ids[i] != seq_ids[0]) ctx->batch_seq_uniform = 0;

@@ -99,10 +99,13 @@ struct hy3a_ctx {
     unsigned int *h_err;  /* pinned */
     int batch_n;
     int batch_contig, batch_seq0, batch_slot0;   /* the batch is rows slot0, slot0+1, ... of one sequence (a prefill chunk) */
+    int batch_pages;                             /* pages of the batch's longest row, */
+    long long batch_pages_all;                   /* and of all its rows */
     int batch_seq_uniform, batch_slot_min;       /* all rows belong to batch_seq0; lowest slot >= 0 of the batch */
     int decode_ctas;
     int bulk_write_pending; /* a kernel that wrote many KV slots was enqueued and no decode launch has followed it yet */
     int use_pdl;          /* launch kernels with programmatic stream serialization (HY3A_NO_PDL=1 turns it off) */
+    int cl_cap[4];        /* decode: clusters of 2^i CTAs that fit on the device at once */
     int decode_stages;    /* pages in the decode kernel's shared-memory ring; < 2 selects the direct-load variant */
 
     /* sequence-shard exchange over peer memory (hy3a_shard_*): one allocation per rank =
@@ -141,6 +144,7 @@ int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq
 int hy3a_launch_init_pages(hy3a_ctx *ctx, size_t first_page, size_t n_pages);
 int hy3a_decode_ring_capacity(int page_bytes, int max_batch);
 int hy3a_decode_max_ctas(void);
+void hy3a_decode_cluster_init(hy3a_ctx *ctx);   /* fills cl_cap */
 int hy3a_fail(hy3a_ctx *ctx, int code, const char *fmt, ...);
 
 /* slots >= ntok of sequence seq (all layers, or one layer if layer >= 0) are about to be rewritten or dropped */

@@ -53,8 +53,10 @@ constexpr int kFixedO = kWarps * 8 * HY3A_D * 4;
 constexpr int kFixedML = ((kWarps * 8 * 2 * 4) + 127) / 128 * 128;
 constexpr int kFixedQ = 8 * 32 * 16;
 constexpr int kFixedNew = 2 * HY3A_D * 4;
-constexpr int kBarBytes = 256;      /* mbarriers of the page ring: empty[8], full[16] */
-constexpr int kFixed = kFixedO + kFixedML + kFixedQ + kFixedNew;   /* bytes of shared memory in front of the page-count prefix */
+constexpr int kBarBytes = 256;      /* mbarriers of the page ring: empty[8], full[16]; of a cluster's meeting: 1 */
+constexpr int kBarClu = 192;
+constexpr int kFixedClu = (kCluBytes + 127) / 128 * 128;
+constexpr int kFixed = kFixedO + kFixedML + kFixedQ + kFixedNew + kFixedClu;   /* bytes of shared memory in front of the page-count prefix */
 static_assert(16 / 8 * 8 >= 8 + 3 && 16 / 7 * 7 >= 7 + 3 && 16 / 6 * 6 >= 6 + 3 && kWarps <= 12, "rounds of the full barriers: see the consumer loop");
 constexpr bool kPSplit = true;                         /* carry the fp16 residual of P in MMA rows 8-15 */
 constexpr int kRecFloats = HY3A_REC_FLOATS;             /* floats per head record in the merge scratch (130 used) */
@@ -313,7 +315,8 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
  * Same arithmetic, same results.                                                          */
 /* SHARD: the sequence-sharded variant (exchange + final fold in the epilogue); a separate instantiation so that the
  * single-GPU kernel's register allocation is untouched by it. */
-template <int DT, bool STAGED, bool SHARD = false>
+/* CL: 0 = any grid, 2 / 4 / 8 = a cluster of CL CTAs per (row, KV head) */
+template <int DT, bool STAGED, bool SHARD = false, int CL = 0>
 __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_kernel(hy3a_cache_view cache, hy3a_batch_view batch, decode_args a) {
     /* dynamic shared memory: [s_o | s_ml | s_q | s_new | page-count prefix | full[8] empty[8] | ring of pages] */
     extern __shared__ __align__(128) uint8_t s_dyn[];
@@ -347,10 +350,13 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         if (STAGED) {
             for (int i = 0; i < a.stages; i++) mbar_init(bar_base + 8 * i, 32 * kGranPage<DT>);   /* empty[stage]: every thread of the warps that share a page */
             for (int i = 0; i < 16; i++) mbar_init(bar_base + 64 + 8 * i, 1);   /* full[page mod n_full]: the producer's expect_tx */
+            if (CL) mbar_init(bar_base + kBarClu, 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            if (CL) mbar_expect_tx(bar_base + kBarClu, kCluBytes);
         }
     }
     __syncthreads();
+    if (CL) cluster_arrive();
     if (warp == 0 && n > 1) {
         int carry = 0;
         for (int base = 0; base < n; base += 32) {
@@ -375,12 +381,15 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
      *    query set-up and the fold twice and becomes the critical path of a small batch);
      *  - many segments: one contiguous, equally sized range per CTA over all units.
      * In both, never more CTAs than units, and the CTAs sharing a segment are contiguous.       */
-    const unsigned L = even_piece_pages(s_prefix, n, G, gridDim.x, lane);      /* 0: shares in proportion to the pages */
-    const bool aligned = split_is_aligned(s_prefix, n, G, gridDim.x, lane, L);
+    const unsigned L = CL ? 0u : even_piece_pages(s_prefix, n, G, gridDim.x, lane);      /* 0: shares in proportion to the pages */
+    const bool aligned = CL || split_is_aligned(s_prefix, n, G, gridDim.x, lane, L);
     int C = (long long)gridDim.x < U ? (int)gridDim.x : (int)U;
     long long u_begin = 0, u_end = 0;
     int al_first = 0, al_pieces = 1;
-    if (idle) {
+    if (CL) {
+        cluster_share<CL ? CL : 1>(s_prefix, G, cta, u_begin, u_end);
+        idle = u_begin == u_end;
+    } else if (idle) {
     } else if (aligned) {
         int rows_ne = 0;
         for (int r = 0; r < n; r++) rows_ne += (s_prefix[r + 1] != s_prefix[r]);
@@ -427,6 +436,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
      * touches memory that the preceding kernel in the stream may produce (queries, the newest KV
      * slot, scratch records), so wait for it -- except the producer lane, which first starts the
      * copies of pages that lie wholly below the newest slot (append-only cache: immutable).       */
+    if (CL) cluster_wait();      /* every CTA of the cluster has set its barrier up */
     const bool is_producer = STAGED && warp == kWarps;
     const unsigned n_full = STAGED ? 16u / (unsigned)a.stages * (unsigned)a.stages : 1u;   /* "full" barriers: a multiple of the stages */
     if (!is_producer) {
@@ -437,7 +447,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
     /* rows with no keys on this rank: zero output / empty partial (hy3_gpu.cu:197-199) */
-    for (int i = cta; i < n; i += gridDim.x) {
+    for (int i = CL ? n : cta; i < n; i += gridDim.x) {
         if (s_prefix[i + 1] != s_prefix[i]) continue;
         if (SHARD) {
             /* sharded: the empty record {m = -inf, l = 0} of every head goes to every other rank now (one flagged line;
@@ -463,7 +473,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         }
     }
 
-    if (idle && !SHARD) return;   /* sharded: idle CTAs may still own the fold of rows without local keys */
+    if (idle && !SHARD && !CL) return;   /* sharded: idle CTAs may still own the fold of rows without local keys */
 
 
     if (STAGED && warp == kWarps) {
@@ -504,6 +514,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 }
             }
         }
+        if (CL) { __syncwarp(); cluster_arrive(); cluster_wait(); }
         return;
     }
 
@@ -758,6 +769,10 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             float4 o4 = *reinterpret_cast<const float4 *>(&s_o[w][h][d4]);
             acc[0] += o4.x * f; acc[1] += o4.y * f; acc[2] += o4.z * f; acc[3] += o4.w * f;
         }
+        if (CL) {
+            if (red) cluster_send<CL ? CL : 1>(smem_u32(s_dyn) + kFixed - kFixedClu, bar_base + kBarClu, cta % (CL ? CL : 1), h, lane, M, L, acc);
+            break;
+        }
         consumer_sync(); /* s_o / s_ml free again */
 
         /* ---- how many CTAs share this segment? */
@@ -928,6 +943,22 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             *reinterpret_cast<float4 *>(a.out + (size_t)row * a.out_stride + head_q * HY3A_D + d4) = o4;
         }
     }
+    if (CL) {
+        constexpr int C1 = CL ? CL : 1, HPC = 8 / C1;
+        const int rank = cta % C1, seg = cta / C1, row = seg / G, hl = seg - row * G;
+        const float none[4] = {0.f, 0.f, 0.f, 0.f};
+        if (idle && warp < 8) cluster_send<C1>(smem_u32(s_dyn) + kFixed - kFixedClu, bar_base + kBarClu, rank, warp, lane, -INFINITY, 0.f, none);
+        if (warp < HPC) {
+            mbar_wait(bar_base + kBarClu, 0u, &s_abort, a.err, 70u);
+            float M, Ls, acc[4];
+            cluster_fold<C1>(s_dyn + kFixed - kFixedClu, warp, lane, M, Ls, acc);
+            cluster_write(a, G, cache.kv_head_begin, row, hl * 8 + rank * HPC + warp, lane, M, Ls, acc);
+        }
+        /* a CTA's shared memory stays until every CTA of the cluster has sent (they have, unless a wait ran out) */
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    }
     /* sharded: rows without keys on this rank were announced at the top; the other ranks' records are folded here */
     if (SHARD)
         for (int i = cta; i < n; i += gridDim.x) {
@@ -972,12 +1003,59 @@ __global__ void hy3a_merge_kernel(const float *partials, int n_parts, int n_rows
 } /* namespace */
 
 template <int DT>
+static const void *decode_cluster_fn(int cl) {
+    return cl == 2 ? (const void *)hy3a_decode_kernel<DT, true, false, 2> : cl == 4 ? (const void *)hy3a_decode_kernel<DT, true, false, 4> : (const void *)hy3a_decode_kernel<DT, true, false, 8>;
+}
+
+cudaError_t hy3a_launch_cluster(hy3a_ctx *ctx, const void *fn, int cl, int clusters, int threads, size_t smem, void **args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cl * clusters); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = ctx->use_pdl ? 2 : 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+/* also sets the kernel's shared-memory limit on the device; 0 where such clusters cannot run */
+int hy3a_cluster_cap(const void *fn, int cl, int threads, size_t smem) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(64 * cl); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.attrs = attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+void hy3a_decode_cluster_init(hy3a_ctx *ctx) {
+    const size_t prefix = ((size_t)(ctx->cfg.max_batch + 1) * sizeof(int) + 127) & ~(size_t)127, smem = kFixed + prefix + kBarBytes + (size_t)ctx->decode_stages * ctx->geom.page_bytes;
+    for (int i = 1; i < 4; i++) {
+        if (ctx->decode_stages < 2) ctx->cl_cap[i] = 0;
+        else if (ctx->geom.dtype == HY3A_KV_INT8) ctx->cl_cap[i] = hy3a_decode_umma_cluster_cap(ctx, 1 << i);
+        else ctx->cl_cap[i] = hy3a_cluster_cap(ctx->geom.dtype == HY3A_KV_FP16 ? decode_cluster_fn<0>(1 << i) : decode_cluster_fn<2>(1 << i), 1 << i, kThreads + 32, smem);
+    }
+}
+
+template <int DT>
 static cudaError_t launch_decode_dt(hy3a_ctx *ctx, const hy3a_cache_view &cv, const hy3a_batch_view &bv, decode_args &a) {
     const size_t prefix = ((size_t)(ctx->batch_n + 1) * sizeof(int) + 127) & ~(size_t)127;
     dim3 grid(ctx->decode_ctas);
     static bool attr_dev[64][3][3];   /* function attributes are per device: [device ordinal][cache type][variant] */
     bool (*attr_set)[3] = attr_dev[ctx->device & 63];
     a.prefix_bytes = (int)prefix;
+    if (a.cluster) {
+        a.stages = ctx->decode_stages;
+        void *args[3] = {(void *)&cv, (void *)&bv, (void *)&a};
+        return hy3a_launch_cluster(ctx, decode_cluster_fn<DT>(a.cluster), a.cluster, ctx->batch_n * ctx->cfg.kv_head_count, kThreads + 32,
+                                   kFixed + prefix + kBarBytes + (size_t)a.stages * ctx->geom.page_bytes, args);
+    }
     if (ctx->decode_stages >= 2) {
         a.stages = ctx->decode_stages;
         const size_t smem = kFixed + prefix + kBarBytes + (size_t)a.stages * ctx->geom.page_bytes;
@@ -1034,6 +1112,33 @@ static int spread_folders(const hy3a_ctx *ctx) {
     return 0;
 }
 
+/* A cluster of CTAs per (row, KV head) instead of the grid, where all clusters run at once: of 2, 4 or 8, the least with which a CTA has
+ * few pages (kPagesCta; a larger cluster meets later), unless the grid's even share is so much smaller that its fold is paid for
+ * (kPagesFold: the difference of 2 to 3 us in pages).  A captured launch meets other lengths when it is replayed, so there the
+ * longest row that the context can hold counts.  Measured back to back, us a layer, grid / clusters of 2 / 4 / 8, 8 KV heads:
+ *   INT8   300  7.8  6.4  6.6  7.5    700  8.4  6.6  6.5  7.8   2 500 10.8  9.5  7.4  8.1    8 192 11.2 25.3 15.0 10.9
+ *   FP16   300  6.2  5.2  4.8  5.8    700  6.6  6.6  5.8  5.9   2 500 10.4 13.7  9.1  8.3    4 096 10.5 20.2 13.0 10.5
+ *   INT4   300  8.6  7.0  6.9  7.7    700  8.7  7.4  7.1  7.8   2 500 11.3 11.1  8.1  8.5   12 000 14.3 29.5 17.6 12.5
+ *   9 rows of 200 / 2 500, clusters of 2: INT8 12.8 -> 10.4 / 17.0 -> 14.9, FP16 10.5 -> 7.6 / 22.0 -> 18.9, INT4 12.4 -> 9.8 / 17.4 -> 14.0 */
+static int cluster_size(const hy3a_ctx *ctx, int most, long long total) {
+    static const int kPagesCta[3] = {1, 5, 4}, kPagesFold[3] = {2, 5, 8};      /* FP16, INT8, INT4 */
+    const int dt = ctx->geom.dtype, segs = ctx->batch_n * ctx->cfg.kv_head_count;
+    if (most < 2 || segs > ctx->cl_cap[1]) return 0;
+    int i = 1;
+    while (i < 3 && ((most - 1) >> i) + 1 > kPagesCta[dt] && segs <= ctx->cl_cap[i + 1]) i++;
+    const long long share = (total * ctx->cfg.kv_head_count + ctx->decode_ctas - 1) / ctx->decode_ctas;
+    return ((most - 1) >> i) + 1 <= share + kPagesFold[dt] ? 1 << i : 0;
+}
+static int decode_cluster(const hy3a_ctx *ctx) {
+    if ((ctx->shard_slot >= 0 && ctx->shard_world > 1) || ctx->decode_ctas < ctx->sm_count) return 0;      /* a world of one has nothing to exchange */
+    const int cl = cluster_size(ctx, ctx->batch_pages, ctx->batch_pages_all);
+    if (!cl) return 0;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) { cudaGetLastError(); st = cudaStreamCaptureStatusActive; }
+    if (st == cudaStreamCaptureStatusNone) return cl;
+    return cluster_size(ctx, ctx->cfg.max_blocks_per_seq, (long long)ctx->cfg.max_blocks_per_seq * ctx->batch_n);
+}
+
 int hy3a_launch_decode(hy3a_ctx *ctx, int layer, const float *q, size_t q_stride, float *out, size_t out_stride, float *partials,
                        const hy3a_step_inputs *step) {
     decode_args a;
@@ -1042,6 +1147,7 @@ int hy3a_launch_decode(hy3a_ctx *ctx, int layer, const float *q, size_t q_stride
     a.scratch = ctx->d_partials; a.counters = ctx->d_counters; a.n_counters = ctx->cfg.max_batch * ctx->cfg.kv_head_count; a.err = ctx->d_err; a.layer = layer;
     a.spread = spread_folders(ctx);
     a.early_prefetch = ctx->use_pdl && !ctx->bulk_write_pending;
+    a.cluster = decode_cluster(ctx);
     if (ctx->shard_slot >= 0) {   /* set by hy3a_decode_step_sharded around this call */
         const int W = ctx->shard_world, slot = ctx->shard_slot;
         const size_t n_seg = (size_t)ctx->shard_rows * ctx->cfg.kv_head_count;

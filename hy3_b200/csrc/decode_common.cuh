@@ -35,6 +35,7 @@ struct hy3a_decode_args {
     int spread;           /* > 0: CTA-aligned segments spread their fold over up to this many of their CTAs (the whole grid is resident) */
     unsigned int *err;
     int layer;
+    int cluster;          /* 0: the grid; 2, 4, 8: a cluster of that many CTAs per (row, KV head) */
     /* fused step (fused != 0): the kernel itself normalises + rotates the queries read from q_in and
      * the CTA that streams the page of the newest slot quantises and appends the new K / V row   */
     int fused;
@@ -51,6 +52,10 @@ struct hy3a_decode_args {
 };
 
 /* the INT8 decode kernel (decode_umma.cu) */
+int hy3a_decode_umma_cluster_cap(hy3a_ctx *ctx, int cl);
+/* clusters of cl CTAs (decode.cu): a launch, and how many of a kernel fit on the current device at once */
+cudaError_t hy3a_launch_cluster(hy3a_ctx *ctx, const void *fn, int cl, int clusters, int threads, size_t smem, void **args);
+int hy3a_cluster_cap(const void *fn, int cl, int threads, size_t smem);
 cudaError_t hy3a_launch_decode_umma(hy3a_ctx *ctx, const hy3a_cache_view &cv, const hy3a_batch_view &bv, hy3a_decode_args &a);
 
 namespace {
@@ -214,6 +219,66 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatil
     return false;
 }
 /* ---- pieces both decode kernels use */
+/* Clusters: the CL CTAs of a (row, KV head) segment take an equal share of its pages each and meet in shared memory.  Rank r finishes
+ * heads [r 8 / CL, (r + 1) 8 / CL): every CTA stores its records of these heads into r's landing zone with st.async, whose bytes
+ * r's mbarrier counts, so that there is no record in memory, no counter and no fetch. */
+constexpr int kCluRec = (HY3A_D + 4) * 4;               /* {acc[128], m, l, -, -} */
+constexpr int kCluBytes = 8 * kCluRec;                  /* a CTA's zone: [CL sources][8 / CL heads] */
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ unsigned cluster_addr(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async16(unsigned addr, float a, float b, float c, float d, unsigned bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar) : "memory");
+}
+/* thread (head h of a warp, 4 dims): this CTA's piece to the CTA that finishes the head */
+template <int CL>
+__device__ __forceinline__ void cluster_send(unsigned zone, unsigned bar, int rank, int h, int lane, float M, float L, const float (&acc)[4]) {
+    constexpr int HPC = 8 / CL;
+    const unsigned to = (unsigned)h / HPC, rec = zone + (unsigned)((rank * HPC + h % HPC) * kCluRec), rb = cluster_addr(bar, to);
+    st_async16(cluster_addr(rec + 16u * (unsigned)lane, to), acc[0], acc[1], acc[2], acc[3], rb);
+    if (lane == 0) st_async16(cluster_addr(rec + 512u, to), M, L, 0.f, 0.f, rb);
+}
+/* warp w < 8 / CL folds its head's pieces in their order (rule of hy3_gpu.cu:233-247); a piece without keys has l = 0 */
+template <int CL>
+__device__ __forceinline__ void cluster_fold(const uint8_t *zone, int w, int lane, float &M, float &L, float (&acc)[4]) {
+    M = -INFINITY; L = 0.f; acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+#pragma unroll
+    for (int c = 0; c < CL; c++) {
+        const uint8_t *rec = zone + (c * (8 / CL) + w) * kCluRec;
+        const float2 ml = *reinterpret_cast<const float2 *>(rec + 512);
+        const float4 v = *reinterpret_cast<const float4 *>(rec + 16 * lane);
+        if (ml.y == 0.f) continue;
+        const float nm = fmaxf(M, ml.x), os = ex2(M - nm), rs = ex2(ml.x - nm);
+        L = L * os + ml.y * rs;
+        acc[0] = acc[0] * os + v.x * rs; acc[1] = acc[1] * os + v.y * rs; acc[2] = acc[2] * os + v.z * rs; acc[3] = acc[3] * os + v.w * rs;
+        M = nm;
+    }
+}
+/* the pages of a cluster's CTA, in units */
+template <int CL>
+__device__ __forceinline__ void cluster_share(const int *s_prefix, int G, int cta, long long &u_begin, long long &u_end) {
+    const int seg = cta / CL, k = cta - seg * CL, row = seg / G, hl = seg - row * G;
+    const int p = s_prefix[row + 1] - s_prefix[row];
+    const long long seg0 = (long long)G * s_prefix[row] + (long long)hl * p;
+    u_begin = seg0 + (long long)k * p / CL;
+    u_end = seg0 + (long long)(k + 1) * p / CL;
+}
+/* head hq (of the context's heads) of a row: final output, or the caller's record */
+__device__ __forceinline__ void cluster_write(const hy3a_decode_args &a, int kv_heads, int kv_head_begin, int row, int hq, int lane, float M, float L, const float (&acc)[4]) {
+    const int d4 = 4 * lane;
+    if (a.user_partials) {
+        float *rec = a.user_partials + ((size_t)row * kv_heads * 8 + hq) * HY3A_PARTIAL_FLOATS;
+        if (lane == 0) { rec[0] = M * kLn2; rec[1] = L; }
+        rec[2 + d4] = acc[0]; rec[3 + d4] = acc[1]; rec[4 + d4] = acc[2]; rec[5 + d4] = acc[3];
+    } else {
+        const float inv = L > 0.f ? 1.f / L : 0.f;
+        *reinterpret_cast<float4 *>(a.out + (size_t)row * a.out_stride + (size_t)(kv_head_begin * 8 + hq) * HY3A_D + d4) = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
+    }
+}
 __device__ __forceinline__ void imma16832(int c[4], const uint4 &a, unsigned b0, unsigned b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])

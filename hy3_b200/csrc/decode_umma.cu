@@ -61,7 +61,7 @@ constexpr int kShardBatchU = 1;                  /* ranks polled at once by the 
 constexpr float kDigits = 32258.f;               /* 127 * 254: the largest two-digit value */
 
 struct u_misc {
-    unsigned long long rfull[8], rempty[8], pfull[kSlots], ofull[kSlots], bk[kSlots], sfree[kSlots], qload;
+    unsigned long long rfull[8], rempty[8], pfull[kSlots], ofull[kSlots], bk[kSlots], sfree[kSlots], qload, clu;
     unsigned tmem;
     int abort_flag, flag, app_ready;         /* app_ready: the fused appends of this CTA are in HBM */
     float qf[8];
@@ -83,10 +83,13 @@ constexpr unsigned kLate = HY3A_LATE, kLateCut = HY3A_LATE_CUT;      /* the last
 constexpr int kOffQ = kOffPt + kSlots * 2048;        /* Q fragments [4 k-steps][32 lanes] x 16 B */
 constexpr int kOffQ8 = kOffQ + 2048;                 /* Q digits [2][8][128] int8 */
 constexpr int kOffMisc = kOffQ8 + 2048;
-constexpr int kOffPrefix = kOffMisc + ((sizeof(u_misc) + 127) / 128) * 128;
+constexpr int kOffClu = kOffMisc + ((sizeof(u_misc) + 127) / 128) * 128;      /* a cluster's landing zone, at the cost of two pages of the ring */
+constexpr int kStagesClu = kStages - 2;
+template <int CL> constexpr int kOffPrefix = kOffClu + (CL ? (kCluBytes + 127) / 128 * 128 : 0);
 static_assert(kShardBatchU * 8 * (HY3A_PARTIAL_FLOATS / 2) * 16 <= kLandBytes, "landing zone too small for the exchange");
 static_assert(8 * kRecFloats * 4 <= kLandBytes && 8 * HY3A_D * 4 <= kLandBytes, "landing zone too small for a record / the hand-over");
-static_assert(kStages >= 2 && kStages <= 8, "ring depth");
+/* score warps 0-3 take the even pages and 4-7 the odd ones: with an even ring each waits for every phase of its stages */
+static_assert(kStages >= 4 && kStages <= 8 && kStages % 2 == 0 && kStagesClu % 2 == 0 && kSlots % 2 == 0, "ring depth");
 
 /* descriptors: K-major, 128-byte swizzle, 8-row groups 1024 B apart (version 1, layout type 2) */
 __device__ __forceinline__ unsigned long long make_desc(unsigned saddr) {
@@ -212,20 +215,22 @@ __device__ __forceinline__ void score_group(u_misc &mi, int slot, unsigned sq, f
     mbar_arrive(UBAR(mi.pfull[slot]));
 }
 
-template <bool SHARD>
+/* CL: 0 = any grid, 2 / 4 / 8 = a cluster of CL CTAs per (row, KV head) */
+template <bool SHARD, int CL = 0>
 __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cache_view cache, hy3a_batch_view batch, decode_args a) {
+    constexpr int kStages = CL ? kStagesClu : HY3A_UMMA_STAGES;
     extern __shared__ __align__(128) uint8_t s_raw[];
     uint8_t *s_dyn = s_raw + ((1024u - (smem_u32(s_raw) & 1023u)) & 1023u);   /* 1024-aligned in the shared window */
     const unsigned s_base = smem_u32(s_dyn);
     u_misc &mi = *reinterpret_cast<u_misc *>(s_dyn + kOffMisc);
-    int *s_prefix = reinterpret_cast<int *>(s_dyn + kOffPrefix);
+    int *s_prefix = reinterpret_cast<int *>(s_dyn + kOffPrefix<CL>);
     const hy3a_geom geom = hy3a_make_geom(1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tig = lane & 3;
     const int n = batch.n, G = cache.kv_heads;
     const int cta = blockIdx.x;
     int *s_pos = s_prefix + n + 1;                                   /* RoPE positions of the rows */
-    const unsigned ring_off = (unsigned)((kOffPrefix + a.prefix_bytes + 1023) & ~1023);
+    const unsigned ring_off = (unsigned)((kOffPrefix<CL> + a.prefix_bytes + 1023) & ~1023);
     const unsigned ring_base = s_base + ring_off;
     const int qw = warp - kQkWarp0, qtid = tid - kQkWarp0 * 32;      /* score-warp numbering (negative for the other roles) */
     const bool is_qk = warp >= kQkWarp0;
@@ -259,9 +264,12 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
             mbar_init(UBAR(mi.sfree[i]), kAccWarps);
         }
         mbar_init(UBAR(mi.qload), 8);
+        if (CL) mbar_init(UBAR(mi.clu), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (CL) mbar_expect_tx(UBAR(mi.clu), kCluBytes);
     }
     __syncthreads();
+    if (CL) cluster_arrive();
     if (n > 1) {
         if (warp == 0) {
             int carry = 0;
@@ -284,11 +292,14 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
     const unsigned Pn = (unsigned)s_prefix[n];
     const long long U = (long long)G * Pn;
     bool idle = (U == 0);
-    const bool aligned = (long long)n * G < (long long)gridDim.x && aligned_split_balanced(s_prefix, n, G, gridDim.x, lane);
+    const bool aligned = CL || ((long long)n * G < (long long)gridDim.x && aligned_split_balanced(s_prefix, n, G, gridDim.x, lane));
     const int C = (long long)gridDim.x < U ? (int)gridDim.x : (int)U;
     long long u_begin = 0, u_end = 0;
     int al_first = 0, al_pieces = 1;
-    if (idle) {
+    if (CL) {
+        cluster_share<CL ? CL : 1>(s_prefix, G, cta, u_begin, u_end);
+        idle = u_begin == u_end;
+    } else if (idle) {
     } else if (aligned && Pn < (1u << 23)) {
         int rows_ne = 0;
         for (int r = 0; r < n; r++) rows_ne += (s_prefix[r + 1] != s_prefix[r]);
@@ -350,7 +361,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         u_end = (long long)(cta + 1) * U / C;
         if (idle) u_begin = u_end = 0;
     }
-    if (idle && !SHARD) {
+    if (idle && !SHARD && !CL) {
         /* nothing to do: give the tensor memory back and leave (sharded: idle CTAs may still own the fold of rows without local keys) */
         fence_before();
         __syncthreads();
@@ -394,6 +405,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
     fence_before();
     __syncthreads();
     fence_after();
+    if (CL) cluster_wait();      /* every CTA of the cluster has set its barrier up */
     const unsigned tmem = mi.tmem;
 
     /* From here on the kernel touches memory that the preceding kernel in the stream may produce (queries, the newest KV
@@ -405,7 +417,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
     /* rows with no keys on this rank: zero output / empty partial (hy3_gpu.cu:197-199) */
-    if (is_qk)
+    if (is_qk && !CL)
         for (int i = cta; i < n; i += gridDim.x) {
             if (s_prefix[i + 1] != s_prefix[i]) continue;
             if (SHARD) {
@@ -707,6 +719,10 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                 const float4 o4 = *reinterpret_cast<const float4 *>(s_dyn + kOffAcc + (h * HY3A_D + d4) * 4);
                 acc[0] = o4.x; acc[1] = o4.y; acc[2] = o4.z; acc[3] = o4.w;
             }
+            if (CL) {
+                cluster_send<CL ? CL : 1>(s_base + kOffClu, UBAR(mi.clu), cta % (CL ? CL : 1), h, lane, M, L, acc);
+                break;
+            }
             qk_sync();   /* everybody holds its share: the accumulators may overwrite the hand-over area (next piece) */
 
             /* ---- how many CTAs share this segment? */
@@ -867,6 +883,18 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                 *reinterpret_cast<float4 *>(a.out + (size_t)row * a.out_stride + head_q * HY3A_D + d4) = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
             }
         }
+        if (CL) {
+            constexpr int C1 = CL ? CL : 1, HPC = 8 / C1;
+            const int rank = cta % C1, seg = cta / C1, row = seg / G, hl = seg - row * G;
+            const float none[4] = {0.f, 0.f, 0.f, 0.f};
+            if (idle) cluster_send<C1>(s_base + kOffClu, UBAR(mi.clu), rank, qw, lane, -INFINITY, 0.f, none);
+            if (qw < HPC) {
+                UWAIT(mi.clu, 0u, 70u);
+                float M, L, acc[4];
+                cluster_fold<C1>(s_dyn + kOffClu, qw, lane, M, L, acc);
+                cluster_write(a, G, cache.kv_head_begin, row, hl * 8 + rank * HPC + qw, lane, M, L, acc);
+            }
+        }
         /* sharded: rows without keys on this rank were announced at the top; the other ranks' records are folded here */
         if (SHARD)
             for (int i = cta; i < n; i += gridDim.x) {
@@ -900,6 +928,8 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         fence_before();
         __syncthreads();
         if (warp == kIssWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kSlots * 64) : "memory");
+        /* a CTA's shared memory stays until every CTA of the cluster has sent (they have, unless a wait ran out) */
+        if (CL) { __syncwarp(); cluster_arrive(); cluster_wait(); }
     }
 }
 
@@ -908,16 +938,33 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
 /* Bytes of dynamic shared memory for a batch capacity (prefix = page counts + positions of the rows). */
 static size_t umma_prefix_bytes(int n) { return ((size_t)(2 * n + 2) * sizeof(int) + 127) & ~(size_t)127; }
 
+/* the launch's shared memory: CL = 0 or any cluster */
+template <int CL>
+static size_t umma_smem(size_t prefix) { return 1024 + ((kOffPrefix<CL> + prefix + 1023) & ~(size_t)1023) + (size_t)(CL ? kStagesClu : kStages) * kStageBytes; }
+
 int hy3a_decode_umma_fits(int max_batch) {
-    return 1024 + ((kOffPrefix + umma_prefix_bytes(max_batch) + 1023) & ~(size_t)1023) + (size_t)kStages * kStageBytes <= (size_t)kSmemMax;
+    return umma_smem<0>(umma_prefix_bytes(max_batch)) <= (size_t)kSmemMax;
+}
+
+static const void *umma_cluster_fn(int cl) {
+    return cl == 2 ? (const void *)hy3a_decode_umma_kernel<false, 2> : cl == 4 ? (const void *)hy3a_decode_umma_kernel<false, 4> : (const void *)hy3a_decode_umma_kernel<false, 8>;
+}
+
+/* clusters of cl CTAs that fit on the device at once */
+int hy3a_decode_umma_cluster_cap(hy3a_ctx *ctx, int cl) {
+    return hy3a_cluster_cap(umma_cluster_fn(cl), cl, kUThreads, umma_smem<1>(umma_prefix_bytes(ctx->cfg.max_batch)));
 }
 
 cudaError_t hy3a_launch_decode_umma(hy3a_ctx *ctx, const hy3a_cache_view &cv, const hy3a_batch_view &bv, hy3a_decode_args &a) {
     const size_t prefix = umma_prefix_bytes(ctx->batch_n);
     a.prefix_bytes = (int)prefix;
     a.stages = kStages;
-    const size_t smem = 1024 + ((kOffPrefix + prefix + 1023) & ~(size_t)1023) + (size_t)kStages * kStageBytes;
+    const size_t smem = umma_smem<0>(prefix);
     const bool shard = a.n_dest > 0;
+    if (a.cluster) {
+        void *args[3] = {(void *)&cv, (void *)&bv, (void *)&a};
+        return hy3a_launch_cluster(ctx, umma_cluster_fn(a.cluster), a.cluster, ctx->batch_n * ctx->cfg.kv_head_count, kUThreads, umma_smem<1>(prefix), args);
+    }
     static bool attr_dev[64][2];   /* function attributes are per device */
     bool *attr_set = attr_dev[ctx->device & 63];
     if (!attr_set[shard ? 1 : 0]) {

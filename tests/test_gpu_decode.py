@@ -403,3 +403,81 @@ def test_errors_are_codes_not_exits(cuda, oracle):
     with pytest.raises(Hy3AttnError):
         ctx._chk(ctx.lib.hy3a_decode(ctx.h, 9, q.data_ptr(), 8192, q.data_ptr(), 8192, None))  # bad layer
     ctx.close()
+
+
+@pytest.mark.parametrize("dt", ["fp16", "int8", "int4"])
+@pytest.mark.parametrize("lens,heads", [
+    ([129], (0, 8)), ([300], (0, 8)), ([640], (3, 5)), ([900], (0, 8)), ([2200], (0, 8)), ([257, 1, 128], (0, 8)), ([1500, 700], (6, 2)),
+    ([4200], (7, 1)), ([200, 130, 256, 255, 129, 300, 384, 200, 140], (0, 8)), ([900, 0, 700], (2, 1)), ([1025] * 5, (4, 3))])
+def test_decode_clusters_equal_the_grid(cuda, oracle, dt, lens, heads):
+    """Steps of few segments run as clusters of 2, 4 or 8 CTAs per (row, KV head).  Fewer pages than CTAs, full and one-token last
+    pages, rows without keys, several heads and rows: against the oracle and the grid (the same kernels on a context that is told
+    of one CTA less than the device has SMs), outputs and the cache; repeated launches bit for bit; partial records; the step
+    captured into a graph and replayed for other lengths.  The two differ by the order of fp32 sums and fp16 digits of P (2^-22):
+    2e-5 is over ten times that at outputs below 4."""
+    import os
+    import torch
+    from hy3_b200 import Hy3Attn
+    h0, nh = heads
+    n = len(lens)
+    rng = np.random.default_rng(5)
+    q, k, v = (torch.from_numpy(rng.standard_normal((n, h, 128)).astype(np.float32)).to(cuda) for h in (64, 8, 8))
+    res = []
+    for ctas in (None, torch.cuda.get_device_properties(0).multi_processor_count - 1):
+        if ctas:
+            os.environ["HY3A_DECODE_CTAS"] = str(ctas)
+        try:
+            ctx = Hy3Attn(kv_dtype=dt, n_layers=2, kv_head_begin=h0, kv_head_count=nh, max_seqs=n, max_batch=n, max_tokens=sum(lens) + 128 * n, max_tokens_per_seq=max(lens) + 128)
+        finally:
+            os.environ.pop("HY3A_DECODE_CTAS", None)
+        for layer in range(2):
+            for i, m in enumerate(lens):
+                if m > 1:
+                    ctx.fill_random(layer, i, 0, m - 1, 100 * layer + i)
+        slots = [m - 1 for m in lens]
+        ctx.batch_set(list(range(n)), slots)
+        outs = []
+        for _ in range(4):
+            for layer in range(2):
+                outs.append(ctx.decode_step(layer, q, k, v, out=torch.full((n, 64, 128), float("nan"), device=cuda)))
+        part = torch.full((n, 8 * nh, 130), float("nan"), device=cuda)
+        ctx.decode_step(0, q, k, v, partials=part)
+        ctx.sync()
+        assert all(torch.equal(outs[i][:, 8 * h0:8 * (h0 + nh)], outs[i % 2][:, 8 * h0:8 * (h0 + nh)]) for i in range(8))
+        qn = torch.zeros((n, 64, 128), device=cuda)
+        ctx.decode_step(0, q, k, v, q_out=qn)
+        ctx.sync()
+        kv = {i: ctx.export_kv(0, i, 0, m) for i, m in enumerate(lens) if m > 0}
+        # a graph captured for these rows, replayed for shorter ones
+        side = torch.cuda.Stream()
+        g_out = torch.zeros((n, 64, 128), device=cuda)
+        ctx.set_stream(side)
+        with torch.cuda.stream(side):
+            ctx.decode_step(1, q, k, v, out=g_out)
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            ctx.decode_step(1, q, k, v, out=g_out)
+        side.synchronize()
+        ctx.use_torch_stream()
+        ctx.batch_set(list(range(n)), [max(-1, m - 3) if m > 2 else m - 1 for m in lens])
+        graph.replay()
+        ctx.sync()
+        res.append((outs[0], outs[1], part, g_out.clone(), kv, qn))
+        del graph
+        ctx.close()
+    own = slice(8 * h0, 8 * (h0 + nh))
+    for a, b in zip(res[0][:2], res[1][:2]):
+        assert torch.isfinite(a[:, own]).all() and (a[:, own] - b[:, own]).abs().max() < 2e-5
+        assert torch.isnan(a[:, :8 * h0]).all() and torch.isnan(a[:, 8 * (h0 + nh):]).all()
+    assert (res[0][3][:, own] - res[1][3][:, own]).abs().max() < 2e-5
+    live = [i for i, m in enumerate(lens) if m > 0]
+    for x in (0, 1):
+        p = res[x][2][live]
+        assert ((p[:, :, 2:] / p[:, :, 1:2]) - res[0][0][live][:, own]).abs().max() < 2e-5
+        assert all((res[x][2][i, :, 1] == 0).all() and torch.isneginf(res[x][2][i, :, 0]).all() for i, m in enumerate(lens) if m == 0)
+    for i in live:
+        assert all(np.array_equal(a, b) for a, b in zip(res[0][4][i], res[1][4][i]))
+        Kf, Vf = (slots_to_float(oracle, x, dt) for x in res[0][4][i])
+        want = oracle.attention(res[0][5][i].cpu().numpy(), Kf, Vf)
+        check_attention(res[0][0][i, own].cpu().numpy(), want[own], "%s row %d of %d tokens" % (dt, i, lens[i]))
