@@ -1,8 +1,9 @@
-"""In-tree build of the two shared libraries for sm_100a with nvcc.
+"""In-tree build of the shared libraries for sm_100a with nvcc.
 
     python -m hy3_b200._build [--force] [--verbose]
 
   libhy3attn.so   the attention library: CUDA kernels + the C ABI of include/hy3_attn.h
+  _native.so      the CPython module with the per-step calls of Hy3Attn (csrc/binding.cpp); links libtorch, not CUDA
   libhy3_gpu.so   the same objects plus hy3_gpu_dropin.cu: hy3_gpu_init / hy3_gpu_free / hy3_eval_gpu for the reference
                   engine (include/hy3_gpu_dropin.h).  It is compiled against the engine's own hy3.h, so it needs the
                   engine's checkout: HY3_REF, or a directory `reference` next to this repository.  Without one a
@@ -20,6 +21,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhy3attn.so")
 DROPIN_LIB = os.path.join(HERE, "libhy3_gpu.so")
+NATIVE = os.path.join(HERE, "_native.so")
 SOURCES = ["append.cu", "decode.cu", "decode_umma.cu", "prefill.cu", "capi.cu", "selftest.cu"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC,-fvisibility=default", "-I", os.path.join(ROOT, "include")]
@@ -61,8 +63,30 @@ def build(force=False, verbose=False):
         if r.returncode:
             print(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_binding(force)
     build_dropin(objs, headers, nvcc, obj_dir, force, verbose)
     return lib_out
+
+
+def build_binding(force=False):
+    """The CPython module with the per-step calls; needs torch's headers and libraries."""
+    src = os.path.join(CSRC, "binding.cpp")
+    if not (force or _newer([src, os.path.join(ROOT, "include", "hy3_attn.h")], NATIVE)):
+        return NATIVE
+    import sysconfig
+
+    import torch
+    t = os.path.dirname(torch.__file__)
+    cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           "-isystem", os.path.join(t, "include"), "-isystem", os.path.join(t, "include", "torch", "csrc", "api", "include"),
+           "-I", sysconfig.get_paths()["include"], src, "-o", NATIVE,
+           "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        print(r.stdout + r.stderr)
+        raise RuntimeError("building the binding failed")
+    return NATIVE
 
 
 def reference_dir():

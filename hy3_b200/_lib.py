@@ -81,3 +81,22 @@ def load_library():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_bound = None
+
+
+def load_native():
+    """The native per-step calls (csrc/binding.cpp, built with the library), bound to the loaded library."""
+    global _bound
+    if _bound is not None:
+        return _bound
+    import torch  # noqa: F401  (its libraries have to be loaded first)
+    lib = load_library()
+    try:
+        from . import _native
+    except ImportError as e:
+        raise Hy3AttnError(-3, "the native binding does not load (%s): build it with `python -m hy3_b200._build`" % e) from e
+    _native.bind(*(C.cast(getattr(lib, "hy3a_" + f), _vp).value for f in ("batch_set", "append", "decode_step", "prefill")))
+    _bound = _native
+    return _bound

@@ -4,7 +4,7 @@ import ctypes as C
 
 import numpy as np
 
-from ._lib import Config, Hy3AttnError, load_library
+from ._lib import Config, Hy3AttnError, load_library, load_native
 
 H, G, D = 64, 8, 128
 PAGE_TOKENS = 128
@@ -12,24 +12,8 @@ PARTIAL_FLOATS = 130
 KV_DTYPES = {"fp16": 0, "int8": 1, "int4": 2}
 
 
-_f32 = None     # torch.float32, fetched with the first tensor (the module itself does not need torch)
-
-
 def _ptr(t):
     return None if t is None else t.data_ptr()
-
-
-def _rows(t, n):
-    """Row stride of an fp32 tensor of n rows whose heads are dense (0 for None)."""
-    if t is None:
-        return 0
-    global _f32
-    if _f32 is None:
-        import torch
-        _f32 = torch.float32
-    st = t.stride()
-    assert len(t) == n and t.dtype is _f32 and st[-1] == 1 and st[-2] == D
-    return st[0]
 
 
 class Hy3Attn:
@@ -38,6 +22,7 @@ class Hy3Attn:
     def __init__(self, kv_dtype="int8", n_layers=80, kv_head_begin=0, kv_head_count=G, max_seqs=1, max_batch=512,
                  max_tokens=8192, max_tokens_per_seq=None, device=None, rms_eps=1e-5, stream=None):
         self.lib = load_library()
+        self._n = load_native()
         self.kv_dtype = kv_dtype
         cfg = Config()
         self.lib.hy3a_default_config(C.byref(cfg))
@@ -56,7 +41,7 @@ class Hy3Attn:
         rc = self.lib.hy3a_create(C.byref(cfg), C.byref(h))
         if rc:
             raise Hy3AttnError(rc, self.lib.hy3a_last_error(None).decode())
-        self.h = h
+        self.h, self._hv = h, h.value
         self.batch_n = 0
         if stream is None:
             # work is enqueued on torch's current stream, so that it is ordered with the allocations,
@@ -73,7 +58,7 @@ class Hy3Attn:
     def close(self):
         if getattr(self, "h", None):
             self.lib.hy3a_destroy(self.h)
-            self.h = None
+            self.h, self._hv = None, 0
 
     def __del__(self):
         try:
@@ -131,30 +116,23 @@ class Hy3Attn:
         s = np.ascontiguousarray(seq_ids, np.int32)
         t = np.ascontiguousarray(slots, np.int32)
         p = t if rope_pos is None else np.ascontiguousarray(rope_pos, np.int32)
-        assert s.size == t.size == p.size
-        rc = self.lib.hy3a_batch_set(self.h, s.size, *(a.__array_interface__["data"][0] for a in (s, t, p)))
+        rc = self._n.batch_set(self._hv, s, t, p)
         if rc:
             self._chk(rc)
-        self.batch_n = int(s.size)
+        self.batch_n = s.size
 
     # ---- hot path
     def append(self, layer, q, k, v, q_out=None, q_out16=None):
         """q [n,64,128] / k,v [n,8,128] fp32 (row stride free, rows dense).  Returns q_out (fp32); q_out=False with a
         q_out16 buffer writes the 16-bit queries only (the chunked prefill reads nothing else)."""
         n = self.batch_n
-        assert (k is None) == (v is None)
-        sq, sk, sv = _rows(q, n), _rows(k, n), _rows(v, n)
         if q_out is False:
             assert q_out16 is not None
             q_out = None
         elif q_out is None:
             import torch
             q_out = torch.empty((n, H, D), dtype=torch.float32, device=q.device)
-        if q_out16 is not None:
-            import torch
-            assert q_out16.dtype == torch.float16 and q_out16.is_contiguous() and q_out16.numel() == n * H * D
-        rc = self.lib.hy3a_append(self.h, layer, q.data_ptr(), sq, _ptr(k), sk, _ptr(v), sv, _ptr(q_out),
-                                  0 if q_out is None else q_out.stride(0), _ptr(q_out16))
+        rc = self._n.append(self._hv, layer, n, q, k, v, q_out, q_out16)
         if rc:
             self._chk(rc)
         return q_out
@@ -175,14 +153,10 @@ class Hy3Attn:
     def decode_step(self, layer, q, k, v, out=None, q_out=None, partials=None):
         """Fused append + decode of one new token per batch row (pre-norm q [n,64,128], k/v [n,8,128])."""
         n = self.batch_n
-        assert (k is None) == (v is None)
-        sq, sk, sv = _rows(q, n), _rows(k, n), _rows(v, n)
         if partials is None and out is None:
             import torch
             out = torch.zeros((n, H, D), dtype=torch.float32, device=q.device)
-        rc = self.lib.hy3a_decode_step(self.h, layer, q.data_ptr(), sq, _ptr(k), sk, _ptr(v), sv, _ptr(q_out),
-                                       0 if q_out is None else q_out.stride(0), _ptr(out),
-                                       0 if out is None else out.stride(0), _ptr(partials))
+        rc = self._n.decode_step(self._hv, layer, n, q, k, v, q_out, out, partials)
         if rc:
             self._chk(rc)
         return out if partials is None else partials
@@ -221,12 +195,12 @@ class Hy3Attn:
         return out
 
     def prefill(self, layer, seq, base_slot, q16, out=None):
-        import torch
-        nq = q16.shape[0]
-        assert q16.dtype == torch.float16 and q16.is_contiguous()
         if out is None:
-            out = torch.zeros((nq, H, D), dtype=torch.float32, device=q16.device)
-        self._chk(self.lib.hy3a_prefill(self.h, layer, seq, base_slot, nq, _ptr(q16), _ptr(out), out.stride(0)))
+            import torch
+            out = torch.zeros((q16.shape[0], H, D), dtype=torch.float32, device=q16.device)
+        rc = self._n.prefill(self._hv, layer, seq, base_slot, q16, out)
+        if rc:
+            self._chk(rc)
         return out
 
     def prefill_cluster(self, base_slot, nq):

@@ -41,6 +41,7 @@ struct append_args {
      * [head][128][mirror_stride], the values the conversion kernel of the chunked prefill would produce */
     __half *mirror_k, *mirror_v;
     int mirror_stride;
+    int wait_first;      /* the preceding kernel may be the one that writes the batch descriptor */
 };
 
 /* grid (10, n_rows), block 256: warp (blockIdx.x*8 + warp) in [0,80) = 64 Q, 8 K, 8 V heads. */
@@ -140,6 +141,7 @@ __global__ void __launch_bounds__(256, 4) hy3a_append_chunk_kernel(hy3a_cache_vi
     const bool is_qb = (int)blockIdx.x >= kv_blocks;
     const int hg = (cache.kv_heads + hpb - 1) / hpb, grp = (int)blockIdx.x / hg;
     __shared__ __align__(16) float s_cos[8][64], s_sin[8][64];
+    if (a.wait_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     {
         const int rows = is_qb ? 1 : 8, row0 = is_qb ? (int)blockIdx.x - kv_blocks : grp * 8;
         for (int i = threadIdx.x; i < rows * 64; i += 256) {
@@ -436,6 +438,7 @@ int hy3a_launch_append(hy3a_ctx *ctx, int layer, const float *q_in, size_t q_str
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
+    a.wait_first = hy3a_take_fresh(ctx);
     cudaError_t e;
     if (ctx->batch_n >= 32) {      /* a chunk: the throughput-shaped kernel */
         const int n = ctx->batch_n, ng = (n + 7) / 8, kvh = ctx->cfg.kv_head_count;

@@ -29,6 +29,49 @@ int hy3a_fail(hy3a_ctx *ctx, int code, const char *fmt, ...) {
     return code;
 }
 
+namespace {
+
+/* The batch descriptor travels as a kernel parameter: a row range of one sequence as four numbers (a decode step of one sequence,
+ * a prefill chunk), other batches by value.  A copy from pinned memory costs the host a staging slot, the copy and an event (8 us with
+ * the call around it, 3 this way) and holds the stream for the copy engine's hand-over; and a kernel keeps the programmatic chain
+ * unbroken, so that the next launch sets itself up meanwhile.  More rows than fit the 4 KB of parameters are copied. */
+constexpr int kBatchParamRows = 336;
+struct batch_run {
+    int seq0, slot0, pos0, n;
+    __device__ __forceinline__ void row(int i, int &seq, int &slot, int &pos) const { seq = seq0; slot = slot0 + i; pos = pos0 + i; }
+};
+template <int N>
+struct batch_rows {
+    int n, seq_[N], slot_[N], pos_[N];
+    batch_rows(int rows, const int *seq, const int *slot, const int *pos) : n(rows) {
+        memcpy(seq_, seq, rows * sizeof(int)); memcpy(slot_, slot, rows * sizeof(int)); memcpy(pos_, pos, rows * sizeof(int));
+    }
+    __device__ __forceinline__ void row(int i, int &seq, int &slot, int &pos) const { seq = seq_[i]; slot = slot_[i]; pos = pos_[i]; }
+};
+template <class B>
+__global__ void __launch_bounds__(128) hy3a_batch_kernel(const __grid_constant__ B b, int *out, int max_batch) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");     /* the next kernel waits before it reads the descriptor */
+    asm volatile("griddepcontrol.wait;" ::: "memory");                  /* the preceding ones are through with the old descriptor */
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i >= max_batch) return;
+    int seq = 0, slot = 0, pos = 0;
+    if (i < b.n) b.row(i, seq, slot, pos);
+    out[i] = seq; out[max_batch + i] = slot; out[2 * max_batch + i] = pos;
+}
+template <class B>
+cudaError_t launch_batch(hy3a_ctx *ctx, const B &b) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((ctx->cfg.max_batch + 127) / 128); cfg.blockDim = dim3(128); cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
+    ctx->batch_fresh = 1;
+    return cudaLaunchKernelEx(&cfg, hy3a_batch_kernel<B>, b, ctx->d_batch, ctx->cfg.max_batch);
+}
+
+} /* namespace */
+
 extern "C" {
 
 const char *hy3a_version(void) { return "hy3attn sm_100a " __DATE__; }
@@ -433,17 +476,28 @@ int hy3a_batch_set(hy3a_ctx *ctx, int n, const int *seq_ids, const int *slots, c
         if (rc) return rc;
         if (slots[i] >= 0) hy3a_mirror_truncate(ctx, seq_ids[i], -1, slots[i]);   /* the slot is about to be written */
     }
-    /* one staging copy of [seq | slot | pos], each padded to max_batch */
-    size_t mb = (size_t)ctx->cfg.max_batch;
-    int *tmp = (int *)malloc(3 * mb * sizeof(int));
-    if (!tmp) return hy3a_fail(ctx, HY3A_ENOMEM, "batch_set: malloc failed");
-    memset(tmp, 0, 3 * mb * sizeof(int));
-    memcpy(tmp, seq_ids, n * sizeof(int));
-    memcpy(tmp + mb, slots, n * sizeof(int));
-    memcpy(tmp + 2 * mb, rope_pos, n * sizeof(int));
-    int rc = stage_h2d(ctx, ctx->d_batch, tmp, 3 * mb * sizeof(int));
-    free(tmp);
-    if (rc) return rc;
+    /* the descriptor is [seq | slot | pos], each padded with zeros to max_batch */
+    const size_t mb = (size_t)ctx->cfg.max_batch;
+    int run = 1;
+    for (int i = 1; i < n && run; i++) run = seq_ids[i] == seq_ids[0] && slots[i] == slots[0] + i && rope_pos[i] == rope_pos[0] + i;
+    if (run) {
+        HY3A_CUDA(ctx, launch_batch(ctx, batch_run{seq_ids[0], slots[0], rope_pos[0], n}));
+    } else if (n <= 32) {
+        HY3A_CUDA(ctx, launch_batch(ctx, batch_rows<32>(n, seq_ids, slots, rope_pos)));
+    } else if (n <= kBatchParamRows) {
+        HY3A_CUDA(ctx, launch_batch(ctx, batch_rows<kBatchParamRows>(n, seq_ids, slots, rope_pos)));
+    } else {
+        int *tmp = (int *)malloc(3 * mb * sizeof(int));
+        if (!tmp) return hy3a_fail(ctx, HY3A_ENOMEM, "batch_set: malloc failed");
+        memset(tmp, 0, 3 * mb * sizeof(int));
+        memcpy(tmp, seq_ids, n * sizeof(int));
+        memcpy(tmp + mb, slots, n * sizeof(int));
+        memcpy(tmp + 2 * mb, rope_pos, n * sizeof(int));
+        int rc = stage_h2d(ctx, ctx->d_batch, tmp, 3 * mb * sizeof(int));
+        free(tmp);
+        if (rc) return rc;
+        ctx->batch_fresh = 0;      /* a copy: the next launch waits for it anyway */
+    }
     ctx->batch_n = n;
     ctx->batch_seq0 = seq_ids[0]; ctx->batch_slot0 = slots[0]; ctx->batch_contig = slots[0] >= 0;
     for (int i = 1; i < n && ctx->batch_contig; i++) ctx->batch_contig = seq_ids[i] == seq_ids[0] && slots[i] == slots[0] + i;

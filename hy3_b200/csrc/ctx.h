@@ -103,6 +103,7 @@ struct hy3a_ctx {
     long long batch_pages_all;                   /* and of all its rows */
     int batch_seq_uniform, batch_slot_min;       /* all rows belong to batch_seq0; lowest slot >= 0 of the batch */
     int decode_ctas;
+    int batch_fresh;      /* the batch descriptor was written by a kernel and no kernel that reads it has been launched since */
     int bulk_write_pending; /* a kernel that wrote many KV slots was enqueued and no decode launch has followed it yet */
     int use_pdl;          /* launch kernels with programmatic stream serialization (HY3A_NO_PDL=1 turns it off) */
     int cl_cap[4];        /* decode: clusters of 2^i CTAs that fit on the device at once */
@@ -167,6 +168,10 @@ static inline hy3a_batch_view hy3a_bview(const hy3a_ctx *c) {
     b.seq = c->d_batch; b.slot = c->d_batch + c->cfg.max_batch; b.pos = c->d_batch + 2 * c->cfg.max_batch; b.n = c->batch_n;
     return b;
 }
+
+/* The decode and append kernels read the batch descriptor before they wait for the preceding kernel.  The first of them behind
+ * hy3a_batch_set has to wait first; those after it find a predecessor that started when the descriptor was complete. */
+static inline int hy3a_take_fresh(hy3a_ctx *c) { const int f = c->batch_fresh; c->batch_fresh = 0; return f; }
 
 #define HY3A_CUDA(ctx, call)                                                                                   \
     do {                                                                                                       \

@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
     const unsigned bar_base = smem_u32(s_dyn + kFixed + a.prefix_bytes);
     const unsigned ring_base = bar_base + kBarBytes;
 
+    if (a.wait_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     /* ---- schedule: prefix of pages per row */
     for (int i = tid; i < n; i += blockDim.x) {
         int len = batch.slot[i] + 1;
@@ -1146,6 +1147,7 @@ int hy3a_launch_decode(hy3a_ctx *ctx, int layer, const float *q, size_t q_stride
     a.q = q; a.q_stride = q_stride; a.out = out; a.out_stride = out_stride; a.user_partials = partials;
     a.scratch = ctx->d_partials; a.counters = ctx->d_counters; a.n_counters = ctx->cfg.max_batch * ctx->cfg.kv_head_count; a.err = ctx->d_err; a.layer = layer;
     a.spread = spread_folders(ctx);
+    a.wait_first = hy3a_take_fresh(ctx);
     a.early_prefetch = ctx->use_pdl && !ctx->bulk_write_pending;
     a.cluster = decode_cluster(ctx);
     if (ctx->shard_slot >= 0) {   /* set by hy3a_decode_step_sharded around this call */
@@ -1224,6 +1226,7 @@ extern "C" int hy3a_decode_noalloc(hy3a_ctx *ctx, int layer, const float *q, siz
     a.counters = reinterpret_cast<unsigned *>(scratch + kNoAllocRecordBytes);
     a.n_counters = kNoAllocRows;
     a.err = ctx->d_err; a.layer = layer;
+    a.wait_first = hy3a_take_fresh(ctx);
     a.early_prefetch = 0;
     hy3a_cache_view cv = hy3a_view(ctx);
     hy3a_batch_view bv = hy3a_bview(ctx);

@@ -39,6 +39,7 @@ struct hy3a_decode_args {
     /* fused step (fused != 0): the kernel itself normalises + rotates the queries read from q_in and
      * the CTA that streams the page of the newest slot quantises and appends the new K / V row   */
     int fused;
+    int wait_first;       /* the preceding kernel may be the one that writes the batch descriptor */
     int early_prefetch;   /* pages below the newest slots may be fetched before griddepcontrol.wait */
     const float *q_in, *k_in, *v_in;
     size_t qi_stride, ki_stride, vi_stride;

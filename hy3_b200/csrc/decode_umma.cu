@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
     const int qw = warp - kQkWarp0, qtid = tid - kQkWarp0 * 32;      /* score-warp numbering (negative for the other roles) */
     const bool is_qk = warp >= kQkWarp0;
 
+    if (a.wait_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     /* ---- prologue: everything here reads only what the host wrote.  The loads are issued together. */
     const int rl_d0 = (lane >> 4) * 64 + (lane & 15) * 4;
     float4 pre_w = make_float4(1.f, 1.f, 1.f, 1.f), pre_f = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -280,3 +280,69 @@ def test_chunk_kernel_head_groups(cuda, oracle, dt, n, heads, slot0, monkeypatch
         ctx.close()
     for what, a, b in zip(("queries", "attention", "K slots", "V slots"), *res):
         assert np.array_equal(a, b), what
+
+
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 336, 337, 600])
+def test_batch_descriptor_forms(cuda, oracle, n):
+    """The batch descriptor reaches the device as a row range, by value (up to 32 or 336 rows) or as a copy: the same tokens as a
+    range and in a shuffled order give the same cache and the same queries, with batches of other forms in between."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    q, k, v = (torch.from_numpy(oracle.fill_normal((n, h, 128), SEED, 700 + h)).to(cuda) for h in (64, 8, 9))
+    v = v[:, :8]
+    perm = np.random.default_rng(n).permutation(n)
+    got = []
+    for order in (np.arange(n), perm):
+        ctx = Hy3Attn(kv_dtype="int8", n_layers=1, max_seqs=2, max_batch=max(n, 40), max_tokens=n + 512, max_tokens_per_seq=n + 128)
+        ctx.batch_set([1] * 3, [5, 4, 9])
+        ctx.batch_set([0] * n, order, 3 * order if n % 2 else None)
+        idx = torch.from_numpy(np.asarray(order)).to(cuda)
+        qo = ctx.append(0, q[idx], k[idx], v[idx])
+        ctx.batch_set([1], [0])
+        ctx.sync()
+        back = torch.empty_like(qo)
+        back[idx] = qo
+        got.append((back, ctx.export_kv(0, 0, 0, n)))
+        ctx.close()
+    assert torch.equal(got[0][0], got[1][0])
+    assert all(np.array_equal(a, b) for a, b in zip(got[0][1], got[1][1]))
+
+
+@pytest.mark.parametrize("kv", ["int8", "fp16"])
+def test_batch_descriptor_is_not_overtaken(cuda, kv):
+    """Steps enqueued without waiting: every launch reads its own step's descriptor (the next one is written by a kernel that may
+    start before the last layer has ended).  Against the same steps with a synchronisation after every call."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(3)
+    steps, B = 40, 3
+    q, k, v = (torch.randn((steps, B, h, 128), device=cuda, generator=gen) for h in (64, 8, 8))
+    res = []
+    for wait in (False, True):
+        ctx = Hy3Attn(kv_dtype=kv, n_layers=2, max_seqs=B, max_batch=48, max_tokens=9000, max_tokens_per_seq=3000)
+        for layer in range(2):
+            for i in range(B):
+                ctx.fill_random(layer, i, 0, 2000, 10 * layer + i)
+        out = torch.zeros((steps, 2, B, 64, 128), device=cuda)
+        pre = torch.zeros((steps, 40, 64, 128), device=cuda)
+        q16 = torch.zeros((40, 64, 128), device=cuda, dtype=torch.float16)
+        torch.cuda.synchronize()
+        for t in range(steps):
+            lens = [100 + 40 * t, 1500 - 30 * t, 7 * t]
+            ctx.batch_set(np.arange(B), np.array(lens))
+            for layer in range(2):
+                ctx.decode_step(layer, q[t], k[t], v[t], out=out[t, layer])
+                if wait:
+                    ctx.sync()
+            if t % 4 == 0:      # a chunk on the first sequence, through the chunk kernel
+                m = 40
+                ctx.batch_set([0] * m, list(range(lens[0], lens[0] + m)))
+                ctx.append(0, q[:m, 0], k[:m, 0], v[:m, 0], q_out=False, q_out16=q16)
+                ctx.prefill(0, 0, lens[0], q16, out=pre[t])
+                if wait:
+                    ctx.sync()
+        ctx.sync()
+        res.append((out, pre))
+        ctx.close()
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
