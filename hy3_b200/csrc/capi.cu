@@ -139,7 +139,7 @@ int hy3a_decode_schedule_kv(int kv_dtype, int n, const int *kv_lens, int kv_head
         for (int r = 0; r < n; r++) {
             const long long p = pages_of(kv_lens[r]);
             if (p == 0) continue;
-            long long c = 1 + spare * p / U;
+            long long c = std::min<long long>(1 + spare * p / U, hy3a_most_pieces((unsigned)p));
             if (c > p) c = p;
             if ((p + c - 1) / c > worst) worst = (p + c - 1) / c;
         }
@@ -150,7 +150,7 @@ int hy3a_decode_schedule_kv(int kv_dtype, int n, const int *kv_lens, int kv_head
         for (int r = 0; r < n; r++) {
             const long long p = pages_of(kv_lens[r]);
             if (p == 0) continue;
-            long long c = L ? (p + L - 1) / L : 1 + spare * p / U;
+            long long c = L ? (p + L - 1) / L : std::min<long long>(1 + spare * p / U, hy3a_most_pieces((unsigned)p));
             if (c > p) c = p;
             if (cta < base + kv_heads * c) {
                 const long long idx = cta - base, hl = idx / c, k = idx % c, seg0 = kv_heads * pre + hl * p, late = c - HY3A_LATE;

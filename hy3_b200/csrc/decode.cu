@@ -402,6 +402,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             const int p = s_prefix[r + 1] - s_prefix[r];
             if (p == 0) continue;
             int c = L ? (p + (int)L - 1) / (int)L : 1 + (int)(spare * p / (P * G));
+            if (!L) c = min(c, (int)hy3a_most_pieces((unsigned)p));
             c = c < p ? c : p;
             if (cta < base + G * c) {
                 const int idx = cta - base, hl = idx / c, k = idx % c;

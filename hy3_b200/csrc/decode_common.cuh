@@ -118,7 +118,7 @@ __device__ __forceinline__ bool aligned_split_balanced(const int *s_prefix, int 
     for (int r = lane; r < n; r += 32) {
         const unsigned p = (unsigned)(s_prefix[r + 1] - s_prefix[r]);
         if (p == 0) continue;
-        unsigned long long c = 1ull + spare * p / PG;
+        unsigned long long c = min(1ull + spare * p / PG, (unsigned long long)hy3a_most_pieces(p));
         if (c > p) c = p;
         const unsigned w = (unsigned)((p + c - 1ull) / c);
         worst = worst > w ? worst : w;

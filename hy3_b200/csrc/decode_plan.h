@@ -16,6 +16,13 @@ constexpr unsigned HY3A_LATE = 4, HY3A_LATE_CUT = 2;
 /* a second segment in a CTA (queries, fold, record: about 6 us) costs more than this many pages */
 constexpr unsigned HY3A_STRADDLE_PAGES = 5;
 
+/* Most pieces of a segment of p pages: every piece is a record to fetch and fold (0.11 us behind the last page), every page 0.57 us of
+ * its CTA, so beyond some sqrt(5 p) more pieces cost more than they save; this line stays near it from 100 to 3 000 pages.  It
+ * matters where few KV heads have many CTAs each.  us a layer without / with it, INT8, FP16, INT4:
+ *   1 head, 20 000 tokens  23.2 -> 10.7  28.1 -> 14.1  30.7 -> 13.1     1 head, 200 000  29.4 -> 26.3  45.2 -> 39.6  39.2 -> 27.3
+ *   2 heads, 60 000        19.9 -> 15.8  27.0 -> 25.5  24.6 -> 18.0     4 heads, 20 000  14.6 -> 11.4  19.7 -> 16.7  18.5 -> 13.4 */
+HY3A_HD unsigned hy3a_most_pieces(unsigned p) { return 24u + p / 32u; }
+
 /* Even pieces (FP16 / INT4 kernel): 2 to 32 rows with fewer than four CTAs per segment; four round well enough */
 HY3A_HD bool hy3a_even_applies(int n, int G, unsigned grid) {
     return n >= 2 && n <= 32 && (unsigned)(n * G) < grid && (unsigned)(n * G) * 4u > grid;

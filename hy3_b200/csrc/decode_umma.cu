@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         for (int r = 0; r < n && !found; r++) {
             const unsigned p = (unsigned)(s_prefix[r + 1] - s_prefix[r]);
             if (p == 0) continue;
-            unsigned c = 1u + spare * p / PG;
+            unsigned c = min(1u + spare * p / PG, hy3a_most_pieces(p));
             c = c < p ? c : p;
             if (cta < base + G * (int)c) {
                 const unsigned idx = (unsigned)(cta - base), hl = idx / c, k = idx - hl * c;
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         for (int r = 0; r < n && !found; r++) {
             const int p = s_prefix[r + 1] - s_prefix[r];
             if (p == 0) continue;
-            int c = 1 + (int)(spare * p / (P * G));
+            int c = min(1 + (int)(spare * p / (P * G)), (int)hy3a_most_pieces((unsigned)p));
             c = c < p ? c : p;
             if (cta < base + G * c) {
                 const int idx = cta - base, hl = idx / c, k = idx % c;

@@ -481,3 +481,24 @@ def test_decode_clusters_equal_the_grid(cuda, oracle, dt, lens, heads):
         Kf, Vf = (slots_to_float(oracle, x, dt) for x in res[0][4][i])
         want = oracle.attention(res[0][5][i].cpu().numpy(), Kf, Vf)
         check_attention(res[0][0][i, own].cpu().numpy(), want[own], "%s row %d of %d tokens" % (dt, i, lens[i]))
+
+
+@pytest.mark.parametrize("dt", ["fp16", "int8", "int4"])
+@pytest.mark.parametrize("n,heads", [(3201, (7, 1)), (20000, (3, 1)), (33000, (2, 2))])
+def test_decode_few_heads_long_row(cuda, oracle, dt, n, heads):
+    """Few KV heads with long rows: segments of as many pieces as their bound allows, on fewer CTAs than the GPU has."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    h0, nh = heads
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, kv_head_begin=h0, kv_head_count=nh, max_batch=1, max_tokens=n + 128)
+    ctx.fill_random(0, 0, 0, n, 31)
+    q = oracle.fill_normal((64, 128), SEED, 811)
+    ctx.batch_set([0], [n - 1])
+    outs = [ctx.decode(0, torch.from_numpy(q[None]).to(cuda)) for _ in range(5)]
+    ctx.sync()
+    ks, vs = ctx.export_kv(0, 0, 0, n)
+    ctx.close()
+    own = slice(8 * h0, 8 * (h0 + nh))
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    want = oracle.attention_f64(q, slots_to_float(oracle, ks, dt), slots_to_float(oracle, vs, dt)).astype(np.float32)
+    check_attention(outs[0][0, own].cpu().numpy(), want[own], "%s %d tokens, %d heads" % (dt, n, nh))

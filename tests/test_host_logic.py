@@ -175,3 +175,15 @@ def test_even_pieces_are_the_least_that_fit(dt):
         else:
             assert max(sizes) - min(sizes) <= 1
     assert seen > 20
+
+
+@pytest.mark.parametrize("dt", ["fp16", "int8", "int4"])
+@pytest.mark.parametrize("length,heads", [(128 * 24, 1), (128 * 25, 1), (20000, 1), (60000, 2), (33000, 4), (32768, 8), (1 << 20, 1), (1 << 20, 8)])
+def test_schedule_bounds_the_pieces_of_a_segment(dt, length, heads):
+    """A segment of p pages is cut into at most 24 + p / 32 pieces, evenly, and every page belongs to one of them."""
+    p = -(-length // 128)
+    ranges = [r for r in (decode_schedule([length], heads, 148, c, dt)[1:] for c in range(148)) if r[1] > r[0]]
+    assert len(ranges) == heads * min(1 + (148 - heads) // heads, 24 + p // 32, p)
+    assert ranges[0][0] == 0 and ranges[-1][1] == p * heads and all(a[1] == b[0] for a, b in zip(ranges, ranges[1:]))
+    sizes = [b - a for a, b in ranges]
+    assert max(sizes) - min(sizes) <= (1 if dt != "int8" else 4)      # INT8: the pieces that start late take two pages less
