@@ -463,16 +463,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             }
             continue;
         }
-        for (int e = tid; e < G * 8 * HY3A_D && !is_producer; e += kThreads) {
-            int hq = e / HY3A_D, d = e % HY3A_D;
-            if (a.user_partials) {
-                float *p = a.user_partials + ((size_t)i * G * 8 + hq) * HY3A_PARTIAL_FLOATS;
-                p[2 + d] = 0.f;
-                if (d == 0) { p[0] = -INFINITY; p[1] = 0.f; }
-            } else {
-                a.out[(size_t)i * a.out_stride + (size_t)(cache.kv_head_begin * 8 + hq) * HY3A_D + d] = 0.f;
-            }
-        }
+        if (!is_producer) HY3A_EMPTY_ROW(i, tid, kThreads);
     }
 
     if (idle && !SHARD && !CL) return;   /* sharded: idle CTAs may still own the fold of rows without local keys */

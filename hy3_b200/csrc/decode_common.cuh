@@ -220,6 +220,22 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatil
     return false;
 }
 /* ---- pieces both decode kernels use */
+/* a row without keys: zero output, or empty partial records {-inf, 0, 0...} (hy3_gpu.cu:197-199); `out`, `partials`: the row's owned heads */
+__device__ __forceinline__ void write_empty_row(float *out, float *partials, int G, int t, int threads) {
+#pragma unroll 1
+    for (int e = t; e < G * 8 * HY3A_D; e += threads) {
+        if (partials) {
+            float *rec = partials + (e / HY3A_D) * HY3A_PARTIAL_FLOATS;
+            rec[2 + e % HY3A_D] = 0.f;
+            if (e % HY3A_D == 0) { rec[0] = -INFINITY; rec[1] = 0.f; }
+        } else {
+            out[e] = 0.f;
+        }
+    }
+}
+#define HY3A_EMPTY_ROW(i, t, threads) \
+    write_empty_row(a.out + (size_t)(i) * a.out_stride + (size_t)cache.kv_head_begin * 8 * HY3A_D, \
+                    a.user_partials ? a.user_partials + (size_t)(i) * G * 8 * HY3A_PARTIAL_FLOATS : nullptr, G, t, threads)
 /* Clusters: the CL CTAs of a (row, KV head) segment take an equal share of its pages each and meet in shared memory.  Rank r finishes
  * heads [r 8 / CL, (r + 1) 8 / CL): every CTA stores its records of these heads into r's landing zone with st.async, whose bytes
  * r's mbarrier counts, so that there is no record in memory, no counter and no fetch. */

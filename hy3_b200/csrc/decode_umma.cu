@@ -363,7 +363,13 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         if (idle) u_begin = u_end = 0;
     }
     if (idle && !SHARD && !CL) {
-        /* nothing to do: give the tensor memory back and leave (sharded: idle CTAs may still own the fold of rows without local keys) */
+        /* No pages: give the tensor memory back and leave -- behind the rows without keys, which belong to idle CTAs as well, and, where
+         * no CTA has pages, behind the wait of CTA 0, so that such a launch too ends after the one before it (hy3a_batch_kernel relies
+         * on that).  (Sharded: idle CTAs may still own the fold of rows without local keys.) */
+        if (cta < n) asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll 1
+        for (int i = cta; i < n; i += gridDim.x)
+            if (s_prefix[i + 1] == s_prefix[i]) HY3A_EMPTY_ROW(i, tid, kUThreads);
         fence_before();
         __syncthreads();
         if (warp == kIssWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(mi.tmem), "n"(kSlots * 64) : "memory");
@@ -429,16 +435,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                 }
                 continue;
             }
-            for (int e = qtid; e < G * 8 * HY3A_D; e += kQkThreads) {
-                const int hq = e / HY3A_D, d = e % HY3A_D;
-                if (a.user_partials) {
-                    float *p = a.user_partials + ((size_t)i * G * 8 + hq) * HY3A_PARTIAL_FLOATS;
-                    p[2 + d] = 0.f;
-                    if (d == 0) { p[0] = -INFINITY; p[1] = 0.f; }
-                } else {
-                    a.out[(size_t)i * a.out_stride + (size_t)(cache.kv_head_begin * 8 + hq) * HY3A_D + d] = 0.f;
-                }
-            }
+            HY3A_EMPTY_ROW(i, qtid, kQkThreads);
         }
 
     if (!idle && warp == kProdWarp) {

@@ -502,3 +502,57 @@ def test_decode_few_heads_long_row(cuda, oracle, dt, n, heads):
     assert all(torch.equal(o, outs[0]) for o in outs)
     want = oracle.attention_f64(q, slots_to_float(oracle, ks, dt), slots_to_float(oracle, vs, dt)).astype(np.float32)
     check_attention(outs[0][0, own].cpu().numpy(), want[own], "%s %d tokens, %d heads" % (dt, n, nh))
+
+
+@pytest.mark.parametrize("dt", ["fp16", "int8", "int4"])
+@pytest.mark.parametrize("lens,heads", [([0], (0, 8)), ([0, 0, 0], (5, 3)), ([1, 0, 0], (0, 1)), ([20000] + [0] * 29, (3, 1))])
+def test_rows_without_keys_are_written(cuda, dt, lens, heads):
+    """A row with slot -1 gets zero outputs, or empty records {-inf, 0, 0...}, also where the CTA it belongs to has no pages, where no CTA
+    has any, and in a captured step whose rows lose their keys before the replay.  Buffers start as NaN; heads of others stay."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    h0, nh = heads
+    n = len(lens)
+    own = slice(8 * h0, 8 * (h0 + nh))
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, kv_head_begin=h0, kv_head_count=nh, max_seqs=n, max_batch=n, max_tokens=sum(lens) + 128 * n, max_tokens_per_seq=max(lens) + 128)
+    for i, m in enumerate(lens):
+        if m:
+            ctx.fill_random(0, i, 0, m, 7 + i)
+    q = torch.randn((n, 64, 128), device=cuda, generator=torch.Generator(cuda).manual_seed(1))
+
+    def fresh():
+        return torch.full((n, 64, 128), float("nan"), device=cuda), torch.full((n, 8 * nh, 130), float("nan"), device=cuda)
+
+    def check(out, part, empty):
+        assert not torch.isnan(out[:, own]).any() and not torch.isnan(part).any()
+        assert torch.isnan(out[:, :8 * h0]).all() and torch.isnan(out[:, 8 * (h0 + nh):]).all()
+        for i in range(n):
+            assert (i in empty) == (not out[i, own].any().item())
+            assert (i in empty) == (torch.isneginf(part[i, :, 0]).all().item() and not part[i, :, 1:].any().item())
+
+    ctx.batch_set(list(range(n)), [m - 1 for m in lens])
+    out, part = fresh()
+    ctx.decode(0, q, out=out)
+    ctx.decode(0, q, partials=part)
+    ctx.sync()
+    check(out, part, [i for i, m in enumerate(lens) if m == 0])
+    # captured with one key more in every row, replayed with these rows and with none that has keys
+    ctx.batch_set(list(range(n)), lens)
+    ctx.sync()
+    side, (g_out, g_part) = torch.cuda.Stream(), fresh()
+    ctx.set_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        ctx.decode(0, q, out=g_out)
+        ctx.decode(0, q, partials=g_part)
+    side.synchronize()
+    ctx.use_torch_stream()
+    for slots in ([m - 1 for m in lens], [-1] * n):
+        ctx.batch_set(list(range(n)), slots)
+        g_out.fill_(float("nan"))
+        g_part.fill_(float("nan"))
+        graph.replay()
+        ctx.sync()
+        check(g_out, g_part, [i for i, s in enumerate(slots) if s < 0])
+    del graph
+    ctx.close()
