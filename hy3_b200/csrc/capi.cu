@@ -67,6 +67,7 @@ cudaError_t launch_batch(hy3a_ctx *ctx, const B &b) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
     ctx->batch_fresh = 1;
+    if (hy3a_capturing(ctx)) ctx->batch_fresh_cap = 1;
     return cudaLaunchKernelEx(&cfg, hy3a_batch_kernel<B>, b, ctx->d_batch, ctx->cfg.max_batch);
 }
 
@@ -496,7 +497,7 @@ int hy3a_batch_set(hy3a_ctx *ctx, int n, const int *seq_ids, const int *slots, c
         int rc = stage_h2d(ctx, ctx->d_batch, tmp, 3 * mb * sizeof(int));
         free(tmp);
         if (rc) return rc;
-        ctx->batch_fresh = 0;      /* a copy: the next launch waits for it anyway */
+        (hy3a_capturing(ctx) ? ctx->batch_fresh_cap : ctx->batch_fresh) = 0;      /* a copy: the next launch waits for it anyway */
     }
     ctx->batch_n = n;
     ctx->batch_seq0 = seq_ids[0]; ctx->batch_slot0 = slots[0]; ctx->batch_contig = slots[0] >= 0;

@@ -104,6 +104,7 @@ struct hy3a_ctx {
     int batch_seq_uniform, batch_slot_min;       /* all rows belong to batch_seq0; lowest slot >= 0 of the batch */
     int decode_ctas;
     int batch_fresh;      /* the batch descriptor was written by a kernel and no kernel that reads it has been launched since */
+    int batch_fresh_cap;  /* the same within stream captures */
     int bulk_write_pending; /* a kernel that wrote many KV slots was enqueued and no decode launch has followed it yet */
     int use_pdl;          /* launch kernels with programmatic stream serialization (HY3A_NO_PDL=1 turns it off) */
     int cl_cap[4];        /* decode: clusters of 2^i CTAs that fit on the device at once */
@@ -169,9 +170,24 @@ static inline hy3a_batch_view hy3a_bview(const hy3a_ctx *c) {
     return b;
 }
 
+/* whether launches on the context's stream are being captured (or the stream cannot be asked, as the default stream during another's capture) */
+static inline bool hy3a_capturing(const hy3a_ctx *c) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) { cudaGetLastError(); return true; }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 /* The decode and append kernels read the batch descriptor before they wait for the preceding kernel.  The first of them behind
- * hy3a_batch_set has to wait first; those after it find a predecessor that started when the descriptor was complete. */
-static inline int hy3a_take_fresh(hy3a_ctx *c) { const int f = c->batch_fresh; c->batch_fresh = 0; return f; }
+ * hy3a_batch_set has to wait first; those after it find a predecessor that started when the descriptor was complete.  A captured
+ * launch does not run now and cannot be that predecessor: it leaves the flag to the next launch that does.  A replayed graph starts
+ * behind everything enqueued before it, so a captured launch itself waits only for a descriptor kernel of its own capture. */
+static inline int hy3a_take_fresh(hy3a_ctx *c) {
+    if (!c->batch_fresh && !c->batch_fresh_cap) return 0;
+    int &flag = hy3a_capturing(c) ? c->batch_fresh_cap : c->batch_fresh;
+    const int f = flag;
+    flag = 0;
+    return f;
+}
 
 #define HY3A_CUDA(ctx, call)                                                                                   \
     do {                                                                                                       \

@@ -1126,9 +1126,7 @@ static int decode_cluster(const hy3a_ctx *ctx) {
     if ((ctx->shard_slot >= 0 && ctx->shard_world > 1) || ctx->decode_ctas < ctx->sm_count) return 0;      /* a world of one has nothing to exchange */
     const int cl = cluster_size(ctx, ctx->batch_pages, ctx->batch_pages_all);
     if (!cl) return 0;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) { cudaGetLastError(); st = cudaStreamCaptureStatusActive; }
-    if (st == cudaStreamCaptureStatusNone) return cl;
+    if (!hy3a_capturing(ctx)) return cl;
     return cluster_size(ctx, ctx->cfg.max_blocks_per_seq, (long long)ctx->cfg.max_blocks_per_seq * ctx->batch_n);
 }
 

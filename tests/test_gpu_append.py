@@ -346,3 +346,68 @@ def test_batch_descriptor_is_not_overtaken(cuda, kv):
         res.append((out, pre))
         ctx.close()
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+
+
+@pytest.mark.parametrize("kv", ["int8", "fp16", "int4"])
+def test_captured_step_leaves_the_descriptor_to_the_next(cuda, kv):
+    """A step captured between a batch descriptor and an eager step does not run, so the eager step is the one that has to wait for the
+    descriptor: work queued in front keeps all of it in flight.  Then the graph, which must follow the descriptors set before each
+    replay, and a capture that holds the descriptor itself.  Against the same steps with a synchronisation after every call."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(4)
+    lens = [1500, 40, 700]
+    q, k, v = (torch.randn((3, h, 128), device=cuda, generator=gen) for h in (64, 8, 8))
+    res = []
+    for wait in (False, True):
+        ctx = Hy3Attn(kv_dtype=kv, n_layers=2, max_seqs=3, max_batch=3, max_tokens=9000, max_tokens_per_seq=3000)
+        for layer in range(2):
+            for i in range(3):
+                ctx.fill_random(layer, i, 0, 2000, 10 * layer + i)
+        out = torch.zeros((8, 3, 64, 128), device=cuda)
+        g_out = torch.zeros((3, 64, 128), device=cuda)
+        torch.cuda.synchronize()
+        side, kept = torch.cuda.Stream(), []
+        ctx.set_stream(side)
+
+        def done():
+            if wait:
+                side.synchronize()
+
+        with torch.cuda.stream(side):
+            for t in range(2):
+                torch.cuda._sleep(20000000)
+                ctx.batch_set([0, 1, 2], [n - 7 * t for n in lens])
+                done()
+                graph = torch.cuda.CUDAGraph()
+                kept.append(graph)
+                graph.capture_begin(capture_error_mode="thread_local")
+                ctx.decode_step(0, q, k, v, out=g_out)
+                graph.capture_end()
+                ctx.decode_step(1, q, k, v, out=out[4 * t])
+                done()
+                ctx.batch_set([0, 1, 2], [n + 9 + t for n in lens])
+                done()
+                graph.replay()
+                done()
+                out[4 * t + 1].copy_(g_out)
+                done()
+                own = torch.cuda.CUDAGraph()
+                kept.append(own)
+                own.capture_begin(capture_error_mode="thread_local")
+                ctx.batch_set([0, 1, 2], [30 + n for n in lens])
+                ctx.decode_step(0, q, k, v, out=g_out)
+                ctx.decode_step(1, q, k, v, out=out[4 * t + 2])
+                own.capture_end()
+                own.replay()
+                done()
+                out[4 * t + 3].copy_(g_out)
+                done()
+        side.synchronize()
+        ctx.use_torch_stream()
+        ctx.sync()
+        res.append(out)
+        del graph, own, kept
+        ctx.close()
+    assert torch.equal(res[0], res[1])
