@@ -261,11 +261,7 @@ int hy3a_create(const hy3a_config *cfg, hy3a_ctx **out) {
         const char *e = getenv("HY3A_DECODE_STAGES");
         if (e) { int v = atoi(e); if (v < ctx->decode_stages) ctx->decode_stages = v; }
     }
-    struct device_guard {   /* the caller's current device is put back on every way out */
-        int prev;
-        device_guard() : prev(-1) { cudaGetDevice(&prev); }
-        ~device_guard() { if (prev >= 0) cudaSetDevice(prev); }
-    } guard;
+    hy3a_device_guard guard(dev);   /* the caller's current device is put back on every way out */
     CREATE_CUDA(cudaSetDevice(dev));
     CREATE_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     ctx->own_stream = 1;
@@ -467,9 +463,19 @@ int hy3a_seq_capacity(hy3a_ctx *ctx, int seq) {
 }
 int hy3a_free_blocks(hy3a_ctx *ctx) { return ctx ? ctx->n_free : HY3A_EINVAL; }
 
+static int check_device(hy3a_ctx *ctx, const char *who) {
+    int cur = -1;
+    if (cudaGetDevice(&cur) != cudaSuccess || cur != ctx->device)
+        return hy3a_fail(ctx, HY3A_ESTATE, "%s: the context lives on device %d but device %d is current (cudaSetDevice first)", who, ctx->device, cur);
+    return 0;
+}
 int hy3a_batch_set(hy3a_ctx *ctx, int n, const int *seq_ids, const int *slots, const int *rope_pos) {
     if (!ctx || !seq_ids || !slots || !rope_pos) return hy3a_fail(ctx, HY3A_EINVAL, "batch_set: NULL argument");
     if (n < 1 || n > ctx->cfg.max_batch) return hy3a_fail(ctx, HY3A_EINVAL, "batch_set: n=%d not in [1,%d]", n, ctx->cfg.max_batch);
+    /* A kernel goes to the current device.  Any may be current where the stream says which one is meant; a default stream is the
+     * current device's. */
+    if ((uintptr_t)ctx->stream <= (uintptr_t)cudaStreamPerThread) { int rc = check_device(ctx, "batch_set"); if (rc) return rc; }
+    hy3a_device_guard guard(ctx->device);
     for (int i = 0; i < n; i++) {
         if (seq_ids[i] < 0 || seq_ids[i] >= ctx->cfg.max_seqs) return hy3a_fail(ctx, HY3A_EINVAL, "batch_set: row %d seq %d out of range", i, seq_ids[i]);
         if (slots[i] < -1) return hy3a_fail(ctx, HY3A_EINVAL, "batch_set: row %d slot %d < -1", i, slots[i]);
@@ -521,10 +527,7 @@ static int check_layer(hy3a_ctx *ctx, int layer, const char *who) {
     if (!ctx) return HY3A_EINVAL;
     if (layer < 0 || layer >= ctx->cfg.n_layers) return hy3a_fail(ctx, HY3A_EINVAL, "%s: layer %d out of range [0,%d)", who, layer, ctx->cfg.n_layers);
     if (ctx->batch_n < 1) return hy3a_fail(ctx, HY3A_ESTATE, "%s: no batch set (call hy3a_batch_set first)", who);
-    int cur = -1;
-    if (cudaGetDevice(&cur) != cudaSuccess || cur != ctx->device)
-        return hy3a_fail(ctx, HY3A_ESTATE, "%s: the context lives on device %d but device %d is current (cudaSetDevice first)", who, ctx->device, cur);
-    return 0;
+    return check_device(ctx, who);
 }
 
 int hy3a_append(hy3a_ctx *ctx, int layer, const float *q_in, size_t q_stride, const float *k_in, size_t k_stride, const float *v_in,
@@ -665,6 +668,8 @@ int hy3a_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq, const
     if (base_slot < 0 || nq < 1) return hy3a_fail(ctx, HY3A_EINVAL, "prefill: base_slot=%d nq=%d", base_slot, nq);
     if (base_slot + nq > ctx->h_seq_blocks[seq] * HY3A_PAGE_TOKENS) return hy3a_fail(ctx, HY3A_ESTATE, "prefill: keys [0,%d) are not all appended", base_slot + nq);
     if (!q16 || !out || (((uintptr_t)q16 | (uintptr_t)out) & 15) || (out_stride & 3)) return hy3a_fail(ctx, HY3A_EINVAL, "prefill: bad pointer");
+    int rc = check_device(ctx, "prefill");
+    if (rc) return rc;
     return hy3a_launch_prefill(ctx, layer, seq, base_slot, nq, q16, out, out_stride);
 }
 

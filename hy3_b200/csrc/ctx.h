@@ -170,6 +170,14 @@ static inline hy3a_batch_view hy3a_bview(const hy3a_ctx *c) {
     return b;
 }
 
+/* makes the context's device current and puts the caller's back */
+struct hy3a_device_guard {
+    int prev;
+    bool moved;
+    explicit hy3a_device_guard(int dev) : prev(-1), moved(false) { if (cudaGetDevice(&prev) != cudaSuccess || prev != dev) moved = cudaSetDevice(dev) == cudaSuccess && prev >= 0; }
+    ~hy3a_device_guard() { if (moved) cudaSetDevice(prev); }
+};
+
 /* whether launches on the context's stream are being captured (or the stream cannot be asked, as the default stream during another's capture) */
 static inline bool hy3a_capturing(const hy3a_ctx *c) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;

@@ -822,6 +822,7 @@ static void plan_chunk(hy3a_ctx *ctx, const int *cap, int base_slot, int nq) {
 extern "C" int hy3a_prefill_cluster(hy3a_ctx *ctx, int base_slot, int nq) {
     if (!ctx) return HY3A_EINVAL;
     if (base_slot < 0 || nq < 1) return hy3a_fail(ctx, HY3A_EINVAL, "prefill_cluster: base_slot %d, nq %d", base_slot, nq);
+    hy3a_device_guard guard(ctx->device);      /* a query: any device may be current */
     const int *cap = NULL;
     int rc = prefill_device(ctx, &cap);
     if (rc) return rc;

@@ -411,3 +411,39 @@ def test_captured_step_leaves_the_descriptor_to_the_next(cuda, kv):
         del graph, own, kept
         ctx.close()
     assert torch.equal(res[0], res[1])
+
+
+def test_calls_with_another_device_current(cuda):
+    """batch_set launches a kernel: with another device current it goes to the context's device where the stream names it, and is refused
+    on a default stream; the prefill's cluster query answers for the context's device; prefill is refused as append and decode are.
+    (Two GPUs: skipped where the box has one.)"""
+    import torch
+    from hy3_b200 import Hy3Attn, Hy3AttnError
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    ctx = Hy3Attn(kv_dtype="int8", n_layers=1, max_batch=64, max_tokens=1024, device=0)
+    ctx.fill_random(0, 0, 0, 600, 3)
+    q16 = torch.randn((45, 64, 128), device="cuda:0").half()
+    q = torch.randn((1, 64, 128), device="cuda:0")
+    ctx.sync()
+    with torch.cuda.device(1):
+        with pytest.raises(Hy3AttnError):
+            ctx.batch_set([0], [500])
+        cluster = ctx.prefill_cluster(500, 45)
+        with pytest.raises(Hy3AttnError):
+            ctx.prefill(0, 0, 500, q16, out=torch.zeros((45, 64, 128), device="cuda:0"))
+        side = torch.cuda.Stream(device=0)
+        ctx.set_stream(side)
+        ctx.batch_set([0], [500])
+        assert torch.cuda.current_device() == 1
+    assert cluster == ctx.prefill_cluster(500, 45) > 1
+    with torch.cuda.stream(side):
+        got = ctx.decode(0, q)
+    side.synchronize()
+    ctx.use_torch_stream()
+    ctx.batch_set([0], [500])
+    want = ctx.decode(0, q)
+    ctx.prefill(0, 0, 500, q16)
+    ctx.sync()
+    assert torch.equal(got, want)
+    ctx.close()
