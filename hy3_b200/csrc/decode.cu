@@ -50,13 +50,17 @@ constexpr int kWarps = HY3A_DECODE_WARPS;              /* consumer warps */
 static_assert(kWarps >= 11, "eight warps for the queries and the reductions, one each for the new V row's scale and the new K and V rows");
 constexpr int kThreads = kWarps * 32;
 constexpr int kFixedO = kWarps * 8 * HY3A_D * 4;
-constexpr int kFixedML = ((kWarps * 8 * 2 * 4) + 127) / 128 * 128;
+constexpr int kFixedML = kWarps * 8 * 2 * 4;
 constexpr int kFixedQ = 8 * 32 * 16;
 constexpr int kFixedNew = 2 * HY3A_D * 4;
-constexpr int kBarBytes = 256;      /* mbarriers of the page ring: empty[8], full[16]; of a cluster's meeting: 1 */
+constexpr int kFixedHead = kFixedO + kFixedML + kFixedQ + kFixedNew;      /* every variant's; a cluster's landing zone follows */
+/* bytes of shared memory in front of the page-count prefix (a multiple of 128), and of the mbarriers behind it: the page ring's empty[8]
+ * and full[16], a cluster's meeting.  The ring starts on 128 bytes.  Nothing is padded further: a context's largest batch is what
+ * the prefix has room for beside two pages (FP16: 12 543 rows). */
+template <int CL> constexpr int kFixed = kFixedHead + (CL ? kCluBytes : 0);
+template <int CL> constexpr int kBarBytes = CL ? 320 : 192;
 constexpr int kBarClu = 192;
-constexpr int kFixedClu = (kCluBytes + 127) / 128 * 128;
-constexpr int kFixed = kFixedO + kFixedML + kFixedQ + kFixedNew + kFixedClu;   /* bytes of shared memory in front of the page-count prefix */
+static_assert(kFixedML % 16 == 0 && kFixedHead % 16 == 0 && (kFixed<0> + kBarBytes<0>) % 128 == 0 && (kFixed<2> + kBarBytes<2>) % 128 == 0, "alignment of the shared-memory map");
 static_assert(16 / 8 * 8 >= 8 + 3 && 16 / 7 * 7 >= 7 + 3 && 16 / 6 * 6 >= 6 + 3 && kWarps <= 12, "rounds of the full barriers: see the consumer loop");
 constexpr bool kPSplit = true;                         /* carry the fp16 residual of P in MMA rows 8-15 */
 constexpr int kRecFloats = HY3A_REC_FLOATS;             /* floats per head record in the merge scratch (130 used) */
@@ -318,7 +322,7 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
 /* CL: 0 = any grid, 2 / 4 / 8 = a cluster of CL CTAs per (row, KV head) */
 template <int DT, bool STAGED, bool SHARD = false, int CL = 0>
 __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_kernel(hy3a_cache_view cache, hy3a_batch_view batch, decode_args a) {
-    /* dynamic shared memory: [s_o | s_ml | s_q | s_new | page-count prefix | full[8] empty[8] | ring of pages] */
+    /* dynamic shared memory: [s_o | s_ml | s_q | s_new | a cluster's landing zone | page-count prefix | empty[8] full[16] meeting | ring of pages] */
     extern __shared__ __align__(128) uint8_t s_dyn[];
     float (*s_o)[8][HY3A_D] = reinterpret_cast<float (*)[8][HY3A_D]>(s_dyn);                       /* per-warp unnormalised outputs */
     float (*s_ml)[8][2] = reinterpret_cast<float (*)[8][2]>(s_dyn + kFixedO);                      /* per-warp {m, l} */
@@ -335,9 +339,9 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
     const int n = batch.n, G = cache.kv_heads;
     const int cta = blockIdx.x;
 
-    int *s_prefix = reinterpret_cast<int *>(s_dyn + kFixed);
-    const unsigned bar_base = smem_u32(s_dyn + kFixed + a.prefix_bytes);
-    const unsigned ring_base = bar_base + kBarBytes;
+    int *s_prefix = reinterpret_cast<int *>(s_dyn + kFixed<CL>);
+    const unsigned bar_base = smem_u32(s_dyn + kFixed<CL> + a.prefix_bytes);
+    const unsigned ring_base = bar_base + kBarBytes<CL>;
 
     if (a.wait_first) asm volatile("griddepcontrol.wait;" ::: "memory");
     /* ---- schedule: prefix of pages per row */
@@ -709,7 +713,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                      * the page in HBM (for later steps). */
                     const int tok = (sg.len - 1) & 127;
                     uint8_t *gp = cache.pool + hy3a_page_index(cache, new_block, a.layer, hl) * (size_t)cache.page_bytes;
-                    uint8_t *sp = s_dyn + kFixed + a.prefix_bytes + kBarBytes + (size_t)stage * geom.page_bytes;
+                    uint8_t *sp = s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + (size_t)stage * geom.page_bytes;
                     float4 r4 = *reinterpret_cast<const float4 *>(&s_new[0][rl_d0]);
                     float y[4] = {r4.x, r4.y, r4.z, r4.w};
                     hy3a_rowops::store_row<DT>(sp, geom, tok, false, y, rl_d0, lane);
@@ -763,7 +767,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             acc[0] += o4.x * f; acc[1] += o4.y * f; acc[2] += o4.z * f; acc[3] += o4.w * f;
         }
         if (CL) {
-            if (red) cluster_send<CL ? CL : 1>(smem_u32(s_dyn) + kFixed - kFixedClu, bar_base + kBarClu, cta % (CL ? CL : 1), h, lane, M, L, acc);
+            if (red) cluster_send<CL ? CL : 1>(smem_u32(s_dyn) + kFixedHead, bar_base + kBarClu, cta % (CL ? CL : 1), h, lane, M, L, acc);
             break;
         }
         consumer_sync(); /* s_o / s_ml free again */
@@ -828,7 +832,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                     }
                     asm volatile("cp.async.wait_all;" ::: "memory");
                     __syncwarp();
-                    const float *zf = reinterpret_cast<const float *>(s_dyn + kFixed + a.prefix_bytes + kBarBytes + zone);
+                    const float *zf = reinterpret_cast<const float *>(s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + zone);
                     for (int c = 0; c < npieces; c++) {
                         const float *pr = zf + (size_t)c * kRecFloats;
                         const float pm = pr[0], pl = pr[1];
@@ -914,7 +918,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 if (STAGED && aligned && (size_t)a.stages * geom.page_bytes >= (size_t)8 * 8 * kShardLines * 16) {
                     /* CTA-aligned segments: the page ring is idle by now and holds all 8 ranks' records at once, so
                      * every rank is polled in the same round */
-                    fa.stage = reinterpret_cast<const uint4 *>(s_dyn + kFixed + a.prefix_bytes + kBarBytes);
+                    fa.stage = reinterpret_cast<const uint4 *>(s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL>);
                     shard_fold<8>(fa);
                 } else {
                     shard_fold<kShardBatch>(fa);
@@ -940,11 +944,11 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         constexpr int C1 = CL ? CL : 1, HPC = 8 / C1;
         const int rank = cta % C1, seg = cta / C1, row = seg / G, hl = seg - row * G;
         const float none[4] = {0.f, 0.f, 0.f, 0.f};
-        if (idle && warp < 8) cluster_send<C1>(smem_u32(s_dyn) + kFixed - kFixedClu, bar_base + kBarClu, rank, warp, lane, -INFINITY, 0.f, none);
+        if (idle && warp < 8) cluster_send<C1>(smem_u32(s_dyn) + kFixedHead, bar_base + kBarClu, rank, warp, lane, -INFINITY, 0.f, none);
         if (warp < HPC) {
             mbar_wait(bar_base + kBarClu, 0u, &s_abort, a.err, 70u);
             float M, Ls, acc[4];
-            cluster_fold<C1>(s_dyn + kFixed - kFixedClu, warp, lane, M, Ls, acc);
+            cluster_fold<C1>(s_dyn + kFixedHead, warp, lane, M, Ls, acc);
             cluster_write(a, G, cache.kv_head_begin, row, hl * 8 + rank * HPC + warp, lane, M, Ls, acc);
         }
         /* a CTA's shared memory stays until every CTA of the cluster has sent (they have, unless a wait ran out) */
@@ -995,6 +999,11 @@ __global__ void hy3a_merge_kernel(const float *partials, int n_parts, int n_rows
 
 } /* namespace */
 
+/* a launch's shared memory */
+static size_t prefix_bytes(int rows) { return ((size_t)(rows + 1) * sizeof(int) + 127) & ~(size_t)127; }
+template <int CL>
+static size_t decode_smem(size_t prefix, size_t ring) { return kFixed<CL> + prefix + kBarBytes<CL> + ring; }
+
 template <int DT>
 static const void *decode_cluster_fn(int cl) {
     return cl == 2 ? (const void *)hy3a_decode_kernel<DT, true, false, 2> : cl == 4 ? (const void *)hy3a_decode_kernel<DT, true, false, 4> : (const void *)hy3a_decode_kernel<DT, true, false, 8>;
@@ -1028,7 +1037,7 @@ int hy3a_cluster_cap(const void *fn, int cl, int threads, size_t smem) {
 }
 
 void hy3a_decode_cluster_init(hy3a_ctx *ctx) {
-    const size_t prefix = ((size_t)(ctx->cfg.max_batch + 1) * sizeof(int) + 127) & ~(size_t)127, smem = kFixed + prefix + kBarBytes + (size_t)ctx->decode_stages * ctx->geom.page_bytes;
+    const size_t smem = decode_smem<2>(prefix_bytes(1), ctx->decode_stages * (size_t)ctx->geom.page_bytes);      /* one CTA per SM at any batch: its registers fill more than half */
     for (int i = 1; i < 4; i++) {
         if (ctx->decode_stages < 2) ctx->cl_cap[i] = 0;
         else if (ctx->geom.dtype == HY3A_KV_INT8) ctx->cl_cap[i] = hy3a_decode_umma_cluster_cap(ctx, 1 << i);
@@ -1038,7 +1047,7 @@ void hy3a_decode_cluster_init(hy3a_ctx *ctx) {
 
 template <int DT>
 static cudaError_t launch_decode_dt(hy3a_ctx *ctx, const hy3a_cache_view &cv, const hy3a_batch_view &bv, decode_args &a) {
-    const size_t prefix = ((size_t)(ctx->batch_n + 1) * sizeof(int) + 127) & ~(size_t)127;
+    const size_t prefix = prefix_bytes(ctx->batch_n);
     dim3 grid(ctx->decode_ctas);
     static bool attr_dev[64][3][3];   /* function attributes are per device: [device ordinal][cache type][variant] */
     bool (*attr_set)[3] = attr_dev[ctx->device & 63];
@@ -1047,11 +1056,11 @@ static cudaError_t launch_decode_dt(hy3a_ctx *ctx, const hy3a_cache_view &cv, co
         a.stages = ctx->decode_stages;
         void *args[3] = {(void *)&cv, (void *)&bv, (void *)&a};
         return hy3a_launch_cluster(ctx, decode_cluster_fn<DT>(a.cluster), a.cluster, ctx->batch_n * ctx->cfg.kv_head_count, kThreads + 32,
-                                   kFixed + prefix + kBarBytes + (size_t)a.stages * ctx->geom.page_bytes, args);
+                                   decode_smem<2>(prefix, a.stages * (size_t)ctx->geom.page_bytes), args);
     }
     if (ctx->decode_stages >= 2) {
         a.stages = ctx->decode_stages;
-        const size_t smem = kFixed + prefix + kBarBytes + (size_t)a.stages * ctx->geom.page_bytes;
+        const size_t smem = decode_smem<0>(prefix, a.stages * (size_t)ctx->geom.page_bytes);
         const bool shard = a.n_dest > 0;
         if (!attr_set[DT][shard ? 2 : 1]) {
             cudaError_t e = shard ? cudaFuncSetAttribute(hy3a_decode_kernel<DT, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax)
@@ -1074,15 +1083,14 @@ static cudaError_t launch_decode_dt(hy3a_ctx *ctx, const hy3a_cache_view &cv, co
             if (e != cudaSuccess) return e;
             attr_set[DT][0] = true;
         }
-        hy3a_decode_kernel<DT, false><<<grid, kThreads, kFixed + prefix + kBarBytes, ctx->stream>>>(cv, bv, a);
+        hy3a_decode_kernel<DT, false><<<grid, kThreads, decode_smem<0>(prefix, 0), ctx->stream>>>(cv, bv, a);
     }
     return cudaGetLastError();
 }
 
 /* Pages that fit in the ring for a given page size and batch capacity. */
 int hy3a_decode_ring_capacity(int page_bytes, int max_batch) {
-    const size_t prefix = ((size_t)(max_batch + 1) * sizeof(int) + 127) & ~(size_t)127;
-    long room = (long)kSmemMax - (long)kFixed - (long)prefix - kBarBytes;
+    long room = (long)kSmemMax - (long)decode_smem<0>(prefix_bytes(max_batch), 0);
     int s = room > 0 ? (int)(room / page_bytes) : 0;
     return s > 8 ? 8 : s;
 }
@@ -1117,6 +1125,8 @@ static int cluster_size(const hy3a_ctx *ctx, int most, long long total) {
     static const int kPagesCta[3] = {1, 5, 4}, kPagesFold[3] = {2, 5, 8};      /* FP16, INT8, INT4 */
     const int dt = ctx->geom.dtype, segs = ctx->batch_n * ctx->cfg.kv_head_count;
     if (most < 2 || segs > ctx->cl_cap[1]) return 0;
+    /* a ring that a context of very large batches has sized to the last byte leaves no room for the landing zone */
+    if (dt != HY3A_KV_INT8 && decode_smem<2>(prefix_bytes(ctx->batch_n), ctx->decode_stages * (size_t)ctx->geom.page_bytes) > (size_t)kSmemMax) return 0;
     int i = 1;
     while (i < 3 && ((most - 1) >> i) + 1 > kPagesCta[dt] && segs <= ctx->cl_cap[i + 1]) i++;
     const long long share = (total * ctx->cfg.kv_head_count + ctx->decode_ctas - 1) / ctx->decode_ctas;

@@ -61,7 +61,7 @@ cudaError_t hy3a_launch_decode_umma(hy3a_ctx *ctx, const hy3a_cache_view &cv, co
 
 namespace {
 
-constexpr int kSmemMax = 232448 - 1024;                /* opt-in limit per block minus the driver's reserve */
+constexpr int kSmemMax = 232448 - 128;                 /* opt-in limit per block minus the 128 bytes that hy3a_decode_kernel declares statically */
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 

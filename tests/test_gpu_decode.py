@@ -556,3 +556,24 @@ def test_rows_without_keys_are_written(cuda, dt, lens, heads):
         check(g_out, g_part, [i for i, s in enumerate(slots) if s < 0])
     del graph
     ctx.close()
+
+
+def test_largest_batch_keeps_the_page_ring(cuda):
+    """The largest FP16 batch whose page counts fit beside a ring of two pages: the fused step needs no q_out there (it does without a
+    ring), and rows at both ends equal those of a small context (the two differ by the order of fp32 sums: 2e-5, as between cluster
+    and grid)."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    n = 12543
+    rows = [0, 1, 6000, n - 2, n - 1]
+    slots = np.arange(n) % 260
+    q = torch.randn((n, 64, 128), device=cuda, generator=torch.Generator(cuda).manual_seed(2))
+    res = []
+    for idx in (np.arange(n), np.array(rows)):
+        ctx = Hy3Attn(kv_dtype="fp16", n_layers=1, max_batch=len(idx), max_tokens=384)
+        ctx.fill_random(0, 0, 0, 384, 5)
+        ctx.batch_set([0] * len(idx), slots[idx], idx)
+        res.append(ctx.decode_step(0, q[torch.from_numpy(idx).to(cuda)], None, None))
+        ctx.sync()
+        ctx.close()
+    assert torch.isfinite(res[0]).all() and (res[0][rows] - res[1]).abs().max() < 2e-5
