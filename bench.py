@@ -613,8 +613,8 @@ def run_ours(args):
         ctx.batch_set([0], [local_slot], [global_pos])
 
     stream.synchronize()
-    launches_before = ctx.launches
     set_positions(0)
+    launches_before = ctx.launches
     with torch.cuda.stream(stream):
         enqueue_step()                                # eager warm-up (also warms NCCL)
     stream.synchronize()

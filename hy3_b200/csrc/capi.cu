@@ -68,6 +68,7 @@ cudaError_t launch_batch(hy3a_ctx *ctx, const B &b) {
     cfg.attrs = attr; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
     ctx->batch_fresh = 1;
     if (hy3a_capturing(ctx)) ctx->batch_fresh_cap = 1;
+    ctx->launches++;
     return cudaLaunchKernelEx(&cfg, hy3a_batch_kernel<B>, b, ctx->d_batch, ctx->cfg.max_batch);
 }
 

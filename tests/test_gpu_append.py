@@ -20,6 +20,11 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 POS = [0, 1, 2, 63, 64, 127, 128, 129, 4095, 4096, 32767, 262143, 262144, 1048575, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14]
 
 
+def torch_rows(cuda, n, heads, seed=1):
+    import torch
+    return torch.randn((n, heads, 128), device=cuda, generator=torch.Generator(cuda).manual_seed(seed + heads))
+
+
 def run_append(cuda, oracle, dt, eps, q, k, v, qw, kw, pos, table=None, probes=(1, 0, 0)):
     import torch
     from hy3_b200 import Hy3Attn
@@ -306,6 +311,22 @@ def test_batch_descriptor_forms(cuda, oracle, n):
         ctx.close()
     assert torch.equal(got[0][0], got[1][0])
     assert all(np.array_equal(a, b) for a, b in zip(got[0][1], got[1][1]))
+
+
+def test_launch_count_includes_the_descriptor_kernel(cuda):
+    """Every kernel counts: the one that carries a descriptor as well; a descriptor that is copied is none."""
+    from hy3_b200 import Hy3Attn
+    ctx = Hy3Attn(kv_dtype="int8", n_layers=1, max_batch=400, max_tokens=512)
+    for n in (1, 400):
+        before = ctx.launches
+        ctx.batch_set([0] * n, list(range(n)))
+        ctx.append(0, *(torch_rows(cuda, n, h) for h in (64, 8, 8)))
+        assert ctx.launches - before == 2
+    before = ctx.launches
+    ctx.batch_set([0] * 400, list(range(399, -1, -1)))
+    assert ctx.launches == before
+    ctx.sync()
+    ctx.close()
 
 
 @pytest.mark.parametrize("kv", ["int8", "fp16"])
