@@ -105,6 +105,7 @@ struct hy3a_ctx {
     int decode_ctas;
     int batch_fresh;      /* the batch descriptor was written by a kernel and no kernel that reads it has been launched since */
     int batch_fresh_cap;  /* the same within stream captures */
+    int batch_unread;     /* no launch outside a capture has read the batch descriptor: the step is replayed from a graph */
     int bulk_write_pending; /* a kernel that wrote many KV slots was enqueued and no decode launch has followed it yet */
     int use_pdl;          /* launch kernels with programmatic stream serialization (HY3A_NO_PDL=1 turns it off) */
     int cl_cap[4];        /* decode: clusters of 2^i CTAs that fit on the device at once */
@@ -190,10 +191,12 @@ static inline bool hy3a_capturing(const hy3a_ctx *c) {
  * launch does not run now and cannot be that predecessor: it leaves the flag to the next launch that does.  A replayed graph starts
  * behind everything enqueued before it, so a captured launch itself waits only for a descriptor kernel of its own capture. */
 static inline int hy3a_take_fresh(hy3a_ctx *c) {
-    if (!c->batch_fresh && !c->batch_fresh_cap) return 0;
-    int &flag = hy3a_capturing(c) ? c->batch_fresh_cap : c->batch_fresh;
+    if (!c->batch_fresh && !c->batch_fresh_cap && !c->batch_unread) return 0;
+    const bool capturing = hy3a_capturing(c);
+    int &flag = capturing ? c->batch_fresh_cap : c->batch_fresh;
     const int f = flag;
     flag = 0;
+    if (!capturing) c->batch_unread = 0;
     return f;
 }
 

@@ -330,6 +330,48 @@ def test_launch_count_includes_the_descriptor_kernel(cuda):
 
 
 @pytest.mark.parametrize("kv", ["int8", "fp16"])
+def test_descriptor_of_a_replayed_step_is_copied(cuda, kv):
+    """The descriptor of a step that only a graph reads travels as a copy (no kernel counts), that of an eager one as a kernel, and the
+    steps may alternate: without waiting between them and with a synchronisation after every call, the same outputs."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    q, k, v = (torch_rows(cuda, 3, h, 9) for h in (64, 8, 8))
+    res = []
+    for wait in (False, True):
+        ctx = Hy3Attn(kv_dtype=kv, n_layers=2, max_seqs=3, max_batch=3, max_tokens=9000, max_tokens_per_seq=3000)
+        for layer in range(2):
+            for i in range(3):
+                ctx.fill_random(layer, i, 0, 2000, 10 * layer + i)
+        out, g_out = torch.zeros((24, 3, 64, 128), device=cuda), torch.zeros((3, 64, 128), device=cuda)
+        side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        ctx.batch_set([0, 1, 2], [99, 5, 700])
+        ctx.decode_step(0, q, k, v, out=g_out)
+        torch.cuda.synchronize()
+        ctx.set_stream(side)
+        with torch.cuda.graph(graph, stream=side):
+            ctx.decode_step(0, q, k, v, out=g_out)
+        ctx.use_torch_stream()
+        kernels = []
+        for t in range(24):
+            before = ctx.launches
+            ctx.batch_set([0, 1, 2], [100 + 50 * t, 1999 - 30 * t, 64 * (t % 5)])
+            kernels.append(ctx.launches - before)
+            if t % 6 == 4:
+                ctx.decode_step(1, q, k, v, out=out[t])
+            else:
+                graph.replay()
+                out[t].copy_(g_out)
+            if wait:
+                torch.cuda.synchronize()
+        ctx.sync()
+        assert kernels == [int(t % 6 == 5 or t == 0) for t in range(24)]
+        res.append(out)
+        del graph
+        ctx.close()
+    assert torch.equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("kv", ["int8", "fp16"])
 def test_batch_descriptor_is_not_overtaken(cuda, kv):
     """Steps enqueued without waiting: every launch reads its own step's descriptor (the next one is written by a kernel that may
     start before the last layer has ended).  Against the same steps with a synchronisation after every call."""
