@@ -249,7 +249,7 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
 #pragma unroll
     for (int nb = 2; nb < NB; nb += 2) mx = fmaxf(mx, fmaxf(fmaxf(s[nb][0], s[nb][1]), fmaxf(s[nb + 1][0], s[nb + 1][1])));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));   /* finite: the first token of this granule is valid */
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));   /* the first token of this granule is valid */
     const bool grow = mx > st.m + kRescaleThreshold;       /* also true while st.m == -inf */
     if (__any_sync(0xffffffffu, grow)) {
         const float m_new = grow ? mx : st.m;
@@ -259,6 +259,7 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
         for (int jn = 0; jn < 16; jn++) { st.o[jn][0] *= alpha; st.o[jn][1] *= alpha; st.o[jn][2] *= alpha; st.o[jn][3] *= alpha; }
         st.m = m_new;
     }
+    const float mref = st.m == -INFINITY ? 0.f : st.m;     /* no finite score yet: -inf weighs 0, NaN stays NaN */
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) {      /* 16 tokens: one k-step of P.V */
         unsigned pa[4];
@@ -268,7 +269,7 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
             for (int nb = 0; nb < 2; nb++) {
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
-                    pe[nb][e] = ex2(s[2 * nt + nb][e] - st.m); /* -inf -> 0 */
+                    pe[nb][e] = ex2(s[2 * nt + nb][e] - mref); /* -inf -> 0 */
                     w[nb][e] = pe[nb][e] * vs[2 * nt + nb][e];
                 }
             }
@@ -759,10 +760,10 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         float L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int w = 0; w < kWarps; w++) {
-            float mw = s_ml[w][h][0];
-            if (mw == -INFINITY) continue;
-            float f = ex2(mw - M);
-            L += s_ml[w][h][1] * f;
+            const float2 ml = *reinterpret_cast<const float2 *>(s_ml[w][h]);
+            if (ml.y == 0.f) continue;
+            const float f = ex2(ml.x - M);
+            L += ml.y * f;
             float4 o4 = *reinterpret_cast<const float4 *>(&s_o[w][h][d4]);
             acc[0] += o4.x * f; acc[1] += o4.y * f; acc[2] += o4.z * f; acc[3] += o4.w * f;
         }
@@ -836,7 +837,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                     for (int c = 0; c < npieces; c++) {
                         const float *pr = zf + (size_t)c * kRecFloats;
                         const float pm = pr[0], pl = pr[1];
-                        if (!(pl > 0.f)) continue;
+                        if (pl == 0.f) continue;
                         const float2 v01 = *reinterpret_cast<const float2 *>(pr + 2 + d4), v23 = *reinterpret_cast<const float2 *>(pr + 4 + d4);
                         const float nm = fmaxf(M, pm), os = ex2(M - nm), rs = ex2(pm - nm);
                         L = L * os + pl * rs;
@@ -878,7 +879,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                         for (int c = 0; c < nc; c++) {
                             const float *pr = land_g + ((size_t)c * 8 + h) * kRecFloats;
                             const float pm = pr[0], pl = pr[1];
-                            if (!(pl > 0.f)) continue;
+                            if (pl == 0.f) continue;
                             const float2 v01 = *reinterpret_cast<const float2 *>(pr + 2 + d4), v23 = *reinterpret_cast<const float2 *>(pr + 4 + d4);
                             const float nm = fmaxf(M, pm), os = ex2(M - nm), rs = ex2(pm - nm);
                             L = L * os + pl * rs;
@@ -935,7 +936,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             if (d4 == 0) { rec[0] = M * kLn2; rec[1] = L; } /* m in natural-log units like the reference record */
             rec[2 + d4] = acc[0]; rec[3 + d4] = acc[1]; rec[4 + d4] = acc[2]; rec[5 + d4] = acc[3];
         } else {
-            float inv = L > 0.f ? 1.f / L : 0.f;
+            float inv = inv_sum(L);
             float4 o4 = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
             *reinterpret_cast<float4 *>(a.out + (size_t)row * a.out_stride + head_q * HY3A_D + d4) = o4;
         }
@@ -986,14 +987,14 @@ __global__ void hy3a_merge_kernel(const float *partials, int n_parts, int n_rows
     for (int s = 0; s < n_parts; s++) {
         const float *p = partials + ((size_t)s * n_rows * n_heads + rh) * HY3A_PARTIAL_FLOATS;
         float pms = p[0], pss = p[1];
-        if (!(pss > 0.f)) continue;
+        if (pss == 0.f) continue;
         float nm = fmaxf(ms, pms), os = __expf(ms - nm), rs = __expf(pms - nm);
         ss = ss * os + pss * rs;
 #pragma unroll
         for (int j = 0; j < 4; j++) ov[j] = ov[j] * os + p[2 + lane * 4 + j] * rs;
         ms = nm;
     }
-    float inv = ss > 0.f ? 1.f / ss : 0.f;
+    float inv = inv_sum(ss);
     *reinterpret_cast<float4 *>(out + (size_t)row * out_stride + (size_t)h * HY3A_D + lane * 4) = make_float4(ov[0] * inv, ov[1] * inv, ov[2] * inv, ov[3] * inv);
 }
 

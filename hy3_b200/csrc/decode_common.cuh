@@ -220,6 +220,9 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatil
     return false;
 }
 /* ---- pieces both decode kernels use */
+/* Folds skip a record only where its denominator is 0, the mark of a piece without keys, and divide by whatever else it is: a NaN score
+ * reaches the output on every route, whichever piece its key is in (a test for l > 0 would drop that piece's other keys too). */
+__device__ __forceinline__ float inv_sum(float l) { return l == 0.f ? 0.f : 1.f / l; }
 /* a row without keys: zero output, or empty partial records {-inf, 0, 0...} (hy3_gpu.cu:197-199); `out`, `partials`: the row's owned heads */
 __device__ __forceinline__ void write_empty_row(float *out, float *partials, int G, int t, int threads) {
 #pragma unroll 1
@@ -292,7 +295,7 @@ __device__ __forceinline__ void cluster_write(const hy3a_decode_args &a, int kv_
         if (lane == 0) { rec[0] = M * kLn2; rec[1] = L; }
         rec[2 + d4] = acc[0]; rec[3 + d4] = acc[1]; rec[4 + d4] = acc[2]; rec[5 + d4] = acc[3];
     } else {
-        const float inv = L > 0.f ? 1.f / L : 0.f;
+        const float inv = inv_sum(L);
         *reinterpret_cast<float4 *>(a.out + (size_t)row * a.out_stride + (size_t)(kv_head_begin * 8 + hq) * HY3A_D + d4) = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
     }
 }
@@ -377,7 +380,7 @@ __device__ __forceinline__ void shard_fold(const shard_fold_args &a) {
                     const uint4 *st = a.stage + (j * 8 + a.h) * kShardLines;
                     const uint4 l0 = st[0];
                     if (l0.y != a.flag || l0.w != a.flag) continue;
-                    if (__uint_as_float(l0.z) > 0.f) {
+                    if (__uint_as_float(l0.z) != 0.f) {
                         const uint4 la = st[a.line_a], lb = st[a.line_a + 1];
                         if (la.y != a.flag || la.w != a.flag || lb.y != a.flag || lb.w != a.flag) continue;
                     }
@@ -404,13 +407,13 @@ __device__ __forceinline__ void shard_fold(const shard_fold_args &a) {
             float pm, pl, pv[4];
             if (base + j == a.my_rank) {
                 pm = a.own_m; pl = a.own_l; pv[0] = a.own_acc[0]; pv[1] = a.own_acc[1]; pv[2] = a.own_acc[2]; pv[3] = a.own_acc[3];
-                if (!(pl > 0.f)) continue;
+                if (pl == 0.f) continue;
             } else {
                 if (gave_up && (pending & (1u << j))) continue;
                 const uint4 *st = a.stage + (j * 8 + a.h) * kShardLines;
                 const uint4 l0 = st[0];
                 pm = __uint_as_float(l0.x); pl = __uint_as_float(l0.z);
-                if (!(pl > 0.f)) continue;
+                if (pl == 0.f) continue;
                 const uint4 la = st[a.line_a], lb = st[a.line_a + 1];
                 pv[0] = __uint_as_float(la.x); pv[1] = __uint_as_float(la.z); pv[2] = __uint_as_float(lb.x); pv[3] = __uint_as_float(lb.z);
             }
@@ -421,7 +424,7 @@ __device__ __forceinline__ void shard_fold(const shard_fold_args &a) {
         }
         __syncwarp();   /* the landing zone is reused by the next batch of ranks */
     }
-    const float inv = ss > 0.f ? 1.f / ss : 0.f;
+    const float inv = inv_sum(ss);
     *reinterpret_cast<float4 *>(a.out) = make_float4(ov[0] * inv, ov[1] * inv, ov[2] * inv, ov[3] * inv);
 }
 

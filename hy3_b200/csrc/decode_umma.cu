@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                         for (int c = 0; c < npieces; c++) {
                             const float *pr = zf + (size_t)c * kRecFloats;
                             const float pm = pr[0], pl = pr[1];
-                            if (!(pl > 0.f)) continue;
+                            if (pl == 0.f) continue;
                             const float2 v01 = *reinterpret_cast<const float2 *>(pr + 2 + d4), v23 = *reinterpret_cast<const float2 *>(pr + 4 + d4);
                             const float nm = fmaxf(M, pm), os = ex2(M - nm), rs = ex2(pm - nm);
                             L = L * os + pl * rs;
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                             for (int c = 0; c < nc; c++) {
                                 const float *pr = land_g + ((size_t)c * 8 + h) * kRecFloats;
                                 const float pm = pr[0], pl = pr[1];
-                                if (!(pl > 0.f)) continue;
+                                if (pl == 0.f) continue;
                                 const float2 v01 = *reinterpret_cast<const float2 *>(pr + 2 + d4), v23 = *reinterpret_cast<const float2 *>(pr + 4 + d4);
                                 const float nm = fmaxf(M, pm), os = ex2(M - nm), rs = ex2(pm - nm);
                                 L = L * os + pl * rs;
@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                 if (d4 == 0) { rec[0] = M * kLn2; rec[1] = L; } /* m in natural-log units like the reference record */
                 rec[2 + d4] = acc[0]; rec[3 + d4] = acc[1]; rec[4 + d4] = acc[2]; rec[5 + d4] = acc[3];
             } else {
-                const float inv = L > 0.f ? 1.f / L : 0.f;
+                const float inv = inv_sum(L);
                 *reinterpret_cast<float4 *>(a.out + (size_t)row * a.out_stride + head_q * HY3A_D + d4) = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
             }
         }

@@ -141,12 +141,12 @@ def merge_partials_numpy(gathered):
             ms, ss, ov = -np.inf, np.float32(0), np.zeros(128, np.float32)
             for s in range(W):
                 pm, pl = gathered[s, r, h, 0], gathered[s, r, h, 1]
-                if not pl > 0:
+                if pl == 0:
                     continue
                 nm = max(ms, pm)
                 os_, rs = np.float32(np.exp(ms - nm)), np.float32(np.exp(pm - nm))
                 ss = ss * os_ + pl * rs
                 ov = ov * os_ + gathered[s, r, h, 2:] * rs
                 ms = nm
-            out[r, h] = ov / ss if ss > 0 else 0
+            out[r, h] = 0 if ss == 0 else ov / ss
     return out

@@ -577,3 +577,44 @@ def test_largest_batch_keeps_the_page_ring(cuda):
         ctx.sync()
         ctx.close()
     assert torch.isfinite(res[0]).all() and (res[0][rows] - res[1]).abs().max() < 2e-5
+
+
+@pytest.mark.parametrize("dt,kind", [("fp16", "nan"), ("fp16", "+inf"), ("int8", "nan"), ("int4", "nan")])
+def test_decode_non_finite_scores(cuda, dt, kind):
+    """A key whose score is NaN or +inf makes the outputs of its KV head's queries NaN, whichever piece it is in, and no others: in one
+    piece, as a cluster, in pieces whose records are folded, captured, through partial records, and with two rows."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    for ntok, at in ((1, 0), (100, 3), (641, 640), (700, 650), (3000, 0), (5000, 2222), (40000, 39999), (40000, 20000)):
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_seqs=2, max_batch=2, max_tokens=2 * ntok + 128, max_tokens_per_seq=40960)
+        for i in range(2):
+            ctx.fill_random(0, i, 0, ntok, 5 + i)
+        ks, vs = ctx.export_kv(0, 0, at, 1)
+        ks[0].view(np.float16)[3 * 128 if dt == "fp16" else 3] = np.float16(kind)       # KV head 3: an element of the key, or its scale
+        ctx.import_kv(0, 0, at, ks, vs)
+        q = torch.randn((2, 64, 128), device=cuda, generator=torch.Generator(cuda).manual_seed(1))
+        outs = []
+        for rows in ([0], [0, 1]):
+            n = len(rows)
+            ctx.batch_set(rows, [ntok - 1] * n)
+            outs.append(ctx.decode(0, q[:n]))
+            part = torch.zeros((n, 64, 130), device=cuda)
+            ctx.decode(0, q[:n], partials=part)
+            merged = torch.zeros((n, 64, 128), device=cuda)
+            ctx.merge_partials(part, 1, n, 64, merged)
+            outs.append(merged)
+            ctx.sync()
+            side, graph, g_out = torch.cuda.Stream(), torch.cuda.CUDAGraph(), torch.zeros((n, 64, 128), device=cuda)
+            torch.cuda.synchronize()
+            ctx.set_stream(side)
+            with torch.cuda.graph(graph, stream=side):
+                ctx.decode(0, q[:n], out=g_out)
+            ctx.use_torch_stream()
+            graph.replay()
+            ctx.sync()
+            outs.append(g_out)
+            del graph
+        ctx.close()
+        for o in outs:
+            assert torch.isnan(o[0, 24:32]).all(), "%d tokens, key %d: dropped" % (ntok, at)
+            assert torch.isfinite(o[0, :24]).all() and torch.isfinite(o[0, 32:]).all() and torch.isfinite(o[1:]).all()
