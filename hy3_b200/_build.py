@@ -3,7 +3,8 @@
     python -m hy3_b200._build [--force] [--verbose]
 
   libhy3attn.so   the attention library: CUDA kernels + the C ABI of include/hy3_attn.h
-  _native.so      the CPython module with the per-step calls of Hy3Attn (csrc/binding.cpp); links libtorch, not CUDA
+  _native.<abi>.so  the CPython module with the per-step calls of Hy3Attn (csrc/binding.cpp); links libtorch, not CUDA.
+                  Built for one Python and one torch; skipped where torch is not installed (the C libraries need neither)
   libhy3_gpu.so   the same objects plus hy3_gpu_dropin.cu: hy3_gpu_init / hy3_gpu_free / hy3_eval_gpu for the reference
                   engine (include/hy3_gpu_dropin.h).  It is compiled against the engine's own hy3.h, so it needs the
                   engine's checkout: HY3_REF, or a directory `reference` next to this repository.  Without one a
@@ -15,13 +16,14 @@ cross-compiles without a GPU.
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhy3attn.so")
 DROPIN_LIB = os.path.join(HERE, "libhy3_gpu.so")
-NATIVE = os.path.join(HERE, "_native.so")
+NATIVE = os.path.join(HERE, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))
 SOURCES = ["append.cu", "decode.cu", "decode_umma.cu", "prefill.cu", "capi.cu", "selftest.cu"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC,-fvisibility=default", "-I", os.path.join(ROOT, "include")]
@@ -63,22 +65,32 @@ def build(force=False, verbose=False):
         if r.returncode:
             print(r.stdout + r.stderr)
             raise RuntimeError("link failed")
-    build_binding(force)
     build_dropin(objs, headers, nvcc, obj_dir, force, verbose)
+    build_binding(force)
     return lib_out
+
+
+def torch_key():
+    """What the binding's C++ ABI depends on besides Python: torch's version and its string ABI."""
+    import torch
+    return "%s cxx11=%d" % (torch.__version__, int(torch._C._GLIBCXX_USE_CXX11_ABI))
 
 
 def build_binding(force=False):
     """The CPython module with the per-step calls; needs torch's headers and libraries."""
+    try:
+        import torch
+    except ImportError:
+        print("hy3_b200._build: torch is not installed: the Python binding is not built")
+        return None
     src = os.path.join(CSRC, "binding.cpp")
-    if not (force or _newer([src, os.path.join(ROOT, "include", "hy3_attn.h")], NATIVE)):
+    key, stamp = torch_key(), NATIVE + ".key"       # beside the module, so that it travels with it
+    built_for = open(stamp).read() if os.path.exists(stamp) else None
+    if not (force or built_for != key or _newer([src, os.path.join(ROOT, "include", "hy3_attn.h")], NATIVE)):
         return NATIVE
-    import sysconfig
-
-    import torch
     t = os.path.dirname(torch.__file__)
     cmd = [os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-DHY3A_TORCH_KEY=\"%s\"" % key,
            "-isystem", os.path.join(t, "include"), "-isystem", os.path.join(t, "include", "torch", "csrc", "api", "include"),
            "-I", sysconfig.get_paths()["include"], src, "-o", NATIVE,
            "-L", os.path.join(t, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
@@ -86,6 +98,8 @@ def build_binding(force=False):
     if r.returncode:
         print(r.stdout + r.stderr)
         raise RuntimeError("building the binding failed")
+    with open(stamp, "w") as f:
+        f.write(key)
     return NATIVE
 
 

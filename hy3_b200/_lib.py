@@ -97,6 +97,9 @@ def load_native():
         from . import _native
     except ImportError as e:
         raise Hy3AttnError(-3, "the native binding does not load (%s): build it with `python -m hy3_b200._build`" % e) from e
+    from ._build import torch_key
+    if _native.torch_key != torch_key():
+        raise Hy3AttnError(-3, "the native binding was built for torch %s, this is %s: build it again with `python -m hy3_b200._build`" % (_native.torch_key, torch_key()))
     _native.bind(*(C.cast(getattr(lib, "hy3a_" + f), _vp).value for f in ("batch_set", "append", "decode_step", "prefill")))
     _bound = _native
     return _bound

@@ -173,4 +173,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods};
 
 } /* namespace */
 
-PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }
+/* `torch_key`: the torch it was built for; the loader compares */
+PyMODINIT_FUNC PyInit__native(void) {
+    PyObject *m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "torch_key", HY3A_TORCH_KEY)) Py_CLEAR(m);
+    return m;
+}

@@ -86,3 +86,17 @@ def test_bad_config_rejected(lib):
     h = C.c_void_p()
     assert lib.hy3a_create(C.byref(cfg), C.byref(h)) == -1 and not h.value
     assert b"kv head range" in lib.hy3a_last_error(None)
+
+
+def test_binding_is_skipped_without_torch_and_refused_for_another(lib, monkeypatch):
+    """The C libraries build where torch is not installed, and a module built for another torch is built again, or refused when loaded."""
+    import sys
+    from hy3_b200 import Hy3AttnError, _build, _lib
+    native = _lib.load_native()
+    assert native.torch_key == _build.torch_key() == open(_build.NATIVE + ".key").read()
+    monkeypatch.setattr(_lib, "_bound", None)
+    monkeypatch.setattr(_build, "torch_key", lambda: "another")
+    with pytest.raises(Hy3AttnError, match="another"):
+        _lib.load_native()
+    monkeypatch.setitem(sys.modules, "torch", None)
+    assert _build.build_binding() is None
