@@ -40,6 +40,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "ctx.h"
 #include "decode_common.cuh"
 #include "rowops.cuh"
@@ -1103,13 +1105,18 @@ static_assert(kRecFloats >= HY3A_PARTIAL_FLOATS && (kRecFloats * 4) % 16 == 0, "
  * exchange (several CTAs store to the peers instead of one); on one GPU the folders only hold their SMs longer, which delays the
  * next launch's CTAs there.  Its folders wait for the other pieces, so every CTA of the grid must be resident.  4 measured best
  * on 8 GPUs (8: 28.8, 4: 27.8, 2: 27.8, 1: 29.2 us per layer).  A folder lands 8 / F heads x pieces records in the page ring: a
- * segment has up to CTAs / KV heads pieces, and with one KV head on 148 CTAs 2 x 148 records (156 KB) exceed the rings of FP16
- * and INT4 pages (131 and 135 KB).  Then 8 folders take one head each; a ring too small for that too keeps the plain fold.
+ * segment has up to CTAs / KV heads pieces, and no more than hy3a_most_pieces of the longest row that the context can hold where
+ * pieces are not of even size (a launch may be replayed for any row, so the batch at hand does not count).  With one KV head and rows
+ * beyond 413 696 (FP16) or 430 080 tokens (INT4), 2 x 125 or 2 x 129 records exceed the rings of 131 and 135 KB.  Then 8 folders take
+ * one head each; a ring too small for that too keeps the plain fold.
  * (Segments of fewer than F pieces have fewer folders: 4 heads x 3 pieces = 6.3 KB at most.) */
 static int spread_folders(const hy3a_ctx *ctx) {
     if (ctx->shard_slot < 0 || ctx->decode_ctas > ctx->sm_count) return 0;
-    const size_t ring = (size_t)(ctx->geom.dtype == HY3A_KV_INT8 ? HY3A_UMMA_STAGES : ctx->decode_stages) * ctx->geom.page_bytes;
-    const size_t pieces = (size_t)(ctx->decode_ctas / ctx->cfg.kv_head_count);
+    const int dt = ctx->geom.dtype, heads = ctx->cfg.kv_head_count;
+    const size_t ring = (size_t)(dt == HY3A_KV_INT8 ? HY3A_UMMA_STAGES : ctx->decode_stages) * ctx->geom.page_bytes;
+    size_t pieces = (size_t)(ctx->decode_ctas / heads);
+    if (dt == HY3A_KV_INT8 || !hy3a_even_applies(ctx->batch_n, heads, (unsigned)ctx->decode_ctas))
+        pieces = std::min(pieces, (size_t)hy3a_most_pieces((unsigned)ctx->cfg.max_blocks_per_seq));
     for (int f = 4; f <= 8; f *= 2) if ((size_t)(8 / f) * pieces * kRecFloats * 4 <= ring) return f;
     return 0;
 }

@@ -57,13 +57,14 @@ def test_world1_push_and_merge_equals_decode_step(cuda, oracle, dt):
 
 
 @pytest.mark.parametrize("dt,heads,lens0,stages", [("fp16", 1, [20000], None), ("int4", 1, [20000], None), ("int8", 1, [20000], None),
+                                                   ("fp16", 1, [520000], None), ("int4", 1, [520000], None), ("int4", 1, [520000], 3),
                                                    ("int4", 2, [20000], 2), ("int4", 4, [300, 9000], 3),
                                                    ("int4", 8, [3007, 129, 0, 4097, 640, 2000, 900], None),
                                                    ("fp16", 8, [3007, 129, 0, 4097, 640, 2000, 900], None),
                                                    ("int4", 8, [9000] + [100] * 8, None)])
 def test_world1_segments_of_many_pieces(cuda, oracle, dt, heads, lens0, stages, monkeypatch):
-    """Few KV heads: up to 148 pieces of a segment, whose records have to fit the page ring that the folders land them in (4 folders
-    of two heads each, 8 of one, or the plain fold).  And 7 or 9 rows of all heads, in pieces of even size or straddling.  Equal to
+    """One KV head and a long row: up to 148 pieces of a segment, whose records have to fit the page ring that the folders land them in (4
+    folders of two heads each, 8 of one, or the plain fold).  And 7 or 9 rows of all heads, in pieces of even size or straddling.  Equal to
     hy3a_decode_step bit for bit."""
     import torch
     from hy3_b200 import Hy3Attn
