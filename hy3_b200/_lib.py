@@ -58,6 +58,7 @@ PROTOTYPES = {
     "hy3a_launch_count": (_u64, [_vp]),
     "hy3a_decode_schedule_kv": (_i, [_i, _i, _ip, _i, _i, _i, _llp, _llp, _llp]),
     "hy3a_decode_schedule": (_i, [_i, _ip, _i, _i, _i, _llp, _llp, _llp]),
+    "hy3a_decode_cluster": (_i, [_vp]),
     "hy3a_prefill_cluster": (_i, [_vp, _i, _i]),
     "hy3a_prefill_schedule": (_i, [_i, _i, _i, _i, _i, _ip, _i]),
     "hy3a_version": (C.c_char_p, []),

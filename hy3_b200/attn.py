@@ -203,6 +203,13 @@ class Hy3Attn:
             self._chk(rc)
         return out
 
+    def decode_cluster(self):
+        """CTAs per (row, KV head) segment of the current batch: 2, 4 or 8 as a cluster, 1: `decode_schedule`."""
+        n = self.lib.hy3a_decode_cluster(self.h)
+        if n < 0:
+            self._chk(n)
+        return n
+
     def prefill_cluster(self, base_slot, nq):
         """CTAs per block of 32 query tokens of such a chunk: 2, 4 or 8 as a cluster, 1: `prefill_schedule`."""
         n = self.lib.hy3a_prefill_cluster(self.h, base_slot, nq)

@@ -256,6 +256,7 @@ int hy3a_create(const hy3a_config *cfg, hy3a_ctx **out) {
     if (ctx->decode_ctas > hy3a_decode_max_ctas()) ctx->decode_ctas = hy3a_decode_max_ctas();
     if (ctx->decode_ctas > 512) ctx->decode_ctas = 512;
     { const char *e = getenv("HY3A_NO_PDL"); ctx->use_pdl = !(e && atoi(e)); }
+    { const char *e = getenv("HY3A_NO_CLUSTERS"); ctx->no_clusters = e && atoi(e); }
     /* fp16 operand mirrors of the chunked prefill: at most this much device memory beside the pool */
     { const char *e = getenv("HY3A_PF_MIRROR_MB"); ctx->pf_mbudget = (size_t)(e ? (atoll(e) > 0 ? atoll(e) : 0) : 8192) << 20; }
     ctx->pf_mseq = -1;

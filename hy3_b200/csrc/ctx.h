@@ -108,6 +108,7 @@ struct hy3a_ctx {
     int batch_unread;     /* no launch outside a capture has read the batch descriptor: the step is replayed from a graph */
     int bulk_write_pending; /* a kernel that wrote many KV slots was enqueued and no decode launch has followed it yet */
     int use_pdl;          /* launch kernels with programmatic stream serialization (HY3A_NO_PDL=1 turns it off) */
+    int no_clusters;      /* HY3A_NO_CLUSTERS=1: decode and prefill keep to the grids (tests, comparisons) */
     int cl_cap[4];        /* decode: clusters of 2^i CTAs that fit on the device at once */
     int decode_stages;    /* pages in the decode kernel's shared-memory ring; < 2 selects the direct-load variant */
 

@@ -1141,11 +1141,18 @@ static int cluster_size(const hy3a_ctx *ctx, int most, long long total) {
     return ((most - 1) >> i) + 1 <= share + kPagesFold[dt] ? 1 << i : 0;
 }
 static int decode_cluster(const hy3a_ctx *ctx) {
-    if ((ctx->shard_slot >= 0 && ctx->shard_world > 1) || ctx->decode_ctas < ctx->sm_count) return 0;      /* a world of one has nothing to exchange */
+    if ((ctx->shard_slot >= 0 && ctx->shard_world > 1) || ctx->decode_ctas < ctx->sm_count || ctx->no_clusters) return 0;      /* a world of one has nothing to exchange */
     const int cl = cluster_size(ctx, ctx->batch_pages, ctx->batch_pages_all);
     if (!cl) return 0;
     if (!hy3a_capturing(ctx)) return cl;
     return cluster_size(ctx, ctx->cfg.max_blocks_per_seq, (long long)ctx->cfg.max_blocks_per_seq * ctx->batch_n);
+}
+
+extern "C" int hy3a_decode_cluster(hy3a_ctx *ctx) {
+    if (!ctx) return HY3A_EINVAL;
+    if (ctx->batch_n < 1) return hy3a_fail(ctx, HY3A_ESTATE, "decode_cluster: no batch set (call hy3a_batch_set first)");
+    const int cl = decode_cluster(ctx);
+    return cl ? cl : 1;
 }
 
 int hy3a_launch_decode(hy3a_ctx *ctx, int layer, const float *q, size_t q_stride, float *out, size_t out_stride, float *partials,

@@ -240,7 +240,11 @@ int hy3a_fill_random(hy3a_ctx *ctx, int layer, int seq, int t0, int n, uint64_t 
 /* ---- introspection ------------------------------------------------------------------*/
 /* Number of kernels this library has launched on ctx since creation. */
 uint64_t hy3a_launch_count(const hy3a_ctx *ctx);
-/* Decode schedule for a batch (pure host arithmetic, no GPU): given n lengths, the number
+/* CTAs that hy3a_decode / hy3a_decode_step give each (row, KV head) segment of the current batch on this context's device: 2, 4 or 8
+ * that share its pages as a thread-block cluster, or 1 (the grid that hy3a_decode_schedule describes), or a negative error.  Within
+ * a stream capture it answers for the captured launch, whose rows may be any that the context can hold. */
+int hy3a_decode_cluster(hy3a_ctx *ctx);
+/* Decode schedule of a batch whose step does not run as clusters (pure host arithmetic, no GPU): given n lengths, the number
  * of page units, and for CTA `cta` of `n_ctas` its unit range [*u0, *u1).  The kernels split
  * the units differently for INT8 and for FP16 / INT4 caches; hy3a_decode_schedule is the
  * schedule of an INT8 cache (the default).                                               */

@@ -9,11 +9,12 @@ from helpers import SEED, check_attention, make_slots, slots_to_float
 pytestmark = pytest.mark.gpu
 
 
-def run_case(cuda, oracle, dt, base, nq, rows=None, eps=1e-6):
+def run_case(cuda, oracle, dt, base, nq, rows=None, eps=1e-6, cluster=None):
     import torch
     from hy3_b200 import Hy3Attn
     ntok = base + nq
     ctx = Hy3Attn(kv_dtype=dt, n_layers=2, max_batch=max(nq, base, 1), max_tokens=ntok + 256, rms_eps=eps)
+    assert cluster is None or ctx.prefill_cluster(base, nq) == cluster
     w = (1.0 + 0.02 * oracle.fill_normal((2, 128), SEED, 3)).astype(np.float32)
     ctx.set_norm_weights(1, w[0], w[1])
     q = oracle.fill_normal((ntok, 64, 128), SEED, 501)
@@ -57,23 +58,26 @@ def test_prefill_chunk_over_prefix(cuda, oracle, dt):
 
 @pytest.mark.parametrize("dt", ["fp16", "int8", "int4"])
 @pytest.mark.parametrize("base,nq", [(2047, 1), (3970, 45), (4090, 37), (4060, 129), (3999, 33)])
-def test_prefill_cut_along_the_keys(cuda, oracle, dt, base, nq):
-    """Chunks whose blocks are cut into several pieces (records + fold): warps without queries, rows whose keys in the last
-    piece are all masked, odd bases."""
+def test_prefill_cut_along_the_keys(cuda, oracle, dt, base, nq, monkeypatch):
+    """Chunks whose blocks are cut into several pieces (records + fold; not as clusters): warps without queries, rows whose keys in the
+    last piece are all masked, odd bases."""
     from hy3_b200.attn import prefill_schedule
+    monkeypatch.setenv("HY3A_NO_CLUSTERS", "1")
     assert (prefill_schedule(base, nq, 8)[:, 5] > 1).any()
-    run_case(cuda, oracle, dt, base, nq, rows=sorted({0, nq // 2, max(nq - 2, 0), nq - 1, min(31, nq - 1), min(32, nq - 1)}))
+    run_case(cuda, oracle, dt, base, nq, cluster=1, rows=sorted({0, nq // 2, max(nq - 2, 0), nq - 1, min(31, nq - 1), min(32, nq - 1)}))
 
 
 @pytest.mark.parametrize("kind", ["nan", "+inf", "-inf"])
-@pytest.mark.parametrize("base,nq,first", [(0, 96, 16), (4060, 37, 4000)])
-def test_prefill_non_finite_scores(cuda, oracle, base, nq, first, kind):
-    """A key whose score is NaN or +inf makes every query that sees it NaN, wherever the key lies in a step (64 positions), uncut and
-    cut; a score of -inf is a weight of 0.  Against softmax in 64 bits."""
+@pytest.mark.parametrize("base,nq,first,clusters", [(0, 96, 16, False), (4060, 37, 4000, False), (4060, 37, 4000, True), (1001, 40, 970, True)])
+def test_prefill_non_finite_scores(cuda, oracle, base, nq, first, clusters, kind, monkeypatch):
+    """A key whose score is NaN or +inf makes every query that sees it NaN, wherever the key lies in a step (64 positions), uncut,
+    cut and in a cluster; a score of -inf is a weight of 0.  Against softmax in 64 bits."""
+    if not clusters:
+        monkeypatch.setenv("HY3A_NO_CLUSTERS", "1")
     import torch
     from hy3_b200 import Hy3Attn
     from hy3_b200.attn import prefill_schedule
-    assert (len(prefill_schedule(base, nq, 8)) > 0) == (base > 0)
+    assert clusters or (len(prefill_schedule(base, nq, 8)) > 0) == (base > 0)
     ntok = base + nq
     q = oracle.fill_normal((nq, 64, 128), SEED, 521).astype(np.float16)
     q[:, :, 0] = 1.0
@@ -82,6 +86,7 @@ def test_prefill_non_finite_scores(cuda, oracle, base, nq, first, kind):
     vs = make_slots(oracle, v, "fp16")
     tq = torch.from_numpy(q).to(cuda)
     ctx = Hy3Attn(kv_dtype="fp16", n_layers=1, max_batch=max(nq, 16), max_tokens=ntok + 128)
+    assert (ctx.prefill_cluster(base, nq) > 1) == clusters
     v64 = v.astype(np.float16).astype(np.float64)
     seen = np.arange(ntok)[None, :] <= base + np.arange(nq)[:, None]
     for r in range(8):
@@ -113,13 +118,14 @@ def test_prefill_non_finite_scores(cuda, oracle, base, nq, first, kind):
     ("fp16", 0, 2048, (0, 8), False), ("int8", 2048, 953, (0, 8), False), ("int4", 40, 700, (0, 8), False), ("fp16", 9930, 97, (0, 8), True),
     ("int8", 1001, 512, (2, 4), True), ("fp16", 500, 1000, (6, 2), True), ("int4", 3000, 200, (7, 1), True), ("fp16", 3000, 300, (5, 3), True),
     ("int8", 100, 2900, (4, 3), False)])
-def test_prefill_every_block_and_head(cuda, oracle, dt, base, nq, heads, cut):
-    """Grids in several groups of blocks (more CTAs than SMs) with a ragged last group, uncut and cut, and contexts that own some of
+def test_prefill_every_block_and_head(cuda, oracle, dt, base, nq, heads, cut, monkeypatch):
+    """Grids (no clusters) in several groups of blocks (more CTAs than SMs) with a ragged last group, uncut and cut, and contexts that own some of
     the KV heads: one query of every 32-token block, every owned head, into an output that starts as NaN; heads of others are not
     written.  Repeated and interleaved with a chunk of another shape on the same records: identical bits."""
     import torch
     from hy3_b200 import Hy3Attn
     from hy3_b200.attn import prefill_schedule
+    monkeypatch.setenv("HY3A_NO_CLUSTERS", "1")
     h0, nh = heads
     plan = prefill_schedule(base, nq, nh)
     assert (len(plan) > 0) == cut
@@ -164,7 +170,7 @@ def test_prefill_clusters(cuda, oracle, dt, base, nq, heads, size):
     for batch in (max(nq, 16), 8):
         ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_batch=batch, max_tokens=ntok + 128, kv_head_begin=h0, kv_head_count=nh)
         ctx.fill_random(0, 0, 0, ntok, 79)
-        assert ctx.prefill_cluster(base, nq) > 1      # `size` on 148 SMs in the usual GPCs
+        assert ctx.prefill_cluster(base, nq) == size or torch.cuda.get_device_properties(0).multi_processor_count != 148
         for _ in range(3):
             outs.append(ctx.prefill(0, 0, base, q16, out=torch.full((nq, 64, 128), float("nan"), device=cuda)))
         ctx.sync()
@@ -183,20 +189,21 @@ def test_prefill_clusters(cuda, oracle, dt, base, nq, heads, size):
 
 
 @pytest.mark.parametrize("dt,base,nq,heads", [("int8", 2500, 500, (3, 5)), ("int4", 500, 1500, (2, 2)), ("fp16", 4500, 150, (0, 8))])
-def test_prefill_records_where_no_cluster_pays(cuda, oracle, dt, base, nq, heads):
+def test_prefill_records_where_no_cluster_pays(cuda, oracle, dt, base, nq, heads, monkeypatch):
     """Chunks that still leave records: the checks of the grids above."""
     from hy3_b200 import Hy3Attn
     ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_batch=nq, max_tokens=base + nq, kv_head_begin=heads[0], kv_head_count=heads[1])
     assert ctx.prefill_cluster(base, nq) == 1
     ctx.close()
-    test_prefill_every_block_and_head(cuda, oracle, dt, base, nq, heads, True)
+    test_prefill_every_block_and_head(cuda, oracle, dt, base, nq, heads, True, monkeypatch)
 
 
-def test_prefill_without_records(cuda, oracle):
-    """A context without piece records (max_batch < 16) runs uncut what another one cuts."""
+def test_prefill_without_records(cuda, oracle, monkeypatch):
+    """A context without piece records (max_batch < 16) runs uncut what another one cuts (where neither takes clusters)."""
     import torch
     from hy3_b200 import Hy3Attn
     from hy3_b200.attn import prefill_schedule
+    monkeypatch.setenv("HY3A_NO_CLUSTERS", "1")
     base, nq = 3970, 45
     assert len(prefill_schedule(base, nq, 8)) > 0 and len(prefill_schedule(base, nq, 8, 148, 0)) == 0
     q16 = torch.from_numpy(oracle.fill_normal((nq, 64, 128), SEED, 541).astype(np.float16)).to(cuda)

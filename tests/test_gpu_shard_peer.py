@@ -21,10 +21,14 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
+@pytest.mark.parametrize("clusters", [False, True])
 @pytest.mark.parametrize("dt", ["int8", "fp16"])
-def test_world1_push_and_merge_equals_decode_step(cuda, oracle, dt):
+def test_world1_push_and_merge_equals_decode_step(cuda, oracle, dt, clusters, monkeypatch):
+    """As a grid, whose sharded variant exchanges with itself, and as clusters where the rule takes them, which leave the exchange out."""
     import torch
     from hy3_b200 import Hy3Attn
+    if not clusters:
+        monkeypatch.setenv("HY3A_NO_CLUSTERS", "1")
     lens0 = [0, 200, 3000]
     B, steps, L = len(lens0), 5, 2
     q = oracle.fill_normal((steps, L, B, 64, 128), SEED, 501)
@@ -51,6 +55,7 @@ def test_world1_push_and_merge_equals_decode_step(cuda, oracle, dt):
                     o = ctx.decode_step(l, tq[t, l], tk[t, l], tv[t, l])
                 outs.append(o)
         ctx.sync()
+        assert clusters or ctx.decode_cluster() == 1
         res[mode] = torch.stack(outs).cpu().numpy()
         ctx.close()
     assert np.array_equal(res["plain"], res["pushed"]), "max diff %.3g" % np.abs(res["plain"] - res["pushed"]).max()
@@ -68,6 +73,7 @@ def test_world1_segments_of_many_pieces(cuda, oracle, dt, heads, lens0, stages, 
     hy3a_decode_step bit for bit."""
     import torch
     from hy3_b200 import Hy3Attn
+    monkeypatch.setenv("HY3A_NO_CLUSTERS", "1")
     if stages is not None:
         monkeypatch.setenv("HY3A_DECODE_STAGES", str(stages))
     B, steps = len(lens0), 4
