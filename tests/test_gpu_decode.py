@@ -593,6 +593,7 @@ def test_decode_non_finite_scores(cuda, dt, kind):
         ks[0].view(np.float16)[3 * 128 if dt == "fp16" else 3] = np.float16(kind)       # KV head 3: an element of the key, or its scale
         ctx.import_kv(0, 0, at, ks, vs)
         q = torch.randn((2, 64, 128), device=cuda, generator=torch.Generator(cuda).manual_seed(1))
+        q[:, :, 0] = 1.0                                                                # the score of the infinite element is +inf
         outs = []
         for rows in ([0], [0, 1]):
             n = len(rows)
