@@ -24,14 +24,15 @@
  * permuted so that every thread's MMA operands are exactly the 16-byte chunks it loads.
  *
  * Scheduling: unit = one 128-token page of one (batch row, KV head); units are laid out
- * row-major, head, page and cut into contiguous ranges, one per CTA, so one launch shape
+ * row-major, head, page and cut into contiguous ranges, one per CTA, so one grid
  * serves every length (lengths come from device memory; nothing is baked into a captured
  * graph, cf. hy3_gpu.cu:774-789).  A producer warp streams the CTA's pages into a shared-
  * memory ring with bulk asynchronous copies (cp.async.bulk + mbarrier transaction counts);
  * the consumer warps take the 16- or 32-token granules of the pages round-robin.  The piece a CTA
  * computes for a (row, head) segment is folded in shared memory; if the segment spans
  * several CTAs each writes an {m, l, acc} record and the LAST CTA to arrive (atomic
- * counter) folds them -- the LSE-merge epilogue, no second launch.
+ * counter) folds them -- the LSE-merge epilogue, no second launch.  Steps of few segments with few pages run as clusters
+ * instead (cluster_size below).
  *
  * Roofline: HBM.  Algorithmic bytes per (token, KV head): 512 (FP16), 132 (INT4); per token and
  * layer x8.

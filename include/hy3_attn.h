@@ -113,7 +113,9 @@ int hy3a_free_blocks(hy3a_ctx *ctx);
  * no private counter, so rolling back (hy3.c:1514) is just passing smaller positions.
  * Reserves capacity for the slots.  slots[i] == -1: the row has no keys in this context (a
  * rank without tokens of the sequence): nothing is stored for it, and decode returns zeros
- * (or an empty partial record).                                                        */
+ * (or an empty partial record).  Launches on the context's device, whichever is current,
+ * unless the stream is a default stream: that is the current device's, so another one than
+ * the context's is refused with HY3A_ESTATE.                                           */
 int hy3a_batch_set(hy3a_ctx *ctx, int n, const int *seq_ids, const int *slots, const int *rope_pos);
 
 /* ---- hot path ----------------------------------------------------------------------*/
@@ -134,8 +136,10 @@ int hy3a_append(hy3a_ctx *ctx, int layer, const float *q_in, size_t q_stride, co
 /* Split-KV GQA decode attention for the n rows of the current batch: row i attends keys
  * [0, slots[i]] of its sequence.  Replaces attention_split_kv[_int4]_kernel +
  * attention_reduce_kernel (hy3_gpu.cu:183, :274, :233) and the split heuristic / graph
- * recapture coupling (:766-789): lengths are read from device memory, one launch shape
- * serves every length.  q: fp32 [n][64][128] (row stride q_stride), out the same shape
+ * recapture coupling (:766-789): lengths are read from device memory, and a captured launch
+ * serves every length that the context can hold.  Steps of few segments with few pages run
+ * as thread-block clusters (hy3a_decode_cluster), all others as one grid; the two, and so an
+ * eager and a captured launch of the same step, may differ in the last bits.  q: fp32 [n][64][128] (row stride q_stride), out the same shape
  * (row stride out_stride).  Only the owned KV groups' 8*kv_head_count heads are written.
  * partials (optional, may be NULL): instead of normalised outputs, write one
  * unnormalised {m, l, acc[128]} record per owned head, [n][8*kv_head_count][130] fp32,
@@ -164,8 +168,9 @@ int hy3a_decode_step(hy3a_ctx *ctx, int layer, const float *q_in, size_t q_strid
  * but it leans on scratch buffers that hy3a_create allocated; this variant keeps the scratch of
  * the cross-CTA merge (the {m, l, acc} records and their arrival counters) in a fixed array that
  * is part of the library image, so it works on a context whatever happened to those buffers and
- * never calls cudaMalloc, cudaFree or any allocating routine.  Same arguments and results as
- * hy3a_decode without `partials`.
+ * never calls cudaMalloc, cudaFree or any allocating routine.  Same arguments as hy3a_decode
+ * without `partials`, same results as its grid (where hy3a_decode runs as clusters, the last
+ * bits may differ).
  * Limits: at most 64 (batch row, owned KV head) pairs per call, i.e. 8 rows with all 8 KV heads;
  * larger batches are refused with HY3A_EINVAL.  The array (2.4 MB) is held by every GPU that
  * loads the library until the process exits.  The first call on a device looks the array's
