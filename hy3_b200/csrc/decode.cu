@@ -1124,11 +1124,15 @@ static int spread_folders(const hy3a_ctx *ctx) {
 
 /* A cluster of CTAs per (row, KV head) instead of the grid, where all clusters run at once: of 2, 4 or 8, the least with which a CTA has
  * few pages (kPagesCta; a larger cluster meets later), unless the grid's even share is so much smaller that its fold is paid for
- * (kPagesFold: the difference of 2 to 3 us in pages).  A captured launch meets other lengths when it is replayed, so there the
+ * (kPagesFold: the difference of 2 to 3 us in pages).  Nor where a CTA's stream counts for more than the fold, a ring of 4 (INT8) instead of
+ * 6 pages with it: INT8 beyond 9 pages for a CTA of 8, or beyond 8 for one of 4 on more than 64 CTAs, unless the grid's CTAs walk 16
+ * rows and more to their piece; INT4 beyond 12 pages that are more than 3 above the share.  A captured launch meets other lengths when it is replayed, so there the
  * longest row that the context can hold counts.  Measured back to back, us a layer, grid / clusters of 2 / 4 / 8, 8 KV heads:
  *   INT8   300  7.8  6.4  6.6  7.5    700  8.4  6.6  6.5  7.8   2 500 10.8  9.5  7.4  8.1    8 192 11.2 25.3 15.0 10.9
  *   FP16   300  6.2  5.2  4.8  5.8    700  6.6  6.6  5.8  5.9   2 500 10.4 13.7  9.1  8.3    4 096 10.5 20.2 13.0 10.5
  *   INT4   300  8.6  7.0  6.9  7.7    700  8.7  7.4  7.1  7.8   2 500 11.3 11.1  8.1  8.5   12 000 14.3 29.5 17.6 12.5
+ *   INT8, where the stream counts, grid / clusters: 1 row of 9 600 11.69 / 11.78, 3 rows of 5 000 12.91 / 13.02, 3 of 8 000 15.58 / 17.81,
+ *   4 rows up to 5 000 12.37 / 13.95; 30 rows of 6 000 with 1 head clusters win by 12 %.  INT4: 1 of 14 000 13.60 / 13.83, 4 up to 8 000 14.70 / 15.96
  *   9 rows of 200 / 2 500, clusters of 2: INT8 12.8 -> 10.4 / 17.0 -> 14.9, FP16 10.5 -> 7.6 / 22.0 -> 18.9, INT4 12.4 -> 9.8 / 17.4 -> 14.0 */
 static int cluster_size(const hy3a_ctx *ctx, int most, long long total) {
     static const int kPagesCta[3] = {1, 5, 4}, kPagesFold[3] = {2, 5, 8};      /* FP16, INT8, INT4 */
@@ -1139,7 +1143,10 @@ static int cluster_size(const hy3a_ctx *ctx, int most, long long total) {
     int i = 1;
     while (i < 3 && ((most - 1) >> i) + 1 > kPagesCta[dt] && segs <= ctx->cl_cap[i + 1]) i++;
     const long long share = (total * ctx->cfg.kv_head_count + ctx->decode_ctas - 1) / ctx->decode_ctas;
-    return ((most - 1) >> i) + 1 <= share + kPagesFold[dt] ? 1 << i : 0;
+    const int pages = ((most - 1) >> i) + 1;      /* of the longest row, a CTA */
+    if (dt == HY3A_KV_INT8 && (i == 3 ? pages > 9 : i == 2 && pages > 8 && segs > 16 && ctx->batch_n < 16)) return 0;
+    if (dt == HY3A_KV_INT4 && i > 1 && pages > 12 && pages > share + 3) return 0;
+    return pages <= share + kPagesFold[dt] ? 1 << i : 0;
 }
 static int decode_cluster(const hy3a_ctx *ctx) {
     if ((ctx->shard_slot >= 0 && ctx->shard_world > 1) || ctx->decode_ctas < ctx->sm_count || ctx->no_clusters) return 0;      /* a world of one has nothing to exchange */

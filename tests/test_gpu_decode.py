@@ -406,16 +406,16 @@ def test_errors_are_codes_not_exits(cuda, oracle):
 
 
 @pytest.mark.parametrize("dt", ["fp16", "int8", "int4"])
-@pytest.mark.parametrize("lens,heads", [
-    ([129], (0, 8)), ([300], (0, 8)), ([640], (3, 5)), ([900], (0, 8)), ([2200], (0, 8)), ([257, 1, 128], (0, 8)), ([1500, 700], (6, 2)),
-    ([4200], (7, 1)), ([200, 130, 256, 255, 129, 300, 384, 200, 140], (0, 8)), ([900, 0, 700], (2, 1)), ([1025] * 5, (4, 3))])
-def test_decode_clusters_equal_the_grid(cuda, oracle, dt, lens, heads):
+@pytest.mark.parametrize("lens,heads,sizes", [      # sizes: CTAs per segment with an FP16, INT8, INT4 cache
+    ([129], (0, 8), (2, 2, 2)), ([300], (0, 8), (4, 2, 2)), ([640], (3, 5), (8, 2, 2)), ([900], (0, 8), (8, 2, 2)), ([2200], (0, 8), (8, 4, 8)),
+    ([257, 1, 128], (0, 8), (4, 2, 2)), ([1500, 700], (6, 2), (8, 4, 4)), ([4200], (7, 1), (1, 8, 8)),
+    ([200, 130, 256, 255, 129, 300, 384, 200, 140], (0, 8), (2, 2, 2)), ([900, 0, 700], (2, 1), (8, 2, 2)), ([1025] * 5, (4, 3), (8, 2, 4))])
+def test_decode_clusters_equal_the_grid(cuda, oracle, dt, lens, heads, sizes, monkeypatch):
     """Steps of few segments run as clusters of 2, 4 or 8 CTAs per (row, KV head).  Fewer pages than CTAs, full and one-token last
-    pages, rows without keys, several heads and rows: against the oracle and the grid (the same kernels on a context that is told
-    of one CTA less than the device has SMs), outputs and the cache; repeated launches bit for bit; partial records; the step
-    captured into a graph and replayed for other lengths.  The two differ by the order of fp32 sums and fp16 digits of P (2^-22):
+    pages, rows without keys, several heads and rows: the sizes that the rule gives, against the oracle and the grid (a context
+    without clusters), outputs and the cache; repeated launches bit for bit; partial records; the step captured into a graph and
+    replayed for shorter and longer rows.  The two differ by the order of fp32 sums and fp16 digits of P (2^-22):
     2e-5 is over ten times that at outputs below 4."""
-    import os
     import torch
     from hy3_b200 import Hy3Attn
     h0, nh = heads
@@ -423,19 +423,17 @@ def test_decode_clusters_equal_the_grid(cuda, oracle, dt, lens, heads):
     rng = np.random.default_rng(5)
     q, k, v = (torch.from_numpy(rng.standard_normal((n, h, 128)).astype(np.float32)).to(cuda) for h in (64, 8, 8))
     res = []
-    for ctas in (None, torch.cuda.get_device_properties(0).multi_processor_count - 1):
-        if ctas:
-            os.environ["HY3A_DECODE_CTAS"] = str(ctas)
-        try:
-            ctx = Hy3Attn(kv_dtype=dt, n_layers=2, kv_head_begin=h0, kv_head_count=nh, max_seqs=n, max_batch=n, max_tokens=sum(lens) + 128 * n, max_tokens_per_seq=max(lens) + 128)
-        finally:
-            os.environ.pop("HY3A_DECODE_CTAS", None)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for clusters in (True, False):
+        monkeypatch.setenv("HY3A_NO_CLUSTERS", str(int(not clusters)))
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=2, kv_head_begin=h0, kv_head_count=nh, max_seqs=n, max_batch=n, max_tokens=sum(lens) + 128 * n, max_tokens_per_seq=max(lens) + 128)
         for layer in range(2):
             for i, m in enumerate(lens):
                 if m > 1:
                     ctx.fill_random(layer, i, 0, m - 1, 100 * layer + i)
         slots = [m - 1 for m in lens]
         ctx.batch_set(list(range(n)), slots)
+        assert ctx.decode_cluster() == (sizes[("fp16", "int8", "int4").index(dt)] if clusters else 1) or sms != 148
         outs = []
         for _ in range(4):
             for layer in range(2):
@@ -448,7 +446,7 @@ def test_decode_clusters_equal_the_grid(cuda, oracle, dt, lens, heads):
         ctx.decode_step(0, q, k, v, q_out=qn)
         ctx.sync()
         kv = {i: ctx.export_kv(0, i, 0, m) for i, m in enumerate(lens) if m > 0}
-        # a graph captured for these rows, replayed for shorter ones
+        # a graph captured for these rows, replayed for shorter and for longer ones
         side = torch.cuda.Stream()
         g_out = torch.zeros((n, 64, 128), device=cuda)
         ctx.set_stream(side)
@@ -460,17 +458,20 @@ def test_decode_clusters_equal_the_grid(cuda, oracle, dt, lens, heads):
             ctx.decode_step(1, q, k, v, out=g_out)
         side.synchronize()
         ctx.use_torch_stream()
-        ctx.batch_set(list(range(n)), [max(-1, m - 3) if m > 2 else m - 1 for m in lens])
-        graph.replay()
-        ctx.sync()
-        res.append((outs[0], outs[1], part, g_out.clone(), kv, qn))
+        replays = []
+        for other in ([max(-1, m - 3) if m > 2 else m - 1 for m in lens], [m + 100 for m in lens]):
+            ctx.batch_set(list(range(n)), other)
+            graph.replay()
+            ctx.sync()
+            replays.append(g_out.clone())
+        res.append((outs[0], outs[1], part, torch.stack(replays, 1), kv, qn))
         del graph
         ctx.close()
     own = slice(8 * h0, 8 * (h0 + nh))
     for a, b in zip(res[0][:2], res[1][:2]):
         assert torch.isfinite(a[:, own]).all() and (a[:, own] - b[:, own]).abs().max() < 2e-5
         assert torch.isnan(a[:, :8 * h0]).all() and torch.isnan(a[:, 8 * (h0 + nh):]).all()
-    assert (res[0][3][:, own] - res[1][3][:, own]).abs().max() < 2e-5
+    assert (res[0][3][:, :, own] - res[1][3][:, :, own]).abs().max() < 2e-5
     live = [i for i, m in enumerate(lens) if m > 0]
     for x in (0, 1):
         p = res[x][2][live]
@@ -619,3 +620,19 @@ def test_decode_non_finite_scores(cuda, dt, kind):
         for o in outs:
             assert torch.isnan(o[0, 24:32]).all(), "%d tokens, key %d: dropped" % (ntok, at)
             assert torch.isfinite(o[0, :24]).all() and torch.isfinite(o[0, 32:]).all() and torch.isfinite(o[1:]).all()
+
+
+@pytest.mark.parametrize("lens,heads,sizes", [      # CTAs per segment with an FP16, INT8, INT4 cache
+    ([128], 8, (1, 1, 1)), ([129] * 9, 8, (2, 2, 2)), ([129] * 10, 8, (1, 1, 1)), ([9216], 8, (1, 8, 8)), ([9217], 8, (1, 1, 8)), ([12000], 8, (1, 1, 8)),
+    ([14000], 8, (1, 1, 1)), ([5000] * 2, 8, (1, 4, 4)), ([5000] * 3, 8, (1, 1, 4)), ([8000] * 3, 8, (1, 1, 1)), ([8000] * 4, 8, (4, 1, 4)),
+    ([6000] * 30, 1, (4, 4, 4)), ([20000], 8, (1, 1, 1))])
+def test_decode_cluster_rule(cuda, lens, heads, sizes):
+    """Where the rule takes clusters and where the grid, on 148 SMs (74 / 33 / 15 clusters of 2 / 4 / 8 at once)."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    for dt, size in zip(("fp16", "int8", "int4"), sizes):
+        ctx = Hy3Attn(kv_dtype=dt, n_layers=1, kv_head_count=heads, max_seqs=len(lens), max_batch=len(lens), max_tokens=sum(lens) + 128 * len(lens), max_tokens_per_seq=max(lens))
+        ctx.batch_set(list(range(len(lens))), [m - 1 for m in lens])
+        assert ctx.decode_cluster() == size or torch.cuda.get_device_properties(0).multi_processor_count != 148, dt
+        ctx.sync()
+        ctx.close()
