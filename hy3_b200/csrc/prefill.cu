@@ -815,7 +815,7 @@ static void plan_chunk(hy3a_ctx *ctx, const int *cap, int base_slot, int nq) {
     if (ctx->pf_plan_base == base_slot && ctx->pf_plan_nq == nq) return;
     float end = 0.f;
     hy3a_pf_plan(base_slot, nq, ctx->cfg.kv_head_count, ctx->sm_count, ctx->d_pf_rec ? HY3A_PF_MAX_SLOTS : 0, &ctx->pf_plan, &end);
-    ctx->pf_plan_cluster = ctx->no_clusters ? 1 : hy3a_pf_cluster(base_slot, nq, ctx->cfg.kv_head_count, cap, end, ctx->pf_plan.count > 0);
+    ctx->pf_plan_cluster = ctx->no_clusters ? 1 : hy3a_pf_cluster(base_slot, nq, ctx->cfg.kv_head_count, cap, end, ctx->pf_plan);
     ctx->pf_plan_base = base_slot; ctx->pf_plan_nq = nq;
 }
 

@@ -130,8 +130,9 @@ static inline void hy3a_pf_plan(int base, int nq, int heads, int sms, int max_sl
 
 /* CTAs per block (1: what the plan above says, whose end in steps is `end`, with blocks cut into records or not).  The blocks of a short chunk may run as clusters of 2,
  * 4 or 8 CTAs that share a block's keys evenly and meet in shared memory instead of through records; cap[i]: clusters of 2^i CTAs
- * that fit at once.  The meeting costs kPfCostMeet[i] steps when all 32 query tokens of a block are in use and less in proportion
- * to the softmax warps that hold some (4 tokens each).  Measured, us a launch, 8 heads, whole / with records / clusters of 2 / 4 / 8:
+ * that fit at once.  The meeting costs kPfCostMeet[i] steps when all 32 query tokens of a block are in use, and down to
+ * kPfCostMeet[0] with the softmax warps that hold some (4 tokens each).  Measured, us a launch, 8 heads,
+ * whole / with records / clusters of 2 / 4 / 8:
  *    45 behind  1 001   21.0  21.0  16.2  14.3  24.9      32 behind  4 064   56.9  28.6  36.2  23.9  20.6
  *     2 behind  1 001   18.2  18.2  13.0   9.3   7.6     128 behind  2 000   35.5  27.1  23.9  19.8  48.7
  *   200 behind  1 000   22.9  23.0  18.1  30.2  60.7     128 behind 16 000  230.6  72.9 110.1  67.8 119.5
@@ -139,12 +140,14 @@ static inline void hy3a_pf_plan(int base, int nq, int heads, int sms, int max_sl
  *   600 behind  4 000  116.1 116.0 107.5 130.7      600 behind 16 000  435.7 324.7 350.1 336.2
  * Clusters of 4 and 8 only where all fit at once.  Records stay the better way for few tokens behind a very long history (more than
  * 8 pieces per block) and for a little more than one block per SM. */
-constexpr float kPfCostMeet[4] = {0.f, 3.5f, 5.5f, 10.f};
-static inline int hy3a_pf_cluster(int base, int nq, int heads, const int cap[4], float end, bool records) {
-    const int nqb = (nq + HY3A_PF_QTOK - 1) / HY3A_PF_QTOK;
-    if (nqb > HY3A_PF_MAX_PIECES || end <= 0.f || hy3a_pf_steps(base, nq, nqb - 1) > 65535) return 1;
+constexpr float kPfCostMeet[4] = {0.8f, 3.5f, 5.5f, 10.f};
+static inline int hy3a_pf_cluster(int base, int nq, int heads, const int cap[4], float end, const hy3a_pf_table &plan) {
+    const int nqb = (nq + HY3A_PF_QTOK - 1) / HY3A_PF_QTOK, longest = hy3a_pf_steps(base, nq, nqb - 1);
+    if (nqb > HY3A_PF_MAX_PIECES || end <= 0.f || longest > 65535) return 1;
     int best = 1;
     const float used = std::min(8, (nq + 3) / 4) * 0.125f;
+    int np = 0;
+    for (int c = 0; c < plan.count; c++) np = std::max(np, (int)plan.e[c].np);
     hy3a_pf_table t;
     t.count = nqb;
     for (int i = 1; i < 4; i++) {
@@ -155,9 +158,13 @@ static inline int hy3a_pf_cluster(int base, int nq, int heads, const int cap[4],
             t.e[c].n = (uint16_t)((hy3a_pf_steps(base, nq, nqb - 1 - c) + cl - 1) / cl);
             t.e[c].np = 1;
         }
-        /* the model of the records is 2 to 4 us low (above), that of several rounds of clusters on every SM a few percent */
-        const float limit = best == 1 ? end * (at_once ? (records ? 1.15f : 1.f) : 0.97f) : end;
-        const float m = hy3a_pf_makespan(&t, heads, cap[i], limit, kPfCostMeet[i] * used);
+        /* the model of the records is up to 4 us low, and 0.6 of their fold goes with the tokens in use; that of several rounds of
+         * clusters on every SM is a few percent low */
+        float limit = end;
+        /* a step of at most 4 tokens takes 0.2 longer (2 behind 16 000: 39.5 with records, 44.4 in clusters of 8; 8 tokens 37.8 and 38.1) */
+        const float slow = nq <= 4 && np > 1 ? 0.2f * longest * (1.f / cl - 1.f / np) : 0.f;
+        if (best == 1) limit = !at_once ? 0.97f * end : np > 1 ? end + 1.f + 3.6f * used - 0.6f * kPfCostFold * np * (1.f - used) - slow : end;
+        const float m = hy3a_pf_makespan(&t, heads, cap[i], limit, kPfCostMeet[0] + (kPfCostMeet[i] - kPfCostMeet[0]) * used);
         if (m < limit) { best = cl; end = m; }
     }
     return best;

@@ -188,6 +188,18 @@ def test_prefill_clusters(cuda, oracle, dt, base, nq, heads, size):
             check_attention(got[i, own], want[i, own], "%s base=%d nq=%d row %d" % (dt, base, nq, i))
 
 
+@pytest.mark.parametrize("base,nq,heads,size", [
+    (100, 8, 8, 1), (500, 2, 4, 8), (8192, 2, 8, 8), (8192, 45, 8, 4), (16000, 2, 8, 1), (16000, 30, 8, 8), (16000, 200, 8, 1), (16000, 256, 8, 2),
+    (30000, 8, 8, 1), (30000, 30, 8, 1), (4064, 300, 4, 1), (16000, 2048, 8, 2)])
+def test_prefill_cluster_rule(cuda, base, nq, heads, size):
+    """Where the rule takes clusters and where records or whole blocks, on 148 SMs (74 / 33 / 15 clusters of 2 / 4 / 8 at once)."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    ctx = Hy3Attn(kv_dtype="int4", n_layers=1, max_batch=max(16, nq), max_tokens=base + nq, kv_head_count=heads)
+    assert ctx.prefill_cluster(base, nq) == size or torch.cuda.get_device_properties(0).multi_processor_count != 148
+    ctx.close()
+
+
 @pytest.mark.parametrize("dt,base,nq,heads", [("int8", 2500, 500, (3, 5)), ("int4", 500, 1500, (2, 2)), ("fp16", 4500, 150, (0, 8))])
 def test_prefill_records_where_no_cluster_pays(cuda, oracle, dt, base, nq, heads, monkeypatch):
     """Chunks that still leave records: the checks of the grids above."""
