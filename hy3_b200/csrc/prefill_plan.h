@@ -158,12 +158,12 @@ static inline int hy3a_pf_cluster(int base, int nq, int heads, const int cap[4],
             t.e[c].n = (uint16_t)((hy3a_pf_steps(base, nq, nqb - 1 - c) + cl - 1) / cl);
             t.e[c].np = 1;
         }
-        /* the model of the records is up to 4 us low, and 0.6 of their fold goes with the tokens in use; that of several rounds of
+        /* the model of the records is up to 4 us low, and 0.7 of their fold goes with the tokens in use; that of several rounds of
          * clusters on every SM is a few percent low */
         float limit = end;
         /* a step of at most 4 tokens takes 0.2 longer (2 behind 16 000: 39.5 with records, 44.4 in clusters of 8; 8 tokens 37.8 and 38.1) */
         const float slow = nq <= 4 && np > 1 ? 0.2f * longest * (1.f / cl - 1.f / np) : 0.f;
-        if (best == 1) limit = !at_once ? 0.97f * end : np > 1 ? end + 1.f + 3.6f * used - 0.6f * kPfCostFold * np * (1.f - used) - slow : end;
+        if (best == 1) limit = !at_once ? 0.97f * end : np > 1 ? end + 1.f + 3.6f * used - 0.7f * kPfCostFold * np * (1.f - used) - slow : end;
         const float m = hy3a_pf_makespan(&t, heads, cap[i], limit, kPfCostMeet[0] + (kPfCostMeet[i] - kPfCostMeet[0]) * used);
         if (m < limit) { best = cl; end = m; }
     }

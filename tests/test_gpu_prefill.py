@@ -189,7 +189,7 @@ def test_prefill_clusters(cuda, oracle, dt, base, nq, heads, size):
 
 
 @pytest.mark.parametrize("base,nq,heads,size", [
-    (100, 8, 8, 1), (500, 2, 4, 8), (8192, 2, 8, 8), (8192, 45, 8, 4), (16000, 2, 8, 1), (16000, 30, 8, 8), (16000, 200, 8, 1), (16000, 256, 8, 2),
+    (100, 8, 8, 1), (500, 2, 4, 8), (8192, 2, 8, 8), (8192, 45, 8, 4), (16000, 2, 8, 1), (16000, 8, 8, 1), (16000, 30, 8, 8), (16000, 200, 8, 1), (16000, 256, 8, 2),
     (30000, 8, 8, 1), (30000, 30, 8, 1), (4064, 300, 4, 1), (16000, 2048, 8, 2)])
 def test_prefill_cluster_rule(cuda, base, nq, heads, size):
     """Where the rule takes clusters and where records or whole blocks, on 148 SMs (74 / 33 / 15 clusters of 2 / 4 / 8 at once)."""
