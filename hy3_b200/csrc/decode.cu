@@ -130,10 +130,16 @@ __device__ __forceinline__ unsigned cvt_u4_hi(unsigned x) {
  * 16+4tig..16+4tig+3) carry head dims kdim32<DT>(kk, tig, 0..7).  In both cases these are
  * exactly the dims whose codes the thread gets out of its own 16-byte loads.              */
 __device__ __forceinline__ int kdim16(int j, int tig, int s) { int c = tig + 4 * (j >> 1); return 8 * c + 4 * (j & 1) + s; }
-/* ---- output-dimension map of P.V: n-block jn (0..15), column n (0..7) -> head dim. */
-template <int DT> __device__ __forceinline__ int vdim(int jn, int n) {
-    if (DT == 2) return 16 * n + jn;
-    return 8 * n + 64 * (jn >> 3) + (jn & 7);
+/* ---- output-dimension map of P.V: n-block jn (0..15), column n (0..7) -> head dim 16 n + jn (INT4) or 8 n + 64 (jn >> 3) + (jn & 7) (FP16):
+ * a lane (columns 2 tig, 2 tig + 1) holds 32 (INT4) or twice 16 (FP16) consecutive dims of its head. */
+
+/* Where a warp's piece keeps 16-byte chunk `chunk` (of 32) of head h's row while the warps of a CTA are folded.  The eight lanes of a
+ * store (two heads, four tig) hold the same chunk of dims that are 128 or 64 bytes apart: unswizzled they met in one (INT4) or
+ * two (FP16) groups of four banks and went out one or two at a time, 256 or 128 wavefronts for each of 11 warps.  us a layer before / with it:
+ * 700 tokens (INT4 clusters) 7.5 -> 6.7 together with the fragments that the queries' warps write themselves, 8 ragged INT4 rows 19.6 -> 18.9,
+ * FP16 32 768 28.1 -> 27.9. */
+template <int DT> __device__ __forceinline__ int stage_chunk(int h, int chunk) {
+    return DT == 2 ? chunk ^ ((chunk >> 3) + 4 * (h & 1)) : chunk ^ (((chunk >> 3) & 1) + 2 * (h & 1));
 }
 
 struct warp_state {
@@ -748,11 +754,17 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             l += __shfl_xor_sync(0xffffffffu, l, 2);
             if (tig == 0) { s_ml[warp][g][0] = st.m; s_ml[warp][g][1] = l; }
             const float inv_ps = 1.f / pscale;
+            /* the lane's 32 dims as eight 16-byte chunks: o[4q + j][b] is dim 16 (2 tig + b) + 4q + j (INT4) or
+             * 64 (q >> 1) + 8 (2 tig + b) + 4 (q & 1) + j (FP16) */
 #pragma unroll
-            for (int jn = 0; jn < 16; jn++) {
-                s_o[warp][g][vdim<DT>(jn, 2 * tig)] = (st.o[jn][0] + st.o[jn][2]) * inv_ps;
-                s_o[warp][g][vdim<DT>(jn, 2 * tig + 1)] = (st.o[jn][1] + st.o[jn][3]) * inv_ps;
-            }
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int b = 0; b < 2; b++) {
+                    const int chunk = DT == 2 ? 8 * tig + 4 * b + q : 16 * (q >> 1) + 4 * tig + 2 * b + (q & 1);
+                    *reinterpret_cast<float4 *>(&s_o[warp][g][4 * stage_chunk<DT>(g, chunk)]) =
+                        make_float4((st.o[4 * q][b] + st.o[4 * q][b + 2]) * inv_ps, (st.o[4 * q + 1][b] + st.o[4 * q + 1][b + 2]) * inv_ps,
+                                    (st.o[4 * q + 2][b] + st.o[4 * q + 2][b + 2]) * inv_ps, (st.o[4 * q + 3][b] + st.o[4 * q + 3][b + 2]) * inv_ps);
+                }
         }
         consumer_sync();
         const bool red = tid < 256;                            /* the first 8 warps do the reductions */
@@ -767,7 +779,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             if (ml.y == 0.f) continue;
             const float f = ex2(ml.x - M);
             L += ml.y * f;
-            float4 o4 = *reinterpret_cast<const float4 *>(&s_o[w][h][d4]);
+            const float4 o4 = *reinterpret_cast<const float4 *>(&s_o[w][h][4 * stage_chunk<DT>(h, lane)]);
             acc[0] += o4.x * f; acc[1] += o4.y * f; acc[2] += o4.z * f; acc[3] += o4.w * f;
         }
         if (CL) {
