@@ -308,14 +308,6 @@ __device__ __forceinline__ float2 unpack_h2(unsigned v) {
     __half2 h = *reinterpret_cast<__half2 *>(&v);
     return __half22float2(h);
 }
-/* INT8/INT4 caches, Q.K^T on m16n8k32: for k-step kk (0..3) the eight k-slots (4tig..4tig+3, 16+4tig..16+4tig+3) of
- * thread-in-group tig carry head dims kdim32<DT>(kk, tig, 0..7): exactly the dims whose codes the thread gets out of its own
- * 16-byte loads of a K row. */
-template <int DT> __device__ __forceinline__ int kdim32(int kk, int tig, int s) {
-    if (DT == 1) return 16 * (tig + 4 * (s >> 2)) + 4 * kk + (s & 3);   /* chunk tig / tig+4, word kk */
-    return 32 * tig + 8 * kk + 2 * (s & 3) + (s >> 2);                   /* word kk: even nibbles, then odd nibbles */
-}
-
 /* Sequence sharding: lines of one head's record in a gather buffer: line 0 = {m, l}, line 1 + j = acc[2j], acc[2j+1]. */
 constexpr int kShardLines = HY3A_PARTIAL_FLOATS / 2;   /* 65 */
 __device__ __forceinline__ void shard_store_line(uint4 *p, float x, float y, unsigned flag) {

@@ -81,8 +81,7 @@ constexpr int kOffLand = 0;                          /* landing zone of records 
 constexpr int kLandBytes = kSlots * 2048;
 constexpr unsigned kLate = HY3A_LATE, kLateCut = HY3A_LATE_CUT;      /* the last pieces of a single-row grid start late: they take fewer pages */
 constexpr int kOffQ = kOffPt + kSlots * 2048;        /* Q fragments [4 k-steps][32 lanes] x 16 B */
-constexpr int kOffQ8 = kOffQ + 2048;                 /* Q digits [2][8][128] int8 */
-constexpr int kOffMisc = kOffQ8 + 2048;
+constexpr int kOffMisc = kOffQ + 2048;
 constexpr int kOffClu = kOffMisc + ((sizeof(u_misc) + 127) / 128) * 128;      /* a cluster's landing zone, at the cost of two pages of the ring */
 constexpr int kStagesClu = kStages - 2;
 template <int CL> constexpr int kOffPrefix = kOffClu + (CL ? (kCluBytes + 127) / 128 * 128 : 0);
@@ -638,14 +637,13 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         const int k_off0 = hy3a_k_chunk_off<1>(g, tig), k_off1 = hy3a_k_chunk_off<1>(g, tig + 4);
         const unsigned sq = s_base + kOffQ + 16u * (unsigned)lane;
         uint4 (*s_q)[32] = reinterpret_cast<uint4 (*)[32]>(s_dyn + kOffQ);
-        signed char *s_q8 = reinterpret_cast<signed char *>(s_dyn + kOffQ8);
         unsigned it = 0;
         long long u = u_begin;
         while (u < u_end) {
             const segment sg = locate(s_prefix, batch, n, G, u, u_end);
             const int row = sg.row, hl = sg.hl, sidx = sg.sidx;
             const int head0 = (cache.kv_head_begin + hl) * 8;
-            /* ---- Q digits of the segment's 8 heads, packed as MMA A fragments (as in decode.cu) */
+            /* ---- Q digits of the segment's 8 heads as MMA A fragments, straight from the registers of the warp that prepared the row */
             if (qw < 8) {
                 float x[4];
                 if (a.fused) {
@@ -672,21 +670,13 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                     hw |= ((unsigned)(int)hi & 0xFFu) << (8 * j);
                     lw |= ((unsigned)(int)lo & 0xFFu) << (8 * j);
                 }
-                *reinterpret_cast<unsigned *>(s_q8 + qw * HY3A_D + rl_d0) = hw;
-                *reinterpret_cast<unsigned *>(s_q8 + (8 + qw) * HY3A_D + rl_d0) = lw;
+                /* MMA k-step kk, k-slots 4tig..4tig+3 / 16+4tig..16+4tig+3 of thread-in-group tig carry head dims 16 tig + 4 kk + 0..3 /
+                 * 64 + the same: exactly what a thread gets out of its own 16-byte loads of a K row.  The lane's four dims are one of these
+                 * halves, kk = lane & 3, tig = (lane & 15) >> 2: words 2 (lane >> 4) (high digits, rows 0-7) and the one behind it (low
+                 * digits, rows 8-15) of that fragment.  (Gathered from a staged copy: a second barrier and 16 byte loads, 700 tokens 7.45
+                 * instead of 7.39 us a layer.) */
+                *reinterpret_cast<uint2 *>(reinterpret_cast<unsigned *>(&s_q[lane & 3][4 * qw + ((lane & 15) >> 2)]) + 2 * (lane >> 4)) = make_uint2(hw, lw);
                 if (lane == 0) mi.qf[qw] = sqv * (1.f / 254.f) * 0.08838834764831845f * kLog2e;
-            }
-            qk_sync();
-            if (qtid < 128) {
-                const int kk = qtid >> 5;
-                unsigned w[4] = {0, 0, 0, 0};
-#pragma unroll
-                for (int s2 = 0; s2 < 8; s2++) {
-                    const int d = kdim32<1>(kk, tig, s2);
-                    w[2 * (s2 >> 2)] |= ((unsigned)(unsigned char)s_q8[g * HY3A_D + d]) << (8 * (s2 & 3));
-                    w[2 * (s2 >> 2) + 1] |= ((unsigned)(unsigned char)s_q8[(8 + g) * HY3A_D + d]) << (8 * (s2 & 3));
-                }
-                s_q[kk][lane] = make_uint4(w[0], w[1], w[2], w[3]);
             }
             qk_sync();
             const float qf = mi.qf[g];
