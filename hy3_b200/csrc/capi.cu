@@ -287,8 +287,8 @@ int hy3a_create(const hy3a_config *cfg, hy3a_ctx **out) {
     CREATE_CUDA(cudaMalloc(&ctx->d_batch, (size_t)3 * cfg->max_batch * sizeof(int)));
     ctx->partial_records = (size_t)ctx->decode_ctas + (size_t)cfg->max_batch * cfg->kv_head_count;
     CREATE_CUDA(cudaMalloc(&ctx->d_partials, ctx->partial_records * 8 * HY3A_REC_FLOATS * sizeof(float)));
-    CREATE_CUDA(cudaMalloc(&ctx->d_counters, (size_t)2 * cfg->max_batch * cfg->kv_head_count * sizeof(unsigned)));
-    CREATE_CUDA(cudaMemsetAsync(ctx->d_counters, 0, (size_t)2 * cfg->max_batch * cfg->kv_head_count * sizeof(unsigned), ctx->stream));
+    CREATE_CUDA(cudaMalloc(&ctx->d_counters, HY3A_COUNTERS((size_t)cfg->max_batch * cfg->kv_head_count) * sizeof(unsigned)));
+    CREATE_CUDA(cudaMemsetAsync(ctx->d_counters, 0, HY3A_COUNTERS((size_t)cfg->max_batch * cfg->kv_head_count) * sizeof(unsigned), ctx->stream));
     CREATE_CUDA(cudaMalloc(&ctx->d_err, HY3A_ERR_WORDS * sizeof(unsigned)));
     CREATE_CUDA(cudaMemsetAsync(ctx->d_err, 0, HY3A_ERR_WORDS * sizeof(unsigned), ctx->stream));
     /* records of the chunked prefill's cut blocks (contexts that take chunks; without room the blocks stay uncut) */
@@ -379,7 +379,7 @@ int hy3a_sync(hy3a_ctx *ctx) {
         unsigned code = ctx->h_err[0], where = ctx->h_err[1], w2 = ctx->h_err[2], w3 = ctx->h_err[3];
         cudaMemsetAsync(ctx->d_err, 0, HY3A_ERR_WORDS * sizeof(unsigned), ctx->stream);
         /* a kernel that gave up may have left merge counters behind */
-        cudaMemsetAsync(ctx->d_counters, 0, (size_t)2 * ctx->cfg.max_batch * ctx->cfg.kv_head_count * sizeof(unsigned), ctx->stream);
+        cudaMemsetAsync(ctx->d_counters, 0, HY3A_COUNTERS((size_t)ctx->cfg.max_batch * ctx->cfg.kv_head_count) * sizeof(unsigned), ctx->stream);
         if (ctx->d_pf_cnt) cudaMemsetAsync(ctx->d_pf_cnt, 0, (size_t)HY3A_PF_MAX_SLOTS * 8 * sizeof(unsigned), ctx->stream);
         return hy3a_fail(ctx, HY3A_ETIMEOUT, "device-side bounded wait or bounds check failed (code %u, where %u, detail %u %u)", code, where, w2, w3);
     }

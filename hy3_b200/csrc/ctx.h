@@ -17,7 +17,8 @@
 #define HY3A_UMMA_STAGES 6    /* pages in the shared-memory ring of the INT8 decode kernel */
 #endif
 #define HY3A_ERR_WORDS 4
-#define HY3A_REC_FLOATS 132   /* a head's {m, l, acc[128]} record in the merge scratch, padded to a multiple of 16 bytes */
+#define HY3A_REC_FLOATS 132   /* a head's {acc[128], m, l} record in the merge scratch, padded to a multiple of 16 bytes */
+#define HY3A_COUNTERS(segments) ((size_t)9 * (segments))   /* counters of the merge: [segments][8] arrivals, [segments] finished folds */
 #define HY3A_RING_SLOTS 16
 
 /* Everything a kernel needs to address the cache; passed by value. */
@@ -67,7 +68,7 @@ struct hy3a_ctx {
     float *d_norm_w;      /* [n_layers][2][128] */
     int *d_batch;         /* [3][max_batch] seq, slot, pos */
     float *d_partials;    /* decode scratch: [(ctas + max_batch*kv_heads)][8][HY3A_REC_FLOATS] */
-    unsigned int *d_counters; /* decode scratch: [2][max_batch*kv_heads] arrival / finished-fold counters (self-resetting) */
+    unsigned int *d_counters; /* decode scratch: HY3A_COUNTERS(max_batch*kv_heads), self-resetting */
     void *d_pf_k, *d_pf_v; /* prefill: fp16 operands shared by all layers, rebuilt per call (used when a layer has no mirror) */
     size_t pf_bytes;
     /* prefill operand mirrors: per layer, the fp16 tensor-core image (K rows, V transposed) of ONE sequence's tokens

@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             if (red) cluster_send<CL ? CL : 1>(smem_u32(s_dyn) + kFixedHead, bar_base + kBarClu, cta % (CL ? CL : 1), h, lane, M, L, acc);
             break;
         }
-        consumer_sync(); /* s_o / s_ml free again */
+        if (SHARD) consumer_sync();      /* s_o / s_ml are landing zones below; else they are written again behind the next segment's queries */
 
         /* ---- how many CTAs share this segment? */
         const int c_first = aligned ? al_first : (int)(((sg.seg_u0 + 1) * C + U - 1) / U) - 1;
@@ -781,21 +781,18 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         /* Which of the 8 heads this CTA finishes (writes out / exchanges): all of them, unless the fold of a
          * segment is spread over several of its CTAs (below). */
         int h_lo = 0, h_hi = 8;
+        bool last = true;      /* this warp has its head's final record */
+        float *const recs = a.scratch + ((size_t)(c_first + rec_base) * 8 + h) * kRecFloats;      /* of the segment's piece 0 */
         if (npieces > 1) {
-            if (red) {
-                float *rec = a.scratch + ((size_t)(cta + rec_base) * 8 + h) * kRecFloats;
-                if (d4 == 0) { rec[0] = M; rec[1] = L; }
-                rec[2 + d4] = acc[0]; rec[3 + d4] = acc[1]; rec[4 + d4] = acc[2]; rec[5 + d4] = acc[3];
-            }
-            consumer_sync();   /* the record is complete in CTA scope; the release below publishes it */
             if (STAGED && aligned && a.spread) {
                 /* ---- CTA-aligned segments (small batches): the fold is SPREAD.  Every CTA announces its record on
                  * the segment's arrival counter; the first F pieces then each fold 8/F of the heads over all pieces
-                 * (one warp per head: 33 16-byte asynchronous copies per record and lane 0 one more, all records in
-                 * flight at once, landing in the idle page ring), instead of one CTA pulling every head of every
-                 * piece while the others have left.  The remaining pieces leave at once.                          */
+                 * (one warp per head), instead of one CTA pulling every head of every piece while the others have
+                 * left.  The remaining pieces leave at once.                                                      */
                 const int Fmax = a.spread, F = npieces >= Fmax ? Fmax : (npieces >= 4 && Fmax >= 4 ? 4 : (npieces >= 2 && Fmax >= 2 ? 2 : 1)), hpf = 8 / F, piece = cta - c_first;
-                if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.counters + sidx) : "memory");
+                if (red) store_record(recs + (size_t)piece * 8 * kRecFloats, lane, M, L, acc);
+                consumer_sync();   /* the record is complete in CTA scope; the release publishes it */
+                if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.counters + 8 * sidx) : "memory");
                 if (piece >= F) continue;   /* CTA-uniform */
                 if (tid == 0) {
                     /* bounded wait for the other pieces (they are resident: one CTA per SM at most) */
@@ -803,7 +800,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                     unsigned long long t0 = 0;
                     bool ok = false;
                     for (unsigned i = 0; i < (1u << 24); i++) {
-                        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.counters + sidx) : "memory");
+                        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.counters + 8 * sidx) : "memory");
                         if (seen >= (unsigned)npieces) { ok = true; break; }
                         if ((i & 255u) == 255u) {
                             unsigned long long t1;
@@ -820,79 +817,27 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 const bool mine = red && h >= h_lo && h < h_hi;
                 M = -INFINITY; L = 0.f; acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
                 if (s_flag && mine) {
-                    /* landing zone of head h: npieces x 528 bytes in the ring (idle: this CTA's pages are consumed) */
-                    const unsigned zone = (unsigned)((h - h_lo) * npieces) * (unsigned)(kRecFloats * 4);
-                    const uint8_t *src = reinterpret_cast<const uint8_t *>(a.scratch + ((size_t)c_first * 8 + h) * kRecFloats);
-                    for (int c = 0; c < npieces; c++) {
-                        const unsigned dst = ring_base + zone + (unsigned)c * (unsigned)(kRecFloats * 4);
-                        const uint8_t *g = src + (size_t)c * 8 * kRecFloats * 4;
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (unsigned)lane), "l"(g + 16 * lane) : "memory");
-                        if (lane == 0) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512u), "l"(g + 512) : "memory");
-                    }
-                    asm volatile("cp.async.wait_all;" ::: "memory");
-                    __syncwarp();
-                    const float *zf = reinterpret_cast<const float *>(s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + zone);
-                    for (int c = 0; c < npieces; c++) {
-                        const float *pr = zf + (size_t)c * kRecFloats;
-                        const float pm = pr[0], pl = pr[1];
-                        if (pl == 0.f) continue;
-                        const float2 v01 = *reinterpret_cast<const float2 *>(pr + 2 + d4), v23 = *reinterpret_cast<const float2 *>(pr + 4 + d4);
-                        const float nm = fmaxf(M, pm), os = ex2(M - nm), rs = ex2(pm - nm);
-                        L = L * os + pl * rs;
-                        acc[0] = acc[0] * os + v01.x * rs; acc[1] = acc[1] * os + v01.y * rs;
-                        acc[2] = acc[2] * os + v23.x * rs; acc[3] = acc[3] * os + v23.y * rs;
-                        M = nm;
-                    }
+                    const int slots = min(32, a.stages * geom.page_bytes / (hpf * 512));      /* the ring is idle: this CTA's pages are consumed */
+                    fold_records(recs, npieces, s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + (h - h_lo) * slots * 512, 512u, slots, lane, M, L, acc);
                 }
                 consumer_sync();   /* every landing zone is read (the sharded exchange lands its lines in the ring too) */
                 if (tid == 0) {
                     /* the last of the F folders puts both counters back to zero for the next launch */
-                    const unsigned old = atomicAdd(a.counters + a.n_counters + sidx, 1u);
-                    if (old == (unsigned)(F - 1)) { a.counters[sidx] = 0u; a.counters[a.n_counters + sidx] = 0u; }
+                    unsigned *done = a.counters + 8 * a.n_counters + sidx;
+                    const unsigned old = atomicAdd(done, 1u);
+                    if (old == (unsigned)(F - 1)) { a.counters[8 * sidx] = 0u; *done = 0u; }
                 }
             } else {
-                /* ---- a CTA may hold pieces of several segments (large batches): the LAST CTA to arrive folds, nobody waits */
-                if (tid == 0) {
-                    unsigned old;
-                    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(a.counters + sidx) : "memory");
-                    s_flag = (old == (unsigned)(npieces - 1));
-                }
-                consumer_sync();
-                if (!s_flag) continue;   /* CTA-uniform */
-                /* fold all pieces with the rule of hy3_gpu.cu:233-247.  The pieces' records (contiguous) are fetched
-                 * into the merge buffer with 16-byte asynchronous copies issued by all threads at once and folded
-                 * from there; larger segments go through it in several rounds.                                    */
-                const unsigned land = smem_u32(s_dyn);
-                const float *land_g = reinterpret_cast<const float *>(s_dyn);
-                const int land_cap = kFixedO / (8 * kRecFloats * 4);
-                M = -INFINITY; L = 0.f; acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-                for (int c0 = 0; c0 < npieces; c0 += land_cap) {
-                    const int nc = min(land_cap, npieces - c0);
-                    const uint8_t *src = reinterpret_cast<const uint8_t *>(a.scratch + (size_t)(c_first + c0 + rec_base) * 8 * kRecFloats);
-                    for (int i = tid; i < nc * (8 * kRecFloats / 4); i += kThreads)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(land + 16u * (unsigned)i), "l"(src + 16 * (size_t)i) : "memory");
-                    asm volatile("cp.async.wait_all;" ::: "memory");
-                    consumer_sync();
-                    if (red) {
-                        for (int c = 0; c < nc; c++) {
-                            const float *pr = land_g + ((size_t)c * 8 + h) * kRecFloats;
-                            const float pm = pr[0], pl = pr[1];
-                            if (pl == 0.f) continue;
-                            const float2 v01 = *reinterpret_cast<const float2 *>(pr + 2 + d4), v23 = *reinterpret_cast<const float2 *>(pr + 4 + d4);
-                            const float nm = fmaxf(M, pm), os = ex2(M - nm), rs = ex2(pm - nm);
-                            L = L * os + pl * rs;
-                            acc[0] = acc[0] * os + v01.x * rs; acc[1] = acc[1] * os + v01.y * rs;
-                            acc[2] = acc[2] * os + v23.x * rs; acc[3] = acc[3] * os + v23.y * rs;
-                            M = nm;
-                        }
-                    }
-                    if (c0 + land_cap < npieces) consumer_sync();   /* landing zone is reused */
-                }
-                if (tid == 0) a.counters[sidx] = 0u; /* self-reset for the next launch */
-                consumer_sync();   /* the landing zone is read; the next segment may reuse the buffer */
+                /* The last CTA to arrive folds, nobody waits.  The records land in the page ring where it is idle (whole CTAs to a segment:
+                 * this CTA's pages are consumed), else in the head's column of s_o, which this warp alone has read. */
+                const bool ring = STAGED && aligned;
+                const int slots = ring ? min(32, a.stages * geom.page_bytes / 4096) : kWarps;
+                uint8_t *const zone = ring ? s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + h * slots * 512 : reinterpret_cast<uint8_t *>(s_o[0][h]);
+                if (red) last = fold_last(recs, cta - c_first, npieces, a.counters + 8 * sidx + h, zone, ring ? 512u : (unsigned)sizeof(s_o[0]), slots, lane, M, L, acc);
+                if (SHARD) consumer_sync();      /* the exchange lands its lines there too */
             }
         }
-        const bool fin = red && h >= h_lo && h < h_hi;   /* this thread finishes its (head, 4 dims) of the segment */
+        const bool fin = red && last && h >= h_lo && h < h_hi;   /* this thread finishes its (head, 4 dims) of the segment */
         if (SHARD) {
             /* sequence sharding: this rank's records of the segment go into every other rank's gather buffer as
              * flagged lines (no fence, no separate flag: a line is valid when both of its flag words carry this
@@ -1100,21 +1045,9 @@ static_assert(kRecFloats >= HY3A_PARTIAL_FLOATS && (kRecFloats * 4) % 16 == 0, "
 /* Folders per segment of the spread fold (0: the last CTA to arrive folds).  It pays off where the epilogue is the cross-GPU
  * exchange (several CTAs store to the peers instead of one); on one GPU the folders only hold their SMs longer, which delays the
  * next launch's CTAs there.  Its folders wait for the other pieces, so every CTA of the grid must be resident.  4 measured best
- * on 8 GPUs (8: 28.8, 4: 27.8, 2: 27.8, 1: 29.2 us per layer).  A folder lands 8 / F heads x pieces records in the page ring: a
- * segment has up to CTAs / KV heads pieces, and no more than hy3a_most_pieces of the longest row that the context can hold where
- * pieces are not of even size (a launch may be replayed for any row, so the batch at hand does not count).  With one KV head and rows
- * beyond 413 696 (FP16) or 430 080 tokens (INT4), 2 x 125 or 2 x 129 records exceed the rings of 131 and 135 KB.  Then 8 folders take
- * one head each; a ring too small for that too keeps the plain fold.
- * (Segments of fewer than F pieces have fewer folders: 4 heads x 3 pieces = 6.3 KB at most.) */
+ * on 8 GPUs (8: 28.8, 4: 27.8, 2: 27.8, 1: 29.2 us per layer). */
 static int spread_folders(const hy3a_ctx *ctx) {
-    if (ctx->shard_slot < 0 || ctx->decode_ctas > ctx->sm_count) return 0;
-    const int dt = ctx->geom.dtype, heads = ctx->cfg.kv_head_count;
-    const size_t ring = (size_t)(dt == HY3A_KV_INT8 ? HY3A_UMMA_STAGES : ctx->decode_stages) * ctx->geom.page_bytes;
-    size_t pieces = (size_t)(ctx->decode_ctas / heads);
-    if (dt == HY3A_KV_INT8 || !hy3a_even_applies(ctx->batch_n, heads, (unsigned)ctx->decode_ctas))
-        pieces = std::min(pieces, (size_t)hy3a_most_pieces((unsigned)ctx->cfg.max_blocks_per_seq));
-    for (int f = 4; f <= 8; f *= 2) if ((size_t)(8 / f) * pieces * kRecFloats * 4 <= ring) return f;
-    return 0;
+    return ctx->shard_slot < 0 || ctx->decode_ctas > ctx->sm_count ? 0 : 4;
 }
 
 /* A cluster of CTAs per (row, KV head) instead of the grid, where all clusters run at once: of 2, 4 or 8, the least with which a CTA has
@@ -1202,11 +1135,12 @@ int hy3a_launch_decode(hy3a_ctx *ctx, int layer, const float *q, size_t q_stride
  * Scratch for hy3a_decode_noalloc: the records and arrival counters of the cross-CTA merge live in
  * this file-scope device array instead of buffers the context allocated.  Every GPU that loads the
  * library holds these 2.4 MB until the process exits.  Layout: [kNoAllocRecords][8][132] floats of
- * records, then two counters (arrivals, finished folds) per segment.                                               */
+ * records, then the counters (HY3A_COUNTERS) of the segments.                                               */
 constexpr int kNoAllocRows = 64;                                   /* most (batch row, KV head) segments per call */
 constexpr int kNoAllocRecords = 512 + kNoAllocRows;                /* one per CTA of the largest grid + one per segment */
 constexpr size_t kNoAllocRecordBytes = (size_t)kNoAllocRecords * 8 * kRecFloats * sizeof(float);
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocRecordBytes + 2 * kNoAllocRows * sizeof(unsigned)];
+constexpr size_t kNoAllocCounterBytes = HY3A_COUNTERS(kNoAllocRows) * sizeof(unsigned);
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocRecordBytes + kNoAllocCounterBytes];
 static unsigned char *g_noalloc_ptr[64];                           /* device address of the array, per device ordinal */
 
 extern "C" int hy3a_decode_noalloc(hy3a_ctx *ctx, int layer, const float *q, size_t q_stride, float *out, size_t out_stride) {
@@ -1236,7 +1170,7 @@ extern "C" int hy3a_decode_noalloc(hy3a_ctx *ctx, int layer, const float *q, siz
     }
     unsigned char *scratch = g_noalloc_ptr[ctx->device];
     /* the arrival counters must start at zero; a call that was cut short may have left some behind */
-    HY3A_CUDA(ctx, cudaMemsetAsync(scratch + kNoAllocRecordBytes, 0, 2 * kNoAllocRows * sizeof(unsigned), ctx->stream));
+    HY3A_CUDA(ctx, cudaMemsetAsync(scratch + kNoAllocRecordBytes, 0, kNoAllocCounterBytes, ctx->stream));
     decode_args a;
     memset(&a, 0, sizeof(a));
     a.q = q; a.q_stride = q_stride; a.out = out; a.out_stride = out_stride;

@@ -86,7 +86,7 @@ constexpr int kOffClu = kOffMisc + ((sizeof(u_misc) + 127) / 128) * 128;      /*
 constexpr int kStagesClu = kStages - 2;
 template <int CL> constexpr int kOffPrefix = kOffClu + (CL ? (kCluBytes + 127) / 128 * 128 : 0);
 static_assert(kShardBatchU * 8 * (HY3A_PARTIAL_FLOATS / 2) * 16 <= kLandBytes, "landing zone too small for the exchange");
-static_assert(8 * kRecFloats * 4 <= kLandBytes && 8 * HY3A_D * 4 <= kLandBytes, "landing zone too small for a record / the hand-over");
+static_assert(8 * HY3A_D * 4 == 4096 && kLandBytes >= 2 * 4096, "the hand-over area, and behind it places for every head's records");
 /* score warps 0-3 take the even pages and 4-7 the odd ones: with an even ring each waits for every phase of its stages */
 static_assert(kStages >= 4 && kStages <= 8 && kStages % 2 == 0 && kStagesClu % 2 == 0 && kSlots % 2 == 0, "ring depth");
 
@@ -700,7 +700,6 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
 
             /* ---- the piece of this CTA, from the accumulators: thread -> (head, 4 dims) */
             epi_sync();
-            const bool red = qtid < 256;
             const int h = (qtid >> 5) & 7, d4 = (qtid & 31) * 4;
             float M = mi.ml[h][0], L = mi.ml[h][1], acc[4];
             {
@@ -711,7 +710,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                 cluster_send<CL ? CL : 1>(s_base + kOffClu, UBAR(mi.clu), cta % (CL ? CL : 1), h, lane, M, L, acc);
                 break;
             }
-            qk_sync();   /* everybody holds its share: the accumulators may overwrite the hand-over area (next piece) */
+            if (SHARD) qk_sync();   /* everybody holds its share: the hand-over area is a landing zone below; else it is written again behind the next piece's queries */
 
             /* ---- how many CTAs share this segment? */
             const int c_first = aligned ? al_first : (int)(((sg.seg_u0 + 1) * C + U - 1) / U) - 1;
@@ -721,24 +720,22 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
             u = sg.seg_u0 + sg.p_end;
 
             int h_lo = 0, h_hi = 8;
+            bool last = true;      /* this warp has its head's final record */
+            float *const recs = a.scratch + ((size_t)(c_first + rec_base) * 8 + h) * kRecFloats;      /* of the segment's piece 0 */
             if (npieces > 1) {
-                if (red) {
-                    float *rec = a.scratch + ((size_t)(cta + rec_base) * 8 + h) * kRecFloats;
-                    if (d4 == 0) { rec[0] = M; rec[1] = L; }
-                    rec[2 + d4] = acc[0]; rec[3 + d4] = acc[1]; rec[4 + d4] = acc[2]; rec[5 + d4] = acc[3];
-                }
-                qk_sync();   /* the record is complete in CTA scope; the release below publishes it */
                 if (aligned && a.spread) {
                     /* CTA-aligned segments: the fold is spread over the first F pieces (see decode.cu) */
                     const int Fmax = a.spread, F = npieces >= Fmax ? Fmax : (npieces >= 4 && Fmax >= 4 ? 4 : (npieces >= 2 && Fmax >= 2 ? 2 : 1)), hpf = 8 / F, piece = cta - c_first;
-                    if (qtid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.counters + sidx) : "memory");
+                    store_record(recs + (size_t)piece * 8 * kRecFloats, lane, M, L, acc);
+                    qk_sync();   /* the record is complete in CTA scope; the release publishes it */
+                    if (qtid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.counters + 8 * sidx) : "memory");
                     if (piece >= F) continue;   /* CTA-uniform */
                     if (qtid == 0) {
                         unsigned seen = 0;
                         unsigned long long t0 = 0;
                         bool ok = false;
                         for (unsigned i = 0; i < (1u << 24); i++) {
-                            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.counters + sidx) : "memory");
+                            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.counters + 8 * sidx) : "memory");
                             if (seen >= (unsigned)npieces) { ok = true; break; }
                             if ((i & 255u) == 255u) {
                                 unsigned long long t1;
@@ -752,81 +749,29 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                     }
                     qk_sync();
                     h_lo = piece * hpf; h_hi = h_lo + hpf;
-                    const bool mine = red && h >= h_lo && h < h_hi;
+                    const bool mine = h >= h_lo && h < h_hi;
                     M = -INFINITY; L = 0.f; acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
                     if (mi.flag && mine) {
-                        /* landing zone of head h: npieces x 528 bytes in the ring (idle: this CTA's pages are consumed) */
-                        const unsigned zone = (unsigned)((h - h_lo) * npieces) * (unsigned)(kRecFloats * 4);
-                        const uint8_t *src = reinterpret_cast<const uint8_t *>(a.scratch + ((size_t)c_first * 8 + h) * kRecFloats);
-                        for (int c = 0; c < npieces; c++) {
-                            const unsigned dst = ring_base + zone + (unsigned)c * (unsigned)(kRecFloats * 4);
-                            const uint8_t *gsrc = src + (size_t)c * 8 * kRecFloats * 4;
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (unsigned)lane), "l"(gsrc + 16 * lane) : "memory");
-                            if (lane == 0) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512u), "l"(gsrc + 512) : "memory");
-                        }
-                        asm volatile("cp.async.wait_all;" ::: "memory");
-                        __syncwarp();
-                        const float *zf = reinterpret_cast<const float *>(s_dyn + ring_off + zone);
-                        for (int c = 0; c < npieces; c++) {
-                            const float *pr = zf + (size_t)c * kRecFloats;
-                            const float pm = pr[0], pl = pr[1];
-                            if (pl == 0.f) continue;
-                            const float2 v01 = *reinterpret_cast<const float2 *>(pr + 2 + d4), v23 = *reinterpret_cast<const float2 *>(pr + 4 + d4);
-                            const float nm = fmaxf(M, pm), os = ex2(M - nm), rs = ex2(pm - nm);
-                            L = L * os + pl * rs;
-                            acc[0] = acc[0] * os + v01.x * rs; acc[1] = acc[1] * os + v01.y * rs;
-                            acc[2] = acc[2] * os + v23.x * rs; acc[3] = acc[3] * os + v23.y * rs;
-                            M = nm;
-                        }
+                        constexpr int kRing = kStages * kStageBytes;      /* idle: this CTA's pages are consumed */
+                        const int slots = min(32, kRing / (hpf * 512));
+                        fold_records(recs, npieces, s_dyn + ring_off + (h - h_lo) * slots * 512, 512u, slots, lane, M, L, acc);
                     }
                     qk_sync();   /* every landing zone is read (the sharded exchange lands its lines in the ring too) */
                     if (qtid == 0) {
-                        const unsigned old = atomicAdd(a.counters + a.n_counters + sidx, 1u);
-                        if (old == (unsigned)(F - 1)) { a.counters[sidx] = 0u; a.counters[a.n_counters + sidx] = 0u; }
+                        unsigned *done = a.counters + 8 * a.n_counters + sidx;
+                        const unsigned old = atomicAdd(done, 1u);
+                        if (old == (unsigned)(F - 1)) { a.counters[8 * sidx] = 0u; *done = 0u; }
                     }
                 } else {
-                    /* the LAST CTA to arrive folds, nobody waits */
-                    if (qtid == 0) {
-                        unsigned old;
-                        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(a.counters + sidx) : "memory");
-                        mi.flag = (old == (unsigned)(npieces - 1));
-                    }
-                    qk_sync();
-                    if (!mi.flag) continue;   /* CTA-uniform */
-                    /* fold all pieces with the rule of hy3_gpu.cu:233-247: the records are fetched with 16-byte asynchronous
-                     * copies issued by all threads at once into the page ring when it is idle (CTA-aligned segments: this
-                     * CTA's pages are consumed), else into the small landing zone, in rounds */
-                    const unsigned land = aligned ? ring_base : s_base + kOffLand;
-                    const float *land_g = reinterpret_cast<const float *>(aligned ? s_dyn + ring_off : s_dyn + kOffLand);
-                    const int land_cap = (aligned ? kStages * kStageBytes : kLandBytes) / (8 * kRecFloats * 4);
-                    M = -INFINITY; L = 0.f; acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-                    for (int c0 = 0; c0 < npieces; c0 += land_cap) {
-                        const int nc = min(land_cap, npieces - c0);
-                        const uint8_t *src = reinterpret_cast<const uint8_t *>(a.scratch + (size_t)(c_first + c0 + rec_base) * 8 * kRecFloats);
-                        for (int i = qtid; i < nc * (8 * kRecFloats / 4); i += kQkThreads)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(land + 16u * (unsigned)i), "l"(src + 16 * (size_t)i) : "memory");
-                        asm volatile("cp.async.wait_all;" ::: "memory");
-                        qk_sync();
-                        if (red) {
-                            for (int c = 0; c < nc; c++) {
-                                const float *pr = land_g + ((size_t)c * 8 + h) * kRecFloats;
-                                const float pm = pr[0], pl = pr[1];
-                                if (pl == 0.f) continue;
-                                const float2 v01 = *reinterpret_cast<const float2 *>(pr + 2 + d4), v23 = *reinterpret_cast<const float2 *>(pr + 4 + d4);
-                                const float nm = fmaxf(M, pm), os = ex2(M - nm), rs = ex2(pm - nm);
-                                L = L * os + pl * rs;
-                                acc[0] = acc[0] * os + v01.x * rs; acc[1] = acc[1] * os + v01.y * rs;
-                                acc[2] = acc[2] * os + v23.x * rs; acc[3] = acc[3] * os + v23.y * rs;
-                                M = nm;
-                            }
-                        }
-                        if (c0 + land_cap < npieces) qk_sync();   /* landing zone is reused */
-                    }
-                    if (qtid == 0) a.counters[sidx] = 0u; /* self-reset for the next launch */
-                    qk_sync();   /* the landing zone is read */
+                    /* The last CTA to arrive folds, nobody waits.  The records land in the page ring where it is idle (whole CTAs to a segment:
+                     * this CTA's pages are consumed), else behind the hand-over area. */
+                    constexpr int kRingSlots = kStages * kStageBytes / 4096 < 32 ? kStages * kStageBytes / 4096 : 32;
+                    uint8_t *const zone = s_dyn + (aligned ? ring_off + h * (kRingSlots * 512) : kOffLand + 4096 + h * 512);
+                    last = fold_last(recs, cta - c_first, npieces, a.counters + 8 * sidx + h, zone, aligned ? 512u : 4096u, aligned ? kRingSlots : kLandBytes / 4096 - 1, lane, M, L, acc);
+                    if (SHARD) qk_sync();      /* the exchange lands its lines there too */
                 }
             }
-            const bool fin = red && h >= h_lo && h < h_hi;   /* this thread finishes its (head, 4 dims) of the segment */
+            const bool fin = last && h >= h_lo && h < h_hi;   /* this thread finishes its (head, 4 dims) of the segment */
             if (SHARD) {
                 /* sequence sharding: this rank's records go into every other rank's gather buffer as flagged lines, then
                  * the same threads collect the other ranks' lines and finish the segment (see decode.cu) */

@@ -147,6 +147,32 @@ def test_few_rows_in_even_pieces(cuda, oracle, dt, heads, lens):
     ctx.close()
 
 
+@pytest.mark.parametrize("dt,stages", [("int8", None), ("int4", None), ("fp16", None), ("int4", 2)])
+@pytest.mark.parametrize("lens", [[32700], [36800], [66000], [9000] * 40])
+def test_folds_of_many_records(cuda, oracle, dt, stages, lens, monkeypatch):
+    """One KV head: 32, 33 and 40 pieces of a segment (one record per lane of the folding warp, one more, and several landings in a ring
+    of two pages), and rows whose few pieces straddle CTAs; twice, because every fold leaves its counters for the next launch."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    if stages:
+        monkeypatch.setenv("HY3A_DECODE_STAGES", str(stages))
+    B = len(lens)
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_seqs=B, max_batch=B, kv_head_count=1, max_tokens=sum(lens) + 128 * B, max_tokens_per_seq=max(lens) + 128)
+    for i, n in enumerate(lens):
+        ctx.fill_random(0, i, 0, n, 170 + i)
+    q = oracle.fill_normal((B, 64, 128), SEED, 443)
+    ctx.batch_set(list(range(B)), [n - 1 for n in lens])
+    outs = [ctx.decode(0, torch.from_numpy(q).to(cuda))[:, :8].clone() for _ in range(2)]
+    ctx.sync()
+    assert torch.equal(outs[0], outs[1])
+    out = outs[0].cpu().numpy()
+    for i in sorted({0, B // 3, B - 1}):
+        ks, vs = ctx.export_kv(0, i, 0, lens[i])
+        want = oracle.attention(q[i], slots_to_float(oracle, ks, dt), slots_to_float(oracle, vs, dt))
+        check_attention(out[i], want[:8], "%s row %d of %d" % (dt, i, B))
+    ctx.close()
+
+
 def test_decode_ragged_batch_and_poison(cuda, oracle):
     """Several sequences of different lengths in one launch; cache bytes past each length are poison."""
     import torch
