@@ -340,6 +340,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
     __shared__ unsigned s_vnew;
     __shared__ int s_flag;
     __shared__ int s_abort;
+    __shared__ cta_plan s_plan;
 
     const hy3a_geom geom = hy3a_make_geom(DT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -352,106 +353,58 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
     const unsigned ring_base = bar_base + kBarBytes<CL>;
 
     if (a.wait_first) asm volatile("griddepcontrol.wait;" ::: "memory");
-    /* ---- schedule: prefix of pages per row */
-    for (int i = tid; i < n; i += blockDim.x) {
-        int len = batch.slot[i] + 1;
-        s_prefix[i + 1] = len > 0 ? (len + HY3A_PT - 1) / HY3A_PT : 0;
-    }
-    if (tid == 0) {
-        s_prefix[0] = 0;
-        s_abort = 0;
-        if (STAGED) {
-            for (int i = 0; i < a.stages; i++) mbar_init(bar_base + 8 * i, 32 * kGranPage<DT>);   /* empty[stage]: every thread of the warps that share a page */
-            for (int i = 0; i < 16; i++) mbar_init(bar_base + 64 + 8 * i, 1);   /* full[page mod n_full]: the producer's expect_tx */
-            if (CL) mbar_init(bar_base + kBarClu, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            if (CL) mbar_expect_tx(bar_base + kBarClu, kCluBytes);
-        }
-    }
-    __syncthreads();
-    if (CL) cluster_arrive();
-    if (warp == 0 && n > 1) {
-        int carry = 0;
-        for (int base = 0; base < n; base += 32) {
-            int i = base + lane;
-            int v = i < n ? s_prefix[i + 1] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int t = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += t;
-            }
-            if (i < n) s_prefix[i + 1] = v + carry;
-            carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-    }
-    __syncthreads();
-
-    const long long U = (long long)G * s_prefix[n];
-    bool idle = (U == 0);
-    /* Two ways to cut the units into per-CTA ranges:
-     *  - few segments (n*G < grid): every segment gets its own whole number of CTAs, for pieces of at
-     *    most L pages or (1 row, more than 32) roughly in proportion to its pages, so no CTA straddles two segments (a straddling CTA pays the
-     *    query set-up and the fold twice and becomes the critical path of a small batch);
-     *  - many segments: one contiguous, equally sized range per CTA over all units.
-     * In both, never more CTAs than units, and the CTAs sharing a segment are contiguous.       */
-    const unsigned L = CL ? 0u : even_piece_pages(s_prefix, n, G, gridDim.x, lane);      /* 0: shares in proportion to the pages */
-    const bool aligned = CL || split_is_aligned(s_prefix, n, G, gridDim.x, lane, L);
-    int C = (long long)gridDim.x < U ? (int)gridDim.x : (int)U;
-    long long u_begin = 0, u_end = 0;
-    int al_first = 0, al_pieces = 1;
-    if (CL) {
-        cluster_share<CL ? CL : 1>(s_prefix, G, cta, u_begin, u_end);
-        idle = u_begin == u_end;
-    } else if (idle) {
-    } else if (aligned) {
-        int rows_ne = 0;
-        for (int r = 0; r < n; r++) rows_ne += (s_prefix[r + 1] != s_prefix[r]);
-        const long long spare = (long long)gridDim.x - (long long)rows_ne * G, P = s_prefix[n];
-        int base = 0;
-        bool found = false;
-        u_begin = u_end = 0;
-        for (int r = 0; r < n && !found; r++) {
-            const int p = s_prefix[r + 1] - s_prefix[r];
-            if (p == 0) continue;
-            int c = L ? (p + (int)L - 1) / (int)L : 1 + (int)(spare * p / (P * G));
-            if (!L) c = min(c, (int)hy3a_most_pieces((unsigned)p));
-            c = c < p ? c : p;
-            if (cta < base + G * c) {
-                const int idx = cta - base, hl = idx / c, k = idx % c;
-                const long long seg0 = (long long)G * s_prefix[r] + (long long)hl * p;
-                u_begin = seg0 + (long long)k * p / c;
-                u_end = seg0 + (long long)(k + 1) * p / c;
-                al_first = base + hl * c;
-                al_pieces = c;
-                found = true;
-            }
-            base += G * c;
-        }
-        if (!found) idle = true;
-    } else {
-        if (cta >= C) idle = true;
-        u_begin = (long long)cta * U / C;
-        u_end = (long long)(cta + 1) * U / C;
-        if (idle) u_begin = u_end = 0;
-    }
-    /* ---- fused step, still before the wait: what the query set-up needs besides the queries themselves
-     * (norm weights, RoPE table, the row's position -> cos/sin) comes from the host, so warps 0-7 (queries)
-     * and 9 (new K row) fetch and compute it now, off the critical path.                               */
+    /* ---- What the query set-up needs besides the queries (norm weights, RoPE table, positions) comes from the host: warps 0-7 (queries) and 9
+     * (new K row) fetch it now, off the critical path; the planning warp sets the barriers up while its rows' slots are on the way. */
+    constexpr int kPlanWarp = STAGED ? kWarps : 0;
     const int rl_d0 = (lane >> 4) * 64 + (lane & 15) * 4;
-    float4 pre_w = make_float4(1.f, 1.f, 1.f, 1.f);
+    float4 pre_w = make_float4(1.f, 1.f, 1.f, 1.f), pre_f = make_float4(0.f, 0.f, 0.f, 0.f);
     float pre_c[4] = {1.f, 1.f, 1.f, 1.f}, pre_s[4] = {0.f, 0.f, 0.f, 0.f};
-    int pre_row = -1;
-    if (a.fused && !idle && (warp < 8 || warp == 9)) {
+    int pre_row = -1, pos_l = 0;           /* pos_l: position of row `lane`, up to 32 rows */
+    const bool ropes = a.fused && (warp < 8 || warp == 9);
+    if (ropes) {
         pre_w = *reinterpret_cast<const float4 *>(a.norm_w + (warp == 9 ? HY3A_D : 0) + rl_d0);
-        pre_row = locate(s_prefix, batch, n, G, u_begin, u_end).row;
-        hy3a_rowops::rope_coeffs(pre_c, pre_s, a.rope, batch.pos[pre_row], lane);
+        pre_f = hy3a_rowops::rope_freqs(a.rope, lane);
+        if (lane < n) pos_l = batch.pos[lane];
     }
+    if (n > 32) {
+        for (int i = tid; i < n; i += blockDim.x) s_prefix[i + 1] = pages_of_slot(batch.slot[i]);
+        __syncthreads();
+    }
+    lane_rows rows = {-1, 0};
+    if (warp == kPlanWarp) {
+        rows = load_rows(batch, n, lane);
+        if (lane == 0) {
+            s_abort = 0;
+            if (STAGED) {
+                for (int i = 0; i < a.stages; i++) mbar_init(bar_base + 8 * i, 32 * kGranPage<DT>);   /* empty[stage]: every thread of the warps that share a page */
+                for (int i = 0; i < 16; i++) mbar_init(bar_base + 64 + 8 * i, 1);   /* full[page mod n_full]: the producer's expect_tx */
+                if (CL) mbar_init(bar_base + kBarClu, 1);
+                asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+                if (CL) mbar_expect_tx(bar_base + kBarClu, kCluBytes);
+            }
+        }
+        plan<DT, CL>(&s_plan, s_prefix, rows.slot, n, G, gridDim.x, cta, lane);
+    }
+    if (CL) cluster_arrive();      /* every CTA of the cluster has set its barrier up; cluster_wait below */
+    const bool is_producer = STAGED && warp == kWarps;
+    if (is_producer) asm volatile("bar.arrive 2, %0;" ::"r"(blockDim.x) : "memory");      /* the others need the plan; the copies need no one */
+    else asm volatile("bar.sync 2, %0;" ::"r"(blockDim.x) : "memory");
+
+    const long long U = (long long)G * s_prefix[n], u_begin = s_plan.u0, u_end = s_plan.u1;
+    const bool aligned = s_plan.aligned, idle = u_begin == u_end;
+    const int C = (long long)gridDim.x < U ? (int)gridDim.x : (int)U;
+    const int al_first = s_plan.first, al_pieces = s_plan.pieces;
+    /* cos / sin of a row's position */
+    auto rope_row = [&](int row) {
+        hy3a_rowops::rope_coeffs(pre_c, pre_s, a.rope, pre_f, n <= 32 ? __shfl_sync(0xffffffffu, pos_l, row) : batch.pos[row]);
+        pre_row = row;
+    };
+    if (ropes && !idle) rope_row(locate(s_prefix, batch, n, G, u_begin, u_end).row);
     /* Everything above reads only what the host wrote (batch descriptor).  From here on the kernel
      * touches memory that the preceding kernel in the stream may produce (queries, the newest KV
      * slot, scratch records), so wait for it -- except the producer lane, which first starts the
      * copies of pages that lie wholly below the newest slot (append-only cache: immutable).       */
-    if (CL) cluster_wait();      /* every CTA of the cluster has set its barrier up */
-    const bool is_producer = STAGED && warp == kWarps;
+    if (CL && !is_producer) cluster_wait();
     const unsigned n_full = STAGED ? 16u / (unsigned)a.stages * (unsigned)a.stages : 1u;   /* "full" barriers: a multiple of the stages */
     if (!is_producer) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -482,18 +435,19 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
 
 
     if (STAGED && warp == kWarps) {
-        /* ================= producer warp: one lane streams the CTA's pages into the ring */
-        if (lane == 0) {
-            unsigned it = 0;
-            bool ok = true;
-            bool waited = false;   /* griddepcontrol.wait executed yet? */
-            const unsigned long long pol = l2_evict_first_policy();
-            if (!a.early_prefetch) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
-            for (long long u = u_begin; u < u_end && ok;) {
-                segment sg = locate(s_prefix, batch, n, G, u, u_end);
-                const int *bt = cache.block_table + (size_t)sg.seq * cache.max_blocks_per_seq;
+        /* ================= producer warp: one lane streams the CTA's pages into the ring (the warp finds the segments).  With every lane in the
+         * loop, each holding a page's block-table entry, INT4 262 144 tokens take 71 us a layer instead of 67. */
+        unsigned it = 0;
+        bool ok = true;
+        bool waited = false;   /* griddepcontrol.wait executed yet? */
+        const unsigned long long pol = l2_evict_first_policy();
+        if (!a.early_prefetch) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
+        for (long long u = u_begin; u < u_end && ok;) {
+            const segment sg = locate(s_prefix, batch, rows, n, G, u, u_end);
+            const int *bt = cache.block_table + (size_t)sg.seq * cache.max_blocks_per_seq;
+            if (lane == 0) {
                 int block_next = bt[sg.p_begin];
-                for (int p = sg.p_begin; p < sg.p_end && ok; p++, it++) {
+                for (int p = sg.p_begin; p < sg.p_end; p++, it++) {
                     const unsigned stage = it % (unsigned)a.stages, phase = (it / (unsigned)a.stages) & 1u;
                     const int block = block_next;
                     if (p + 1 < sg.p_end) block_next = bt[p + 1];   /* in flight while we wait for the stage */
@@ -507,19 +461,20 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                     mbar_expect_tx(full, (unsigned)geom.page_bytes);
                     bulk_g2s(ring_base + stage * (unsigned)geom.page_bytes, page, (unsigned)geom.page_bytes, full, pol);
                 }
-                u = sg.seg_u0 + sg.p_end;
             }
-            if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
-            if (!ok) {
-                /* gave up: let the copies already issued land before the CTA's shared memory goes away */
-                const unsigned first = it > (unsigned)a.stages ? it - (unsigned)a.stages : 0u;
-                for (unsigned j = first; j < it; j++) {
-                    const unsigned fb = j % n_full, fphase = (j / n_full) & 1u;
-                    for (unsigned spin = 0; spin < (1u << 20) && !mbar_test(bar_base + 64 + 8 * fb, fphase); spin++) __nanosleep(64);
-                }
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            u = sg.seg_u0 + sg.p_end;
+        }
+        if (lane == 0 && !waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (lane == 0 && !ok) {
+            /* gave up: let the copies already issued land before the CTA's shared memory goes away */
+            const unsigned first = it > (unsigned)a.stages ? it - (unsigned)a.stages : 0u;
+            for (unsigned j = first; j < it; j++) {
+                const unsigned fb = j % n_full, fphase = (j / n_full) & 1u;
+                for (unsigned spin = 0; spin < (1u << 20) && !mbar_test(bar_base + 64 + 8 * fb, fphase); spin++) __nanosleep(64);
             }
         }
-        if (CL) { __syncwarp(); cluster_arrive(); cluster_wait(); }
+        if (CL) { __syncwarp(); cluster_wait(); cluster_arrive(); cluster_wait(); }
         return;
     }
 
@@ -576,7 +531,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             if (a.fused) {
                 const float4 xv = *reinterpret_cast<const float4 *>(a.q_in + (size_t)row * a.qi_stride + (size_t)(head0 + warp) * HY3A_D + d0);
                 x[0] = xv.x; x[1] = xv.y; x[2] = xv.z; x[3] = xv.w;
-                if (row != pre_row) { hy3a_rowops::rope_coeffs(pre_c, pre_s, a.rope, batch.pos[row], lane); pre_row = row; }
+                if (row != pre_row) rope_row(row);
                 hy3a_rowops::norm_rope_apply(x, pre_w, a.eps, pre_c, pre_s, lane);
                 if (a.q_out && sg.p_begin == 0)
                     *reinterpret_cast<float4 *>(a.q_out + (size_t)row * a.q_out_stride + (size_t)(head0 + warp) * HY3A_D + d0) = make_float4(x[0], x[1], x[2], x[3]);
@@ -636,7 +591,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             if (warp == 9) {
                 const float4 k4 = *reinterpret_cast<const float4 *>(a.k_in + (size_t)row * a.ki_stride + kvh);
                 float y[4] = {k4.x, k4.y, k4.z, k4.w};
-                if (row != pre_row) { hy3a_rowops::rope_coeffs(pre_c, pre_s, a.rope, batch.pos[row], lane); pre_row = row; }
+                if (row != pre_row) rope_row(row);
                 hy3a_rowops::norm_rope_apply(y, pre_w, a.eps, pre_c, pre_s, lane);
                 *reinterpret_cast<float4 *>(&s_new[0][rl_d0]) = make_float4(y[0], y[1], y[2], y[3]);
             } else if (warp == 10) {
@@ -772,8 +727,8 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         if (SHARD) consumer_sync();      /* s_o / s_ml are landing zones below; else they are written again behind the next segment's queries */
 
         /* ---- how many CTAs share this segment? */
-        const int c_first = aligned ? al_first : (int)(((sg.seg_u0 + 1) * C + U - 1) / U) - 1;
-        const int npieces = aligned ? al_pieces : (int)((sg.seg_u1 * C + U - 1) / U) - 1 - c_first + 1;
+        const int c_first = aligned ? al_first : cta_of_unit(sg.seg_u0, U, C);
+        const int npieces = aligned ? al_pieces : cta_of_unit(sg.seg_u1 - 1, U, C) - c_first + 1;
         const int rec_base = aligned ? 0 : sidx;   /* record index = CTA (+ segment when CTAs may hold several pieces) */
         const size_t head_q = (size_t)(cache.kv_head_begin + hl) * 8 + h; /* global query head */
         u = sg.seg_u0 + sg.p_end;

@@ -80,7 +80,7 @@ struct segment {
 
 /* Locate the (row, local head) segment that contains unit u and the page range of it that
  * falls into [u, u_end).                                                                   */
-__device__ __forceinline__ segment locate(const int *s_prefix, const hy3a_batch_view &batch, int n, int G, long long u, long long u_end) {
+__device__ __forceinline__ segment locate_pages(const int *s_prefix, int n, int G, long long u, long long u_end) {
     segment sg;
     int lo = 0, hi = n - 1;
     while (lo < hi) {
@@ -96,36 +96,27 @@ __device__ __forceinline__ segment locate(const int *s_prefix, const hy3a_batch_
     sg.p_begin = (int)(u - sg.seg_u0);
     sg.p_end = (int)((sg.seg_u1 < u_end ? sg.seg_u1 : u_end) - sg.seg_u0);
     sg.sidx = lo * G + sg.hl;
-    sg.len = batch.slot[lo] + 1;
-    sg.seq = batch.seq[lo];
     return sg;
 }
-
-/* The CTA-aligned split gives every (row, KV head) segment whole CTAs in proportion to its pages.  With few segments that is
- * balanced to a page; when the segments are about as many as the CTAs the rounding leaves some CTAs with far more pages than
- * the even share (64 rows of one KV head on 148 CTAs: up to 1.75 x), and the plain equal split over all units is the better
- * one.  Returns whether the aligned split stays within 5/4 of the even share.  Every lane takes rows lane, lane + 32, ...;
- * call with all lanes of the warp; the result is the same in every warp. */
-__device__ __forceinline__ bool aligned_split_balanced(const int *s_prefix, int n, int G, unsigned grid, int lane) {
-    if ((unsigned)(n * G) * 4u <= grid) return true;   /* at least four CTAs per segment */
-    const unsigned long long P = (unsigned)s_prefix[n];
-    int ne = 0;
-    for (int r = lane; r < n; r += 32) ne += (s_prefix[r + 1] != s_prefix[r]);
-    ne = __reduce_add_sync(0xffffffffu, ne);
-    const unsigned long long spare = grid - (unsigned)(ne * G), PG = P * (unsigned)G;
-    if (PG == 0) return true;
-    unsigned worst = 0;
-    for (int r = lane; r < n; r += 32) {
-        const unsigned p = (unsigned)(s_prefix[r + 1] - s_prefix[r]);
-        if (p == 0) continue;
-        unsigned long long c = min(1ull + spare * p / PG, (unsigned long long)hy3a_most_pieces(p));
-        if (c > p) c = p;
-        const unsigned w = (unsigned)((p + c - 1ull) / c);
-        worst = worst > w ? worst : w;
-    }
-    worst = __reduce_max_sync(0xffffffffu, worst);
-    const unsigned long long even = (PG + grid - 1ull) / grid;
-    return (unsigned long long)worst * 4ull <= even * 5ull + 4ull;
+__device__ __forceinline__ segment locate(const int *s_prefix, const hy3a_batch_view &batch, int n, int G, long long u, long long u_end) {
+    segment sg = locate_pages(s_prefix, n, G, u, u_end);
+    sg.len = batch.slot[sg.row] + 1;
+    sg.seq = batch.seq[sg.row];
+    return sg;
+}
+/* the rows of the producer's warp: lane = row, up to 32 of them; its segments then wait for no load */
+struct lane_rows { int slot, seq; };
+__device__ __forceinline__ lane_rows load_rows(const hy3a_batch_view &batch, int n, int lane) {
+    lane_rows r = {-1, 0};
+    if (n <= 32 && lane < n) { r.slot = batch.slot[lane]; r.seq = batch.seq[lane]; }
+    return r;
+}
+__device__ __forceinline__ segment locate(const int *s_prefix, const hy3a_batch_view &batch, const lane_rows &rows, int n, int G, long long u, long long u_end) {
+    if (n > 32) return locate(s_prefix, batch, n, G, u, u_end);
+    segment sg = locate_pages(s_prefix, n, G, u, u_end);
+    sg.len = __shfl_sync(0xffffffffu, rows.slot, sg.row) + 1;
+    sg.seq = __shfl_sync(0xffffffffu, rows.seq, sg.row);
+    return sg;
 }
 
 /* 2 to 32 rows with fewer than four CTAs per segment: the least number of pages L for which pieces of at most L pages fit the
@@ -140,14 +131,125 @@ __device__ __noinline__ unsigned even_piece_search(const int *s_prefix, int n, i
     return hy3a_least_piece((P + cap - 1u) / cap, hy3a_piece_bound(P, cap, (unsigned)n, __reduce_max_sync(0xffffffffu, p)), cap,
                             [&](unsigned L) { return __reduce_add_sync(0xffffffffu, (p + L - 1u) / L); });
 }
-__device__ __forceinline__ unsigned even_piece_pages(const int *s_prefix, int n, int G, unsigned grid, int lane) {
-    return hy3a_even_applies(n, G, grid) ? even_piece_search(s_prefix, n, G, grid, lane) : 0u;
+/* the pages of a cluster's CTA, in units */
+template <int CL>
+__device__ __forceinline__ void cluster_share(const int *s_prefix, int G, int cta, long long &u_begin, long long &u_end) {
+    const int seg = cta / CL, k = cta - seg * CL, row = seg / G, hl = seg - row * G;
+    const int p = s_prefix[row + 1] - s_prefix[row];
+    const long long seg0 = (long long)G * s_prefix[row] + (long long)hl * p;
+    u_begin = seg0 + (long long)k * p / CL;
+    u_end = seg0 + (long long)(k + 1) * p / CL;
 }
-/* whether segments get whole CTAs; `L` from above */
-__device__ __forceinline__ bool split_is_aligned(const int *s_prefix, int n, int G, unsigned grid, int lane, unsigned L) {
-    if (!((long long)n * G < (long long)grid)) return false;
-    if (L == 0u) return aligned_split_balanced(s_prefix, n, G, grid, lane);
-    return hy3a_even_accepted(L, (unsigned)s_prefix[n], G, grid);
+/* ---- the CTA's range of units.  One warp (the producer's, which then starts its copies without a word from the others) plans for the CTA.
+ *  - few segments (n G < grid): every segment gets its own whole number of CTAs, for pieces of at most L pages or (1 row, more than 32,
+ *    INT8) roughly in proportion to its pages, so that no CTA straddles two segments (a straddling CTA pays the query set-up and the
+ *    fold twice and becomes the critical path of a small batch).  In proportion is balanced to a page with few segments; when the
+ *    segments are about as many as the CTAs the rounding leaves some with far more pages than the even share (64 rows of one KV head
+ *    on 148 CTAs: up to 1.75 x), so with fewer than four CTAs per segment it is kept only within 5/4 of the even share;
+ *  - else one contiguous, equally sized range per CTA over all units.
+ * In both, never more CTAs than units, and the CTAs sharing a segment are contiguous.  A lane takes a row, 32 at a time, and the
+ * arithmetic is 32-bit (T) unless the units are too many for it: this stands in front of every launch's first copy.  Planned by
+ * every warp for itself, row by row and with 64-bit divisions, it took 1.1 us of a launch of one row, 3.3 of 8 rows, 2.3 of 64. */
+struct cta_plan { long long u0, u1; int first, pieces, aligned; };
+template <int DT, class T>
+__device__ __noinline__ void plan_cta(cta_plan *out, const int *s_prefix, int n, int G, unsigned grid, unsigned cta, int lane) {
+    const unsigned Pn = (unsigned)s_prefix[n], g = (unsigned)G;
+    const T U = (T)Pn * g;
+    auto pages = [&](int r) { return r < n ? (unsigned)(s_prefix[r + 1] - s_prefix[r]) : 0u; };
+    unsigned ne = 0, L = 0;
+    for (int r = lane; r < n; r += 32) ne += pages(r) != 0u;
+    ne = __reduce_add_sync(0xffffffffu, ne);
+    const T spare = (T)grid - (T)ne * g;
+    auto pieces = [&](unsigned p) {
+        const unsigned c = L ? (p + L - 1u) / L : min(1u + (unsigned)(spare * p / U), hy3a_most_pieces(p));
+        return c < p ? c : p;
+    };
+    bool aligned = Pn != 0u && (unsigned)n * g < grid;
+    if (aligned && DT != 1 && hy3a_even_applies(n, G, grid)) {
+        L = even_piece_search(s_prefix, n, G, grid, lane);
+        aligned = hy3a_even_accepted(L, Pn, G, grid);
+    } else if (aligned && (unsigned)n * g * 4u > grid) {
+        unsigned worst = 0;
+        for (int r = lane; r < n; r += 32) {
+            const unsigned p = pages(r), c = p ? pieces(p) : 1u;
+            worst = max(worst, (p + c - 1u) / c);
+        }
+        worst = __reduce_max_sync(0xffffffffu, worst);
+        aligned = (T)worst * 4u <= (U + grid - 1u) / grid * 5u + 4u;
+    }
+    if (lane == 0) {
+        const T C = U < grid ? U : (T)grid;
+        const bool mine = !aligned && cta < C;
+        out->u0 = mine ? (long long)(cta * U / C) : 0;
+        out->u1 = mine ? (long long)((cta + 1u) * U / C) : 0;
+        out->first = 0; out->pieces = 1; out->aligned = aligned;
+    }
+    __syncwarp();
+    unsigned base0 = 0;
+    for (int r0 = 0; aligned && r0 < n && base0 <= cta; r0 += 32) {
+        const unsigned p = pages(r0 + lane), c = p ? pieces(p) : 0u;
+        unsigned end = c * g;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned t = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += t;
+        }
+        const unsigned base = base0 + end - c * g;
+        if (c && cta >= base && cta < base0 + end) {      /* one lane at most */
+            const unsigned idx = cta - base, hl = idx / c, k = idx - hl * c, k1 = k + 1u;
+            const long long seg0 = (long long)g * s_prefix[r0 + lane] + (long long)hl * p;
+            T b = (T)k * p / c, e = (T)k1 * p / c;
+            /* The CTAs with the highest indices are dispatched last, onto the SMs that the preceding launch's folding CTAs held
+             * longest: they start their ring fill late and would finish last (and then fold, and hold their SMs again).  In a
+             * single-row grid the last HY3A_LATE pieces of the INT8 kernel therefore take HY3A_LATE_CUT pages less each and the other
+             * pieces of that segment share them: 18.83 instead of 19.02 us per launch on the benchmark. */
+            if (DT == 1 && ne == 1u && hl == g - 1u && c > 2u * HY3A_LATE && p >= 8u * c && Pn < (1u << 23)) {
+                const unsigned pp = p + HY3A_LATE * HY3A_LATE_CUT, late = c - HY3A_LATE;
+                b = (T)k * pp / c - HY3A_LATE_CUT * (k > late ? k - late : 0u);
+                e = (T)k1 * pp / c - HY3A_LATE_CUT * (k1 > late ? k1 - late : 0u);
+            }
+            out->u0 = seg0 + (long long)b; out->u1 = seg0 + (long long)e;
+            out->first = (int)(base + hl * c); out->pieces = (int)c;
+        }
+        base0 += __shfl_sync(0xffffffffu, end, 31);
+    }
+}
+__device__ __forceinline__ int pages_of_slot(int slot) { return slot >= 0 ? slot / HY3A_PT + 1 : 0; }
+/* the planning warp: prefix of pages per row (rows beyond 32 come as page counts in s_prefix), then the plan, in shared memory */
+template <int DT, int CL>
+__device__ __forceinline__ void plan(cta_plan *out, int *s_prefix, int slot /* of row `lane`, -1 behind the last */, int n, int G, unsigned grid, int cta, int lane) {
+    int carry = 0;
+    for (int base = 0; base < n; base += 32) {
+        const int i = base + lane;
+        int v = n <= 32 ? pages_of_slot(slot) : (i < n ? s_prefix[i + 1] : 0);
+        if (n > 1) {
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += t;
+            }
+        }
+        if (i < n) s_prefix[i + 1] = v + carry;
+        carry += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) s_prefix[0] = 0;
+    __syncwarp();
+    if (CL) {
+        if (lane == 0) {
+            cluster_share<CL ? CL : 1>(s_prefix, G, cta, out->u0, out->u1);
+            out->first = 0; out->pieces = 1; out->aligned = 1;
+        }
+    } else if ((unsigned long long)(unsigned)s_prefix[n] * (unsigned)G * (grid + 1u) >> 32) {
+        plan_cta<DT, unsigned long long>(out, s_prefix, n, G, grid, (unsigned)cta, lane);
+    } else {
+        plan_cta<DT, unsigned>(out, s_prefix, n, G, grid, (unsigned)cta, lane);
+    }
+    __syncwarp();
+}
+/* pieces of a segment where units are dealt in equal ranges: CTA of unit u is the least c with (c + 1) U / C > u */
+__device__ __forceinline__ int cta_of_unit(long long u, long long U, int C) {
+    const unsigned long long x = (unsigned long long)(u + 1) * (unsigned)C + (unsigned long long)U - 1ull;
+    return (int)((x >> 32 ? x / (unsigned long long)U : (unsigned)x / (unsigned)U) - 1ull);
 }
 
 /* ---- shared-memory / mbarrier / bulk-copy primitives ---------------------------------- */
@@ -351,15 +453,6 @@ __device__ __forceinline__ void cluster_fold(const uint8_t *zone, int w, int lan
         acc[0] = acc[0] * os + v.x * rs; acc[1] = acc[1] * os + v.y * rs; acc[2] = acc[2] * os + v.z * rs; acc[3] = acc[3] * os + v.w * rs;
         M = nm;
     }
-}
-/* the pages of a cluster's CTA, in units */
-template <int CL>
-__device__ __forceinline__ void cluster_share(const int *s_prefix, int G, int cta, long long &u_begin, long long &u_end) {
-    const int seg = cta / CL, k = cta - seg * CL, row = seg / G, hl = seg - row * G;
-    const int p = s_prefix[row + 1] - s_prefix[row];
-    const long long seg0 = (long long)G * s_prefix[row] + (long long)hl * p;
-    u_begin = seg0 + (long long)k * p / CL;
-    u_end = seg0 + (long long)(k + 1) * p / CL;
 }
 /* head hq (of the context's heads) of a row: final output, or the caller's record */
 __device__ __forceinline__ void cluster_write(const hy3a_decode_args &a, int kv_heads, int kv_head_begin, int row, int hq, int lane, float M, float L, const float (&acc)[4]) {

@@ -47,7 +47,8 @@ HY3A_HD unsigned hy3a_least_piece(unsigned lo, unsigned hi, unsigned cap, Pieces
 }
 /* whether pieces of at most L of the P pages per head are kept, or units are dealt in equal contiguous ranges instead */
 HY3A_HD bool hy3a_even_accepted(unsigned L, unsigned P, int G, unsigned grid) {
-    const unsigned long long even = ((unsigned long long)P * (unsigned)G + grid - 1ull) / grid;
+    const unsigned long long sum = (unsigned long long)P * (unsigned)G + grid - 1ull;
+    const unsigned long long even = sum >> 32 ? sum / grid : (unsigned)sum / grid;      /* a 64-bit division costs hundreds of cycles */
     return L * 4ull <= even * 5ull + 4ull || L <= even + HY3A_STRADDLE_PAGES;
 }
 

@@ -20,7 +20,7 @@
  *               also run the fused append (one warp per new row).
  *   warp 8      page producer (one lane): bulk copies (cp.async.bulk + mbarrier transaction counts, evict-first in L2) into a
  *               ring of pages; the first ring fill runs before the preceding kernel is known to be complete (pages below
- *               the newest slot are immutable), and once the queries are loaded it asks L2 for the pages beyond the ring.
+ *               the newest slot are immutable).  It plans for the CTA first (decode_common.cuh).
  *   warp 9      MMA issuer (one lane): when the four groups' digits of a page are in shared memory it issues the four
  *               tcgen05.mma back to back, one tcgen05.commit for the accumulators and one that frees the ring stage.  It
  *               does nothing else: scalar code between two MMAs of a lane costs more than the MMA.
@@ -61,9 +61,10 @@ constexpr int kShardBatchU = 1;                  /* ranks polled at once by the 
 constexpr float kDigits = 32258.f;               /* 127 * 254: the largest two-digit value */
 
 struct u_misc {
-    unsigned long long rfull[8], rempty[8], pfull[kSlots], ofull[kSlots], bk[kSlots], sfree[kSlots], qload, clu;
+    unsigned long long rfull[8], rempty[8], pfull[kSlots], ofull[kSlots], bk[kSlots], sfree[kSlots], clu;
     unsigned tmem;
     int abort_flag, flag, app_ready;         /* app_ready: the fused appends of this CTA are in HBM */
+    cta_plan plan;
     float qf[8];
     float ml[8][2];                              /* {M, L} of the segment piece the accumulators just finished */
     float meta_m[kSlots][4][8], meta_l[kSlots][4][8], meta_wb[kSlots][4];
@@ -79,7 +80,6 @@ constexpr int kOffPt = 0;                            /* kSlots x [16 rows][128 B
 constexpr int kOffAcc = 0;                           /* [8 heads][128 dims] fp32: the finished piece, handed to the epilogue */
 constexpr int kOffLand = 0;                          /* landing zone of records / exchange lines when the page ring is not idle */
 constexpr int kLandBytes = kSlots * 2048;
-constexpr unsigned kLate = HY3A_LATE, kLateCut = HY3A_LATE_CUT;      /* the last pieces of a single-row grid start late: they take fewer pages */
 constexpr int kOffQ = kOffPt + kSlots * 2048;        /* Q fragments [4 k-steps][32 lanes] x 16 B */
 constexpr int kOffMisc = kOffQ + 2048;
 constexpr int kOffClu = kOffMisc + ((sizeof(u_misc) + 127) / 128) * 128;      /* a cluster's landing zone, at the cost of two pages of the ring */
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
     float4 pre_w = make_float4(1.f, 1.f, 1.f, 1.f), pre_f = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.fused && is_qk && qw < 8) {
         pre_w = *reinterpret_cast<const float4 *>(a.norm_w + rl_d0);
-        pre_f = *reinterpret_cast<const float4 *>(a.rope.inv_freq + (lane & 15) * 4);
+        pre_f = hy3a_rowops::rope_freqs(a.rope, lane);
     }
     if (warp == kIssWarp) {
         /* TMEM: kSlots pages x 4 groups x 16 columns (allocated by every CTA up front: the allocation takes about a microsecond) */
@@ -248,119 +248,41 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int i = tid; i < n; i += kUThreads) {
-        const int len = batch.slot[i] + 1;
-        s_prefix[i + 1] = len > 0 ? (len + HY3A_PT - 1) / HY3A_PT : 0;
+        if (n > 32) s_prefix[i + 1] = pages_of_slot(batch.slot[i]);
         s_pos[i] = batch.pos[i];
     }
-    if (tid == 0) {
-        s_prefix[0] = 0;
-        mi.abort_flag = 0;
-        mi.app_ready = 0;
-        for (int i = 0; i < kStages; i++) { mbar_init(UBAR(mi.rfull[i]), 1); mbar_init(UBAR(mi.rempty[i]), 1); }
-        for (int i = 0; i < kSlots; i++) {
-            mbar_init(UBAR(mi.pfull[i]), 128);      /* the four score warps of a page, every lane */
-            mbar_init(UBAR(mi.ofull[i]), 1);
-            mbar_init(UBAR(mi.bk[i]), 1);
-            mbar_init(UBAR(mi.sfree[i]), kAccWarps);
-        }
-        mbar_init(UBAR(mi.qload), 8);
-        if (CL) mbar_init(UBAR(mi.clu), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (CL) mbar_expect_tx(UBAR(mi.clu), kCluBytes);
-    }
-    __syncthreads();
-    if (CL) cluster_arrive();
-    if (n > 1) {
-        if (warp == 0) {
-            int carry = 0;
-            for (int base = 0; base < n; base += 32) {
-                const int i = base + lane;
-                int v = i < n ? s_prefix[i + 1] : 0;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, v, o);
-                    if (lane >= o) v += t;
-                }
-                if (i < n) s_prefix[i + 1] = v + carry;
-                carry += __shfl_sync(0xffffffffu, v, 31);
+    if (n > 32) __syncthreads();
+    const bool is_producer = warp == kProdWarp;
+    lane_rows rows = {-1, 0};
+    if (is_producer) {
+        /* the planning warp sets the barriers up while its rows' slots are on the way */
+        rows = load_rows(batch, n, lane);
+        if (lane == 0) {
+            mi.abort_flag = 0;
+            mi.app_ready = 0;
+            for (int i = 0; i < kStages; i++) { mbar_init(UBAR(mi.rfull[i]), 1); mbar_init(UBAR(mi.rempty[i]), 1); }
+            for (int i = 0; i < kSlots; i++) {
+                mbar_init(UBAR(mi.pfull[i]), 128);      /* the four score warps of a page, every lane */
+                mbar_init(UBAR(mi.ofull[i]), 1);
+                mbar_init(UBAR(mi.bk[i]), 1);
+                mbar_init(UBAR(mi.sfree[i]), kAccWarps);
             }
+            if (CL) mbar_init(UBAR(mi.clu), 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            if (CL) mbar_expect_tx(UBAR(mi.clu), kCluBytes);
         }
-        __syncthreads();
+        plan<1, CL>(&mi.plan, s_prefix, rows.slot, n, G, gridDim.x, cta, lane);
     }
-    /* ---- schedule: the unit split of decode.cu, in 32-bit arithmetic where the counts allow it (a 64-bit division costs
-     * hundreds of cycles, and a CTA that starts late has this code on the launch's critical path) */
-    const unsigned Pn = (unsigned)s_prefix[n];
-    const long long U = (long long)G * Pn;
-    bool idle = (U == 0);
-    const bool aligned = CL || ((long long)n * G < (long long)gridDim.x && aligned_split_balanced(s_prefix, n, G, gridDim.x, lane));
+    if (CL) cluster_arrive();      /* every CTA of the cluster has set its barrier up; cluster_wait below */
+    fence_before();
+    /* the others need the plan; the copies need no one.  A barrier of its own: the producer may be at the CTA's last one before the others are here */
+    if (is_producer) asm volatile("bar.arrive 4, %0;" ::"n"(kUThreads) : "memory");
+    else asm volatile("bar.sync 4, %0;" ::"n"(kUThreads) : "memory");
+    fence_after();
+    const long long U = (long long)G * s_prefix[n], u_begin = mi.plan.u0, u_end = mi.plan.u1;
+    const bool aligned = mi.plan.aligned, idle = u_begin == u_end;
     const int C = (long long)gridDim.x < U ? (int)gridDim.x : (int)U;
-    long long u_begin = 0, u_end = 0;
-    int al_first = 0, al_pieces = 1;
-    if (CL) {
-        cluster_share<CL ? CL : 1>(s_prefix, G, cta, u_begin, u_end);
-        idle = u_begin == u_end;
-    } else if (idle) {
-    } else if (aligned && Pn < (1u << 23)) {
-        int rows_ne = 0;
-        for (int r = 0; r < n; r++) rows_ne += (s_prefix[r + 1] != s_prefix[r]);
-        const unsigned spare = gridDim.x - (unsigned)(rows_ne * G), PG = Pn * (unsigned)G;   /* spare < 2^8, pages < 2^23 */
-        int base = 0;
-        bool found = false;
-        for (int r = 0; r < n && !found; r++) {
-            const unsigned p = (unsigned)(s_prefix[r + 1] - s_prefix[r]);
-            if (p == 0) continue;
-            unsigned c = min(1u + spare * p / PG, hy3a_most_pieces(p));
-            c = c < p ? c : p;
-            if (cta < base + G * (int)c) {
-                const unsigned idx = (unsigned)(cta - base), hl = idx / c, k = idx - hl * c;
-                const unsigned seg0 = (unsigned)G * (unsigned)s_prefix[r] + hl * p;
-                u_begin = seg0 + k * p / c;
-                u_end = seg0 + (k + 1u) * p / c;
-                /* The CTAs with the highest indices are dispatched last, onto the SMs that the preceding launch's folding CTAs
-                 * held longest: they start their ring fill late and would finish last (and then fold, and hold their SMs again).
-                 * In a single-row grid the last kLate pieces therefore take kLateCut pages less each and the other pieces of that
-                 * segment share them: 18.83 instead of 19.02 us per launch on the benchmark. */
-                if (rows_ne == 1 && hl == (unsigned)G - 1u && c > 2u * kLate && p >= 8u * c) {
-                    const unsigned pp = p + kLate * kLateCut, k1 = k + 1u;
-                    u_begin = seg0 + k * pp / c - kLateCut * (k > c - kLate ? k - (c - kLate) : 0u);
-                    u_end = seg0 + k1 * pp / c - kLateCut * (k1 > c - kLate ? k1 - (c - kLate) : 0u);
-                }
-                al_first = base + (int)(hl * c);
-                al_pieces = (int)c;
-                found = true;
-            }
-            base += G * (int)c;
-        }
-        if (!found) idle = true;
-    } else if (aligned) {
-        int rows_ne = 0;
-        for (int r = 0; r < n; r++) rows_ne += (s_prefix[r + 1] != s_prefix[r]);
-        const long long spare = (long long)gridDim.x - (long long)rows_ne * G, P = s_prefix[n];
-        int base = 0;
-        bool found = false;
-        for (int r = 0; r < n && !found; r++) {
-            const int p = s_prefix[r + 1] - s_prefix[r];
-            if (p == 0) continue;
-            int c = min(1 + (int)(spare * p / (P * G)), (int)hy3a_most_pieces((unsigned)p));
-            c = c < p ? c : p;
-            if (cta < base + G * c) {
-                const int idx = cta - base, hl = idx / c, k = idx % c;
-                const long long seg0 = (long long)G * s_prefix[r] + (long long)hl * p;
-                u_begin = seg0 + (long long)k * p / c;
-                u_end = seg0 + (long long)(k + 1) * p / c;
-                al_first = base + hl * c;
-                al_pieces = c;
-                found = true;
-            }
-            base += G * c;
-        }
-        if (!found) idle = true;
-    } else {
-        if (cta >= C) idle = true;
-        u_begin = (long long)cta * U / C;
-        u_end = (long long)(cta + 1) * U / C;
-        if (idle) u_begin = u_end = 0;
-    }
+    const int al_first = mi.plan.first, al_pieces = mi.plan.pieces;
     if (idle && !SHARD && !CL) {
         /* No pages: give the tensor memory back and leave -- behind the rows without keys, which belong to idle CTAs as well, and, where
          * no CTA has pages, behind the wait of CTA 0, so that such a launch too ends after the one before it (hy3a_batch_kernel relies
@@ -376,21 +298,13 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
     }
     segment sg0;                                                    /* the CTA's first piece */
     sg0.row = 0; sg0.hl = 0;
-    if (!idle) sg0 = locate(s_prefix, batch, n, G, u_begin, u_end);
+    if (!idle && !is_producer) sg0 = locate(s_prefix, batch, n, G, u_begin, u_end);
 
     /* fused step: cos / sin of the first segment's row (positions are in shared memory, the table in registers) */
     float pre_c[4] = {1.f, 1.f, 1.f, 1.f}, pre_s[4] = {0.f, 0.f, 0.f, 0.f};
     int pre_row = -1;
     auto rope_of_row = [&](int row) {
-        const int ti = s_pos[row];
-        const int pos = (ti + (ti >= a.rope.pos_jump_at ? a.rope.pos_jump : 0)) * a.rope.pos_stride;
-        const float fr4[4] = {pre_f.x, pre_f.y, pre_f.z, pre_f.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float fr = (float)pos * fr4[j];
-            pre_c[j] = cosf(fr) * a.rope.attn_factor;
-            pre_s[j] = sinf(fr) * a.rope.attn_factor;
-        }
+        hy3a_rowops::rope_coeffs(pre_c, pre_s, a.rope, pre_f, s_pos[row]);
         pre_row = row;
     };
     if (a.fused && !idle && is_qk && qw < 8) rope_of_row(sg0.row);
@@ -408,16 +322,12 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
             asm volatile("prefetch.global.L2 [%0];" ::"l"(kp));
         }
     }
-    fence_before();
-    __syncthreads();
-    fence_after();
-    if (CL) cluster_wait();      /* every CTA of the cluster has set its barrier up */
-    const unsigned tmem = mi.tmem;
+    if (CL && !is_producer) cluster_wait();
+    const unsigned tmem = is_producer ? 0u : mi.tmem;      /* the producer has not waited for it */
 
     /* From here on the kernel touches memory that the preceding kernel in the stream may produce (queries, the newest KV
      * slot, scratch records): wait for it -- except the producer lane, which first starts the copies of pages that lie
      * wholly below the newest slot (append-only cache: immutable). */
-    const bool is_producer = warp == kProdWarp;
     if (!is_producer) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -438,70 +348,54 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         }
 
     if (!idle && warp == kProdWarp) {
-        /* ================= producer: one lane streams the CTA's pages into the ring */
-        if (lane == 0) {
-            unsigned it = 0;
-            bool waited = false;   /* griddepcontrol.wait executed yet? */
-            bool app_seen = false; /* the CTA's fused appends are known to be complete */
-            const unsigned long long pol = l2_evict_first_policy();
-            /* once the preceding kernel is complete: ask L2 for the pages that do not fit the ring, so that HBM works
-             * while the queries are being prepared and the ring's own copies later hit L2 */
-            auto prefetch_rest = [&]() {
-                unsigned k = 0;
-                for (long long u2 = u_begin; u2 < u_end;) {
-                    const segment s2 = locate(s_prefix, batch, n, G, u2, u_end);
-                    const int *bt2 = cache.block_table + (size_t)s2.seq * cache.max_blocks_per_seq;
-                    for (int p2 = s2.p_begin; p2 < s2.p_end; p2++, k++) {
-                        if (k < (unsigned)kStages) continue;
-                        if (k >= (unsigned)kStages + 24u) return;    /* far enough ahead */
-                        const uint8_t *pg = cache.pool + hy3a_page_index(cache, bt2[p2], a.layer, s2.hl) * (size_t)cache.page_bytes;
-                        asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;" ::"l"(pg), "r"((unsigned)geom.page_bytes), "l"(pol) : "memory");
-                    }
-                    u2 = s2.seg_u0 + s2.p_end;
-                }
-            };
-            if (!a.early_prefetch) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
-            for (long long u = u_begin; u < u_end;) {
-                const segment sg = locate(s_prefix, batch, n, G, u, u_end);
-                const int *bt = cache.block_table + (size_t)sg.seq * cache.max_blocks_per_seq;
+        /* ================= producer: one lane streams the CTA's pages into the ring (the warp finds the segments).  Nothing is asked of L2 beyond the
+         * ring: the first copies of a launch are what HBM has to bring first, and a request for the next 24 pages at once took
+         * its bandwidth from the CTAs that start late (32 768 tokens 20.1 us a layer with it, 18.8 for 6 pages, 17.6 without; one page at a
+         * time, each behind its block-table entry, 17.5 against 17.6 with all entries held by the warp's lanes). */
+        unsigned it = 0;
+        bool waited = false;   /* griddepcontrol.wait executed yet? */
+        bool app_seen = false; /* the CTA's fused appends are known to be complete */
+        const unsigned long long pol = l2_evict_first_policy();
+        if (!a.early_prefetch) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
+        for (long long u = u_begin; u < u_end;) {
+            const segment sg = locate(s_prefix, batch, rows, n, G, u, u_end);
+            const int *bt = cache.block_table + (size_t)sg.seq * cache.max_blocks_per_seq;
+            if (lane == 0) {
                 int block_next = bt[sg.p_begin];
                 for (int p = sg.p_begin; p < sg.p_end; p++, it++) {
-                    const unsigned stage = it % (unsigned)kStages, phase = (it / (unsigned)kStages) & 1u;
                     const int block = block_next;
                     if (p + 1 < sg.p_end) block_next = bt[p + 1];   /* in flight while we wait for the stage */
+                    const unsigned stage = it % (unsigned)kStages, phase = (it / (unsigned)kStages) & 1u;
                     /* before the preceding kernel is known to be complete only pages that lie wholly below the newest
                      * slot may be fetched, and only into stages that were never used */
                     if (!waited && (it >= (unsigned)kStages || (p + 1) * HY3A_PT > sg.len - 2)) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
-                    if (it == (unsigned)kStages) {
-                        /* the ring is full and nothing is consumed yet: once the score warps hold their queries (their loads are
-                         * not to queue behind this burst), ask L2 for the rest */
-                        UWAIT(mi.qload, 0u, 4u);
-                        prefetch_rest();
-                    }
-                    if (!UWAIT(mi.rempty[stage], phase ^ 1u, 1u)) continue;      /* gave up: issue nothing more */
                     const uint8_t *page = cache.pool + hy3a_page_index(cache, block, a.layer, sg.hl) * (size_t)cache.page_bytes;
-                    if (a.fused && a.k_in && p == ((sg.len - 1) >> 7) && !app_seen) {
-                        /* the page that holds a newest slot: the accumulator warps append those rows at the start of the
-                         * kernel; their stores must be in HBM / L2 before the copy reads the page */
-                        volatile int *ready = &mi.app_ready;
-                        unsigned long long t0 = 0;
-                        for (unsigned i = 0; !*ready && i < (1u << 24); i++) {
-                            if ((i & 255u) == 255u) {
-                                unsigned long long t1;
-                                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-                                if (t0 == 0) t0 = t1;
-                                if (mi.abort_flag || (i >= (1u << 14) && t1 - t0 > 500000000ull)) { mi.abort_flag = 1; if (atomicCAS(a.err, 0u, 5u) == 0u) a.err[1] = 60u; break; }
+                    const bool newest = a.fused && a.k_in && p == ((sg.len - 1) >> 7);
+                    if (UWAIT(mi.rempty[stage], phase ^ 1u, 1u)) {      /* else gave up: issue nothing more */
+                        if (newest && !app_seen) {
+                            /* the page that holds a newest slot: the accumulator warps append those rows at the start of the
+                             * kernel; their stores must be in HBM / L2 before the copy reads the page */
+                            volatile int *ready = &mi.app_ready;
+                            unsigned long long t0 = 0;
+                            for (unsigned i = 0; !*ready && i < (1u << 24); i++) {
+                                if ((i & 255u) == 255u) {
+                                    unsigned long long t1;
+                                    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+                                    if (t0 == 0) t0 = t1;
+                                    if (mi.abort_flag || (i >= (1u << 14) && t1 - t0 > 500000000ull)) { mi.abort_flag = 1; if (atomicCAS(a.err, 0u, 5u) == 0u) a.err[1] = 60u; break; }
+                                }
                             }
+                            app_seen = true;
                         }
-                        app_seen = true;
+                        mbar_expect_tx(UBAR(mi.rfull[stage]), (unsigned)geom.page_bytes);
+                        bulk_g2s(ring_base + stage * (unsigned)kStageBytes, page, (unsigned)geom.page_bytes, UBAR(mi.rfull[stage]), pol);
                     }
-                    mbar_expect_tx(UBAR(mi.rfull[stage]), (unsigned)geom.page_bytes);
-                    bulk_g2s(ring_base + stage * (unsigned)kStageBytes, page, (unsigned)geom.page_bytes, UBAR(mi.rfull[stage]), pol);
                 }
-                u = sg.seg_u0 + sg.p_end;
             }
-            if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+            __syncwarp();
+            u = sg.seg_u0 + sg.p_end;
         }
+        if (lane == 0 && !waited) asm volatile("griddepcontrol.wait;" ::: "memory");
     } else if (!idle && warp == kIssWarp) {
         /* ================= MMA issuer: one lane; per page one wait, four MMAs back to back, one commit (the scalar code
          * between two tcgen05.mma of a thread costs more than the MMA itself, so this loop does nothing else) */
@@ -660,7 +554,6 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                 float m = fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3])));
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-                if (u == u_begin && lane == 0) mbar_arrive(UBAR(mi.qload));   /* the first piece's queries have arrived */
                 const float sqv = m > 0.f ? m * (1.f / 127.f) : 1.f, inv = 1.f / sqv;
                 unsigned hw = 0, lw = 0;
 #pragma unroll
@@ -713,8 +606,8 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
             if (SHARD) qk_sync();   /* everybody holds its share: the hand-over area is a landing zone below; else it is written again behind the next piece's queries */
 
             /* ---- how many CTAs share this segment? */
-            const int c_first = aligned ? al_first : (int)(((sg.seg_u0 + 1) * C + U - 1) / U) - 1;
-            const int npieces = aligned ? al_pieces : (int)((sg.seg_u1 * C + U - 1) / U) - 1 - c_first + 1;
+            const int c_first = aligned ? al_first : cta_of_unit(sg.seg_u0, U, C);
+            const int npieces = aligned ? al_pieces : cta_of_unit(sg.seg_u1 - 1, U, C) - c_first + 1;
             const int rec_base = aligned ? 0 : sidx;   /* record index = CTA (+ segment when CTAs may hold several pieces) */
             const size_t head_q = (size_t)(cache.kv_head_begin + hl) * 8 + h; /* global query head */
             u = sg.seg_u0 + sg.p_end;
@@ -862,7 +755,7 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
         __syncthreads();
         if (warp == kIssWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kSlots * 64) : "memory");
         /* a CTA's shared memory stays until every CTA of the cluster has sent (they have, unless a wait ran out) */
-        if (CL) { __syncwarp(); cluster_arrive(); cluster_wait(); }
+        if (CL) { __syncwarp(); if (is_producer) cluster_wait(); cluster_arrive(); cluster_wait(); }
     }
 }
 

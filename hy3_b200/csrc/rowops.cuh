@@ -73,10 +73,8 @@ __device__ __forceinline__ unsigned store_row(uint8_t *page, const hy3a_geom &g,
 
 /* cos/sin (times attn_factor) of the RoPE angles of this lane's 4 dim pairs at token index ti
  * (hy3_gpu.cu:152, :161-162). */
-__device__ __forceinline__ void rope_coeffs(float c[4], float s[4], const hy3a_rope_params &rope, int ti, int lane) {
-    const int idx = lane & 15;
+__device__ __forceinline__ void rope_coeffs(float c[4], float s[4], const hy3a_rope_params &rope, const float4 fv /* of the lane's dims */, int ti) {
     const int pos = (ti + (ti >= rope.pos_jump_at ? rope.pos_jump : 0)) * rope.pos_stride;
-    const float4 fv = *reinterpret_cast<const float4 *>(rope.inv_freq + idx * 4);
     const float fr4[4] = {fv.x, fv.y, fv.z, fv.w};
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -85,6 +83,8 @@ __device__ __forceinline__ void rope_coeffs(float c[4], float s[4], const hy3a_r
         s[j] = sinf(fr) * rope.attn_factor;
     }
 }
+__device__ __forceinline__ float4 rope_freqs(const hy3a_rope_params &rope, int lane) { return *reinterpret_cast<const float4 *>(rope.inv_freq + (lane & 15) * 4); }
+__device__ __forceinline__ void rope_coeffs(float c[4], float s[4], const hy3a_rope_params &rope, int ti, int lane) { rope_coeffs(c, s, rope, rope_freqs(rope, lane), ti); }
 
 /* RMSNorm (this lane's 4 weights wv, eps) + RoPE with precomputed coefficients of the warp's row y[4]. */
 __device__ __forceinline__ void norm_rope_apply(float y[4], const float4 wv, float eps, const float c[4], const float s[4], int lane) {
