@@ -140,6 +140,20 @@ template <int DT> __device__ __forceinline__ int stage_chunk(int h, int chunk) {
     return DT == 2 ? chunk ^ ((chunk >> 3) + 4 * (h & 1)) : chunk ^ (((chunk >> 3) & 1) + 2 * (h & 1));
 }
 
+/* ---- packed fp32 pairs, one instruction for two values (the same bits): the softmax of INT4 32-token granules, us a layer 68.6 -> 66.5 at 262 144
+ * tokens, 8 ragged rows 17.1 -> 17.0 */
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 w, x, y;\n mov.b64 {%0, %1}, w;\n}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 w, x, y;\n mov.b64 {%0, %1}, w;\n}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
 struct warp_state {
     float m;      /* reference max (base-2 logits), identical in the 4 lanes of a head; may lag the true max by 2^8 */
     float l;      /* this lane's share of the denominator */
@@ -233,8 +247,8 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
         /* rows 0-7 carry the high digit of q, rows 8-15 the low digit: q ~ sq*(hi + lo/254) */
 #pragma unroll
         for (int nb = 0; nb < NB; nb++) {
-            r[nb][0] = (float)(c[nb][0] * 254 + c[nb][2]) * qf;
-            r[nb][1] = (float)(c[nb][1] * 254 + c[nb][3]) * qf;
+            const float2 x = mul2(make_float2((float)(c[nb][0] * 254 + c[nb][2]), (float)(c[nb][1] * 254 + c[nb][3])), make_float2(qf, qf));
+            r[nb][0] = x.x; r[nb][1] = x.y;
         }
     }
     /* ---- logits (base 2) and V scales */
@@ -244,10 +258,11 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
         float2 kf = make_float2(1.f, 1.f), vf = make_float2(1.f, 1.f);
         if (DT != 0) { kf = unpack_h2(ksw[nb]); vf = unpack_h2(vsw[nb]); }
         const int t0 = kGran<DT> * gi + 8 * nb + 2 * tig;
-        s[nb][0] = (FULL || t0 < valid) ? r[nb][0] * kf.x : -INFINITY;
-        s[nb][1] = (FULL || t0 + 1 < valid) ? r[nb][1] * kf.y : -INFINITY;
-        vs[nb][0] = (FULL || t0 < valid) ? vf.x * pscale : 0.f;
-        vs[nb][1] = (FULL || t0 + 1 < valid) ? vf.y * pscale : 0.f;
+        const float2 x = mul2(make_float2(r[nb][0], r[nb][1]), kf), y = mul2(vf, make_float2(pscale, pscale));
+        s[nb][0] = (FULL || t0 < valid) ? x.x : -INFINITY;
+        s[nb][1] = (FULL || t0 + 1 < valid) ? x.y : -INFINITY;
+        vs[nb][0] = (FULL || t0 < valid) ? y.x : 0.f;
+        vs[nb][1] = (FULL || t0 + 1 < valid) ? y.y : 0.f;
     }
     /* ---- online softmax with a lazily updated reference max: O and l are only rescaled when
      * the granule's max exceeds the reference by more than 2^8; until then p <= 2^8, which the
@@ -274,11 +289,10 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
             float w[2][2], pe[2][2];
 #pragma unroll
             for (int nb = 0; nb < 2; nb++) {
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    pe[nb][e] = ex2(s[2 * nt + nb][e] - mref); /* -inf -> 0 */
-                    w[nb][e] = pe[nb][e] * vs[2 * nt + nb][e];
-                }
+                const float2 t = add2(make_float2(s[2 * nt + nb][0], s[2 * nt + nb][1]), make_float2(-mref, -mref));
+                pe[nb][0] = ex2(t.x); pe[nb][1] = ex2(t.y);      /* -inf -> 0 */
+                const float2 wv = mul2(make_float2(pe[nb][0], pe[nb][1]), make_float2(vs[2 * nt + nb][0], vs[2 * nt + nb][1]));
+                w[nb][0] = wv.x; w[nb][1] = wv.y;
             }
             st.l += (pe[0][0] + pe[0][1]) + (pe[1][0] + pe[1][1]);
             pa[0] = pack_h2(w[0][0], w[0][1]);
