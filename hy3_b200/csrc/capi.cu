@@ -260,8 +260,8 @@ int hy3a_create(const hy3a_config *cfg, hy3a_ctx **out) {
     /* fp16 operand mirrors of the chunked prefill: at most this much device memory beside the pool */
     { const char *e = getenv("HY3A_PF_MIRROR_MB"); ctx->pf_mbudget = (size_t)(e ? (atoll(e) > 0 ? atoll(e) : 0) : 8192) << 20; }
     ctx->pf_mseq = -1;
-    {   /* ring depth: as many pages as fit in shared memory beside the merge buffers, at most 8 */
-        ctx->decode_stages = hy3a_decode_ring_capacity(ctx->geom.page_bytes, cfg->max_batch);
+    {   /* ring depth: as many stages as fit in shared memory beside the merge buffers, at most 8 */
+        ctx->decode_stages = hy3a_decode_ring_capacity(ctx->geom.dtype, cfg->max_batch);
         const char *e = getenv("HY3A_DECODE_STAGES");
         if (e) { int v = atoi(e); if (v < ctx->decode_stages) ctx->decode_stages = v; }
     }

@@ -111,7 +111,7 @@ struct hy3a_ctx {
     int use_pdl;          /* launch kernels with programmatic stream serialization (HY3A_NO_PDL=1 turns it off) */
     int no_clusters;      /* HY3A_NO_CLUSTERS=1: decode and prefill keep to the grids (tests, comparisons) */
     int cl_cap[4];        /* decode: clusters of 2^i CTAs that fit on the device at once */
-    int decode_stages;    /* pages in the decode kernel's shared-memory ring; < 2 selects the direct-load variant */
+    int decode_stages;    /* stages of the decode kernel's shared-memory ring (pages; FP16: half pages); < 2 selects the direct-load variant */
 
     /* sequence-shard exchange over peer memory (hy3a_shard_*): one allocation per rank =
      * [n_slots][world][rows*heads][65] flagged 16-byte lines {value, flag, value, flag} of gathered records,
@@ -147,7 +147,7 @@ int hy3a_launch_fill_random(hy3a_ctx *ctx, int layer, int seq, int t0, int n, ui
 int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq, const void *q16, float *out,
                         size_t out_stride);
 int hy3a_launch_init_pages(hy3a_ctx *ctx, size_t first_page, size_t n_pages);
-int hy3a_decode_ring_capacity(int page_bytes, int max_batch);
+int hy3a_decode_ring_capacity(int dtype, int max_batch);
 int hy3a_decode_max_ctas(void);
 void hy3a_decode_cluster_init(hy3a_ctx *ctx);   /* fills cl_cap */
 int hy3a_fail(hy3a_ctx *ctx, int code, const char *fmt, ...);

@@ -167,7 +167,13 @@ __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;"
  * independent score chains cover each other's latency: 262 144 positions 82.9 -> 73.8 us a layer (3.3 -> 3.75 TB/s), 8 ragged
  * sequences of up to 8 000 tokens 27.3 -> 26.2 us.  FP16 keeps 16: its K and V registers would not fit twice. */
 template <int DT> constexpr int kGran = DT == 2 ? 32 : 16;
-template <int DT> constexpr int kGranPage = HY3A_PT / kGran<DT>;
+/* A stage of the ring: an INT4 page, half an FP16 page (64 tokens: K and V rows in one copy each).  Halves fill what two whole pages leave
+ * of the shared memory (5 x 32 KB instead of 2 x 64), come and go in smaller steps, and the half behind a row's last token is not fetched: 16 000
+ * tokens 17.3 -> 16.5 us a layer, 32 768 26.6 -> 25.8. */
+template <int DT> constexpr int kStageTok = DT == 0 ? 64 : 128;
+template <int DT> constexpr int kStageBytes = DT == 0 ? 32768 : 16896;
+template <int DT> constexpr int kStageV = DT == 0 ? 16384 : 8192;      /* V area of a stage */
+template <int DT, bool STAGED> constexpr int kGranStage = (STAGED ? kStageTok<DT> : HY3A_PT) / kGran<DT>;
 
 /* One granule of one warp: loads, S = Q.K^T, online softmax, O += P.V.
  * SM: operands come from a shared-memory copy of the page (32-bit shared addresses) instead
@@ -181,8 +187,8 @@ __device__ __forceinline__ void granule(warp_state &st, unsigned sq, float qf, c
     constexpr int NK = DT == 0 ? 4 : 1;
     constexpr int NV = DT == 0 ? 8 : 2;                      /* V chunks per 16 tokens */
     constexpr int NB = kGran<DT> / 8, NT = kGran<DT> / 16;   /* 8-token blocks, 16-token halves */
-    /* page-relative byte offsets of granule gi (16 tokens = 16 K rows = 8 V pair-rows) */
-    const int gk = gi * kGran<DT> * geom.k_row, gv = geom.v_off + gi * (DT == 0 ? 16 : 8 * NT) * geom.v_prow, gs = gi * 2 * kGran<DT>;
+    /* byte offsets of granule gi in the stage (or page) */
+    const int gk = gi * kGran<DT> * geom.k_row, gv = (SM ? kStageV<DT> : geom.v_off) + gi * (DT == 0 ? 16 : 8 * NT) * geom.v_prow, gs = gi * 2 * kGran<DT>;
     uint4 kr[NB][NK];
 #pragma unroll
     for (int nb = 0; nb < NB; nb++) {
@@ -390,8 +396,8 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
         if (lane == 0) {
             s_abort = 0;
             if (STAGED) {
-                for (int i = 0; i < a.stages; i++) mbar_init(bar_base + 8 * i, 32 * kGranPage<DT>);   /* empty[stage]: every thread of the warps that share a page */
-                for (int i = 0; i < 16; i++) mbar_init(bar_base + 64 + 8 * i, 1);   /* full[page mod n_full]: the producer's expect_tx */
+                for (int i = 0; i < a.stages; i++) mbar_init(bar_base + 8 * i, 32 * kGranStage<DT, STAGED>);   /* empty[stage]: every thread of the warps that share it */
+                for (int i = 0; i < 16; i++) mbar_init(bar_base + 64 + 8 * i, 1);   /* full[ring position mod n_full]: the producer's expect_tx */
                 if (CL) mbar_init(bar_base + kBarClu, 1);
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
                 if (CL) mbar_expect_tx(bar_base + kBarClu, kCluBytes);
@@ -461,19 +467,28 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             const int *bt = cache.block_table + (size_t)sg.seq * cache.max_blocks_per_seq;
             if (lane == 0) {
                 int block_next = bt[sg.p_begin];
-                for (int p = sg.p_begin; p < sg.p_end; p++, it++) {
-                    const unsigned stage = it % (unsigned)a.stages, phase = (it / (unsigned)a.stages) & 1u;
+                for (int p = sg.p_begin; p < sg.p_end; p++) {
                     const int block = block_next;
                     if (p + 1 < sg.p_end) block_next = bt[p + 1];   /* in flight while we wait for the stage */
-                    /* before the preceding kernel is known to be complete only pages that lie wholly below
-                     * the newest slot may be fetched, and only into stages that were never used            */
-                    if (!waited && (it >= (unsigned)a.stages || (p + 1) * HY3A_PT > sg.len - 2)) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
-                    ok = mbar_wait(bar_base + 8 * stage, phase ^ 1u, &s_abort, a.err, 1u);
-                    if (!ok) break;
                     const uint8_t *page = cache.pool + hy3a_page_index(cache, block, a.layer, sg.hl) * (size_t)cache.page_bytes;
-                    const unsigned full = bar_base + 64 + 8 * (it % n_full);
-                    mbar_expect_tx(full, (unsigned)geom.page_bytes);
-                    bulk_g2s(ring_base + stage * (unsigned)geom.page_bytes, page, (unsigned)geom.page_bytes, full, pol);
+#pragma unroll 1
+                    for (int t0 = p * HY3A_PT, half = 0; t0 < min(sg.len, (p + 1) * HY3A_PT); t0 += kStageTok<DT>, half++, it++) {
+                        const unsigned stage = it % (unsigned)a.stages, phase = (it / (unsigned)a.stages) & 1u;
+                        /* before the preceding kernel is known to be complete only tokens that lie wholly below
+                         * the newest slot may be fetched, and only into stages that were never used            */
+                        if (!waited && (it >= (unsigned)a.stages || t0 + kStageTok<DT> > sg.len - 2)) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
+                        ok = mbar_wait(bar_base + 8 * stage, phase ^ 1u, &s_abort, a.err, 1u);
+                        if (!ok) break;
+                        const unsigned full = bar_base + 64 + 8 * (it % n_full), dst = ring_base + stage * (unsigned)kStageBytes<DT>;
+                        mbar_expect_tx(full, (unsigned)kStageBytes<DT>);
+                        if (DT == 0) {
+                            bulk_g2s(dst, page + half * kStageV<DT>, kStageV<DT>, full, pol);
+                            bulk_g2s(dst + kStageV<DT>, page + geom.v_off + half * kStageV<DT>, kStageV<DT>, full, pol);
+                        } else {
+                            bulk_g2s(dst, page, (unsigned)kStageBytes<DT>, full, pol);
+                        }
+                    }
+                    if (!ok) break;
                 }
             }
             ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -637,14 +652,16 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
 #pragma unroll
         for (int jn = 0; jn < 16; jn++) { st.o[jn][0] = st.o[jn][1] = st.o[jn][2] = st.o[jn][3] = 0.f; }
 
-        /* granule slot x = GP*(ring position of the page) + granule-in-page; warp w takes slots
-         * x = w (mod kWarps), so any number of consumer warps shares the GP granules of a page and
-         * each page is released by exactly GP warps (one arrival per thread per slot).            */
-        constexpr unsigned GP = kGranPage<DT>;
-        constexpr int GT = kGran<DT>;
-        const unsigned it_end = it + (unsigned)(sg.p_end - sg.p_begin);
+        /* granule slot x = GP*(ring position of the stage) + granule-in-stage; warp w takes slots
+         * x = w (mod kWarps), so any number of consumer warps shares the GP granules of a stage and
+         * each stage is released by exactly GP warps (one arrival per thread per slot).  (Direct variant: stage = page.) */
+        constexpr unsigned GP = kGranStage<DT, STAGED>;
+        constexpr int GT = kGran<DT>, ST = STAGED ? kStageTok<DT> : HY3A_PT;
+        /* stages of the piece, and of those in the sequence's last page */
+        const int t_end = min(sg.len, sg.p_end * HY3A_PT), tail_t0 = (sg.pages - 1) * HY3A_PT;
+        const unsigned it_end = it + (unsigned)((t_end - sg.p_begin * HY3A_PT + ST - 1) / ST);
         unsigned x = it * GP + ((unsigned)warp + kWarps - (it * GP) % kWarps) % kWarps, pit = x / GP;
-        /* ring position of page pit, its "full" barrier and that barrier's phase, carried along (no divisions per granule) */
+        /* ring position of stage pit, its "full" barrier and that barrier's phase, carried along (no divisions per granule) */
         unsigned stage = STAGED ? pit % (unsigned)a.stages : 0u, fb = pit % n_full, fphase = (pit / n_full) & 1u;
         auto advance = [&]() {
             x += kWarps;
@@ -658,42 +675,46 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             }
         };
         if (STAGED) {
-            /* A warp holds granules in GP of every 11 pages, so it may skip a use of a stage, and an mbarrier wait only knows
+            /* A warp holds granules in GP of every 11 stages, so it may skip a use of a stage, and an mbarrier wait only knows
              * the parity of a phase: with one "full" barrier per stage the warp's next wait on that stage could pass on the
-             * stale phase while the skipped page is still landing (seen with the two-stage ring of FP16 pages).  So the
-             * barriers are cycled over n_full pages: page pit - n_full, whose phase a wait for pit could mistake, has long
-             * been consumed, because this warp's last page pit' >= pit - ceil(11 / GP) was issued after page pit' - stages
+             * stale phase while the skipped copy is still landing (seen with a two-stage ring of FP16 pages).  So the
+             * barriers are cycled over n_full ring positions: position pit - n_full, whose phase a wait for pit could mistake, has
+             * long been consumed, because this warp's last position pit' >= pit - ceil(11 / GP) was issued after pit' - stages
              * had been consumed, and n_full >= stages + ceil(11 / GP). */
             auto page_wait = [&]() {
                 mbar_wait(bar_base + 64 + 8 * fb, fphase, &s_abort, a.err, 2u);
-                return ring_base + stage * (unsigned)geom.page_bytes;
+                return ring_base + stage * (unsigned)kStageBytes<DT>;
             };
             /* The sequence's last page has its masks and the fused append; it stands behind the loop (a warp has one granule of it at most),
              * whose body is then one granule's code
              * (INT4 8 ragged rows 18.0 -> 17.3 us a layer, 32 768 tokens 17.0 -> 16.5; FP16 32 768 26.8 -> 26.6). */
-            const unsigned whole = it_end - (sg.p_end == sg.pages ? 1u : 0u);
+            const unsigned whole = it_end - (sg.p_end == sg.pages ? (unsigned)((sg.len - tail_t0 + ST - 1) / ST) : 0u);
             for (; x < whole * GP; advance()) {
                 const unsigned spage = page_wait();
                 granule<DT, true, true>(st, sq, qf, nullptr, spage, geom, k_off, v_off, sc_off, (int)(x % GP), tig, HY3A_PT, pscale);
                 mbar_arrive(bar_base + 8 * stage); /* every thread of the warps that share a page releases it */
             }
             if (x < it_end * GP) {
-                const int gi = (int)(x % GP), valid = sg.len - (sg.p_end - 1) * HY3A_PT;
+                /* valid: tokens from the stage's first one on; the newest is number valid - 1 */
+                const int gi = (int)(x % GP), valid = sg.len - tail_t0 - (int)(pit - whole) * ST;
                 const unsigned spage = page_wait();
-                if (has_new && gi == ((sg.len - 1) & 127) / GT) {
+                if (has_new && valid <= ST && gi == (valid - 1) / GT) {
                     /* fused append: this warp holds the only granule that contains the newest slot.  It quantises the new rows
                      * exactly as the append kernel does and writes them into the shared-memory copy it is about to read and to
                      * the page in HBM (for later steps). */
                     const int tok = (sg.len - 1) & 127;
                     uint8_t *gp = cache.pool + hy3a_page_index(cache, new_block, a.layer, hl) * (size_t)cache.page_bytes;
-                    uint8_t *sp = s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + (size_t)stage * geom.page_bytes;
+                    uint8_t *sp = s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + (size_t)stage * kStageBytes<DT>;
+                    hy3a_geom sgeom = geom;      /* of the stage: its rows are swizzled alike */
+                    sgeom.v_off = kStageV<DT>;
+                    const int stok = valid - 1;
                     float4 r4 = *reinterpret_cast<const float4 *>(&s_new[0][rl_d0]);
                     float y[4] = {r4.x, r4.y, r4.z, r4.w};
-                    hy3a_rowops::store_row<DT>(sp, geom, tok, false, y, rl_d0, lane);
+                    hy3a_rowops::store_row<DT>(sp, sgeom, stok, false, y, rl_d0, lane);
                     hy3a_rowops::store_row<DT>(gp, geom, tok, false, y, rl_d0, lane);
                     r4 = *reinterpret_cast<const float4 *>(&s_new[1][rl_d0]);
                     y[0] = r4.x; y[1] = r4.y; y[2] = r4.z; y[3] = r4.w;
-                    const unsigned sb = hy3a_rowops::store_row<DT>(sp, geom, tok, true, y, rl_d0, lane);
+                    const unsigned sb = hy3a_rowops::store_row<DT>(sp, sgeom, stok, true, y, rl_d0, lane);
                     hy3a_rowops::store_row<DT>(gp, geom, tok, true, y, rl_d0, lane);
                     if (DT != 0 && lane == 0) atomicMax(cache.vs_max + a.layer * G + hl, sb);
                     __syncwarp();
@@ -801,7 +822,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 const bool mine = red && h >= h_lo && h < h_hi;
                 M = -INFINITY; L = 0.f; acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
                 if (s_flag && mine) {
-                    const int slots = min(32, a.stages * geom.page_bytes / (hpf * 512));      /* the ring is idle: this CTA's pages are consumed */
+                    const int slots = min(32, a.stages * kStageBytes<DT> / (hpf * 512));      /* the ring is idle: this CTA's pages are consumed */
                     fold_records(recs, npieces, s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + (h - h_lo) * slots * 512, 512u, slots, lane, M, L, acc);
                 }
                 consumer_sync();   /* every landing zone is read (the sharded exchange lands its lines in the ring too) */
@@ -815,7 +836,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 /* The last CTA to arrive folds, nobody waits.  The records land in the page ring where it is idle (whole CTAs to a segment:
                  * this CTA's pages are consumed), else in the head's column of s_o, which this warp alone has read. */
                 const bool ring = STAGED && aligned;
-                const int slots = ring ? min(32, a.stages * geom.page_bytes / 4096) : kWarps;
+                const int slots = ring ? min(32, a.stages * kStageBytes<DT> / 4096) : kWarps;
                 uint8_t *const zone = ring ? s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL> + h * slots * 512 : reinterpret_cast<uint8_t *>(s_o[0][h]);
                 if (red) last = fold_last(recs, cta - c_first, npieces, a.counters + 8 * sidx + h, zone, ring ? 512u : (unsigned)sizeof(s_o[0]), slots, lane, M, L, acc);
                 if (SHARD) consumer_sync();      /* the exchange lands its lines there too */
@@ -843,7 +864,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 fa.out = a.out + (size_t)row * a.out_stride + ((size_t)(cache.kv_head_begin + hl) * 8 + h) * HY3A_D + d4;
                 fa.n_ranks = a.n_dest; fa.my_rank = a.my_rank; fa.line_a = 1 + (d4 >> 1); fa.flag = flag; fa.stage = reinterpret_cast<const uint4 *>(s_dyn); fa.h = h; fa.lane = lane;
                 fa.own_m = m_nat; fa.own_l = L; fa.own_acc[0] = acc[0]; fa.own_acc[1] = acc[1]; fa.own_acc[2] = acc[2]; fa.own_acc[3] = acc[3];
-                if (STAGED && aligned && (size_t)a.stages * geom.page_bytes >= (size_t)8 * 8 * kShardLines * 16) {
+                if (STAGED && aligned && (size_t)a.stages * kStageBytes<DT> >= (size_t)8 * 8 * kShardLines * 16) {
                     /* CTA-aligned segments: the page ring is idle by now and holds all 8 ranks' records at once, so
                      * every rank is polled in the same round */
                     fa.stage = reinterpret_cast<const uint4 *>(s_dyn + kFixed<CL> + a.prefix_bytes + kBarBytes<CL>);
@@ -929,6 +950,7 @@ __global__ void hy3a_merge_kernel(const float *partials, int n_parts, int n_rows
 
 /* a launch's shared memory */
 static size_t prefix_bytes(int rows) { return ((size_t)(rows + 1) * sizeof(int) + 127) & ~(size_t)127; }
+static size_t ring_bytes(const hy3a_ctx *ctx) { return (size_t)ctx->decode_stages * (ctx->geom.dtype == HY3A_KV_FP16 ? kStageBytes<0> : kStageBytes<2>); }      /* not INT8's */
 template <int CL>
 static size_t decode_smem(size_t prefix, size_t ring) { return kFixed<CL> + prefix + kBarBytes<CL> + ring; }
 
@@ -965,7 +987,7 @@ int hy3a_cluster_cap(const void *fn, int cl, int threads, size_t smem) {
 }
 
 void hy3a_decode_cluster_init(hy3a_ctx *ctx) {
-    const size_t smem = decode_smem<2>(prefix_bytes(1), ctx->decode_stages * (size_t)ctx->geom.page_bytes);      /* one CTA per SM at any batch: its registers fill more than half */
+    const size_t smem = decode_smem<2>(prefix_bytes(1), ring_bytes(ctx));      /* one CTA per SM at any batch: its registers fill more than half */
     for (int i = 1; i < 4; i++) {
         if (ctx->decode_stages < 2) ctx->cl_cap[i] = 0;
         else if (ctx->geom.dtype == HY3A_KV_INT8) ctx->cl_cap[i] = hy3a_decode_umma_cluster_cap(ctx, 1 << i);
@@ -984,11 +1006,11 @@ static cudaError_t launch_decode_dt(hy3a_ctx *ctx, const hy3a_cache_view &cv, co
         a.stages = ctx->decode_stages;
         void *args[3] = {(void *)&cv, (void *)&bv, (void *)&a};
         return hy3a_launch_cluster(ctx, decode_cluster_fn<DT>(a.cluster), a.cluster, ctx->batch_n * ctx->cfg.kv_head_count, kThreads + 32,
-                                   decode_smem<2>(prefix, a.stages * (size_t)ctx->geom.page_bytes), args);
+                                   decode_smem<2>(prefix, ring_bytes(ctx)), args);
     }
     if (ctx->decode_stages >= 2) {
         a.stages = ctx->decode_stages;
-        const size_t smem = decode_smem<0>(prefix, a.stages * (size_t)ctx->geom.page_bytes);
+        const size_t smem = decode_smem<0>(prefix, ring_bytes(ctx));
         const bool shard = a.n_dest > 0;
         if (!attr_set[DT][shard ? 2 : 1]) {
             cudaError_t e = shard ? cudaFuncSetAttribute(hy3a_decode_kernel<DT, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax)
@@ -1016,11 +1038,11 @@ static cudaError_t launch_decode_dt(hy3a_ctx *ctx, const hy3a_cache_view &cv, co
     return cudaGetLastError();
 }
 
-/* Pages that fit in the ring for a given page size and batch capacity. */
-int hy3a_decode_ring_capacity(int page_bytes, int max_batch) {
-    long room = (long)kSmemMax - (long)decode_smem<0>(prefix_bytes(max_batch), 0);
-    int s = room > 0 ? (int)(room / page_bytes) : 0;
-    return s > 8 ? 8 : s;
+/* Stages that fit in the ring for a cache type and batch capacity, at most 8; none where two whole pages do not fit (the direct variant). */
+int hy3a_decode_ring_capacity(int dtype, int max_batch) {
+    const long room = (long)kSmemMax - (long)decode_smem<0>(prefix_bytes(max_batch), 0);
+    const int page = hy3a_make_geom(dtype).page_bytes, stage = dtype == HY3A_KV_FP16 ? kStageBytes<0> : page;
+    return room < 2l * page ? 0 : (int)std::min(8l, room / stage);
 }
 /* Largest grid the last-arrival merge can stage in the merge buffer. */
 int hy3a_decode_max_ctas(void) { return kFixedO / 64; }
@@ -1051,7 +1073,7 @@ static int cluster_size(const hy3a_ctx *ctx, int most, long long total) {
     const int dt = ctx->geom.dtype, segs = ctx->batch_n * ctx->cfg.kv_head_count;
     if (most < 2 || segs > ctx->cl_cap[1]) return 0;
     /* a ring that a context of very large batches has sized to the last byte leaves no room for the landing zone */
-    if (dt != HY3A_KV_INT8 && decode_smem<2>(prefix_bytes(ctx->batch_n), ctx->decode_stages * (size_t)ctx->geom.page_bytes) > (size_t)kSmemMax) return 0;
+    if (dt != HY3A_KV_INT8 && decode_smem<2>(prefix_bytes(ctx->batch_n), ring_bytes(ctx)) > (size_t)kSmemMax) return 0;
     int i = 1;
     while (i < 3 && ((most - 1) >> i) + 1 > kPagesCta[dt] && segs <= ctx->cl_cap[i + 1]) i++;
     const long long share = (total * ctx->cfg.kv_head_count + ctx->decode_ctas - 1) / ctx->decode_ctas;

@@ -48,7 +48,7 @@ struct hy3a_decode_args {
     const float *norm_w;  /* [2][128] of this layer */
     float eps;
     hy3a_rope_params rope;
-    int stages;           /* staged variant: pages in the shared-memory ring (2..8) */
+    int stages;           /* staged variant: stages of the shared-memory ring (2..8) */
     int prefix_bytes;     /* bytes reserved for the page-count prefix */
 };
 
