@@ -455,9 +455,11 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
 
 
     if (STAGED && warp == kWarps) {
-        /* ================= producer warp: one lane streams the CTA's pages into the ring (the warp finds the segments).  With every lane in the
-         * loop, each holding a page's block-table entry, INT4 262 144 tokens take 71 us a layer instead of 67. */
-        unsigned it = 0;
+        /* ================= producer warp: one lane streams the CTA's pages into the ring (the warp finds the segments).  It shares a
+         * scheduler with two consumer warps, so the loop is short: stage, parity and barrier are carried along, addresses are a base and a
+         * stride.  INT4 262 144 tokens 66.5 -> 62.5 us a layer, 8 ragged rows 17.0 -> 16.7; with every lane in the loop, each holding a
+         * page's block-table entry, 71. */
+        unsigned it = 0, stage = 0, phase = 1, fb = 0;      /* ring position, its stage, the parity to wait for there and its "full" barrier, carried along */
         bool ok = true;
         bool waited = false;   /* griddepcontrol.wait executed yet? */
         const unsigned long long pol = l2_evict_first_policy();
@@ -466,27 +468,32 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
             const segment sg = locate(s_prefix, batch, rows, n, G, u, u_end);
             const int *bt = cache.block_table + (size_t)sg.seq * cache.max_blocks_per_seq;
             if (lane == 0) {
+                const uint8_t *page0 = cache.pool + hy3a_page_index(cache, 0, a.layer, sg.hl) * (size_t)cache.page_bytes;
+                const size_t block_bytes = (hy3a_page_index(cache, 1, a.layer, sg.hl) - hy3a_page_index(cache, 0, a.layer, sg.hl)) * (size_t)cache.page_bytes;
                 int block_next = bt[sg.p_begin];
                 for (int p = sg.p_begin; p < sg.p_end; p++) {
-                    const int block = block_next;
+                    const uint8_t *page = page0 + block_next * block_bytes;
                     if (p + 1 < sg.p_end) block_next = bt[p + 1];   /* in flight while we wait for the stage */
-                    const uint8_t *page = cache.pool + hy3a_page_index(cache, block, a.layer, sg.hl) * (size_t)cache.page_bytes;
-#pragma unroll 1
-                    for (int t0 = p * HY3A_PT, half = 0; t0 < min(sg.len, (p + 1) * HY3A_PT); t0 += kStageTok<DT>, half++, it++) {
-                        const unsigned stage = it % (unsigned)a.stages, phase = (it / (unsigned)a.stages) & 1u;
+#pragma unroll
+                    for (int half = 0; half < HY3A_PT / kStageTok<DT>; half++) {
+                        const int t_end = p * HY3A_PT + (half + 1) * kStageTok<DT>;
+                        if (half && t_end - kStageTok<DT> >= sg.len) break;
                         /* before the preceding kernel is known to be complete only tokens that lie wholly below
                          * the newest slot may be fetched, and only into stages that were never used            */
-                        if (!waited && (it >= (unsigned)a.stages || t0 + kStageTok<DT> > sg.len - 2)) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
-                        ok = mbar_wait(bar_base + 8 * stage, phase ^ 1u, &s_abort, a.err, 1u);
+                        if (!waited && (it >= (unsigned)a.stages || t_end > sg.len - 2)) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
+                        ok = mbar_wait(bar_base + 8 * stage, phase, &s_abort, a.err, 1u);
                         if (!ok) break;
-                        const unsigned full = bar_base + 64 + 8 * (it % n_full), dst = ring_base + stage * (unsigned)kStageBytes<DT>;
+                        const unsigned full = bar_base + 64 + 8 * fb, dst = ring_base + stage * (unsigned)kStageBytes<DT>;
                         mbar_expect_tx(full, (unsigned)kStageBytes<DT>);
                         if (DT == 0) {
                             bulk_g2s(dst, page + half * kStageV<DT>, kStageV<DT>, full, pol);
-                            bulk_g2s(dst + kStageV<DT>, page + geom.v_off + half * kStageV<DT>, kStageV<DT>, full, pol);
+                            bulk_g2s(dst + kStageV<DT>, page + HY3A_PT * 256 + half * kStageV<DT>, kStageV<DT>, full, pol);
                         } else {
                             bulk_g2s(dst, page, (unsigned)kStageBytes<DT>, full, pol);
                         }
+                        it++;
+                        if (++stage == (unsigned)a.stages) { stage = 0; phase ^= 1u; }
+                        if (++fb == n_full) fb = 0;
                     }
                     if (!ok) break;
                 }
@@ -686,8 +693,7 @@ __global__ void __launch_bounds__(kThreads + (STAGED ? 32 : 0), 1) hy3a_decode_k
                 return ring_base + stage * (unsigned)kStageBytes<DT>;
             };
             /* The sequence's last page has its masks and the fused append; it stands behind the loop (a warp has one granule of it at most),
-             * whose body is then one granule's code
-             * (INT4 8 ragged rows 18.0 -> 17.3 us a layer, 32 768 tokens 17.0 -> 16.5; FP16 32 768 26.8 -> 26.6). */
+             * whose body is then one granule's code (INT4 8 ragged rows 18.0 -> 17.3 us a layer, 32 768 tokens 17.0 -> 16.5; FP16 32 768 26.8 -> 26.6). */
             const unsigned whole = it_end - (sg.p_end == sg.pages ? (unsigned)((sg.len - tail_t0 + ST - 1) / ST) : 0u);
             for (; x < whole * GP; advance()) {
                 const unsigned spage = page_wait();

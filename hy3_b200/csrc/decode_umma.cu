@@ -361,15 +361,16 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
             const segment sg = locate(s_prefix, batch, rows, n, G, u, u_end);
             const int *bt = cache.block_table + (size_t)sg.seq * cache.max_blocks_per_seq;
             if (lane == 0) {
+                const uint8_t *page0 = cache.pool + hy3a_page_index(cache, 0, a.layer, sg.hl) * (size_t)cache.page_bytes;
+                const size_t block_bytes = (hy3a_page_index(cache, 1, a.layer, sg.hl) - hy3a_page_index(cache, 0, a.layer, sg.hl)) * (size_t)cache.page_bytes;
                 int block_next = bt[sg.p_begin];
                 for (int p = sg.p_begin; p < sg.p_end; p++, it++) {
-                    const int block = block_next;
+                    const uint8_t *page = page0 + block_next * block_bytes;
                     if (p + 1 < sg.p_end) block_next = bt[p + 1];   /* in flight while we wait for the stage */
                     const unsigned stage = it % (unsigned)kStages, phase = (it / (unsigned)kStages) & 1u;
                     /* before the preceding kernel is known to be complete only pages that lie wholly below the newest
                      * slot may be fetched, and only into stages that were never used */
                     if (!waited && (it >= (unsigned)kStages || (p + 1) * HY3A_PT > sg.len - 2)) { asm volatile("griddepcontrol.wait;" ::: "memory"); waited = true; }
-                    const uint8_t *page = cache.pool + hy3a_page_index(cache, block, a.layer, sg.hl) * (size_t)cache.page_bytes;
                     const bool newest = a.fused && a.k_in && p == ((sg.len - 1) >> 7);
                     if (UWAIT(mi.rempty[stage], phase ^ 1u, 1u)) {      /* else gave up: issue nothing more */
                         if (newest && !app_seen) {
