@@ -13,7 +13,7 @@
  *      K-major operands for the tensor cores.  The operands of a layer are kept across chunks (the
  *      context's per-layer mirrors), so a chunk only converts the pages it appended.
  *   2. hy3a_prefill_kernel: one CTA per (32 query tokens x the 8 query heads of one KV head) = two
- *      128-row Q tiles (GQA packing: the 8 heads share every K/V tile).  Warp-specialised:
+ *      128-row Q tiles (one in the clusters of short chunks) (GQA packing: the 8 heads share every K/V tile).  Warp-specialised:
  *        TMA producer: Q once, then 64-key K / V tiles into 4-stage rings (cp.async.bulk.tensor,
  *                 128-byte swizzle, mbarrier transaction counts)
  *        MMA issuers (one warp per Q tile, one elected lane): S = Q.K^T (M=128, N=64, K=16) and
@@ -177,20 +177,20 @@ __device__ __forceinline__ float ex2v(float x) { float r; asm volatile("ex2.appr
  * rounding of P is a zero-mean 2^-12 relative error per term, far below the tolerance).  One pair in eight goes through the FMA
  * pipe: 512 tokens behind 4 096 take 73.0 us with none, 70.8 with one, 73.0 with two (the FMA form costs issue slots that the
  * waiting tile's maximum wants); 2 048 fresh tokens 82.1 / 81.6 / 82.3. */
-template <bool CUT>
+template <bool CUT, bool TURNS>
 __device__ __forceinline__ float2 softmax_exp(const unsigned (&v)[64], float m, unsigned (&pk)[32], int x, bool pass) {
     /* m == -inf: every key of the row so far is masked; the arguments are then -inf, not NaN, and all P are 0 */
     const float2 sc = splat(kScaleLog2), nm = splat(CUT && m == -INFINITY ? 0.f : -m);
     float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, t[32];
 #pragma unroll
     for (int i = 0; i < 32; i++) t[i] = fma2(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sc, nm);
-    turn_wait(x);
+    if (TURNS) turn_wait(x);
 #pragma unroll
     for (int i = 0; i < 32; i++) {
         if ((i & 7) == 7) t[i] = ex2_fma(t[i]);
         else { t[i].x = ex2v(t[i].x); t[i].y = ex2v(t[i].y); }
     }
-    if (pass) turn_pass(x);
+    if (TURNS && pass) turn_pass(x);
 #pragma unroll
     for (int i = 0; i < 32; i++) {
         pk[i] = pack_h2(t[i].x, t[i].y);
@@ -335,7 +335,10 @@ __device__ __forceinline__ void st_cluster16(unsigned addr, float a, float b, fl
 __device__ __forceinline__ void st_cluster8(unsigned addr, float a, float b) {
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
 }
-template <int MODE, int CL>
+/* TILES: query tiles of a CTA.  One only in clusters, where blocks of 16 tokens fit at once as well (hy3a_launch_prefill): a block then
+ * has half the exchange and half the softmax, and none for a second tile without tokens; warps 4-7 and 10 have nothing to do.  us a layer with its
+ * append, two tiles / one: 45 tokens behind 1 001 19.7 / 15.2, 64 behind 8 192 43.6 / 34.2, 16 behind 500 13.9 / 12.7. */
+template <int MODE, int CL, int TILES = 2>
 __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUtensorMap &tm_k, const CUtensorMap &tm_v, const prefill_args &a, const pf_where &w) {
     extern __shared__ uint8_t s_raw[];
     uint8_t *sm = s_raw + ((1024u - (smem_u32(s_raw) & 1023u)) & 1023u);
@@ -348,13 +351,14 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr bool CUT = MODE != PF_WHOLE;
     const int hl = w.hl, qblk = w.qblk, ntiles = w.ntiles, j0 = CUT ? w.j0 : 0, np = MODE == PF_CUT ? w.np : 1, piece = w.piece, rec0 = w.rec0;
-    const int q0 = qblk * kQTok2;
+    constexpr int kRows = 128 * TILES;
+    const int q0 = qblk * kQTok * TILES;
 
     if (tid == 0) {
         *s_abort = 0;
         mbar_init(BAR(B3_Q), 1);
-        for (int i = 0; i < 2; i++) { mbar_init(BAR(B3_K0F + i), 1); mbar_init(BAR(B3_K0E + i), 2); }
-        for (int i = 0; i < kSt3; i++) { mbar_init(BAR(B3_DF + i), 1); mbar_init(BAR(B3_DE + i), 2); }   /* K0E, DE: one commit per issuer */
+        for (int i = 0; i < 2; i++) { mbar_init(BAR(B3_K0F + i), 1); mbar_init(BAR(B3_K0E + i), TILES); }
+        for (int i = 0; i < kSt3; i++) { mbar_init(BAR(B3_DF + i), 1); mbar_init(BAR(B3_DE + i), TILES); }   /* K0E, DE: one commit per issuer */
         for (int i = 0; i < 4; i++) { mbar_init(BAR(B3_SF + i), 1); mbar_init(BAR(B3_P + i), 4); }   /* P: one arrival per softmax warp of the tile */
         for (int i = 0; i < 4; i++) mbar_init(BAR(B3_O + i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -380,8 +384,8 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
              * operands are complete from here on (all global reads of this CTA follow this thread's copies) */
             asm volatile("griddepcontrol.wait;" ::: "memory");
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-            mbar_expect_tx(BAR(B3_Q), 2 * kTileBytes);
-            for (int x = 0; x < 2; x++) {
+            mbar_expect_tx(BAR(B3_Q), TILES * kTileBytes);
+            for (int x = 0; x < TILES; x++) {
                 tma_load_3d(sbase + kOff3Q + x * kTileBytes, &tm_q, BAR(B3_Q), 0, (a.kv_head_begin + hl) * 8, q0 + x * kQTok);
                 tma_load_3d(sbase + kOff3Q + x * kTileBytes + 16384, &tm_q, BAR(B3_Q), 64, (a.kv_head_begin + hl) * 8, q0 + x * kQTok);
             }
@@ -407,6 +411,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
             }
         }
     } else if (warp >= 9) {
+        if (warp < 9 + TILES) {
         /* ===================== MMA issuer of tile x (whole warp, one elected lane issues) =====================
          * order: S_x(0) S_x(1) | PV_x(0) S_x(2) | PV_x(1) S_x(3) | ...   tcgen05.commit covers what this thread issued, so
          * a K or V stage is released by one commit of each issuer */
@@ -458,7 +463,8 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
             if (j2 < ntiles) issue_qk(j2);
             umma_commit_lead(BAR(B3_DE + st), lead);
         }
-    } else {
+        }
+    } else if (warp < 4 * TILES) {
         /* ===================== softmax warps: tile x = warp / 4; thread = one row of Q tile x ===================== */
         const int x = warp >> 2, t_local = (tid & 127) >> 3;
         const int tq0 = q0 + x * kQTok;                          /* first query token of this tile */
@@ -468,7 +474,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
         float m = -INFINITY;
         float2 l2 = make_float2(0.f, 0.f);
         bool ok = true;
-        if (x == 1 && (MODE != PF_CLUSTER || ntiles > 0)) turn_pass(1);      /* tile A has the first turn (a piece of a cluster may have no steps) */
+        if (TILES == 2 && x == 1 && (MODE != PF_CLUSTER || ntiles > 0)) turn_pass(1);      /* tile A has the first turn (a piece of a cluster may have no steps) */
         for (int j = 0; j < ntiles; j++) {       /* to the end also after a wait ran out: the turns have to match */
             const unsigned tm_s = tmem + 128u * x + 64u * (j & 1) + lane_base;
             ok = __all_sync(0xffffffffu, mbar_wait_blocking(BAR(B3_SF + 2 * x + (j & 1)), (unsigned)(j >> 1) & 1u, s_abort, a.err, 30u));   /* keep the warp together */
@@ -514,7 +520,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
                 m = m_new;
             }
             unsigned pk[32];
-            const float2 ls = softmax_exp<CUT>(v, m, pk, x, x == 0 || j + 1 < ntiles);
+            const float2 ls = softmax_exp<CUT, TILES == 2>(v, m, pk, x, x == 0 || j + 1 < ntiles);
             l2 = add2(l2, ls);
             /* P over the first 32 columns of this S buffer (column c = keys 2c, 2c+1) */
             tmem_st32(tm_s, pk);
@@ -532,18 +538,18 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
         ok = __all_sync(0xffffffffu, ok);                     /* warp-uniform: tcgen05.ld is warp-collective */
         if (MODE == PF_CLUSTER) {
             /* The CL pieces of a block meet in shared memory: CTA r of the cluster finishes columns [128 r / CL, 128 (r + 1) / CL) of
-             * all 256 rows.  Every piece sends the others their columns of its O and every row's {m, l}; the zones lie over the Q
+             * all rows.  Every piece sends the others their columns of its O and every row's {m, l}; the zones lie over the Q
              * tiles and the K ring, which are free in all CTAs once all have arrived behind their last P.V.  Bound by the bytes
-             * between the SMs (98 KB out of and into each CTA of 4): 45 tokens behind 1 001 take 14.3 us a launch, 21.0 with
-             * records through memory, and 19.0 with chunks of a row side by side (a store then crosses as 32 pieces of 16 bytes). */
+             * between the SMs (98 KB out of and into each CTA of 4): 45 tokens behind 1 001 in two tiles a CTA take 14.3 us a launch,
+             * 21.0 with records through memory, and 19.0 with chunks of a row side by side (a store then crosses as 32 pieces of 16 bytes). */
             constexpr int W4 = 32 / CL;                          /* float4 chunks of a row that a CTA finishes */
-            constexpr int kZone = W4 * 4096;                     /* one source's zone: [W4 chunks][256 rows] */
-            constexpr int kOffMl = CL * kZone, kOffWt = kOffMl + CL * 256 * 8;
-            static_assert(kOffWt + CL * 256 * 4 <= kOff3Bar, "the zones overlap the barriers");
+            constexpr int kZone = W4 * kRows * 16;               /* one source's zone: [W4 chunks][rows] */
+            constexpr int kOffMl = CL * kZone, kOffWt = kOffMl + CL * kRows * 8;
+            static_assert(kOffWt + CL * kRows * 4 <= kOff3Bar, "the zones overlap the barriers");
             const int me = w.piece, row = tid;
             /* chunk c of all rows is contiguous, so that a warp's store crosses as 512 consecutive bytes; rows are permuted within
              * groups of 8 by the chunk, so that 8 lanes which read a row's chunks (CL = 8: two rows') hit all banks */
-            auto zone_off = [](int r, int c) { return c * 4096 + ((r & ~7) | ((r ^ (CL == 8 ? 2 * c : c)) & 7)) * 16; };
+            auto zone_off = [](int r, int c) { return c * (kRows * 16) + ((r & ~7) | ((r ^ (CL == 8 ? 2 * c : c)) & 7)) * 16; };
             const bool live = tq0 + (warp & 3) * 4 < a.nq;       /* the warp has query tokens: else nothing to send or finish */
             cluster_arrive();
             cluster_wait();
@@ -564,14 +570,14 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
                 }
             }
 #pragma unroll
-            for (int r = 0; r < CL; r++) if (live) st_cluster8(cluster_addr(sbase + kOffMl + (me * 256 + row) * 8, r), m, l);
+            for (int r = 0; r < CL; r++) if (live) st_cluster8(cluster_addr(sbase + kOffMl + (me * kRows + row) * 8, r), m, l);
             cluster_arrive();
             cluster_wait();
             /* weights of the pieces for this thread's row (a piece of masked keys has m = -inf: weight 0; key 0 is never masked) */
             if (live) {
                 float2 ml[CL];
 #pragma unroll
-                for (int r = 0; r < CL; r++) ml[r] = *reinterpret_cast<const float2 *>(sm + kOffMl + (r * 256 + row) * 8);
+                for (int r = 0; r < CL; r++) ml[r] = *reinterpret_cast<const float2 *>(sm + kOffMl + (r * kRows + row) * 8);
                 float M = ml[0].x, L = 0.f;
 #pragma unroll
                 for (int r = 1; r < CL; r++) M = fmaxf(M, ml[r].x);
@@ -579,7 +585,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
                 for (int r = 0; r < CL; r++) { ml[r].x = ex2f(ml[r].x - M); L += ml[r].y * ml[r].x; }
                 const float inv = L > 0.f ? 1.f / L : 0.f;
 #pragma unroll
-                for (int r = 0; r < CL; r++) *reinterpret_cast<float *>(sm + kOffWt + (r * 256 + row) * 4) = ml[r].x * inv;
+                for (int r = 0; r < CL; r++) *reinterpret_cast<float *>(sm + kOffWt + (r * kRows + row) * 4) = ml[r].x * inv;
             }
             __syncwarp();                                        /* a warp folds its own 32 rows */
             const int c = lane % W4;
@@ -591,7 +597,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
 #pragma unroll
                 for (int p = 0; p < CL; p++) {
                     const float4 v = *reinterpret_cast<const float4 *>(sm + p * kZone + zone_off(r, c));
-                    const float f = *reinterpret_cast<const float *>(sm + kOffWt + (p * 256 + r) * 4);
+                    const float f = *reinterpret_cast<const float *>(sm + kOffWt + (p * kRows + r) * 4);
                     acc.x = fmaf(v.x, f, acc.x); acc.y = fmaf(v.y, f, acc.y); acc.z = fmaf(v.z, f, acc.z); acc.w = fmaf(v.w, f, acc.w);
                 }
                 if (t < a.nq) *reinterpret_cast<float4 *>(o0 + (size_t)t * a.out_stride + (r & 7) * HY3A_D) = acc;
@@ -698,7 +704,7 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
             }
         }
     }
-    if (MODE == PF_CLUSTER && warp >= 8) {       /* the other roles arrive for the two meetings of the epilogue */
+    if (MODE == PF_CLUSTER && warp >= 4 * TILES) {       /* the other roles arrive for the two meetings of the epilogue */
         __syncwarp();
         cluster_arrive(); cluster_wait();
         cluster_arrive(); cluster_wait();
@@ -737,7 +743,7 @@ hy3a_prefill_cut_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     prefill_body<PF_CUT, 1>(tm_q, tm_k, tm_v, a, w);
 }
 /* blocks cut into CL pieces, one per CTA of a cluster */
-template <int CL>
+template <int CL, int TILES>
 __global__ void __launch_bounds__(kPf3Threads, 1)
 hy3a_prefill_cluster_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ prefill_args a) {
     pf_where w = {0, 0, 0, 0, 0, 1, 0};
@@ -745,17 +751,18 @@ hy3a_prefill_cluster_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     w.piece = blockIdx.x - blk * CL;                              /* = rank in the cluster */
     w.hl = blk - ent * a.kv_heads;
     w.qblk = a.entries - 1 - ent;
-    const int nt = (min(a.base + (w.qblk + 1) * kQTok2, a.base + a.nq) + kKeys3 - 1) / kKeys3;
+    const int nt = (min(a.base + (w.qblk + 1) * kQTok * TILES, a.base + a.nq) + kKeys3 - 1) / kKeys3;
     w.j0 = w.piece * nt / CL;
     w.ntiles = (w.piece + 1) * nt / CL - w.j0;
-    prefill_body<PF_CLUSTER, CL>(tm_q, tm_k, tm_v, a, w);
+    prefill_body<PF_CLUSTER, CL, TILES>(tm_q, tm_k, tm_v, a, w);
 }
 
 
 } /* namespace */
 
+template <int TILES>
 static const void *pf_cluster_fn(int cl) {
-    return cl == 2 ? (const void *)hy3a_prefill_cluster_kernel<2> : cl == 4 ? (const void *)hy3a_prefill_cluster_kernel<4> : (const void *)hy3a_prefill_cluster_kernel<8>;
+    return cl == 2 ? (const void *)hy3a_prefill_cluster_kernel<2, TILES> : cl == 4 ? (const void *)hy3a_prefill_cluster_kernel<4, TILES> : (const void *)hy3a_prefill_cluster_kernel<8, TILES>;
 }
 
 typedef CUresult (*hy3a_encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
@@ -794,8 +801,9 @@ static int prefill_device(hy3a_ctx *ctx, const int **cap) {
         HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
         HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_cut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
         for (int i = 1; i < 4; i++) {
-            const void *f = pf_cluster_fn(1 << i);
+            const void *f = pf_cluster_fn<2>(1 << i);
             HY3A_CUDA(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
+            HY3A_CUDA(ctx, cudaFuncSetAttribute(pf_cluster_fn<1>(1 << i), cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 1 << i; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
             cudaLaunchConfig_t cfg = {};
@@ -937,12 +945,15 @@ int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq
         at[0] = attr[0];
         cfg.attrs = at; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
         if (cl > 1) {
-            a.entries = blocks;
+            /* blocks of one tile where they fit at once too: as many SMs again share the softmax and the exchange */
+            const int blocks1 = (nq + kQTok - 1) / kQTok;
+            const bool one = blocks1 * kvh <= cl_cap[cl == 2 ? 1 : cl == 4 ? 2 : 3];
+            a.entries = one ? blocks1 : blocks;
             cudaLaunchAttribute &ca = at[cfg.numAttrs++];
             ca.id = cudaLaunchAttributeClusterDimension; ca.val.clusterDim.x = cl; ca.val.clusterDim.y = ca.val.clusterDim.z = 1;
-            cfg.gridDim = dim3(blocks * kvh * cl);
+            cfg.gridDim = dim3(a.entries * kvh * cl);
             void *args[4] = {&tq, &tk, &tv, &a};
-            HY3A_CUDA(ctx, cudaLaunchKernelExC(&cfg, pf_cluster_fn(cl), args));
+            HY3A_CUDA(ctx, cudaLaunchKernelExC(&cfg, one ? pf_cluster_fn<1>(cl) : pf_cluster_fn<2>(cl), args));
         } else {
             const int entries = ctx->pf_plan.count ? ctx->pf_plan.count : blocks;
             a.entries = entries; a.group = entries * kvh <= ctx->sm_count ? entries : kGroup;

@@ -188,6 +188,17 @@ def test_prefill_clusters(cuda, oracle, dt, base, nq, heads, size):
             check_attention(got[i, own], want[i, own], "%s base=%d nq=%d row %d" % (dt, base, nq, i))
 
 
+@pytest.mark.parametrize("dt,base,nq,heads", [("fp16", 700, 15, (0, 8)), ("int8", 1001, 16, (0, 8)), ("int4", 1001, 17, (0, 8)), ("fp16", 3000, 64, (0, 8)), ("int8", 2000, 65, (2, 3))])
+def test_prefill_clusters_of_one_tile(cuda, oracle, dt, base, nq, heads):
+    """Blocks of 16 tokens: a last block of one token, of 15 and a full one, several blocks per head."""
+    from hy3_b200 import Hy3Attn
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_batch=nq, max_tokens=base + nq, kv_head_begin=heads[0], kv_head_count=heads[1])
+    size = ctx.prefill_cluster(base, nq)
+    ctx.close()
+    assert size > 1
+    test_prefill_clusters(cuda, oracle, dt, base, nq, heads, size)
+
+
 @pytest.mark.parametrize("base,nq,heads,size", [
     (100, 8, 8, 1), (500, 2, 4, 8), (8192, 2, 8, 8), (8192, 45, 8, 4), (16000, 2, 8, 1), (16000, 8, 8, 1), (16000, 30, 8, 8), (16000, 200, 8, 1), (16000, 256, 8, 2),
     (30000, 8, 8, 1), (30000, 30, 8, 1), (4064, 300, 4, 1), (16000, 2048, 8, 2)])
