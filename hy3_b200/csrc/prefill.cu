@@ -335,9 +335,10 @@ __device__ __forceinline__ void st_cluster16(unsigned addr, float a, float b, fl
 __device__ __forceinline__ void st_cluster8(unsigned addr, float a, float b) {
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
 }
-/* TILES: query tiles of a CTA.  One only in clusters, where blocks of 16 tokens fit at once as well (hy3a_launch_prefill): a block then
- * has half the exchange and half the softmax, and none for a second tile without tokens; warps 4-7 and 10 have nothing to do.  us a layer with its
- * append, two tiles / one: 45 tokens behind 1 001 19.7 / 15.2, 64 behind 8 192 43.6 / 34.2, 16 behind 500 13.9 / 12.7. */
+/* TILES: query tiles of a CTA.  One where blocks of 16 tokens fit at once as well (hy3a_launch_prefill; never where blocks are cut): a block then
+ * has half the softmax and half the exchange of a cluster, and none for a second tile without tokens; warps 4-7 and 10 have nothing to do.  us a layer with its
+ * append, two tiles / one: 45 tokens behind 1 001 19.7 / 15.2, 64 behind 8 192 43.6 / 34.2, 16 behind 500 13.9 / 12.7; uncut,
+ * 30 behind 300 16.7 / 12.8, 256 fresh ones 15.4 / 13.0. */
 template <int MODE, int CL, int TILES = 2>
 __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUtensorMap &tm_k, const CUtensorMap &tm_v, const prefill_args &a, const pf_where &w) {
     extern __shared__ uint8_t s_raw[];
@@ -721,15 +722,16 @@ __device__ __forceinline__ void prefill_body(const CUtensorMap &tm_q, const CUte
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 #undef BAR
 }
-/* blocks uncut (full grids) */
+/* blocks uncut (full grids; of one tile where these do not fill the SMs) */
+template <int TILES>
 __global__ void __launch_bounds__(kPf3Threads, 1)
 hy3a_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ prefill_args a) {
     pf_where w = {0, 0, 0, 0, 0, 1, 0};
     int ent;
     entry_of(a, ent, w.hl);
     w.qblk = a.entries - 1 - ent;
-    w.ntiles = (min(a.base + (w.qblk + 1) * kQTok2, a.base + a.nq) + kKeys3 - 1) / kKeys3;      /* keys behind these do not matter for this CTA */
-    prefill_body<PF_WHOLE, 1>(tm_q, tm_k, tm_v, a, w);
+    w.ntiles = (min(a.base + (w.qblk + 1) * kQTok * TILES, a.base + a.nq) + kKeys3 - 1) / kKeys3;      /* keys behind these do not matter for this CTA */
+    prefill_body<PF_WHOLE, 1, TILES>(tm_q, tm_k, tm_v, a, w);
 }
 /* blocks cut along the keys (grids that would leave SMs idle); a separate kernel, because the offsets and the -inf test of its
  * inner loop cost the other one 5 % */
@@ -798,7 +800,8 @@ static int prefill_device(hy3a_ctx *ctx, const int **cap) {
     static int cap_dev[64][4];
     const int dev = ctx->device & 63;
     if (!done_dev[dev]) {
-        HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
+        HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
+        HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
         HY3A_CUDA(ctx, cudaFuncSetAttribute(hy3a_prefill_cut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf3Smem));
         for (int i = 1; i < 4; i++) {
             const void *f = pf_cluster_fn<2>(1 << i);
@@ -939,14 +942,14 @@ int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq
     {
         plan_chunk(ctx, cl_cap, base_slot, nq);
         const int cl = ctx->pf_plan_cluster, blocks = (nq + kQTok2 - 1) / kQTok2;
+        /* blocks of one tile where they fit at once too: as many SMs again share the softmax, and the exchange of clusters */
+        const int blocks1 = (nq + kQTok - 1) / kQTok;
         cudaLaunchConfig_t cfg = {};
         cfg.stream = ctx->stream; cfg.blockDim = dim3(kPf3Threads); cfg.dynamicSmemBytes = kPf3Smem;
         cudaLaunchAttribute at[2];
         at[0] = attr[0];
         cfg.attrs = at; cfg.numAttrs = ctx->use_pdl ? 1 : 0;
         if (cl > 1) {
-            /* blocks of one tile where they fit at once too: as many SMs again share the softmax and the exchange */
-            const int blocks1 = (nq + kQTok - 1) / kQTok;
             const bool one = blocks1 * kvh <= cl_cap[cl == 2 ? 1 : cl == 4 ? 2 : 3];
             a.entries = one ? blocks1 : blocks;
             cudaLaunchAttribute &ca = at[cfg.numAttrs++];
@@ -955,11 +958,12 @@ int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq
             void *args[4] = {&tq, &tk, &tv, &a};
             HY3A_CUDA(ctx, cudaLaunchKernelExC(&cfg, one ? pf_cluster_fn<1>(cl) : pf_cluster_fn<2>(cl), args));
         } else {
-            const int entries = ctx->pf_plan.count ? ctx->pf_plan.count : blocks;
+            const bool one = !ctx->pf_plan.count && blocks1 * kvh <= ctx->sm_count;
+            const int entries = ctx->pf_plan.count ? ctx->pf_plan.count : one ? blocks1 : blocks;
             a.entries = entries; a.group = entries * kvh <= ctx->sm_count ? entries : kGroup;
             cfg.gridDim = dim3(entries * kvh);
             if (ctx->pf_plan.count) HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_cut_kernel, tq, tk, tv, a, ctx->pf_plan));
-            else HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, hy3a_prefill_kernel, tq, tk, tv, a));
+            else HY3A_CUDA(ctx, cudaLaunchKernelEx(&cfg, one ? hy3a_prefill_kernel<1> : hy3a_prefill_kernel<2>, tq, tk, tv, a));
         }
     }
     ctx->launches++;

@@ -188,6 +188,12 @@ def test_prefill_clusters(cuda, oracle, dt, base, nq, heads, size):
             check_attention(got[i, own], want[i, own], "%s base=%d nq=%d row %d" % (dt, base, nq, i))
 
 
+@pytest.mark.parametrize("dt,base,nq,heads", [("fp16", 0, 33, (0, 8)), ("int8", 30, 48, (0, 8)), ("int4", 0, 288, (0, 8)), ("int8", 0, 289, (0, 8)), ("fp16", 0, 49, (2, 3))])
+def test_prefill_uncut_blocks_of_one_tile(cuda, oracle, dt, base, nq, heads, monkeypatch):
+    """Uncut grids whose blocks of 16 tokens fit at once (up to 288 tokens of 8 heads), with a last block of one token and a full one; one token more."""
+    test_prefill_every_block_and_head(cuda, oracle, dt, base, nq, heads, False, monkeypatch)
+
+
 @pytest.mark.parametrize("dt,base,nq,heads", [("fp16", 700, 15, (0, 8)), ("int8", 1001, 16, (0, 8)), ("int4", 1001, 17, (0, 8)), ("fp16", 3000, 64, (0, 8)), ("int8", 2000, 65, (2, 3))])
 def test_prefill_clusters_of_one_tile(cuda, oracle, dt, base, nq, heads):
     """Blocks of 16 tokens: a last block of one token, of 15 and a full one, several blocks per head."""
