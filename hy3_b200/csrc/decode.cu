@@ -30,8 +30,8 @@
  * memory ring with bulk asynchronous copies (cp.async.bulk + mbarrier transaction counts);
  * the consumer warps take the 16- or 32-token granules of the pages round-robin.  The piece a CTA
  * computes for a (row, head) segment is folded in shared memory; if the segment spans
- * several CTAs each writes an {m, l, acc} record and the LAST CTA to arrive (atomic
- * counter) folds them -- the LSE-merge epilogue, no second launch.  Steps of few segments with few pages run as clusters
+ * several CTAs each writes an {acc, m, l} record per query head and the LAST warp to arrive
+ * (atomic counter per head) folds them -- the LSE-merge epilogue, no second launch.  Steps of few segments with few pages run as clusters
  * instead (cluster_size below).
  *
  * Roofline: HBM.  Algorithmic bytes per (token, KV head): 512 (FP16), 132 (INT4); per token and
