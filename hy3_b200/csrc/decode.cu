@@ -1073,7 +1073,10 @@ static int spread_folders(const hy3a_ctx *ctx) {
  *   INT4   300  8.6  7.0  6.9  7.7    700  8.7  7.4  7.1  7.8   2 500 11.3 11.1  8.1  8.5   12 000 14.3 29.5 17.6 12.5
  *   INT8, where the stream counts, grid / clusters: 1 row of 9 600 11.69 / 11.78, 3 rows of 5 000 12.91 / 13.02, 3 of 8 000 15.58 / 17.81,
  *   4 rows up to 5 000 12.37 / 13.95; 30 rows of 6 000 with 1 head clusters win by 12 %.  INT4: 1 of 14 000 13.60 / 13.83, 4 up to 8 000 14.70 / 15.96
- *   9 rows of 200 / 2 500, clusters of 2: INT8 12.8 -> 10.4 / 17.0 -> 14.9, FP16 10.5 -> 7.6 / 22.0 -> 18.9, INT4 12.4 -> 9.8 / 17.4 -> 14.0 */
+ *   9 rows of 200 / 2 500, clusters of 2: INT8 12.8 -> 10.4 / 17.0 -> 14.9, FP16 10.5 -> 7.6 / 22.0 -> 18.9, INT4 12.4 -> 9.8 / 17.4 -> 14.0
+ * The lines were drawn before the fold ran per head and one warp planned, which gave the grid 1 to 2 us and the clusters 0.1 to 0.5; they still
+ * hold (66 shapes, grid / as the rule has it): INT8 1 000 9.0 / 7.4, 4 096 11.0 / 9.0, 9 000 12.0 / 11.8; FP16 1 000 6.7 / 5.9, 3 500 9.5 / 8.5;
+ * INT4 2 500 10.1 / 7.7, 9 000 11.0 / 11.1, 12 000 12.5 / 11.6 */
 static int cluster_size(const hy3a_ctx *ctx, int most, long long total) {
     static const int kPagesCta[3] = {1, 5, 4}, kPagesFold[3] = {2, 5, 8};      /* FP16, INT8, INT4 */
     const int dt = ctx->geom.dtype, segs = ctx->batch_n * ctx->cfg.kv_head_count;
