@@ -411,6 +411,7 @@ __device__ __forceinline__ bool fold_last(float *rec0, int piece, int np, unsign
     unsigned old = 0;
     if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(arrivals) : "memory");
     if (__shfl_sync(0xffffffffu, old, 0) != (unsigned)(np - 1)) return false;
+    __syncwarp();      /* lane 0 has acquired the other pieces' records; a shuffle orders no memory, and every lane reads them */
     if (lane == 0) *arrivals = 0u;      /* for the next launch */
     fold_records(rec0, np, zone, stride, slots, lane, M, L, acc);
     return true;

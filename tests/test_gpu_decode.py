@@ -173,6 +173,37 @@ def test_folds_of_many_records(cuda, oracle, dt, stages, lens, monkeypatch):
     ctx.close()
 
 
+@pytest.mark.parametrize("dt", ["int8", "int4", "fp16"])
+@pytest.mark.parametrize("lens,heads", [([30000] + [100] * 198, 1), ([40000] + [200] * 30, 8)])
+def test_folds_of_straddling_segments(cuda, oracle, dt, lens, heads):
+    """Equal ranges of units: the pieces of a segment that straddles CTAs meet in the few places that the ring leaves (11; INT8: 3), in
+    several landings, while the other warps of the CTA go on to its next segment.  Every lane of the folding warp reads records that
+    only one lane has waited for: back to back, bit for bit, and against the oracle."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    from hy3_b200.attn import decode_schedule
+    B = len(lens)
+    ranges = [decode_schedule(lens, heads, 148, c, kv_dtype=dt)[1:] for c in range(148)]
+    first = (lens[0] + 127) // 128                                            # units of row 0's first head
+    mine = [r for r in ranges if r[0] < first]
+    assert len(mine) > 11 and mine[-1][1] > first                             # many pieces, the last CTA holds the next segment as well
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, max_seqs=B, max_batch=B, kv_head_count=heads, max_tokens=sum(lens) + 128 * B, max_tokens_per_seq=max(lens) + 128)
+    for i, n in enumerate(lens):
+        ctx.fill_random(0, i, 0, n, 270 + i)
+    q = oracle.fill_normal((B, 64, 128), SEED, 445)
+    tq = torch.from_numpy(q).to(cuda)
+    ctx.batch_set(list(range(B)), [n - 1 for n in lens])
+    outs = [ctx.decode(0, tq)[:, :8 * heads].clone() for _ in range(40)]
+    ctx.sync()
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+    out = outs[0].cpu().numpy()
+    for i in (0, 1, 2, B - 1):
+        ks, vs = ctx.export_kv(0, i, 0, lens[i])
+        want = oracle.attention(q[i], slots_to_float(oracle, ks, dt), slots_to_float(oracle, vs, dt))
+        check_attention(out[i], want[:8 * heads], "%s row %d of %d" % (dt, i, B))
+    ctx.close()
+
+
 def test_decode_ragged_batch_and_poison(cuda, oracle):
     """Several sequences of different lengths in one launch; cache bytes past each length are poison."""
     import torch
