@@ -341,9 +341,10 @@ __device__ __forceinline__ void write_empty_row(float *out, float *partials, int
 #define HY3A_EMPTY_ROW(i, t, threads) \
     write_empty_row(a.out + (size_t)(i) * a.out_stride + (size_t)cache.kv_head_begin * 8 * HY3A_D, \
                     a.user_partials ? a.user_partials + (size_t)(i) * G * 8 * HY3A_PARTIAL_FLOATS : nullptr, G, t, threads)
-/* ---- a segment that several CTAs share, one warp per query head.  Records in memory: {acc[128], m, l, -, -}. */
+/* ---- a segment that several CTAs share, one warp per query head.  Records in memory: {acc[128], m, l, -, -}.  A piece without keys (l = 0)
+ * leaves acc = 0, and its weight in the fold is 0: the sums of a piece whose scores are all -inf may hold 0 x infinity (a V scale). */
 __device__ __forceinline__ void store_record(float *rec, int lane, float M, float L, const float (&acc)[4]) {
-    *reinterpret_cast<float4 *>(rec + 4 * lane) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<float4 *>(rec + 4 * lane) = L != 0.f ? make_float4(acc[0], acc[1], acc[2], acc[3]) : make_float4(0.f, 0.f, 0.f, 0.f);
     if (lane == 0) *reinterpret_cast<float2 *>(rec + HY3A_D) = make_float2(M, L);
 }
 __device__ __forceinline__ float warp_max(float x) {

@@ -679,6 +679,34 @@ def test_decode_non_finite_scores(cuda, dt, kind):
             assert torch.isfinite(o[0, :24]).all() and torch.isfinite(o[0, 32:]).all() and torch.isfinite(o[1:]).all()
 
 
+@pytest.mark.parametrize("dt", ["int8", "int4"])
+@pytest.mark.parametrize("heads", [1, 8])
+@pytest.mark.parametrize("no_clusters", ["1", "0"])
+def test_pieces_whose_scores_are_all_minus_infinity(cuda, oracle, dt, heads, no_clusters, monkeypatch):
+    """Keys whose scores are -inf weigh nothing, and a piece that holds no others (denominator 0) is skipped on every route: infinite V
+    scales beside such keys, which make 0 x infinity of the piece's sums, do not reach the output."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    monkeypatch.setenv("HY3A_NO_CLUSTERS", no_clusters)
+    n, cut = 2048, 1024                                 # pieces of one page in the grid, of four in a cluster: both end at the cut
+    ctx = Hy3Attn(kv_dtype=dt, n_layers=1, kv_head_count=heads, max_tokens=n + 128)
+    ctx.fill_random(0, 0, 0, n, 3)
+    ks, vs = ctx.export_kv(0, 0, 0, n)
+    want_k, want_v = slots_to_float(oracle, ks[cut:].copy(), dt), slots_to_float(oracle, vs[cut:].copy(), dt)
+    ks[:cut, :16].view(np.float16)[:] = -np.inf
+    vs[:cut, :16].view(np.float16)[:] = np.inf
+    ks[:cut, 16:] = 1 if dt == "int8" else 0x11         # positive codes and queries: every score is -inf
+    ctx.import_kv(0, 0, 0, ks, vs)
+    q = np.abs(oracle.fill_normal((1, 64, 128), SEED, 451)) + 0.1
+    ctx.batch_set([0], [n - 1])
+    assert (ctx.decode_cluster() > 1) == (no_clusters == "0")
+    out = ctx.decode(0, torch.from_numpy(q.astype(np.float32)).to(cuda))
+    ctx.sync()
+    want = oracle.attention(q[0].astype(np.float32), want_k, want_v)
+    check_attention(out[0, :8 * heads].cpu().numpy(), want[:8 * heads], "%s, %d heads" % (dt, heads))
+    ctx.close()
+
+
 @pytest.mark.parametrize("lens,heads,sizes", [      # CTAs per segment with an FP16, INT8, INT4 cache
     ([128], 8, (1, 1, 1)), ([129] * 9, 8, (2, 2, 2)), ([129] * 10, 8, (1, 1, 1)), ([9216], 8, (1, 8, 8)), ([9217], 8, (1, 1, 8)), ([12000], 8, (1, 1, 8)),
     ([14000], 8, (1, 1, 1)), ([5000] * 2, 8, (1, 4, 4)), ([5000] * 3, 8, (1, 1, 4)), ([8000] * 3, 8, (1, 1, 1)), ([8000] * 4, 8, (4, 1, 4)),
