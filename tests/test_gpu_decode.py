@@ -122,6 +122,32 @@ def test_ring_depth_does_not_matter(cuda, dt, n, monkeypatch):
         assert all(torch.equal(outs[i], outs[i - i % 8]) for i in range(len(outs)))
 
 
+@pytest.mark.parametrize("lens", [[40017], [351], [351, 65, 700, 129, 1, 64] * 4])
+def test_half_page_ring_depth_does_not_matter(cuda, lens, monkeypatch):
+    """An FP16 ring holds half pages, 5 of them or as few as 2 (4 beside the largest batches): every depth gives the same bits, back to
+    back.  The rows of the batch are more segments than CTAs, and a row that ends in the first half of a page puts the CTA's next
+    segment at an odd position of the ring."""
+    import torch
+    from hy3_b200 import Hy3Attn
+    B = len(lens)
+    q = torch.randn((B, 64, 128), device=cuda, generator=torch.Generator(device=cuda).manual_seed(7))
+    ref = None
+    for stages in ("5", "4", "3", "2"):
+        monkeypatch.setenv("HY3A_DECODE_STAGES", stages)
+        ctx = Hy3Attn(kv_dtype="fp16", n_layers=1, max_seqs=B, max_batch=B, max_tokens=sum(lens) + 128 * B, max_tokens_per_seq=max(lens) + 128)
+        for i, n in enumerate(lens):
+            ctx.fill_random(0, i, 0, n, 30 + i)
+        outs = []
+        for cut in (1, 2, 33, 64, 65):
+            ctx.batch_set(list(range(B)), [max(0, n - cut) for n in lens])
+            outs += [ctx.decode(0, q).clone() for _ in range(8)]
+        ctx.sync()
+        ctx.close()
+        ref = ref or outs
+        assert all(torch.equal(a, b) for a, b in zip(outs, ref)), "stages=%s" % stages
+        assert all(torch.equal(outs[i], outs[i - i % 8]) for i in range(len(outs)))
+
+
 @pytest.mark.parametrize("dt", ["int4", "fp16"])
 @pytest.mark.parametrize("heads", [8, 3])
 @pytest.mark.parametrize("lens", [[3007, 129, 1, 4097, 640], [300] * 17, [1, 5000, 128, 2, 3, 257, 127, 255, 31, 33, 700, 900, 11]])
