@@ -253,8 +253,7 @@ int hy3a_create(const hy3a_config *cfg, hy3a_ctx **out) {
     ctx->sm_count = prop.multiProcessorCount;
     ctx->decode_ctas = prop.multiProcessorCount;
     { const char *e = getenv("HY3A_DECODE_CTAS"); if (e && atoi(e) > 0) ctx->decode_ctas = atoi(e); }
-    if (ctx->decode_ctas > hy3a_decode_max_ctas()) ctx->decode_ctas = hy3a_decode_max_ctas();
-    if (ctx->decode_ctas > 512) ctx->decode_ctas = 512;
+    if (ctx->decode_ctas > 512) ctx->decode_ctas = 512;      /* the records that hy3a_decode_noalloc's scratch has for CTAs */
     { const char *e = getenv("HY3A_NO_PDL"); ctx->use_pdl = !(e && atoi(e)); }
     { const char *e = getenv("HY3A_NO_CLUSTERS"); ctx->no_clusters = e && atoi(e); }
     /* fp16 operand mirrors of the chunked prefill: at most this much device memory beside the pool */

@@ -148,7 +148,6 @@ int hy3a_launch_prefill(hy3a_ctx *ctx, int layer, int seq, int base_slot, int nq
                         size_t out_stride);
 int hy3a_launch_init_pages(hy3a_ctx *ctx, size_t first_page, size_t n_pages);
 int hy3a_decode_ring_capacity(int dtype, int max_batch);
-int hy3a_decode_max_ctas(void);
 void hy3a_decode_cluster_init(hy3a_ctx *ctx);   /* fills cl_cap */
 int hy3a_fail(hy3a_ctx *ctx, int code, const char *fmt, ...);
 

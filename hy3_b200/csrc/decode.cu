@@ -1050,8 +1050,6 @@ int hy3a_decode_ring_capacity(int dtype, int max_batch) {
     const int page = hy3a_make_geom(dtype).page_bytes, stage = dtype == HY3A_KV_FP16 ? kStageBytes<0> : page;
     return room < 2l * page ? 0 : (int)std::min(8l, room / stage);
 }
-/* Largest grid the last-arrival merge can stage in the merge buffer. */
-int hy3a_decode_max_ctas(void) { return kFixedO / 64; }
 static_assert(kRecFloats >= HY3A_PARTIAL_FLOATS && (kRecFloats * 4) % 16 == 0, "a head's record must start on a 16-byte boundary");
 
 /* Folders per segment of the spread fold (0: the last CTA to arrive folds).  It pays off where the epilogue is the cross-GPU
