@@ -211,7 +211,7 @@ class Hy3Attn:
         return n
 
     def prefill_cluster(self, base_slot, nq):
-        """CTAs per block of 32 query tokens of such a chunk: 2, 4 or 8 as a cluster, 1: `prefill_schedule`."""
+        """CTAs per block of 32 (or, where those fit at once too, 16) query tokens of such a chunk: 2, 4 or 8 as a cluster, 1: `prefill_schedule`."""
         n = self.lib.hy3a_prefill_cluster(self.h, base_slot, nq)
         if n < 0:
             self._chk(n)

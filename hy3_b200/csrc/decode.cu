@@ -1072,9 +1072,13 @@ static int spread_folders(const hy3a_ctx *ctx) {
  *   INT8, where the stream counts, grid / clusters: 1 row of 9 600 11.69 / 11.78, 3 rows of 5 000 12.91 / 13.02, 3 of 8 000 15.58 / 17.81,
  *   4 rows up to 5 000 12.37 / 13.95; 30 rows of 6 000 with 1 head clusters win by 12 %.  INT4: 1 of 14 000 13.60 / 13.83, 4 up to 8 000 14.70 / 15.96
  *   9 rows of 200 / 2 500, clusters of 2: INT8 12.8 -> 10.4 / 17.0 -> 14.9, FP16 10.5 -> 7.6 / 22.0 -> 18.9, INT4 12.4 -> 9.8 / 17.4 -> 14.0
- * The lines were drawn before the fold ran per head and one warp planned, which gave the grid 1 to 2 us and the clusters 0.1 to 0.5; they still
- * hold (66 shapes, grid / as the rule has it): INT8 1 000 9.0 / 7.4, 4 096 11.0 / 9.0, 9 000 12.0 / 11.8; FP16 1 000 6.7 / 5.9, 3 500 9.5 / 8.5;
- * INT4 2 500 10.1 / 7.7, 9 000 11.0 / 11.1, 12 000 12.5 / 11.6 */
+ * The lines were drawn before the fold ran per head and one warp planned, which gave the grid 1 to 2 us and the clusters 0.1 to 0.5.  For 1 to 4
+ * rows they still hold (66 shapes, grid / as the rule has it): INT8 1 000 9.0 / 7.4, 4 096 11.0 / 9.0, 9 000 12.0 / 11.8; FP16 1 000 6.7 / 5.9,
+ * 3 500 9.5 / 8.5; INT4 2 500 10.1 / 7.7, 9 000 11.0 / 11.1, 12 000 12.5 / 11.6.  Of 96 shapes of 9 to 64 ragged rows, 1 to 8 heads and up to
+ * 1 000 to 12 000 tokens, the rule takes what is within 3 % of the best in 74.  It takes clusters that the grid beats by 5 to 14 % in 5, all INT4 up
+ * to 3 000 and 6 000 (9 rows x 4 heads 10.3 / 11.7, 32 x 1 11.2 / 12.6), and the grid where clusters win, because the grid's CTAs get more
+ * than the even share that the rule compares with (INT8 and more than 32 rows have no even pieces): INT8 up to 3 000, 16 rows x 4 heads
+ * 20.5 / 13.3, 32 x 2 19.4 / 13.3, 64 x 1 20.5 / 13.5, up to 6 000 24.6 / 19.7; 64 x 1 FP16 up to 3 000 18.5 / 15.3, INT4 up to 6 000 22.2 / 16.5 */
 static int cluster_size(const hy3a_ctx *ctx, int most, long long total) {
     static const int kPagesCta[3] = {1, 5, 4}, kPagesFold[3] = {2, 5, 8};      /* FP16, INT8, INT4 */
     const int dt = ctx->geom.dtype, segs = ctx->batch_n * ctx->cfg.kv_head_count;

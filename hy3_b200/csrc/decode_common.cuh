@@ -120,11 +120,13 @@ __device__ __forceinline__ segment locate(const int *s_prefix, const hy3a_batch_
 }
 
 /* 2 to 32 rows with fewer than four CTAs per segment: the least number of pages L for which pieces of at most L pages fit the
- * grid (sum of ceil(pages / L) over the rows <= CTAs per head), a lane per row; 0: not this case.  Shares in proportion (above)
+ * grid (sum of ceil(pages / L) over the rows <= CTAs per head), a lane per row; 0: not this case.  Shares in proportion (plan_cta, below)
  * round down, and a row that just misses its second CTA holds the launch up: 8 rows of 22 to 56 pages x 8 heads on 148 CTAs get at
  * most 24 pages a CTA that way, 19 this way (INT4: 27.3 -> 21.1 us a layer with the straddling split that 24 pages fall back to;
- * 12 rows of up to 2 646 tokens 27.1 -> 17.7, FP16 24.9 -> 20.6).  The FP16 / INT4 kernel only: the INT8 kernel gains as much
- * there, but its batch-1 launch loses 0.4 % to the registers of this code.  The result is the same in every warp. */
+ * 12 rows of up to 2 646 tokens 27.1 -> 17.7, FP16 24.9 -> 20.6).  The FP16 / INT4 kernel only: the INT8 kernel would gain
+ * as much there (8 rows of 300 to 8 000 x 8 heads 26.6 -> 18.4, 12 up to 2 646 28.2 -> 15.8, 30 up to 16 000 x 2 38.4 -> 32.8), but its batch-1
+ * launch loses 1 % with this code in the planning warp (32 768 tokens 17.60 -> 17.78, 16 000 12.94 -> 13.11), at the same registers and
+ * spills.  Called by a whole warp, the result is the same in every lane. */
 __device__ __noinline__ unsigned even_piece_search(const int *s_prefix, int n, int G, unsigned grid, int lane) {
     const unsigned P = (unsigned)s_prefix[n], cap = grid / (unsigned)G, p = lane < n ? (unsigned)(s_prefix[lane + 1] - s_prefix[lane]) : 0u;
     if (P == 0u) return 0u;

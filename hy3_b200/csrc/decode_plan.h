@@ -13,14 +13,19 @@
 
 /* INT8 kernel, single-row grid: the last kLate pieces of the last segment take kLateCut pages less each (they start late) */
 constexpr unsigned HY3A_LATE = 4, HY3A_LATE_CUT = 2;
-/* a second segment in a CTA (queries, fold, record: about 6 us) costs more than this many pages */
+/* A second segment in a CTA (queries, fold, record) costs more than this many pages.  The line was drawn when it cost about 6 us, before the
+ * fold ran per head; 14 ragged batches since, us a layer with 0 / 5 / 12 pages, FP16, INT4: 14 rows up to 1 412 tokens x 8 heads
+ * 17.2 / 12.0 / 12.0, 18.6 / 10.8 / 10.8; 30 up to 1 510 x 4 22.9 / 15.6 / 15.6, 30.8 / 13.7 / 13.6; 20 up to 9 594 x 4 43.2 / 43.4 / 34.8,
+ * 38.2 / 38.2 / 20.3; 25 up to 1 020 x 4, INT4, 12.3 / 12.3 / 12.6; the others within 1 %.  So more than 5 would pay now for long rows. */
 constexpr unsigned HY3A_STRADDLE_PAGES = 5;
 
-/* Most pieces of a segment of p pages: every piece is a record to fetch and fold (0.11 us behind the last page), every page 0.57 us of
- * its CTA, so beyond some sqrt(5 p) more pieces cost more than they save; this line stays near it from 100 to 3 000 pages.  It
- * matters where few KV heads have many CTAs each.  us a layer without / with it, INT8, FP16, INT4:
- *   1 head, 20 000 tokens  23.2 -> 10.7  28.1 -> 14.1  30.7 -> 13.1     1 head, 200 000  29.4 -> 26.3  45.2 -> 39.6  39.2 -> 27.3
- *   2 heads, 60 000        19.9 -> 15.8  27.0 -> 25.5  24.6 -> 18.0     4 heads, 20 000  14.6 -> 11.4  19.7 -> 16.7  18.5 -> 13.4 */
+/* Most pieces of a segment of p pages: every piece is a record to fetch and fold behind the last page, every page time of its CTA.  It
+ * matters where few KV heads have many CTAs each.  The line was drawn when every record was a dependent step of the fold (0.11 us; a page 0.57);
+ * the folding warp takes the first 32 in one step now, and a segment that keeps to 32 still gains most.  us a layer with 36 + p / 32 / without
+ * a line / with this one, INT8, FP16, INT4:
+ *   1 head, 20 000 tokens  11.3 / 23.3 / 10.3  11.5 / 21.0 / 11.1  11.6 / 22.6 / 10.3     1 head, 200 000  25.6 / 30.9 / 25.2  30.8 / 35.9 / 30.8  22.0 / 27.4 / 22.2
+ *   2 heads, 60 000        17.1 / 22.2 / 17.6  21.1 / 24.3 / 22.0  15.3 / 19.6 / 15.8     4 heads, 20 000  16.6 / 16.6 / 11.5  16.8 / 16.8 / 13.1  14.8 / 14.8 / 11.0
+ *   1 head, 60 000         14.5 / 24.7 / 15.9  17.7 / 26.0 / 18.3  14.6 / 23.1 / 15.3 */
 HY3A_HD unsigned hy3a_most_pieces(unsigned p) { return 24u + p / 32u; }
 
 /* Even pieces (FP16 / INT4 kernel): 2 to 32 rows with fewer than four CTAs per segment; four round well enough */

@@ -567,8 +567,8 @@ __global__ void __launch_bounds__(kUThreads, 1) hy3a_decode_umma_kernel(hy3a_cac
                 /* MMA k-step kk, k-slots 4tig..4tig+3 / 16+4tig..16+4tig+3 of thread-in-group tig carry head dims 16 tig + 4 kk + 0..3 /
                  * 64 + the same: exactly what a thread gets out of its own 16-byte loads of a K row.  The lane's four dims are one of these
                  * halves, kk = lane & 3, tig = (lane & 15) >> 2: words 2 (lane >> 4) (high digits, rows 0-7) and the one behind it (low
-                 * digits, rows 8-15) of that fragment.  (Gathered from a staged copy: a second barrier and 16 byte loads, 700 tokens 7.45
-                 * instead of 7.39 us a layer.) */
+                 * digits, rows 8-15) of that fragment.  (Gathered from a staged copy: a second barrier and 16 byte loads; no
+                 * difference beyond noise at 700 tokens, 7.45 and 7.39 us a layer.) */
                 *reinterpret_cast<uint2 *>(reinterpret_cast<unsigned *>(&s_q[lane & 3][4 * qw + ((lane & 15) >> 2)]) + 2 * (lane >> 4)) = make_uint2(hw, lw);
                 if (lane == 0) mi.qf[qw] = sqv * (1.f / 254.f) * 0.08838834764831845f * kLog2e;
             }

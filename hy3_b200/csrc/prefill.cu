@@ -13,7 +13,8 @@
  *      K-major operands for the tensor cores.  The operands of a layer are kept across chunks (the
  *      context's per-layer mirrors), so a chunk only converts the pages it appended.
  *   2. hy3a_prefill_kernel: one CTA per (32 query tokens x the 8 query heads of one KV head) = two
- *      128-row Q tiles (one in the clusters of short chunks) (GQA packing: the 8 heads share every K/V tile).  Warp-specialised:
+ *      128-row Q tiles (GQA packing: the 8 heads share every K/V tile); where blocks of 16 tokens fit on the device at once, in
+ *      clusters or uncut, one tile.  Warp-specialised:
  *        TMA producer: Q once, then 64-key K / V tiles into 4-stage rings (cp.async.bulk.tensor,
  *                 128-byte swizzle, mbarrier transaction counts)
  *        MMA issuers (one warp per Q tile, one elected lane): S = Q.K^T (M=128, N=64, K=16) and

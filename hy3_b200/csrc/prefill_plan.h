@@ -34,7 +34,9 @@ struct hy3a_pf_table {
     hy3a_pf_piece e[HY3A_PF_MAX_PIECES];
 };
 
-/* Costs in steps of both query tiles (0.79 us in a CTA by itself, 0.9 with 128 CTAs): start and end of a CTA, writing a record,
+/* The plan and the choice of clusters compare blocks of 32 tokens, two query tiles a CTA.  The launch takes blocks of 16, one tile a CTA, where
+ * these fit at once as well (hy3a_launch_prefill); what that saves (blocks cut into records never take it) is not in these costs.
+ * Costs in steps of both query tiles (0.79 us in a CTA by itself, 0.9 with 128 CTAs): start and end of a CTA, writing a record,
  * folding one record.  To derive them again: a one-step launch takes 6.5 us; 32 tokens behind 4 064 (8 CTAs uncut, 56.9 us) in 2 /
  * 4 / 8 / 16 pieces a block take 42.5 / 32.1 / 28.1 / 33.6 us, i.e. 10.7 / 13.0 / 15.3 / 24 us beside the steps and the 6.5, where
  * 5 + 1.5 pieces say 6.3 / 8.7 / 13.4 / 22.9.  The model is 2 to 4 us low for few pieces, which the 0.88 below allows for. */
@@ -131,13 +133,21 @@ static inline void hy3a_pf_plan(int base, int nq, int heads, int sms, int max_sl
 /* CTAs per block (1: what the plan above says, whose end in steps is `end`, with blocks cut into records or not).  The blocks of a short chunk may run as clusters of 2,
  * 4 or 8 CTAs that share a block's keys evenly and meet in shared memory instead of through records; cap[i]: clusters of 2^i CTAs
  * that fit at once.  The meeting costs kPfCostMeet[i] steps when all 32 query tokens of a block are in use, and down to
- * kPfCostMeet[0] with the softmax warps that hold some (4 tokens each).  Measured, us a launch, 8 heads,
+ * kPfCostMeet[0] with the softmax warps that hold some (4 tokens each).  Measured with two tiles a CTA throughout, us a launch, 8 heads,
  * whole / with records / clusters of 2 / 4 / 8:
  *    45 behind  1 001   21.0  21.0  16.2  14.3  24.9      32 behind  4 064   56.9  28.6  36.2  23.9  20.6
  *     2 behind  1 001   18.2  18.2  13.0   9.3   7.6     128 behind  2 000   35.5  27.1  23.9  19.8  48.7
  *   200 behind  1 000   22.9  23.0  18.1  30.2  60.7     128 behind 16 000  230.6  72.9 110.1  67.8 119.5
  *    30 behind    300   11.1  11.1  10.8  11.1  13.9      64 behind  8 192  113.4  39.6  64.2  39.1  53.1
  *   600 behind  4 000  116.1 116.0 107.5 130.7      600 behind 16 000  435.7 324.7 350.1 336.2
+ * and with one tile where the launch takes it (uncut up to 18 blocks of 16 a head, clusters of 2 / 4 / 8 up to 9 / 4 / 1):
+ *    45 behind  1 001   15.1  15.2  11.8  10.6  25.3      32 behind  4 064   44.5  28.8  25.9  16.8  20.7
+ *     2 behind  1 001   13.7  13.8  10.0   7.3   6.1     128 behind  2 000   26.2  27.6  17.7  20.4  48.1
+ *   200 behind  1 000   17.0  17.1  18.3  30.2  60.0     128 behind 16 000  164.1  76.7  87.6  69.7 120.4
+ *    30 behind    300    8.3   8.3   8.0   7.8  13.9      64 behind  8 192   86.2  40.4  47.8  29.7  53.4
+ *     8 behind 16 000  158.8  38.0  84.0  45.0  26.7
+ * The choice below was fitted to the first table.  Of 51 shapes measured so, it is more than 3 % behind the best in 11: 8 behind 16 000
+ * 37.8, 32 behind 4 064 20.7, 128 behind 2 000 19.9, 200 behind 1 000 18.3, the others by 3 to 10 %.
  * Clusters of 4 and 8 only where all fit at once.  Records stay the better way for few tokens behind a very long history (more than
  * 8 pieces per block) and for a little more than one block per SM. */
 constexpr float kPfCostMeet[4] = {0.8f, 3.5f, 5.5f, 10.f};

@@ -257,13 +257,14 @@ int hy3a_decode_schedule_kv(int kv_dtype, int n, const int *kv_lens, int kv_head
                             long long *total_units, long long *u0, long long *u1);
 int hy3a_decode_schedule(int n, const int *kv_lens, int kv_heads, int n_ctas, int cta, long long *total_units,
                          long long *u0, long long *u1);
-/* CTAs that hy3a_prefill gives each block of 32 query tokens and KV head of such a chunk on this context's device: 2, 4 or 8 that
- * share the block's keys as a thread-block cluster, or 1 (hy3a_prefill_schedule), or a negative error. */
+/* CTAs that hy3a_prefill gives each block of query tokens (32; 16 where blocks of 16 fit on the device at once too) and KV head of such a
+ * chunk on this context's device: 2, 4 or 8 that share the block's keys as a thread-block cluster, or 1 (hy3a_prefill_schedule), or a
+ * negative error. */
 int hy3a_prefill_cluster(hy3a_ctx *ctx, int base_slot, int nq);
 /* How hy3a_prefill cuts a chunk that does not run as clusters into CTAs (pure host arithmetic, no GPU): the pieces of one KV head in launch order, six
  * ints each {query block of 32 tokens, first step, steps (of 64 keys), first record, piece, pieces of the block}.  `sms` SMs,
  * `max_records` piece records over all heads (0: blocks stay uncut).  Writes at most cap pieces, returns their number
- * (0: uncut blocks in descending order) or a negative error.                                                         */
+ * (0: uncut blocks in descending order, of 16 tokens where these fit on the device at once) or a negative error.     */
 int hy3a_prefill_schedule(int base_slot, int nq, int kv_heads, int sms, int max_records, int *pieces, int cap);
 /* Library build info, e.g. "hy3attn sm_100a <date>". */
 const char *hy3a_version(void);
